@@ -239,8 +239,8 @@ int launch_wna16_to_awq(const uint8_t* w, const __half* scales, const uint8_t* z
 bool moe_wt_supported(int H, int I, int group);
 int launch_wt_grouped(int mode, int tile_rows, const __half* a, int64_t a_rows, const uint32_t* w, int experts,
                       const __half* scales, const uint32_t* qzeros, const int4* tiles,
-                      const int32_t* n_tiles, __half* out, int K, int N, int group, int half_cols,
-                      cudaStream_t stream);
+                      const int32_t* n_tiles, const float* row_weights, __half* out, int K, int N, int group,
+                      int half_cols, cudaStream_t stream);
 
 int launch_topk_softmax(const void* gating, int gating_dtype, int T, int E, int topk,
                         int renormalize, float* topk_weights, int32_t* topk_ids,

@@ -37,8 +37,8 @@
 // tile table that moe_gather_kernel wrote: entry (expert, first row, rows) of the permuted list.
 //   MODE 1  gate_up: each CTA holds 64 gate columns (lane quarters 0, 1) and the matching 64 up columns
 //           (quarters 2, 3); epilogue act[pos, c] = silu(gate) * up.
-//   MODE 2  down: epilogue y[pos, c] = D, in permuted order (the routed weight is applied when a
-//           token's slots are summed).
+//   MODE 2  down: epilogue y[pos, c] = routed weight * D, in permuted order, so that a row is rounded once
+//           and what is rounded is the weighted row: D alone may lie outside the range of fp16.
 //
 // TMEM columns: accumulators first (two of 64 or 128 tokens, one of 256), then A[slots][8 steps][8]: four
 // slots, six up to 64 tokens.  With as many slots as teams a team waits for the MMAs of its own last
@@ -107,6 +107,7 @@ struct WtParams {
   // grouped modes
   const int4* tiles;           // (expert, first row, rows, -)
   const int32_t* n_tiles;
+  const float* row_weights;    // MODE 2: routed weight of every permuted row
   int half_cols;               // MODE 1: I (gate columns [0, I), up columns [I, 2 I))
 };
 
@@ -209,6 +210,14 @@ __device__ __forceinline__ void wt_epilogue(const WtParams& p, const Work& work,
     const int kb = work.k_begin(seg), ke = work.k_end(seg);
     const int buf = seg & (p.nbuf - 1);
     const bool handover = MODE == 0 && ke < p.KT;  // another pair holds the tile's last stage
+    // MODE 2: routed weights of tokens 8 k + 2 t4, + 1 of a chunk of 32, fetched a chunk ahead
+    float2 rw_next[4];
+    auto fetch_weights = [&](int c0) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        rw_next[k] = __ldcg(reinterpret_cast<const float2*>(p.row_weights + t.m0 + c0 + 8 * k + 2 * t4));
+    };
+    if (MODE == 2) fetch_weights(0);
     // CTAs whose partial tiles are added: blockIdx.x - 2 gather .. blockIdx.x - 2
     int gather = 0;
     if (MODE == 0 && kb > 0 && !handover) gather = work.worker - work.tile_id(seg) * p.KT / p.chunk;
@@ -331,6 +340,14 @@ __device__ __forceinline__ void wt_epilogue(const WtParams& p, const Work& work,
           __syncwarp();
           if (lane == 0 && ok && piece + kWtPartRing < pieces) load_part(piece + kWtPartRing);
         }
+      }
+      if (MODE == 2) {
+        float2 rw[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) rw[k] = rw_next[k];
+        if (c0 + 32 < t.n) fetch_weights(c0 + 32);
+#pragma unroll
+        for (int i = 0; i < 32; ++i) d[i >> 4][i & 15] *= (i & 1) ? rw[(i & 15) >> 2].y : rw[(i & 15) >> 2].x;
       }
       wt_store<4>(d, dst + (size_t)c0 * pitch, pitch, ok ? rows - c0 : 0);
     }
@@ -973,11 +990,12 @@ int launch_wt_moe(const __half* a, int64_t a_rows, const uint32_t* w, int expert
 
 // Grouped expert GEMM of a fused-MoE layer (MODE 1 / 2 of the kernel) over the tile table of
 // moe_gather_kernel, of at most tile_rows rows each.  a: activations in permuted row order [a_rows, K];
-// w: packed expert weights stacked along the rows [experts * K, N / 8].
+// w: packed expert weights stacked along the rows [experts * K, N / 8].  row_weights (mode 2): a routed
+// weight per row of a, readable up to 32 rows past the last tile.
 int launch_wt_grouped(int mode, int tile_rows, const __half* a, int64_t a_rows, const uint32_t* w, int experts,
                       const __half* scales, const uint32_t* qzeros, const int4* tiles,
-                      const int32_t* n_tiles, __half* out, int K, int N, int group, int half_cols,
-                      cudaStream_t stream) {
+                      const int32_t* n_tiles, const float* row_weights, __half* out, int K, int N, int group,
+                      int half_cols, cudaStream_t stream) {
   if ((group != 128 && group != 64) || K % kWtBK != 0 || N % 32 != 0) return AWQ_B200_ERR_SHAPE;
   WtParams p = {};
   p.scales = scales;
@@ -988,6 +1006,7 @@ int launch_wt_grouped(int mode, int tile_rows, const __half* a, int64_t a_rows, 
   p.K = K;
   p.tiles = tiles;
   p.n_tiles = n_tiles;
+  p.row_weights = row_weights;
   p.half_cols = half_cols;
   if (mode == 1)
     return group == 128 ? launch_wt_moe<1, 128>(a, a_rows, w, experts, tile_rows, p, stream)

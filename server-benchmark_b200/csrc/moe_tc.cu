@@ -3,11 +3,11 @@
 // The (token, slot) pairs are already sorted by expert with every expert's run padded to whole
 // row blocks (moe_align_kernel; 128 rows, or 8 or 16 for batches in between):
 //
-//   moe_gather_kernel   x_perm[pos] = x[token(pos)], the inverse permutation, and the tile table of the
-//                       grouped GEMMs: up to 256 rows of one expert per entry
+//   moe_gather_kernel   x_perm[pos] = x[token(pos)], the inverse permutation, the routed weight of every
+//                       row, and the tile table of the grouped GEMMs: up to 256 rows of one expert per entry
 //   gemm_wt_kernel<1>   gate_up with silu(gate) * up in the epilogue -> act[pos]
-//   gemm_wt_kernel<2>   down -> y[pos], over x_perm, which nobody reads any more
-//   moe_combine_kernel  out[t] = sum over the slots of routed weight * y[pos(t, slot)]
+//   gemm_wt_kernel<2>   routed weight * down -> y[pos], over x_perm, which nobody reads any more
+//   moe_combine_kernel  out[t] = sum over the slots of y[pos(t, slot)]
 //
 // Rows move in permuted order between the kernels, so the GEMM epilogues store whole row segments at
 // a fixed pitch; what is scattered is the last kernel's reads, 4 KB at a time.
@@ -91,15 +91,15 @@ __device__ void moe_tile_table(const int32_t* sorted_ids,
   if (tid == 0) n_tiles[0] = count_carry;
 }
 
-// x_perm[pos, :] = x[token(pos), :] and inverse[pair] = pos for the rows of the used blocks (padding
-// rows are left as they are: what the GEMMs compute from them is stored nowhere).
+// x_perm[pos, :] = x[token(pos), :], row_weights[pos] = weights[pair] and inverse[pair] = pos for the rows
+// of the used blocks (padding rows are left as they are: what the GEMMs compute from them is stored nowhere).
 // One warp per row, eight rows per CTA; a lane keeps four 16-byte loads in flight.  The
 // first CTA writes the tile table instead of rows.
 constexpr int kGatherRows = kGatherThreads / 32;
 __global__ void __launch_bounds__(kGatherThreads)
 moe_gather_kernel(const __half* x, const int32_t* sorted_ids,
-                  const int32_t* expert_ids, const int32_t* num_post_pad,
-                  __half* __restrict__ x_perm, int32_t* __restrict__ inverse,
+                  const int32_t* expert_ids, const int32_t* num_post_pad, const float* weights,
+                  __half* __restrict__ x_perm, int32_t* __restrict__ inverse, float* __restrict__ row_weights,
                   int4* __restrict__ tiles, int32_t* __restrict__ n_tiles, int64_t capacity,
                   int numel, int topk, int H, int rows_per_block, int tile_rows) {
   pdl_launch_dependents();
@@ -119,7 +119,10 @@ moe_gather_kernel(const __half* x, const int32_t* sorted_ids,
   uint4* dst = reinterpret_cast<uint4*>(x_perm + (size_t)pos * H);
   const int units = H / 8;
   if (fid >= numel) return;
-  if (lane == 0) inverse[fid] = (int32_t)pos;
+  if (lane == 0) {
+    inverse[fid] = (int32_t)pos;
+    row_weights[pos] = __ldcg(weights + fid);
+  }
   const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)(fid / topk) * H);
   int i = lane;
   for (; i + 96 < units; i += 128) {
@@ -133,11 +136,10 @@ moe_gather_kernel(const __half* x, const int32_t* sorted_ids,
   for (; i < units; i += 32) dst[i] = __ldcg(src + i);
 }
 
-// out[t] = sum over the slots, in slot order, of weight * y[inverse[t, slot]] in fp32; a negative
+// out[t] = sum over the slots, in slot order, of y[inverse[t, slot]] in fp32; a negative
 // position is a pair whose expert lives on another rank.  One thread per 8 columns.
 __global__ void __launch_bounds__(256)
-moe_combine_kernel(const __half* y, const int32_t* inverse,
-                   const float* weights, __half* __restrict__ out, int T, int topk,
+moe_combine_kernel(const __half* y, const int32_t* inverse, __half* __restrict__ out, int T, int topk,
                    int H) {
   const int units = H / 8;
   const long long idx = (long long)blockIdx.x * 256 + threadIdx.x;
@@ -146,14 +148,13 @@ moe_combine_kernel(const __half* y, const int32_t* inverse,
   if (idx >= (long long)T * units) return;
   const int t = (int)(idx / units), u = (int)(idx % units);
   const int32_t* pos = inverse + (size_t)t * topk;
-  const float* w = weights + (size_t)t * topk;
   float v[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) v[j] = 0.f;
-  auto add = [&](const uint4& r, float rw) {
+  auto add = [&](const uint4& r) {
     const __half* h = reinterpret_cast<const __half*>(&r);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = fmaf(rw, __half2float(h[j]), v[j]);
+    for (int j = 0; j < 8; ++j) v[j] += __half2float(h[j]);
   };
   auto fetch = [&](int s) {
     const int p = __ldcg(pos + s);
@@ -163,12 +164,12 @@ moe_combine_kernel(const __half* y, const int32_t* inverse,
   int s = 0;
   for (; s + 4 <= topk; s += 4) {
     const uint4 a = fetch(s), b = fetch(s + 1), c = fetch(s + 2), d = fetch(s + 3);
-    add(a, __ldcg(w + s));
-    add(b, __ldcg(w + s + 1));
-    add(c, __ldcg(w + s + 2));
-    add(d, __ldcg(w + s + 3));
+    add(a);
+    add(b);
+    add(c);
+    add(d);
   }
-  for (; s < topk; ++s) add(fetch(s), __ldcg(w + s));
+  for (; s < topk; ++s) add(fetch(s));
   __align__(16) __half o[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) o[j] = __float2half_rn(v[j]);
@@ -187,13 +188,14 @@ bool moe_tc_supported(int H, int I, int group) {
 
 namespace {
 // Scratch of a call with `rows` permuted rows: gathered activations (later the down projection's
-// output), silu(gate) * up, inverse permutation, tile table.
+// output), silu(gate) * up, inverse permutation, routed weights by row, tile table.
 struct TcScratch {
-  size_t act, inverse, tiles, n_tiles, bytes;
+  size_t act, inverse, weights, tiles, n_tiles, bytes;
   TcScratch(int64_t rows, int64_t pairs, int H, int I, int block) {
     act = align_up((size_t)rows * H * 2, 256);
     inverse = act + align_up((size_t)rows * I * 2, 256);
-    tiles = inverse + align_up((size_t)pairs * sizeof(int32_t), 256);
+    weights = inverse + align_up((size_t)pairs * sizeof(int32_t), 256);
+    tiles = weights + align_up((size_t)(rows + 32) * sizeof(float), 256);
     n_tiles = tiles + align_up((size_t)(rows / block) * sizeof(int4), 256);
     bytes = n_tiles + 256;
   }
@@ -222,6 +224,7 @@ int launch_moe_experts_tc(const MoeArgs& a, void* workspace, size_t workspace_by
   __half* x_perm = reinterpret_cast<__half*>(ws);
   __half* act = reinterpret_cast<__half*>(ws + at.act);
   int32_t* inverse = reinterpret_cast<int32_t*>(ws + at.inverse);
+  float* row_weights = reinterpret_cast<float*>(ws + at.weights);
   int4* tiles = reinterpret_cast<int4*>(ws + at.tiles);
   int32_t* n_tiles = reinterpret_cast<int32_t*>(ws + at.n_tiles);
 
@@ -230,21 +233,21 @@ int launch_moe_experts_tc(const MoeArgs& a, void* workspace, size_t workspace_by
     if (cudaMemsetAsync(inverse, 0xFF, (size_t)numel * sizeof(int32_t), stream) != cudaSuccess)
       return AWQ_B200_ERR_LAUNCH;
   }
-  if (launch_pdl(moe_gather_kernel, dim3((unsigned)((rows + kGatherRows - 1) / kGatherRows + 1)), dim3(kGatherThreads), 0,
-                 stream, a.x, a.sorted_ids, a.expert_ids, a.num_post_pad, x_perm, inverse, tiles,
-                 n_tiles, a.sorted_capacity, numel, a.topk, a.H, a.block, max_rows) != cudaSuccess) {
+  if (launch_pdl(moe_gather_kernel, dim3((unsigned)((rows + kGatherRows - 1) / kGatherRows + 1)),
+                 dim3(kGatherThreads), 0, stream, a.x, a.sorted_ids, a.expert_ids, a.num_post_pad,
+                 a.topk_weights, x_perm, inverse, row_weights, tiles, n_tiles, a.sorted_capacity, numel, a.topk, a.H, a.block, max_rows) != cudaSuccess) {
     cudaGetLastError();
     return AWQ_B200_ERR_LAUNCH;
   }
-  if (int rc = launch_wt_grouped(1, max_rows, x_perm, rows, a.w13_q, a.E, a.w13_s, a.w13_z, tiles, n_tiles, act,
-                                 a.H, 2 * a.I, a.group, a.I, stream))
+  if (int rc = launch_wt_grouped(1, max_rows, x_perm, rows, a.w13_q, a.E, a.w13_s, a.w13_z, tiles, n_tiles,
+                                 nullptr, act, a.H, 2 * a.I, a.group, a.I, stream))
     return rc;
-  if (int rc = launch_wt_grouped(2, max_rows, act, rows, a.w2_q, a.E, a.w2_s, a.w2_z, tiles, n_tiles, x_perm,
-                                 a.I, a.H, a.group, 0, stream))
+  if (int rc = launch_wt_grouped(2, max_rows, act, rows, a.w2_q, a.E, a.w2_s, a.w2_z, tiles, n_tiles,
+                                 row_weights, x_perm, a.I, a.H, a.group, 0, stream))
     return rc;
   const long long work = (long long)a.T * (a.H / 8);
   if (launch_pdl(moe_combine_kernel, dim3((unsigned)((work + 255) / 256)), dim3(256), 0, stream,
-                 (const __half*)x_perm, (const int32_t*)inverse, a.topk_weights, a.out, a.T, a.topk,
+                 (const __half*)x_perm, (const int32_t*)inverse, a.out, a.T, a.topk,
                  a.H) != cudaSuccess) {
     cudaGetLastError();
     return AWQ_B200_ERR_LAUNCH;

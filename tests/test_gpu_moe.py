@@ -243,6 +243,42 @@ def test_small_batch_experts_edges(A, t, k, e, h, i, parallel):
         assert O.rel_err(y, ref) < TOL
 
 
+# Tokens of one expert each: whole prompts (grouped tiles), a server's batch (a tile per row block).
+@pytest.mark.parametrize("t,e", [(300, 4), (40, 8)])
+def test_rows_leave_the_range_of_fp16_only_before_their_weight(A, t, e):
+    """Rows of the down projection beyond 65504 whose routed weight brings them back: the weight is
+    applied in fp32, ahead of the rounding to fp16."""
+    h, i, k = 512, 256, 2
+    w1, w2, x, logits = _moe_case(e, h, i, t, k, seed=t)
+    _, ids, _ = O.topk_softmax(logits.numpy(), k, True)
+    one = np.ones((t, k), dtype=np.float32)
+    rows = O.fused_experts_fp32(x.numpy(), *[a.numpy() for a in w1], *[a.numpy() for a in w2], one, ids)
+    # row sums far beyond 65504, the weighted ones (by 2^-6, exact) inside
+    w2 = (w2[0], w2[1] * float(2 ** np.round(np.log2(4e5 / np.abs(rows).max()))), w2[2])
+    w = one * 2.0 ** -6
+    ref = O.fused_experts_fp32(x.numpy(), *[a.numpy() for a in w1], *[a.numpy() for a in w2], w, ids)
+    assert 2 ** 6 * np.abs(ref).max() > 2 * 65504 and np.abs(ref).max() < 30000
+    y = A.fused_experts(x.cuda(), tuple(a.cuda() for a in w1), tuple(a.cuda() for a in w2),
+                        torch.from_numpy(w).cuda(), torch.from_numpy(ids).cuda()).float().cpu().numpy()
+    assert np.isfinite(y).all()
+    assert O.rel_err(y, ref) < TOL
+
+
+# Grouped tiles (75 rows per expert and slot; no tile is split along K).
+@pytest.mark.parametrize("t,e,h,i,k", [(300, 4, 512, 384, 2)])
+def test_a_slot_is_rounded_once_weighted_and_then_added(A, t, e, h, i, k):
+    """Every (token, slot) row is rounded to fp16 after its routed weight and a token's rows are added
+    in fp32: the output is the rounded sum of what the slots give one by one, bit for bit."""
+    w1, w2, x, logits = _moe_case(e, h, i, t, k, seed=7 * t)
+    w1d, w2d, xd = tuple(a.cuda() for a in w1), tuple(a.cuda() for a in w2), x.cuda()
+    w, ids, _ = A.fused_topk(xd, logits.cuda(), k, True)
+    y = A.fused_experts(xd, w1d, w2d, w, ids)
+    total = torch.zeros(t, h, device="cuda")
+    for s in range(k):
+        total += A.fused_experts(xd, w1d, w2d, w[:, s:s + 1].contiguous(), ids[:, s:s + 1].contiguous()).float()
+    assert torch.equal(y, total.half())
+
+
 def test_wna16_layout_converts_back_bit_exact(A, golden):
     """uint8 [E, N, K/2] (vLLM's MoE WNA16 layout) -> AWQ layout on the device: vLLM's own
     converted tensors give back the AWQ tensors they were made from, and stacked random experts
