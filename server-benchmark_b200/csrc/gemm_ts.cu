@@ -32,10 +32,9 @@
 //           x by index (TMA gather) from the permuted list.  Direct form (no permutation): block b is
 //           pair b alone.  (128 gate and 128 up columns side by side in a unit, as two boxes of 64-byte
 //           rows, took 2 to 7 us longer at every batch size: the words arrive slower.)
-//   MODE 2  down: rows of act; epilogue pair_out[pair] = routed weight * D.
-//   MODE 3  down, direct form: a tile is (token, slab) and its K range runs over the token's experts one
-//           after the other, each unit weighted by its pair's routed weight: out[token] is complete
-//           without a sum kernel, in fp32.
+//   MODE 2  down: rows of act; epilogue pair_out[pair] = routed weight * D, rounded as in the other expert
+//           kernels, for a sum over the slots afterwards.  Direct form: a pair without an expert here
+//           (negative id) gets a row of zeros.
 //
 // unit_full counts the conversion warps, the announcement of the tokens and the fold warps of the unit
 // four before, whose accumulators the MMAs overwrite.  mma_done counts the MMA warp's commit and the
@@ -184,18 +183,15 @@ __device__ __forceinline__ void tmem_ld<16>(uint32_t taddr, uint32_t (&r)[16]) {
       : "memory");
 }
 
-// Routing tables are read through L2: MODE 2 and 3 read them ahead of pdl_wait.
-template <int MODE>
-__device__ __forceinline__ int ts_expert(const TsParams& p, int tile, int k) {
-  const int block = tile / p.slabs;
-  return __ldcg(p.expert_ids + (MODE == 3 ? block * p.topk + k / p.KT : block));
+// Routing tables are read through L2: MODE 2 reads them ahead of pdl_wait.
+__device__ __forceinline__ int ts_expert(const TsParams& p, int tile) {
+  return __ldcg(p.expert_ids + tile / p.slabs);
 }
 template <int MT, int MODE>
 __device__ __forceinline__ Work ts_work(const TsParams& p) {
   if (MODE == 0) return Work(blockIdx.x, gridDim.x, p.slabs, p.KT, p.chunk);
-  const int blocks = MODE == 3 ? p.numel / p.topk
-                               : (p.sorted_ids ? __ldcg(p.num_post) / MT : p.numel);
-  const int KT = MODE == 1 ? 2 * p.KT : (MODE == 3 ? p.KT * p.topk : p.KT), tiles = blocks * p.slabs;
+  const int blocks = p.sorted_ids ? __ldcg(p.num_post) / MT : p.numel;
+  const int KT = MODE == 1 ? 2 * p.KT : p.KT, tiles = blocks * p.slabs;
   const int even = (tiles * KT + (int)gridDim.x - 1) / (int)gridDim.x;
   const int least = (KT + p.max_split - 1) / p.max_split;
   return Work(blockIdx.x, gridDim.x, tiles, KT, max(1, max(even, least)));
@@ -207,43 +203,33 @@ template <int MODE>
 struct TsWalk {
   const TsParams& p;
   const Work& work;
-  int u = 0, seg = 0, k = 0, k_end = 0, kk = 0, tile = 0, slab = 0;
+  int u = 0, seg = 0, k = 0, k_end = 0, tile = 0, slab = 0;
   int expert = 0, expert_next = 0;
   bool fetched = false;
   __device__ __forceinline__ TsWalk(const TsParams& p_, const Work& w_) : p(p_), work(w_) {}
-  // Positions on unit u; returns whether a new matrix begins.  MODE 1: kk counts gate units, then up.
+  // Positions on unit u; returns whether a new tile begins.  MODE 1: k counts gate units, then up.
   __device__ __forceinline__ bool settle() {
-    bool matrix = false;
-    if (k == k_end) {
-      tile = work.tile_id(seg);
-      k = work.k_begin(seg);
-      k_end = work.k_end(seg++);
-      kk = MODE == 3 ? k % p.KT : k;
-      slab = MODE == 0 ? tile : tile - tile / p.slabs * p.slabs;
-      matrix = true;
-    } else if (MODE == 3 && kk == p.KT) {
-      kk = 0;
-      matrix = true;
-    }
-    if (MODE != 0 && matrix) {
+    if (k != k_end) return false;
+    tile = work.tile_id(seg);
+    k = work.k_begin(seg);
+    k_end = work.k_end(seg++);
+    slab = MODE == 0 ? tile : tile - tile / p.slabs * p.slabs;
+    if (MODE != 0) {
       if (!fetched) {
-        expert_next = ts_expert<MODE>(p, tile, k);
+        expert_next = ts_expert(p, tile);
         fetched = true;
       }
       expert = max(expert_next, 0);  // absent (negative): any matrix, nothing of it is used
-      const int k_next = (k / p.KT + 1) * p.KT;
-      if (MODE == 3 && k_next < k_end) expert_next = ts_expert<MODE>(p, tile, k_next);
-      else if (seg < work.segs) expert_next = ts_expert<MODE>(p, work.tile_id(seg), work.k_begin(seg));
+      if (seg < work.segs) expert_next = ts_expert(p, work.tile_id(seg));
     }
-    return matrix;
+    return true;
   }
   __device__ __forceinline__ void next() {
     ++u;
     ++k;
-    ++kk;
   }
-  __device__ __forceinline__ bool up() const { return MODE == 1 && kk >= p.KT; }
-  __device__ __forceinline__ int unit() const { return up() ? kk - p.KT : kk; }  // inside the matrix
+  __device__ __forceinline__ bool up() const { return MODE == 1 && k >= p.KT; }
+  __device__ __forceinline__ int unit() const { return up() ? k - p.KT : k; }  // inside the matrix
   __device__ __forceinline__ int column() const { return slab * kTsBN + (up() ? p.half_cols : 0); }
 };
 
@@ -363,8 +349,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     while (x.u < work.count && ok) {
       if (x.settle() && MODE != 0) {
         const int block = x.tile / p.slabs;
-        if (MODE == 3) row = block * p.topk + x.k / p.KT;  // the pair's row of act
-        if (MODE == 2) row = block * MT;
+        if (MODE == 2) row = p.sorted_ids != nullptr ? block * MT : block;  // of act
         if (MODE == 1 && p.sorted_ids == nullptr) row = block / p.topk;  // the pair's token
         if (MODE == 1 && p.sorted_ids != nullptr) {
           const int fid = fid_next >= 0 ? fid_next : block_fid(x.seg - 1);
@@ -575,22 +560,14 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       const int id = work.tile_id(seg), kb = work.k_begin(seg), ke = work.k_end(seg);
       const int block = MODE == 0 ? 0 : id / p.slabs, slab = MODE == 0 ? id : id - block * p.slabs;
       // What the end of the segment needs, fetched ahead of its units.  MODE 2: lane m knows pair and
-      // routed weight of row m.  MODE 3: weight and expert of the first and the following slot.
+      // routed weight of row m.
       int fid = p.numel;
       float fw = 0.f;
       bool valid = true;  // false: an expert of another rank
       if (MODE == 1 || MODE == 2) valid = __ldcg(p.expert_ids + block) >= 0;
       if (MODE == 2 && lane < MT) {
-        fid = __ldcg(p.sorted_ids + block * MT + lane);
+        fid = p.sorted_ids != nullptr ? __ldcg(p.sorted_ids + block * MT + lane) : (lane == 0 ? block : p.numel);
         fw = fid < p.numel ? __ldcg(p.topk_weights + fid) : 0.f;
-      }
-      int slot_end = MODE == 3 ? kb : 0, pair = MODE == 3 ? block * p.topk + kb / p.KT : 0;
-      float rw = 1.f, rw_next = 0.f;
-      int e_next = 0;
-      bool absent = false;
-      if (MODE == 3) {
-        rw_next = __ldcg(p.topk_weights + pair);
-        e_next = __ldcg(p.expert_ids + pair);
       }
       uint64_t tot[MT / 2];
 #pragma unroll
@@ -603,17 +580,6 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             gate[(2 * m) * 32] = v.x;
             gate[(2 * m + 1) * 32] = v.y;
             tot[m] = 0ull;
-          }
-        }
-        if (MODE == 3 && k >= slot_end) {
-          const int slot = k / p.KT;
-          slot_end = (slot + 1) * p.KT;
-          rw = rw_next;
-          absent = e_next < 0;
-          if (slot_end < ke) {
-            ++pair;
-            rw_next = __ldcg(p.topk_weights + pair);
-            e_next = __ldcg(p.expert_ids + pair);
           }
         }
         if (ok) ok = mbar_wait(mma_done(u), unit_phase(u), &s_abort, 28);
@@ -630,8 +596,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
           uint16_t sh;
           asm volatile("ld.shared.u16 %0, [%1];" : "=h"(sh) : "r"(s_addr + ring * kSz + h * kTsScaleBytes));
           const uint32_t zw = lds32(z_addr + ring * kSz + h * kTsZeroBytes);
-          float sc = __half2float(__ushort_as_half(sh));
-          if (MODE == 3) sc *= rw;
+          const float sc = __half2float(__ushort_as_half(sh));
           const float nz = fmaf(__uint_as_float(((zw >> z_shift) & 0xFu) | 0x4B000000u), zf, zc);
           sc2[h] = pack2(sc, sc);
           nz2[h] = pack2(nz, nz);
@@ -640,7 +605,6 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(unit_full(u + NDB));
-        if (MODE == 3 && absent) continue;
 #pragma unroll
         for (int h = 0; h < G; ++h) {
           const uint32_t sx = sx_base + ring * kSums + h * (NT * 4);
@@ -750,18 +714,15 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                                  (size_t)p.half_cols, first,
                                  ok && valid && n0 < p.half_cols ? (p.sorted_ids != nullptr ? MT : 1) : 0,
                                  odd);
-      } else if (MODE == 3) {
-        handover::store_rows<MT>(v, p.out + (size_t)(block + first) * p.N + n0, (size_t)p.N, first,
-                                 ok && n0 < p.N ? 1 : 0, odd);
       } else {
         const uint32_t sel = odd ? 0x3276u : 0x5410u;
 #pragma unroll
         for (int m = 0; m < MT; m += 2) {
           const float w0 = __shfl_sync(0xffffffffu, fw, m), w1 = __shfl_sync(0xffffffffu, fw, m + 1);
           const int f = __shfl_sync(0xffffffffu, fid, m + first);
-          const uint32_t own = as_u32(__floats2half2_rn(v[m] * w0, v[m + 1] * w1));
+          const uint32_t own = valid ? as_u32(__floats2half2_rn(v[m] * w0, v[m + 1] * w1)) : 0u;
           const uint32_t other = __shfl_xor_sync(0xffffffffu, own, 1);
-          if (ok && valid && n0 < p.N && f < p.numel)
+          if (ok && n0 < p.N && f < p.numel)
             *reinterpret_cast<uint32_t*>(p.out + (size_t)f * p.N + n0) = prmt(own, other, sel);
         }
       }
@@ -900,7 +861,7 @@ int launch_ts_dense(const __half* x, const uint32_t* qweight, const __half* scal
 }
 
 // Expert GEMMs: gate_up, then down.
-template <int MT, int MODE2>
+template <int MT>
 int launch_ts_experts(const MoeArgs& a, __half* act, int64_t act_rows, __half* pair_out, TsParams p,
                       cudaStream_t stream) {
   const int ctas = ts_ctas();
@@ -933,12 +894,12 @@ int launch_ts_experts(const MoeArgs& a, __half* act, int64_t act_rows, __half* p
   p.N = a.H;
   p.KT = a.I / kTsBK;
   p.slabs = (a.H + kTsBN - 1) / kTsBN;
-  p.out = MODE2 == 3 ? a.out : pair_out;
+  p.out = pair_out;
   TsMaps maps;
   if (int rc = ts_weight_maps(&maps, a.w2_q, a.w2_s, a.w2_z, (uint64_t)a.E * a.I, (uint64_t)a.H))
     return rc;
   if (int rc = encode_map_x(&maps.x, act, (uint64_t)act_rows, I, 16)) return rc;
-  return launch_ts<MT, MODE2>(maps, p, ctas, stream);
+  return launch_ts<MT, 2>(maps, p, ctas, stream);
 }
 
 int ts_tokens(int M) { return M <= 4 ? 4 : (M <= 8 ? 8 : 16); }
@@ -983,17 +944,17 @@ size_t moe_ts_partial_bytes(int block) {
 
 bool moe_ts_ready(const void* workspace) { return handover::sync_block(workspace) != nullptr; }
 
-// Both expert GEMMs of a small batch.  Permuted: act rows by position, pair_out by pair.  Direct (no
-// permutation): act rows by pair, a.out complete.
+// Both expert GEMMs of a small batch, pair_out by pair.  Rows of act by position, direct (no
+// permutation) by pair.
 int launch_moe_ts(const MoeArgs& a, __half* act, int64_t act_rows, __half* pair_out, float* partial,
                   void* workspace, cudaStream_t stream) {
   TsParams p = {};
   p.partial = partial;
   p.sync = handover::sync_block(workspace);
   if (p.sync == nullptr) return AWQ_B200_ERR_LIMIT;
-  if (a.direct) return launch_ts_experts<4, 3>(a, act, act_rows, pair_out, p, stream);
-  return a.block == 8 ? launch_ts_experts<8, 2>(a, act, act_rows, pair_out, p, stream)
-                      : launch_ts_experts<16, 2>(a, act, act_rows, pair_out, p, stream);
+  if (a.direct) return launch_ts_experts<4>(a, act, act_rows, pair_out, p, stream);
+  return a.block == 8 ? launch_ts_experts<8>(a, act, act_rows, pair_out, p, stream)
+                      : launch_ts_experts<16>(a, act, act_rows, pair_out, p, stream);
 }
 
 int ts_device_status(int* out, int clear) { return read_tc_status(out, clear); }

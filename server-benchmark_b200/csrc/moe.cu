@@ -829,14 +829,14 @@ int launch_moe_experts(const MoeArgs& a, void* workspace, size_t workspace_bytes
   const bool ts = moe_ts_supported(a) && workspace_bytes >= at + moe_ts_partial_bytes(a.block) &&
                   moe_ts_ready(workspace);
   float* ts_partial = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + at);
-  if (ts && a.direct) return launch_moe_ts(a, act, rows, pair_out, ts_partial, workspace, stream);
-  // direct mode: the down GEMM sums a token's slots itself when the counters fit and every pair counts
+  // direct mode on the mma.sync kernels: the down GEMM sums a token's slots itself when the counters fit
+  // and every pair counts
   uint32_t* tickets = nullptr;
-  if (a.direct && !a.absent && (size_t)a.T * ((a.H + kBN - 1) / kBN) * sizeof(uint32_t) <= kMoeDirectTicketBytes)
+  if (!ts && a.direct && !a.absent && (size_t)a.T * ((a.H + kBN - 1) / kBN) * sizeof(uint32_t) <= kMoeDirectTicketBytes)
     tickets = reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(pair_out) +
                                           align_up((size_t)numel * a.H * sizeof(__half), 256));
 
-  if (a.expert_parallel || a.absent) {
+  if (a.expert_parallel || (a.absent && !ts)) {
     // pairs routed to experts of other ranks are never written: they must read as zero
     if (cudaMemsetAsync(pair_out, 0, (size_t)numel * a.H * sizeof(__half), stream) != cudaSuccess)
       return AWQ_B200_ERR_LAUNCH;

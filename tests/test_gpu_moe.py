@@ -264,8 +264,9 @@ def test_rows_leave_the_range_of_fp16_only_before_their_weight(A, t, e):
     assert O.rel_err(y, ref) < TOL
 
 
-# Grouped tiles (75 rows per expert and slot; no tile is split along K).
-@pytest.mark.parametrize("t,e,h,i,k", [(300, 4, 512, 384, 2)])
+# Grouped tiles (75 rows per expert and slot; no tile is split along K), and the direct mode (a unit of K
+# per CTA in all of its calls, so that their sums have one order).
+@pytest.mark.parametrize("t,e,h,i,k", [(300, 4, 512, 384, 2), (1, 16, 512, 384, 8), (2, 16, 512, 384, 4)])
 def test_a_slot_is_rounded_once_weighted_and_then_added(A, t, e, h, i, k):
     """Every (token, slot) row is rounded to fp16 after its routed weight and a token's rows are added
     in fp32: the output is the rounded sum of what the slots give one by one, bit for bit."""
