@@ -213,3 +213,20 @@ def test_back_to_back_layers_see_each_others_outputs(A, m):
             ref = A.awq_gemm(ref, qw, s, qz, 8)
             torch.cuda.synchronize()
             assert torch.equal(ref, o)
+
+
+@pytest.mark.parametrize("m,group", [(8, 128), (16, 128), (16, 64), (17, 64), (24, 64), (32, 64), (32, 32)])
+def test_small_batches_apply_the_scales_in_fp32(A, m, group):
+    """Up to 16 tokens, and 32 with the finer groups, nothing but the output is rounded to fp16: its error
+    against 64 bits is that of the rounding alone, which weights rounded to (q - z) * s would exceed by
+    a third."""
+    from awq_b200 import synth
+    k, n = 2048, 1056
+    qw, s, qz = synth.awq_linear_tensors(k, n, group, seed=m + group)
+    x = synth.activations(m, k, seed=3)
+    # the oracle's weights are exact in fp32: 5 bits of q - z times 11 of s
+    ref = x.double().numpy() @ O.dequantize_fp32(qw.numpy(), s.numpy(), qz.numpy(), group).astype(np.float64)
+    y = A.awq_gemm(*dev(x, qw, s, qz), 8).cpu().numpy()
+    error = np.linalg.norm(y - ref)
+    # 5 %: the fp32 sums, K * 2^-24 of their terms' size at most, move few values to the other side
+    assert error < 1.05 * np.linalg.norm(ref.astype(np.float16) - ref)
