@@ -15,8 +15,8 @@
 //   moe_sum_kernel        out[t] = sum over the k slots of token t, fp32 accumulation.
 // These GEMMs split K across a thread-block cluster and reduce through distributed shared memory,
 // exactly like the dense small-M kernel.  They serve quantisation groups of 32 and 64, the decode
-// copies and scratch without room for partial tiles; group 128 goes to gemm_ts.cu (a tile per row block)
-// and, with more rows per expert, all groups go to gemm_wt.cu (moe_tc.cu).
+// copies and scratch without room for partial tiles; group 128 goes to gemm_ts.cu (a tile per row block).
+// All of these apply the scales in fp32.  Row blocks of 128 (prefill) go to gemm_wt.cu (moe_tc.cu).
 #include <cooperative_groups.h>
 
 #include <mutex>
@@ -716,13 +716,11 @@ int launch_moe_align(const int32_t* topk_ids, int numel, int E, int block,
   return AWQ_B200_OK;
 }
 
-// Row block of the permutation: 128 (tcgen05 grouped GEMMs) once an expert sees 36 rows or more
-// on average and the shapes fit that kernel's tiles (measured at 128 experts, top-8: the grouped
-// kernels take 271 us from T = 256 to 768, the streaming kernels 169 / 215 / 254 / 336 us at
-// T = 256 / 384 / 512 / 768); 8 up to eight rows per expert on
-// average (one 8-token tile streams a third faster than two, which outweighs the experts that
-// need a second block up to there: measured crossover between T = 128 and 192 at 128 experts,
-// top-8); else 16.
+// Row block of the permutation.  128, the grouped tiles of gemm_wt.cu, from 36 rows per expert on average if
+// the shapes fit them.  They win from about 17 rows (128 experts of 2048 x 768, top-8: 128 against 146 us at
+// 20 rows, 135 against 204 at 35; 64 of 4096 x 1536, top-4: 222 against 319 at 32), but round (q - z) * s to
+// fp16, which the kernels of smaller blocks do not (error of the layer against 64 bits 5.0e-4 and 3.6e-4):
+// fewer rows stay with those.  8 up to eight rows per expert on average; else 16.
 int moe_block_size(int T, int topk, int E, int H, int I, int group) {
   const long long pairs = (long long)T * topk;
   if (pairs >= 36LL * E && moe_tc_supported(H, I, group)) return 128;
@@ -745,7 +743,8 @@ size_t moe_workspace_bytes(int T, int topk, int E, int H, int I) {
   const size_t small = align_up((size_t)rows * I * sizeof(__half), 256) +
                        align_up((size_t)T * topk * H * sizeof(__half), 256) +
                        (size_t)kMoeDirectTicketBytes + moe_ts_partial_bytes(picked == 8 ? 8 : 16);
-  const size_t big = moe_tc_workspace_bytes(T, topk, E, H, I, picked < 16 ? 16 : picked);
+  if (picked != 128) return small;
+  const size_t big = moe_tc_workspace_bytes(T, topk, E, H, I);
   return big > small ? big : small;
 }
 
@@ -796,25 +795,11 @@ int launch_moe_gemms(const MoeArgs& a, __half* act, __half* pair_out, uint32_t* 
   return AWQ_B200_OK;
 }
 
-// Row blocks of 16 on the grouped GEMMs of prefill (up to 256 rows of an expert per tile) once experts
-// have more than a block or so: a tile converts an expert's weights once however many blocks it has.
-// Against a tile per block of gemm_ts (group 128): at 128 experts of 2048 x 768, top-8, 137 / 136 /
-// 137 / 138 us with tiles and 115 / 128 / 149 / 162 without at 14 / 16 / 20 / 24 rows per expert; at 64
-// experts of 4096 x 1536, top-4, 221 / 222 / 225 / 229 and 185 / 217 / 256 / 307.  The streaming kernels
-// of the other groups lose earlier.
-static bool moe_tiles_pay(const MoeArgs& a) {
-  const int rows = moe_ts_supported(a) ? 17 : 13;
-  return !a.decode_layout && !a.direct && moe_tc_supported(a.H, a.I, a.group) &&
-         (long long)a.T * a.topk >= (long long)rows * a.E;
-}
-
 int launch_moe_experts(const MoeArgs& a, void* workspace, size_t workspace_bytes,
                        cudaStream_t stream) {
   // the decode-layout copy is read by the streaming kernels only (group 128, K % 128)
   if (a.decode_layout && (a.block == 128 || a.group != 128)) return AWQ_B200_ERR_SHAPE;
   if (a.block == 128) return launch_moe_experts_tc(a, workspace, workspace_bytes, stream);
-  if (moe_tiles_pay(a) && workspace != nullptr && workspace_bytes >= moe_tc_layout_bytes(a))
-    return launch_moe_experts_tc(a, workspace, workspace_bytes, stream);
   const size_t need = moe_layout_bytes(a);
   if (workspace == nullptr || workspace_bytes < need) return AWQ_B200_ERR_WORKSPACE;
   const int numel = a.T * a.topk;

@@ -1,7 +1,7 @@
 // Fused-MoE experts for prefill-sized token counts (many rows per expert), group 128 or 64.
 //
 // The (token, slot) pairs are already sorted by expert with every expert's run padded to whole
-// row blocks (moe_align_kernel; 128 rows, or 8 or 16 for batches in between):
+// row blocks (moe_align_kernel, 128 rows):
 //
 //   moe_gather_kernel   x_perm[pos] = x[token(pos)], the inverse permutation, the routed weight of every
 //                       row, and the tile table of the grouped GEMMs: up to 256 rows of one expert per entry
@@ -17,16 +17,13 @@ namespace awq {
 
 namespace {
 
+constexpr int kMBM = 128;      // rows of a block of the permutation
 constexpr int kTileRows = 256;  // rows of a grouped GEMM's tile, at most
 
-// Rows of a tile: with up to 128 (64) rows most experts are one tile, two accumulators fit beside the
-// weights, and the next tile's MMAs run under the epilogue of the last one.  Average rows per expert up
-// to which nearly all experts fit: 100 and 40.  Router + experts, 128 experts of 2048 x 768, top-8: 1000
-// tokens 148 -> 141 us, 1600 tokens 184 -> 167.
-int tile_rows(long long pairs, int E, int block) {
-  if (block <= 64 && pairs <= 40LL * E) return 64;
-  return pairs <= 100LL * E ? 128 : kTileRows;
-}
+// Rows of a tile: with up to 128 most experts are one tile, two accumulators fit beside the weights, and the
+// next tile's MMAs run under the epilogue of the last one.  Up to 100 rows per expert on average nearly all
+// experts fit: router + experts, 128 experts of 2048 x 768, top-8, 1600 tokens 184 -> 167 us.
+int tile_rows(long long pairs, int E) { return pairs <= 100LL * E ? 128 : kTileRows; }
 
 // Tile table of the grouped GEMMs in gemm_wt.cu: up to `tile_rows` rows of one expert per entry, i.e.
 // every expert's run of row blocks cut into pieces of tile_rows / block blocks.  One CTA; blocks are scanned 256 at
@@ -191,34 +188,33 @@ namespace {
 // output), silu(gate) * up, inverse permutation, routed weights by row, tile table.
 struct TcScratch {
   size_t act, inverse, weights, tiles, n_tiles, bytes;
-  TcScratch(int64_t rows, int64_t pairs, int H, int I, int block) {
+  TcScratch(int64_t rows, int64_t pairs, int H, int I) {
     act = align_up((size_t)rows * H * 2, 256);
     inverse = act + align_up((size_t)rows * I * 2, 256);
     weights = inverse + align_up((size_t)pairs * sizeof(int32_t), 256);
     tiles = weights + align_up((size_t)(rows + 32) * sizeof(float), 256);
-    n_tiles = tiles + align_up((size_t)(rows / block) * sizeof(int4), 256);
+    n_tiles = tiles + align_up((size_t)(rows / kMBM) * sizeof(int4), 256);
     bytes = n_tiles + 256;
   }
 };
-int64_t padded_rows(int64_t capacity, int block) { return (capacity + block - 1) / block * block; }
+int64_t padded_rows(int64_t capacity) { return (capacity + kMBM - 1) / kMBM * kMBM; }
 }  // namespace
 
-size_t moe_tc_workspace_bytes(int T, int topk, int E, int H, int I, int block) {
+size_t moe_tc_workspace_bytes(int T, int topk, int E, int H, int I) {
   const int64_t pairs = (int64_t)T * topk;
-  return TcScratch(padded_rows(awq_b200_moe_sorted_capacity(pairs, E, block), block), pairs, H, I, block)
-      .bytes;
+  return TcScratch(padded_rows(awq_b200_moe_sorted_capacity(pairs, E, kMBM)), pairs, H, I).bytes;
 }
 
 size_t moe_tc_layout_bytes(const MoeArgs& a) {
-  return TcScratch(padded_rows(a.sorted_capacity, a.block), (int64_t)a.T * a.topk, a.H, a.I, a.block).bytes;
+  return TcScratch(padded_rows(a.sorted_capacity), (int64_t)a.T * a.topk, a.H, a.I).bytes;
 }
 
 int launch_moe_experts_tc(const MoeArgs& a, void* workspace, size_t workspace_bytes,
                           cudaStream_t stream) {
-  if (kTileRows % a.block != 0 || !moe_tc_supported(a.H, a.I, a.group)) return AWQ_B200_ERR_SHAPE;
-  const int numel = a.T * a.topk, max_rows = tile_rows(numel, a.E, a.block);
-  const int64_t rows = padded_rows(a.sorted_capacity, a.block);
-  const TcScratch at(rows, numel, a.H, a.I, a.block);
+  if (a.block != kMBM || !moe_tc_supported(a.H, a.I, a.group)) return AWQ_B200_ERR_SHAPE;
+  const int numel = a.T * a.topk, max_rows = tile_rows(numel, a.E);
+  const int64_t rows = padded_rows(a.sorted_capacity);
+  const TcScratch at(rows, numel, a.H, a.I);
   if (workspace == nullptr || workspace_bytes < at.bytes) return AWQ_B200_ERR_WORKSPACE;
   uint8_t* ws = static_cast<uint8_t*>(workspace);
   __half* x_perm = reinterpret_cast<__half*>(ws);

@@ -280,6 +280,36 @@ def test_a_slot_is_rounded_once_weighted_and_then_added(A, t, e, h, i, k):
     assert torch.equal(y, total.half())
 
 
+# Rows per expert on average: 5, 9, 15, 25, 35.
+@pytest.mark.parametrize("group", [128, 64])
+@pytest.mark.parametrize("t", [20, 36, 60, 100, 140])
+def test_batches_below_prefill_apply_the_scales_in_fp32(A, t, group):
+    """Below 36 rows per expert the error against 64 bits is that of the roundings of activations, rows and
+    output, which weights rounded to (q - z) * s would exceed by a third."""
+    from awq_b200 import synth
+    e, h, i, k = 8, 512, 256, 2
+    w1, w2 = synth.moe_layer_tensors(e, h, i, group, seed=t)
+    x, logits = synth.activations(t, h, seed=t + 1), synth.gating_logits(t, e, seed=t + 2)
+    w, ids, _ = O.topk_softmax(logits.numpy(), k, True)
+    y = A.fused_experts(x.cuda(), tuple(a.cuda() for a in w1), tuple(a.cuda() for a in w2),
+                        torch.from_numpy(w).cuda(), torch.from_numpy(ids).cuda(), group_size=group)
+
+    def layer(r):  # in 64 bits, r at the places where the kernels round
+        out = np.zeros((t, h))
+        for n in range(e):
+            tok, slot = np.nonzero(ids == n)
+            m1, m2 = (O.dequantize_fp32(*[a[n].numpy() for a in ws], group).astype(np.float64) for ws in (w1, w2))
+            gu = x.double().numpy()[tok] @ m1
+            act = r(gu[:, :i] / (1 + np.exp(-gu[:, :i])) * gu[:, i:])
+            np.add.at(out, tok, r(act @ m2 * w[tok, slot, None]))
+        return r(out)
+
+    exact = layer(lambda v: v)
+    rounded = np.linalg.norm(layer(lambda v: v.astype(np.float16).astype(np.float64)) - exact)
+    # 10 %: another set of the same roundings (fp32 sums, __expf), 10^4 values and more
+    assert np.linalg.norm(y.double().cpu().numpy() - exact) < 1.1 * rounded
+
+
 def test_wna16_layout_converts_back_bit_exact(A, golden):
     """uint8 [E, N, K/2] (vLLM's MoE WNA16 layout) -> AWQ layout on the device: vLLM's own
     converted tensors give back the AWQ tensors they were made from, and stacked random experts
