@@ -133,11 +133,13 @@ moe_gather_kernel(const __half* x, const int32_t* sorted_ids,
   for (; i < units; i += 32) dst[i] = __ldcg(src + i);
 }
 
-// out[t] = sum over the slots, in slot order, of y[inverse[t, slot]] in fp32; a negative
-// position is a pair whose expert lives on another rank.  One thread per 8 columns.
+// out[t] = sum over the slots, in slot order, of y[inverse[t, slot]] in fp32.  A pair that the permutation
+// dropped (its expert lives on another rank, or its id is no expert's) has no entry in `inverse`: what
+// stands there is left over from other calls.  So an entry counts only if the permuted list has the pair at
+// that place, which also keeps every read inside y.  One thread per 8 columns.
 __global__ void __launch_bounds__(256)
-moe_combine_kernel(const __half* y, const int32_t* inverse, __half* __restrict__ out, int T, int topk,
-                   int H) {
+moe_combine_kernel(const __half* y, const int32_t* inverse, const int32_t* sorted_ids,
+                   __half* __restrict__ out, int64_t capacity, int T, int topk, int H) {
   const int units = H / 8;
   const long long idx = (long long)blockIdx.x * 256 + threadIdx.x;
   pdl_launch_dependents();
@@ -155,8 +157,11 @@ moe_combine_kernel(const __half* y, const int32_t* inverse, __half* __restrict__
   };
   auto fetch = [&](int s) {
     const int p = __ldcg(pos + s);
-    return p >= 0 ? __ldcg(reinterpret_cast<const uint4*>(y + (size_t)p * H) + u)
-                  : make_uint4(0, 0, 0, 0);
+    const bool inside = p >= 0 && p < capacity;
+    const int pair = inside ? __ldcg(sorted_ids + p) : -1;
+    const uint4 r = inside ? __ldcg(reinterpret_cast<const uint4*>(y + (size_t)p * H) + u)
+                           : make_uint4(0, 0, 0, 0);
+    return pair == t * topk + s ? r : make_uint4(0, 0, 0, 0);
   };
   int s = 0;
   for (; s + 4 <= topk; s += 4) {
@@ -224,11 +229,6 @@ int launch_moe_experts_tc(const MoeArgs& a, void* workspace, size_t workspace_by
   int4* tiles = reinterpret_cast<int4*>(ws + at.tiles);
   int32_t* n_tiles = reinterpret_cast<int32_t*>(ws + at.n_tiles);
 
-  if (a.expert_parallel) {
-    // pairs routed to experts of other ranks appear nowhere in the permuted list
-    if (cudaMemsetAsync(inverse, 0xFF, (size_t)numel * sizeof(int32_t), stream) != cudaSuccess)
-      return AWQ_B200_ERR_LAUNCH;
-  }
   if (launch_pdl(moe_gather_kernel, dim3((unsigned)((rows + kGatherRows - 1) / kGatherRows + 1)),
                  dim3(kGatherThreads), 0, stream, a.x, a.sorted_ids, a.expert_ids, a.num_post_pad,
                  a.topk_weights, x_perm, inverse, row_weights, tiles, n_tiles, a.sorted_capacity, numel, a.topk, a.H, a.block, max_rows) != cudaSuccess) {
@@ -243,8 +243,8 @@ int launch_moe_experts_tc(const MoeArgs& a, void* workspace, size_t workspace_by
     return rc;
   const long long work = (long long)a.T * (a.H / 8);
   if (launch_pdl(moe_combine_kernel, dim3((unsigned)((work + 255) / 256)), dim3(256), 0, stream,
-                 (const __half*)x_perm, (const int32_t*)inverse, a.out, a.T, a.topk,
-                 a.H) != cudaSuccess) {
+                 (const __half*)x_perm, (const int32_t*)inverse, a.sorted_ids, a.out, a.sorted_capacity, a.T,
+                 a.topk, a.H) != cudaSuccess) {
     cudaGetLastError();
     return AWQ_B200_ERR_LAUNCH;
   }

@@ -310,6 +310,29 @@ def test_batches_below_prefill_apply_the_scales_in_fp32(A, t, group):
     assert np.linalg.norm(y.double().cpu().numpy() - exact) < 1.1 * rounded
 
 
+def test_prefill_ids_of_no_expert_contribute_nothing(A):
+    """Without an expert_map the permutation drops ids outside [0, E) (padding tokens carry -1): such a
+    (token, slot) pair adds zero, whatever earlier calls left in the scratch."""
+    e, h, i, t, k = 8, 512, 256, 500, 2
+    w1, w2, x, logits = _moe_case(e, h, i, t, k, seed=17)
+    w1d, w2d = tuple(a.cuda() for a in w1), tuple(a.cuda() for a in w2)
+    w, ids, _ = O.topk_softmax(logits.numpy(), k, True)
+    # a larger batch first: its entries, rows beyond the next call's among them, stay in the scratch
+    wl, il = (torch.from_numpy(np.tile(a, (4, 1))).cuda() for a in (w, ids))
+    A.fused_experts(torch.full((4 * t, h), 3e4, dtype=torch.float16, device="cuda"), w1d, w2d, wl, il)
+    rng = np.random.default_rng(5)
+    some = ids.copy()
+    some[rng.random((t, k)) < 0.3] = -1
+    some[rng.random((t, k)) < 0.1] = e
+    some[7] = -1
+    w_ref = np.where((some >= 0) & (some < e), w, 0).astype(np.float32)
+    ref = O.fused_experts_fp32(x.numpy(), *[a.numpy() for a in w1], *[a.numpy() for a in w2], w_ref, ids)
+    y = A.fused_experts(x.cuda(), w1d, w2d, torch.from_numpy(w).cuda(), torch.from_numpy(some).cuda())
+    y = y.float().cpu().numpy()
+    assert not y[7].any()
+    assert np.isfinite(y).all() and O.rel_err(y, ref) < TOL
+
+
 def test_wna16_layout_converts_back_bit_exact(A, golden):
     """uint8 [E, N, K/2] (vLLM's MoE WNA16 layout) -> AWQ layout on the device: vLLM's own
     converted tensors give back the AWQ tensors they were made from, and stacked random experts
