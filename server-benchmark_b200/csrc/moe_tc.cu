@@ -229,6 +229,13 @@ int launch_moe_experts_tc(const MoeArgs& a, void* workspace, size_t workspace_by
   int4* tiles = reinterpret_cast<int4*>(ws + at.tiles);
   int32_t* n_tiles = reinterpret_cast<int32_t*>(ws + at.n_tiles);
 
+  if (a.expert_parallel) {
+    // Most pairs are routed to experts of other ranks, and what an earlier call left of them would cost the
+    // combine kernel a row each: one of eight ranks of 128 experts (2048 x 768, top-8), 2500
+    // tokens, 93 us without and 76 with this.
+    if (cudaMemsetAsync(inverse, 0xFF, (size_t)numel * sizeof(int32_t), stream) != cudaSuccess)
+      return AWQ_B200_ERR_LAUNCH;
+  }
   if (launch_pdl(moe_gather_kernel, dim3((unsigned)((rows + kGatherRows - 1) / kGatherRows + 1)),
                  dim3(kGatherThreads), 0, stream, a.x, a.sorted_ids, a.expert_ids, a.num_post_pad,
                  a.topk_weights, x_perm, inverse, row_weights, tiles, n_tiles, a.sorted_capacity, numel, a.topk, a.H, a.block, max_rows) != cudaSuccess) {
