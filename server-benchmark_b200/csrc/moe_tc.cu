@@ -23,7 +23,16 @@ constexpr int kTileRows = 256;  // rows of a grouped GEMM's tile, at most
 // Rows of a tile: with up to 128 most experts are one tile, two accumulators fit beside the weights, and the
 // next tile's MMAs run under the epilogue of the last one.  Up to 100 rows per expert on average nearly all
 // experts fit: router + experts, 128 experts of 2048 x 768, top-8, 1600 tokens 184 -> 167 us.
-int tile_rows(long long pairs, int E) { return pairs <= 100LL * E ? 128 : kTileRows; }
+// `experts` counts those that the pairs are spread over, on all ranks.
+int tile_rows(long long pairs, long long experts) { return pairs <= 100 * experts ? 128 : kTileRows; }
+
+// Experts that the permutation was built for: those of all ranks under expert parallelism, where `E` counts
+// the local ones.  Read off the capacity of the permuted list, which has room for kMBM - 1 entries of padding
+// per expert (awq_b200_moe_sorted_capacity; a batch of 36 rows per expert has more pairs than experts).
+long long routed_experts(const MoeArgs& a) {
+  const long long from_capacity = (a.sorted_capacity - (long long)a.T * a.topk) / (kMBM - 1);
+  return a.expert_parallel && from_capacity > a.E ? from_capacity : a.E;
+}
 
 // Tile table of the grouped GEMMs in gemm_wt.cu: up to `tile_rows` rows of one expert per entry, i.e.
 // every expert's run of row blocks cut into pieces of tile_rows / block blocks.  One CTA; blocks are scanned 256 at
@@ -217,7 +226,7 @@ size_t moe_tc_layout_bytes(const MoeArgs& a) {
 int launch_moe_experts_tc(const MoeArgs& a, void* workspace, size_t workspace_bytes,
                           cudaStream_t stream) {
   if (a.block != kMBM || !moe_tc_supported(a.H, a.I, a.group)) return AWQ_B200_ERR_SHAPE;
-  const int numel = a.T * a.topk, max_rows = tile_rows(numel, a.E);
+  const int numel = a.T * a.topk, max_rows = tile_rows(numel, routed_experts(a));
   const int64_t rows = padded_rows(a.sorted_capacity);
   const TcScratch at(rows, numel, a.H, a.I);
   if (workspace == nullptr || workspace_bytes < at.bytes) return AWQ_B200_ERR_WORKSPACE;

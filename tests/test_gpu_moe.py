@@ -402,6 +402,33 @@ def test_fused_experts_expert_parallel_shards_sum(A, t):
     assert O.rel_err(acc.cpu().numpy(), full.cpu().numpy()) < 5e-3
 
 
+def test_expert_parallel_batch_takes_the_kernels_of_its_rows_per_expert(A):
+    """64 tokens on one of eight ranks are four rows per expert however few experts live here: the calls
+    below prefill run the same kernels with and without an expert_map."""
+    from torch.profiler import ProfilerActivity, profile
+    e, h, i, t, k = 128, 512, 256, 64, 8
+    w1, w2, x, logits = _moe_case(16, h, i, t, 8, seed=3)
+    w1d, w2d, xd = tuple(a.cuda() for a in w1), tuple(a.cuda() for a in w2), x.cuda()
+    logits = torch.randn(t, e, generator=torch.Generator().manual_seed(4)).cuda()
+    w, ids, _ = A.fused_topk(xd, logits, k, True)
+    emap = torch.full((e,), -1, dtype=torch.int32, device="cuda")
+    emap[32:48] = torch.arange(16, dtype=torch.int32, device="cuda")
+
+    def call():
+        return A.fused_experts(xd, w1d, w2d, w, ids, global_num_experts=e, expert_map=emap)
+
+    call()
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as prof:
+        call()
+        torch.cuda.synchronize()
+    names = [event.key for event in prof.key_averages() if "awq::" in event.key]
+    if not names:
+        pytest.skip("the profiler sees no kernels here")
+    assert any("gemm_ts_kernel" in n for n in names), names
+    assert not any("gemm_wt_kernel" in n for n in names), names
+
+
 def test_fused_moe_full_size_rows_are_independent(A):
     """Benchmark-size check without the oracle: a token's output does not depend on which other
     tokens share the batch, so the first rows of the T = 4096 layer (tcgen05 grouped GEMMs)
