@@ -272,10 +272,9 @@ struct MoeArgs {
 constexpr int kMoeDirectTicketBytes = 4096;  // AWQ_B200_MOE_DIRECT_MAX_PAIRS tokens x 64 slabs
 // gemm_ts.cu: expert GEMMs of small batches
 bool moe_ts_supported(const MoeArgs& a);
-bool moe_ts_ready(const void* workspace);
 size_t moe_ts_partial_bytes(int block);
 int launch_moe_ts(const MoeArgs& a, __half* act, int64_t act_rows, __half* pair_out, float* partial,
-                  void* workspace, cudaStream_t stream);
+                  cudaStream_t stream);
 int launch_moe_local_ids(const int32_t* topk_ids, int n, const int32_t* expert_map, int E,
                          int32_t* out, cudaStream_t stream);
 bool moe_supported(int H, int I, int group, int block);

@@ -121,7 +121,7 @@ struct TsParams {
   int numel, topk, half_cols;
   int max_split;               // CTAs a tile is split over at most, about
   float* partial;          // [CTA][MT][256] partial tiles handed over (MODE 1: gate and up, [CTA][2])
-  handover::Sync* sync;
+  handover::Flags flags;
 };
 
 // Pairs of fp32 values in 64-bit registers: one instruction for two FMAs.
@@ -244,7 +244,6 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   extern __shared__ uint8_t smem_raw[];
   __shared__ volatile int s_abort;
   __shared__ uint32_t s_tmem_base;
-  __shared__ unsigned int s_epoch;
   __shared__ float s_gate[MODE == 1 ? kTsFoldWarps * MT * 32 : 1];  // gate sums during the up units
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -548,12 +547,6 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     if (lane == 0)
       for (int u = 0; u < NDB; ++u) mbar_arrive(unit_full(u));
     pdl_wait();  // orders this thread's writes after the kernel before this one
-    unsigned int epoch = 0;
-    if (work.chunked) {
-      if (tid == kTsFold0 * 32) s_epoch = handover::take_ticket(p.sync);
-      asm volatile("bar.sync 1, %0;" ::"n"(kTsFoldWarps * 32) : "memory");
-      epoch = s_epoch;
-    }
     bool ok = true;
     int u = 0;
     for (int seg = 0; seg < work.segs; ++seg) {
@@ -639,17 +632,15 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
           for (int m = 0; m < MT; ++m) part[m * kTsBN] = gate[m * 32];
         }
         __syncwarp();
-        if (lane == 0 && ok && !s_abort)
-          handover::st_release(&p.sync->flags[blockIdx.x][fold], epoch);
+        if (lane == 0 && ok && !s_abort) p.flags.raise(blockIdx.x, fold);
         continue;
       }
-      int gather = 0;  // CTAs before this one that share the tile
-      if (kb > 0) {
-        gather = blockIdx.x - id * work.KT / work.chunk;
+      const int gather = work.helpers(seg);  // CTAs before this one that share the tile
+      if (gather > 0) {
         if (ok)
           for (int c = 1 + lane; c <= gather; c += 32) {
             uint32_t polls = 0;
-            while (handover::ld_acquire(&p.sync->flags[blockIdx.x - c][fold]) != epoch) {
+            while (!p.flags.raised(blockIdx.x - c, fold)) {
               if (++polls >= kSpinLimit || s_abort) {
                 s_abort = 1;
                 atomicCAS(&g_tc_status, 0, 29);
@@ -657,6 +648,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 break;
               }
             }
+            p.flags.lower(blockIdx.x - c, fold);
           }
         ok = __all_sync(0xffffffffu, ok);
         __syncwarp();  // what a lane acquired holds for the warp's reads of the partial tiles
@@ -737,6 +729,10 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     const long long t_end = clock64() + 2000000;
     while (clock64() < t_end) {
     }
+    // flags raised meanwhile: a replay of this launch must not find them
+    if (warp >= kTsFold0 && warp < kTsIssue && work.segs > 0)
+      for (int c = 1 + lane; c <= work.helpers(work.segs - 1); c += 32)
+        p.flags.lower(blockIdx.x - c, warp - kTsFold0);
   }
   tc_fence_before();
   __syncthreads();
@@ -839,6 +835,11 @@ int ts_weight_maps(TsMaps* m, const uint32_t* w, const __half* scales, const uin
                        kTsBN / kPack, box, CU_TENSOR_MAP_SWIZZLE_NONE);
 }
 
+// Partial tiles of all CTAs.
+constexpr size_t ts_partial_bytes(int tokens) {
+  return (size_t)handover::kMaxCtas * tokens * kTsBN * sizeof(float);
+}
+
 template <int MT, int GROUP>
 int launch_ts_dense(const __half* x, const uint32_t* qweight, const __half* scales,
                     const uint32_t* qzeros, TsParams p, void* workspace, size_t workspace_bytes,
@@ -848,10 +849,10 @@ int launch_ts_dense(const __half* x, const uint32_t* qweight, const __half* scal
   const long units = (long)p.slabs * p.KT;
   int ctas = ts_ctas() < p.slabs ? ts_ctas() : p.slabs;
   const int chunk = ts_chunk(p.slabs, p.KT, MT);
-  if (chunk > 0 && workspace != nullptr && workspace_bytes >= gemm_ts_workspace_bytes(p.M, p.N, p.K, GROUP) &&
-      (p.sync = handover::sync_block(workspace)) != nullptr) {
+  if (chunk > 0 && workspace != nullptr && workspace_bytes >= gemm_ts_workspace_bytes(p.M, p.N, p.K, GROUP)) {
     p.chunk = chunk;
     p.partial = static_cast<float*>(workspace);
+    p.flags = handover::make_flags(workspace, ts_partial_bytes(MT));
     ctas = (int)((units + p.chunk - 1) / p.chunk);
   }
   TsMaps maps;
@@ -865,6 +866,7 @@ template <int MT>
 int launch_ts_experts(const MoeArgs& a, __half* act, int64_t act_rows, __half* pair_out, TsParams p,
                       cudaStream_t stream) {
   const int ctas = ts_ctas();
+  p.flags = handover::make_flags(p.partial, 2 * ts_partial_bytes(MT));
   p.sorted_ids = a.sorted_ids;
   p.expert_ids = a.expert_ids;
   p.num_post = a.num_post_pad;
@@ -895,6 +897,7 @@ int launch_ts_experts(const MoeArgs& a, __half* act, int64_t act_rows, __half* p
   p.KT = a.I / kTsBK;
   p.slabs = (a.H + kTsBN - 1) / kTsBN;
   p.out = pair_out;
+  p.flags.token = handover::next_token();
   TsMaps maps;
   if (int rc = ts_weight_maps(&maps, a.w2_q, a.w2_s, a.w2_z, (uint64_t)a.E * a.I, (uint64_t)a.H))
     return rc;
@@ -913,7 +916,7 @@ bool gemm_ts_supported(int M, int N, int K, int group) {
 
 size_t gemm_ts_workspace_bytes(int M, int N, int K, int group) {
   if (!gemm_ts_supported(M, N, K, group)) return 0;
-  return (size_t)handover::kMaxCtas * ts_tokens(M) * kTsBN * sizeof(float);
+  return ts_partial_bytes(ts_tokens(M)) + handover::kFlagBytes;
 }
 
 int launch_gemm_ts(const __half* x, const uint32_t* qweight, const __half* scales,
@@ -937,21 +940,15 @@ bool moe_ts_supported(const MoeArgs& a) {
   return a.group == kTsBK && !a.decode_layout && a.H % kTsBK == 0 && a.I % kTsBK == 0;
 }
 
-// Partial tiles of gate and up, rows of the largest block.
-size_t moe_ts_partial_bytes(int block) {
-  return (size_t)handover::kMaxCtas * 2 * block * kTsBN * sizeof(float);
-}
-
-bool moe_ts_ready(const void* workspace) { return handover::sync_block(workspace) != nullptr; }
+// Partial tiles of gate and up, rows of the largest block, and the flags.
+size_t moe_ts_partial_bytes(int block) { return 2 * ts_partial_bytes(block) + handover::kFlagBytes; }
 
 // Both expert GEMMs of a small batch, pair_out by pair.  Rows of act by position, direct (no
 // permutation) by pair.
 int launch_moe_ts(const MoeArgs& a, __half* act, int64_t act_rows, __half* pair_out, float* partial,
-                  void* workspace, cudaStream_t stream) {
+                  cudaStream_t stream) {
   TsParams p = {};
   p.partial = partial;
-  p.sync = handover::sync_block(workspace);
-  if (p.sync == nullptr) return AWQ_B200_ERR_LIMIT;
   if (a.direct) return launch_ts_experts<4>(a, act, act_rows, pair_out, p, stream);
   return a.block == 8 ? launch_ts_experts<8>(a, act, act_rows, pair_out, p, stream)
                       : launch_ts_experts<16>(a, act, act_rows, pair_out, p, stream);

@@ -103,7 +103,7 @@ struct WtParams {
   int slots, acol;             // A slots behind them (64 columns each) and the first one's column
   int xstage;                  // bytes of an x stage
   float* partial;              // [CTA][4][nt][32] partial tiles handed over
-  handover::Sync* sync;        // flags of the hand-over
+  handover::Flags flags;       // of the hand-over
   // grouped modes
   const int4* tiles;           // (expert, first row, rows, -)
   const int32_t* n_tiles;
@@ -187,29 +187,19 @@ template <int MODE, int GROUP>
 __device__ __forceinline__ void wt_epilogue(const WtParams& p, const Work& work, uint32_t tmem,
                                             int rank, int q, int lane, uint32_t d_full0,
                                             uint32_t d_empty0, float* ex, uint32_t part_ring,
-                                            uint32_t part_full, volatile int* abort_flag,
-                                            unsigned int* s_epoch) {
+                                            uint32_t part_full, volatile int* abort_flag) {
   const uint32_t lane_q = (uint32_t)(q * 32) << 16;
   const int g = lane >> 2, t4 = lane & 3;  // row and column pair of the accumulator fragments
   const uint32_t d_empty_leader = map_rank(d_empty0, 0);
   pdl_wait();  // orders this thread's writes after the kernel before this one
-  unsigned int epoch = 0;
-  if (MODE == 0 && work.chunked) {
-    if (q == 0 && lane == 0) {
-      *s_epoch = handover::take_ticket(p.sync);
-    }
-    named_barrier<1, kWtEpiWarps * 32>();
-    epoch = *s_epoch;
-  }
   // After a wait that gave up the loop still runs to its end, without waiting and without storing:
   // every warp then passes the same named barriers.
   bool ok = true;
   int flip = 0;
   for (int seg = 0; seg < work.segs; ++seg) {
     const WtTile t = wt_tile<MODE, GROUP>(p, work.tile_id(seg));
-    const int kb = work.k_begin(seg), ke = work.k_end(seg);
     const int buf = seg & (p.nbuf - 1);
-    const bool handover = MODE == 0 && ke < p.KT;  // another pair holds the tile's last stage
+    const bool handover = MODE == 0 && work.k_end(seg) < p.KT;  // another pair holds the tile's last stage
     // MODE 2: routed weights of tokens 8 k + 2 t4, + 1 of a chunk of 32, fetched a chunk ahead
     float2 rw_next[4];
     auto fetch_weights = [&](int c0) {
@@ -219,14 +209,13 @@ __device__ __forceinline__ void wt_epilogue(const WtParams& p, const Work& work,
     };
     if (MODE == 2) fetch_weights(0);
     // CTAs whose partial tiles are added: blockIdx.x - 2 gather .. blockIdx.x - 2
-    int gather = 0;
-    if (MODE == 0 && kb > 0 && !handover) gather = work.worker - work.tile_id(seg) * p.KT / p.chunk;
+    const int gather = MODE == 0 ? work.helpers(seg) : 0;
     if (ok) ok = mbar_wait(d_full0 + 8 * buf, (uint32_t)(p.nbuf == 2 ? seg >> 1 : seg) & 1u, abort_flag,
                           38);
     if (MODE == 0 && ok)
       for (int c = 1 + lane; c <= gather; c += 32) {
         uint32_t polls = 0;
-        while (handover::ld_acquire(&p.sync->flags[blockIdx.x - 2 * c][q]) != epoch) {
+        while (!p.flags.raised(blockIdx.x - 2 * c, q)) {
           if (++polls >= kSpinLimit || *abort_flag) {
             *abort_flag = 1;
             atomicCAS(&g_tc_status, 0, 39);
@@ -234,6 +223,7 @@ __device__ __forceinline__ void wt_epilogue(const WtParams& p, const Work& work,
             break;
           }
         }
+        p.flags.lower(blockIdx.x - 2 * c, q);
       }
     ok = __all_sync(0xffffffffu, ok);
     __syncwarp();  // what a lane acquired holds for the warp's reads of the partial tiles
@@ -354,7 +344,7 @@ __device__ __forceinline__ void wt_epilogue(const WtParams& p, const Work& work,
     if (MODE == 0 && handover) {
       fence_proxy_async_all();
       __syncwarp();
-      if (lane == 0 && ok && !*abort_flag) handover::st_release(&p.sync->flags[blockIdx.x][q], epoch);
+      if (lane == 0 && ok && !*abort_flag) p.flags.raise(blockIdx.x, q);
     }
   }
 }
@@ -366,7 +356,6 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   extern __shared__ uint8_t smem_raw[];
   __shared__ volatile int s_abort;
   __shared__ uint32_t s_tmem_base;
-  __shared__ unsigned int s_epoch;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int rank = blockIdx.x & 1;  // cluster of two along x: rank 0 is the leader
@@ -704,8 +693,7 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                              reinterpret_cast<float*>(smem_raw + (bar_base + kWtBarBytes -
                                                                   smem_u32(smem_raw))),
                              x_base + (warp - kWtEpiWarp0) * (kWtPartRing * kWtPartBytes),
-                             part_full(warp - kWtEpiWarp0),
-                             &s_abort, &s_epoch);
+                             part_full(warp - kWtEpiWarp0), &s_abort);
   }
 
   // ---- teardown ----
@@ -716,6 +704,10 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     const long long t_end = clock64() + 2000000;
     while (clock64() < t_end) {
     }
+    // flags raised meanwhile: a replay of this launch must not find them
+    if (MODE == 0 && warp >= kWtEpiWarp0 && warp < kWtEpiWarp0 + kWtEpiWarps && work.segs > 0)
+      for (int c = 1 + lane; c <= work.helpers(work.segs - 1); c += 32)
+        p.flags.lower(blockIdx.x - 2 * c, warp - kWtEpiWarp0);
   }
   tc_fence_before();
   __syncthreads();
@@ -803,10 +795,9 @@ int make_wt_map(CUtensorMap* map_w, const uint32_t* qweight, int64_t wrows, int 
                        box_words == 16 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
 }
 
-// Scratch of the chunked split: one partial tile per CTA.
-size_t wt_scratch_bytes(int nt, int pairs) {
-  return (size_t)2 * pairs * nt * kWtCols * sizeof(float);
-}
+// Scratch of the chunked split: one partial tile per CTA, and the flags.
+size_t wt_partial_bytes(int nt, int pairs) { return (size_t)2 * pairs * nt * kWtCols * sizeof(float); }
+size_t wt_scratch_bytes(int nt, int pairs) { return wt_partial_bytes(nt, pairs) + handover::kFlagBytes; }
 
 // How a dense call is cut: tokens of a tile, and units of a pair's range (0: whole tiles, strided).
 struct WtPlan {
@@ -914,11 +905,12 @@ int launch_wt_dense(const __half* x, const uint32_t* qweight, WtParams p, void* 
   const int most = wt_pairs<0, GROUP>(kWtSmemLimit);
   WtPlan plan = wt_plan(p.M, p.slabs, p.KT, most, true);
   if (plan.chunk > 0) {
-    if (workspace != nullptr && workspace_bytes >= wt_scratch_bytes(plan.nt, plan.pairs) &&
-        (p.sync = handover::sync_block(workspace)) != nullptr)
+    if (workspace != nullptr && workspace_bytes >= wt_scratch_bytes(plan.nt, plan.pairs)) {
       p.partial = static_cast<float*>(workspace);
-    else
+      p.flags = handover::make_flags(workspace, wt_partial_bytes(plan.nt, plan.pairs));
+    } else {
       plan = wt_plan(p.M, p.slabs, p.KT, most, false);
+    }
   }
   p.nt = plan.nt;
   p.chunk = plan.chunk;

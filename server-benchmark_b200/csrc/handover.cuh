@@ -8,7 +8,7 @@
 // started before it and do not wait for it.
 #pragma once
 
-#include <mutex>
+#include <chrono>
 
 #include "common.cuh"
 
@@ -16,32 +16,44 @@ namespace awq {
 
 namespace handover {
 
-// Flags of the hand-over, one block of them per scratch buffer (calls that share a scratch buffer
-// never overlap).  Every CTA of a launch takes a ticket; a launch takes 512 in all, so ticket / 512
-// numbers the launches and is the same in all CTAs of one.  A flag holds the number of the launch
-// that raised it last: nothing has to be cleared, also not between replays of a captured launch.
-constexpr unsigned int kTickets = 512;
+// Flags of the hand-over, one per CTA and epilogue warp, behind the partial tiles in the caller's scratch,
+// which comes with any content.  A flag is raised by storing the token of its launch, a 64-bit number that
+// no other launch of the process has and that other data holds with a chance of 2^-64; the one warp that
+// waits for it lowers it again (to 0, no token), so a replay of a captured launch, whose token is the same
+// every time, does not find it raised.  Nothing outlives the call but these zeros.  Calls that share a
+// scratch buffer must not overlap.
 constexpr int kMaxCtas = 256;
-constexpr int kMaxWarps = 16;
-struct Sync {
-  unsigned int tickets;
-  unsigned int pad[31];
-  unsigned int flags[kMaxCtas][kMaxWarps];  // one per epilogue warp
-};
-constexpr int kSyncBlocks = 64;
-static __device__ Sync g_sync[kSyncBlocks];  // one copy per .cu file; zero-initialised: no launch yet
+constexpr int kMaxWarps = 8;
+constexpr size_t kFlagBytes = (size_t)kMaxCtas * kMaxWarps * sizeof(unsigned long long);
 
-__device__ __forceinline__ unsigned int take_ticket(Sync* sync) {
-  const unsigned int n = blockIdx.x == 0 ? kTickets - gridDim.x + 1 : 1;
-  return atomicAdd(&sync->tickets, n) / kTickets + 1;
+struct Flags {
+  unsigned long long* base;  // [CTA][kMaxWarps]
+  unsigned long long token;
+  __device__ __forceinline__ unsigned long long* at(int cta, int warp) const {
+    return base + cta * kMaxWarps + warp;
+  }
+  __device__ __forceinline__ void raise(int cta, int warp) const {
+    asm volatile("st.release.gpu.global.b64 [%0], %1;" ::"l"(at(cta, warp)), "l"(token) : "memory");
+  }
+  __device__ __forceinline__ bool raised(int cta, int warp) const {
+    unsigned long long v;
+    asm volatile("ld.acquire.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(at(cta, warp)) : "memory");
+    return v == token;
+  }
+  __device__ __forceinline__ void lower(int cta, int warp) const { *at(cta, warp) = 0; }
+};
+
+// Token of a launch: a counter, started by the clock and spread over 64 bits by an odd factor.
+inline unsigned long long next_token() {
+  static std::atomic<unsigned long long> counter{
+      (unsigned long long)std::chrono::system_clock::now().time_since_epoch().count()};
+  const unsigned long long token = ++counter * 0x9E3779B97F4A7C15ull;
+  return token != 0 ? token : next_token();
 }
-__device__ __forceinline__ unsigned int ld_acquire(const unsigned int* p) {
-  unsigned int v;
-  asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ void st_release(unsigned int* p, unsigned int v) {
-  asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+
+// Flags of a launch whose partial tiles take `partial_bytes` (a multiple of 8) of `workspace`.
+inline Flags make_flags(void* workspace, size_t partial_bytes) {
+  return {reinterpret_cast<unsigned long long*>(static_cast<uint8_t*>(workspace) + partial_bytes), next_token()};
 }
 
 // A worker's units: segments of consecutive stages of one tile, walked in the same order by every
@@ -81,6 +93,10 @@ struct Work {
     return chunked && seg == segs - 1 ? begin : 0;
   }
   __device__ __forceinline__ int k_end(int seg) const { return chunked && seg == 0 ? end : KT; }
+  // Workers before this one that share the tile of a segment which this worker finishes.
+  __device__ __forceinline__ int helpers(int seg) const {
+    return k_begin(seg) > 0 && k_end(seg) == KT ? worker - tile_id(seg) * KT / chunk : 0;
+  }
 };
 
 // Two tokens of 32 columns per step: this lane's column of tokens c, c + 1 packed to fp16, then
@@ -99,30 +115,6 @@ __device__ __forceinline__ void store_rows(const float (&v)[COUNT], __half* dst,
     if (m + c < rows) *reinterpret_cast<uint32_t*>(dst) = prmt(own, other, sel);
     dst += 2 * pitch;
   }
-}
-
-// Flag block of a scratch buffer on the current device; nullptr once more scratch buffers have been
-// seen than there are blocks, and the caller then does without the hand-over.
-static Sync* sync_block(const void* workspace) {
-  static std::mutex mu;
-  static const void* owner[64][kSyncBlocks];
-  static Sync* base[64];
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
-  std::lock_guard<std::mutex> lock(mu);
-  if (base[dev] == nullptr) {
-    void* ptr = nullptr;
-    if (cudaGetSymbolAddress(&ptr, g_sync) != cudaSuccess) {
-      (void)cudaGetLastError();
-      return nullptr;
-    }
-    base[dev] = static_cast<Sync*>(ptr);
-  }
-  for (int i = 0; i < kSyncBlocks; ++i) {
-    if (owner[dev][i] == nullptr) owner[dev][i] = workspace;
-    if (owner[dev][i] == workspace) return base[dev] + i;
-  }
-  return nullptr;
 }
 
 }  // namespace handover

@@ -811,8 +811,7 @@ int launch_moe_experts(const MoeArgs& a, void* workspace, size_t workspace_bytes
   // Expert GEMMs on tcgen05 (gemm_ts.cu) when the scratch has room for their partial tiles; the
   // mma.sync kernels below serve group sizes 32 and 64, decode-layout copies and smaller scratch.
   const size_t at = align_up(need, 256);
-  const bool ts = moe_ts_supported(a) && workspace_bytes >= at + moe_ts_partial_bytes(a.block) &&
-                  moe_ts_ready(workspace);
+  const bool ts = moe_ts_supported(a) && workspace_bytes >= at + moe_ts_partial_bytes(a.block);
   float* ts_partial = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + at);
   // direct mode on the mma.sync kernels: the down GEMM sums a token's slots itself when the counters fit
   // and every pair counts
@@ -828,7 +827,7 @@ int launch_moe_experts(const MoeArgs& a, void* workspace, size_t workspace_bytes
   }
   int rc;
   if (ts)
-    rc = launch_moe_ts(a, act, rows, pair_out, ts_partial, workspace, stream);
+    rc = launch_moe_ts(a, act, rows, pair_out, ts_partial, stream);
   else if (a.decode_layout)
     rc = a.block == 8 ? launch_moe_gemms<1, 128, true>(a, act, pair_out, tickets, numel, nblk, stream)
                       : launch_moe_gemms<2, 128, true>(a, act, pair_out, tickets, numel, nblk, stream);

@@ -137,3 +137,31 @@ def test_ts_groups_of_64(A, m, k, n, bias):
     assert torch.equal(y[0], y[1])
     # fp32 sums of exact products; the output's 2^-11 is far inside TOL
     assert O.rel_err(y[0].cpu().numpy(), ref) < TOL
+
+
+@pytest.mark.parametrize("kernel,m,k,n", [("KERNEL_TS", 5, 8192, 1280), ("KERNEL_WT", 40, 8192, 1312)])
+def test_scratch_may_be_any_buffer_with_any_content(A, kernel, m, k, n):
+    """Shared slabs and tiles with more scratch buffers, one after the other, than a table of them could hold,
+    each full of other data, and one buffer again and again: always the same bits."""
+    from awq_b200 import _lib, synth
+    qw, s, qz = (t.cuda() for t in synth.awq_linear_tensors(k, n, 128, seed=1))
+    x = synth.activations(m, k, seed=2).cuda()
+    lib, kernel = _lib.load(), getattr(A, kernel)
+    need = lib.awq_b200_gemm_workspace_bytes(m, n, k, 128, kernel)
+    assert need > 0
+    step = -(-need // 256) * 256
+    pool = torch.randint(0, 256, (150 * step,), dtype=torch.uint8, device="cuda",
+                         generator=torch.Generator(device="cuda").manual_seed(3))
+    pool[:step] = 255
+    pool[step:2 * step] = 0
+    outs = torch.full((300, m, n), float("nan"), dtype=torch.float16, device="cuda")
+    for i in range(300):
+        scratch = pool[min(i, 149) * step:]
+        rc = lib.awq_b200_gemm(x.data_ptr(), qw.data_ptr(), s.data_ptr(), qz.data_ptr(), None,
+                               outs[i].data_ptr(), m, n, k, 128, kernel, scratch.data_ptr(), step,
+                               torch.cuda.current_stream().cuda_stream)
+        assert rc == 0
+    torch.cuda.synchronize()
+    assert device_status() == 0, "a bounded wait ran out"
+    assert torch.isfinite(outs[0].float()).all()
+    assert all(torch.equal(outs[0], y) for y in outs[1:])
