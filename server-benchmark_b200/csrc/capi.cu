@@ -37,9 +37,9 @@ int check_awq_shape(int N, int K, int group) {
 // tensor-parallel shards):
 //   M <= 16     unpacked weights in TMEM, zero point and scale applied to the accumulators (gemm_ts),
 //               groups of 128 and 64: faster than the mma.sync streaming kernel on every layer, 4.9
-//               against 7.6 us on K 1024 x N 8192 up to 45 against 56 us on K 8192 x N 59136.  Without
-//               scratch it distributes whole slabs, and the streaming kernel's cluster split is the
-//               better one.
+//               against 7.6 us on K 1024 x N 8192 up to 45 against 56 us on K 8192 x N 59136.  Without the
+//               scratch it asks for it distributes whole slabs, and the streaming kernel's cluster split
+//               is the better one.
 //   M <= 32     groups of 64 and 32: kernels that apply the scales in fp32 (gemm_wt rounds (q - z) * s to
 //               fp16: error against 64 bits 2.9e-4 instead of 2.1e-4).  Groups of 64: gemm_ts, 16 rows of x
 //               at a time: M 24 12.5 (streaming kernel) and 12.6 us on K 2048 x N 5120, 25.1 -> 21.2 on
@@ -164,7 +164,9 @@ int awq_b200_gemm(const void* x, const void* qweight, const void* scales, const 
   if (int rc = check_device()) return rc;
   const bool automatic = kernel == AWQ_B200_KERNEL_AUTO;
   if (automatic)
-    kernel = pick_gemm_kernel(M, N, K, group, workspace != nullptr && workspace_bytes > 0);
+    kernel = pick_gemm_kernel(M, N, K, group,
+                              workspace != nullptr && (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0 &&
+                                  workspace_bytes >= awq_b200_gemm_workspace_bytes(M, N, K, group, kernel));
 
   const __half* xh = static_cast<const __half*>(x);
   const uint32_t* qw = static_cast<const uint32_t*>(qweight);

@@ -165,3 +165,21 @@ def test_scratch_may_be_any_buffer_with_any_content(A, kernel, m, k, n):
     assert device_status() == 0, "a bounded wait ran out"
     assert torch.isfinite(outs[0].float()).all()
     assert all(torch.equal(outs[0], y) for y in outs[1:])
+
+
+@pytest.mark.parametrize("m,group", [(5, 128), (20, 64)])
+def test_automatic_choice_without_enough_scratch_takes_the_streaming_kernel(A, m, group):
+    """Scratch that is too small or misaligned serves no hand-over: the call runs as without any."""
+    from awq_b200 import _lib, synth
+    k, n = 8192, 1280
+    dev = [t.cuda() for t in (synth.activations(m, k, seed=2), *synth.awq_linear_tensors(k, n, group, seed=1))]
+    lib = _lib.load()
+    need = lib.awq_b200_gemm_workspace_bytes(m, n, k, group, 0)
+    pool = torch.empty(need + 512, dtype=torch.uint8, device="cuda")
+    want = A.awq_gemm(*dev, 8, kernel=A.KERNEL_STREAM)
+    for ptr, size in ((None, 0), (pool.data_ptr(), need - 1), (pool.data_ptr() + 16, need)):
+        y = torch.empty_like(want)
+        rc = lib.awq_b200_gemm(*[t.data_ptr() for t in dev], None, y.data_ptr(), m, n, k, group, 0, ptr, size,
+                               torch.cuda.current_stream().cuda_stream)
+        assert rc == 0
+        assert torch.equal(y, want)
