@@ -47,10 +47,11 @@ def _require(t: torch.Tensor, name: str, dtype, ndim: int | None = None) -> None
 
 
 def reserve_workspace(nbytes: int, device: torch.device | str | None = None) -> None:
-    """Make the current stream's scratch buffer at least ``nbytes`` large (load-time call, before
-    any CUDA-graph capture: a buffer cannot grow while its stream is being captured).
-    ``moe_workspace_bytes`` gives the need of the fused-MoE layer for a token count; the dense
-    kernels never need more than the default."""
+    """Make the current stream's scratch buffer at least ``nbytes`` large (load-time call: the buffer
+    otherwise grows when a call needs more).  ``moe_workspace_bytes`` gives the need of the fused-MoE
+    layer for a token count; the dense kernels never need more than the default.  Calls captured into
+    a CUDA graph do not use it: they take their scratch from the graph's memory pool, so that graphs
+    captured on one stream may be replayed on several at a time."""
     dev = torch.device(device) if device is not None else torch.device("cuda",
                                                                       torch.cuda.current_device())
     if nbytes > 0:

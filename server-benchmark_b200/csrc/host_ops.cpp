@@ -116,41 +116,31 @@ at::Tensor empty_like_device(const at::Tensor& ref, at::ScalarType dtype, Sizes.
 
 PyObject* wrap(at::Tensor t) { return THPVariable_Wrap(std::move(t)); }
 
-// ---- scratch: one buffer per (device, stream) -----------------------------------------------
-// A buffer is replaced only when a call needs more than it holds; the old one is kept alive (a
-// CUDA graph captured earlier has its address baked in).  Growing while the stream is being
-// captured would put the new buffer into the graph's private pool, so that raises.
+// ---- scratch: one buffer per (device, stream), one per call while the stream is captured ----------
+// The partial tiles of a call and the flags that announce them lie in its scratch, so calls that may
+// overlap must not share one.  Calls of one stream never overlap; captured on one stream, they do as
+// soon as their graphs are replayed on several.  A captured call therefore takes its scratch from the
+// graph's own memory pool and gives it back to the pool at the end of the call, like any temporary
+// tensor of a captured operator.
 constexpr int64_t kMinWorkspace = 24 << 20;  // covers every dense kernel's scratch need
 
-// Callers hold the GIL, which is what makes the table safe with several threads.
-struct Workspaces {
-  std::map<std::pair<int, void*>, at::Tensor> current;
-  std::vector<at::Tensor> retired;
-};
-
-Workspaces& workspaces() {
+// Callers hold the GIL, which is what makes the table safe with several threads.  Growing replaces a
+// buffer; the old one goes back to the caching allocator, which hands it on in stream order.
+std::map<std::pair<int, void*>, at::Tensor>& workspaces() {
   // never destroyed: tensors must not be freed after the interpreter and CUDA are gone
-  static Workspaces* w = new Workspaces;
+  static auto* w = new std::map<std::pair<int, void*>, at::Tensor>;
   return *w;
 }
 
 at::Tensor workspace(const at::Device& device, int64_t nbytes) {
   const int dev = device.has_index() ? device.index() : c10::cuda::current_device();
-  const std::pair<int, void*> key{dev, stream_now()};
-  Workspaces& w = workspaces();
-  at::Tensor& ws = w.current[key];
-  if (!ws.defined() || ws.numel() < nbytes) {
-    if (ws.defined()) {
-      if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None)
-        fail(PyExc_RuntimeError,
-             "the scratch buffer of this stream (%lld bytes) would have to grow to %lld bytes during "
-             "stream capture; call awq_b200.reserve_workspace(nbytes) on this stream before capturing",
-             (long long)ws.numel(), (long long)nbytes);
-      w.retired.push_back(ws);
-    }
-    ws = at::detail::empty_cuda({nbytes > kMinWorkspace ? nbytes : kMinWorkspace}, at::kByte,
-                                at::Device(at::kCUDA, dev), std::nullopt);
-  }
+  const auto fresh = [&](int64_t size) {
+    return at::detail::empty_cuda({size}, at::kByte, at::Device(at::kCUDA, dev), std::nullopt);
+  };
+  if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None)
+    return fresh(nbytes);
+  at::Tensor& ws = workspaces()[{dev, stream_now()}];
+  if (!ws.defined() || ws.numel() < nbytes) ws = fresh(nbytes > kMinWorkspace ? nbytes : kMinWorkspace);
   return ws;
 }
 

@@ -183,3 +183,54 @@ def test_automatic_choice_without_enough_scratch_takes_the_streaming_kernel(A, m
                                torch.cuda.current_stream().cuda_stream)
         assert rc == 0
         assert torch.equal(y, want)
+
+
+def _layers(A, m):
+    from awq_b200 import synth
+    dense = [t.cuda() for t in (synth.activations(m, 8192, seed=m), *synth.awq_linear_tensors(8192, 1280, 128, seed=1))]
+    e, h, i, k = 16, 1024, 256, 4
+    w1, w2 = (tuple(t.cuda() for t in w) for w in synth.moe_layer_tensors(e, h, i, 128, seed=2))
+    x, logits = synth.activations(m, h, seed=m).cuda(), synth.gating_logits(m, e, seed=m).cuda()
+    return lambda: (A.awq_gemm(*dense, 8), A.fused_moe(x, w1, w2, logits, k, True))
+
+
+def test_graphs_captured_on_one_stream_run_side_by_side(A):
+    """Two captured steps with shared slabs and tiles, from one capture stream, replayed on two streams at
+    a time: each has scratch of its own."""
+    steps = [_layers(A, 5), _layers(A, 40)]
+    want = [[y.clone() for y in step()] for step in steps]
+    torch.cuda.synchronize()
+    graphs, outs = [], []
+    for step in steps:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):       # the default capture stream, the same for both
+            outs.append(step())
+        graphs.append(graph)
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    for _ in range(20):
+        for graph, stream in zip(graphs, streams):
+            with torch.cuda.stream(stream):
+                for _ in range(10):
+                    graph.replay()
+        torch.cuda.synchronize()
+        for ys, refs in zip(outs, want):
+            assert all(torch.equal(y, ref) for y, ref in zip(ys, refs))
+    assert device_status() == 0, "a bounded wait ran out"
+
+
+def test_capture_on_a_new_stream_takes_calls_of_any_size(A):
+    """A stream's first captured calls: a linear, then a fused-MoE layer with a larger need."""
+    from awq_b200 import synth
+    small = _layers(A, 5)
+    e, h, i, k, t = 16, 2048, 768, 8, 1024
+    w1, w2 = (tuple(a.cuda() for a in w) for w in synth.moe_layer_tensors(e, h, i, 128, seed=2))
+    x, logits = synth.activations(t, h, seed=t).cuda(), synth.gating_logits(t, e, seed=t).cuda()
+    want = A.fused_moe(x, w1, w2, logits, k, True)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=torch.cuda.Stream()):
+        small()
+        y = A.fused_moe(x, w1, w2, logits, k, True)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, want)
