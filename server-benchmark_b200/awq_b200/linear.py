@@ -52,7 +52,8 @@ class AWQConfig:
 
 
 def kmajor_pays(qweight: torch.Tensor, group_size: int) -> bool:
-    """Whether the K-major decode kernel is the faster one for a layer of this size."""
+    """Whether ``decode_kmajor`` makes a copy of a layer of this size (from about which size the K-major
+    kernel is faster than the decode-layout one)."""
     k, words = qweight.shape
     if group_size != 128 or k % 128 != 0 or k // 128 > 256:
         return False

@@ -182,8 +182,8 @@ def parser() -> argparse.ArgumentParser:
     ap.add_argument("--pipeline-parallel-size", type=int, default=1)
     ap.add_argument("--extra-args", default="--max-model-len 8192")
     ap.add_argument("--plugin", default="on", choices=["on", "fill", "off"])
-    ap.add_argument("--repack-decode", action="store_true")
-    ap.add_argument("--decode-kmajor", action="store_true")
+    ap.add_argument("--repack-decode", action="store_true", help="accepted; the plug-in makes no copies")
+    ap.add_argument("--decode-kmajor", action="store_true", help="accepted; the plug-in makes no copies")
     ap.add_argument("--policy", default="round_robin", choices=["round_robin", "least_conn"])
     ap.add_argument("--concurrency", default="1", help="one value or a comma-separated list")
     ap.add_argument("--num-prompts", default="100", help="one value, or one per concurrency")

@@ -16,7 +16,6 @@ from vllm.model_executor.layers.quantization.utils.quant_utils import is_layer_s
 from vllm.model_executor.utils import set_weight_attrs
 
 from . import ops, torch_ops
-from .linear import kmajor_pays
 from .vllm_plugin import _name_seed, _options, calls, fill_awq_tensors
 
 
@@ -31,25 +30,15 @@ class B200AWQLinearMethod(AWQLinearMethod):
         if _options["dummy_fill"] is not None:
             fill_awq_tensors(layer.qweight.data, layer.scales.data, layer.qzeros.data,
                              _options["dummy_fill"] + _name_seed(layer))
-        k, words = layer.qweight.shape
-        group = k // layer.scales.shape[0]
-        layer.qweight_decode = None
-        layer.qweight_kmajor = None
-        if _options["repack_decode"] and group == 128 and k % 128 == 0 and words % 4 == 0:
-            layer.qweight_decode = ops.awq_repack(layer.qweight.data)
-        if _options["decode_kmajor"] and kmajor_pays(layer.qweight.data, group):
-            layer.qweight_kmajor = ops.awq_repack_kmajor(layer.qweight.data)
 
     def apply(self, layer, x, bias=None):
-        # traced by torch.compile inside vLLM: one registered operator, layout choice inside
+        # traced by torch.compile inside vLLM: one registered operator for every token count
         calls["linear"] += 1
         if x.dtype != torch.float16:
             raise ValueError("AWQ on B200 computes in fp16: start vLLM with --dtype half")
         out_shape = x.shape[:-1] + (layer.scales.shape[-1],)
         x2 = x.reshape(-1, x.shape[-1]).contiguous()
-        out = torch_ops.linear(x2, layer.qweight, layer.scales, layer.qzeros, bias,
-                               getattr(layer, "qweight_decode", None),
-                               getattr(layer, "qweight_kmajor", None))
+        out = torch_ops.linear(x2, layer.qweight, layer.scales, layer.qzeros, bias, None, None)
         return out.reshape(out_shape)
 
 
@@ -97,10 +86,6 @@ class B200AWQMoEMethod(FusedMoEMethodBase):
             fill_awq_tensors(layer.w2_qweight.data, layer.w2_scales.data,
                              layer.w2_qzeros.data, seed + 2)
         self.moe_quant_config = None   # rebuilt from the final parameters on first use
-        layer.w13_decode = layer.w2_decode = None
-        if _options["repack_decode"] and self.quant_config.group_size == 128:
-            layer.w13_decode = ops.awq_repack(layer.w13_qweight.data)
-            layer.w2_decode = ops.awq_repack(layer.w2_qweight.data)
 
     def get_fused_moe_quant_config(self, layer):
         # built after loading (layer.ensure_moe_quant_config_init): scales and zero points
@@ -128,8 +113,6 @@ class B200AWQMoEMethod(FusedMoEMethodBase):
             apply_router_weight_on_input=getattr(layer, "apply_router_weight_on_input", False),
             global_num_experts=getattr(layer, "global_num_experts", -1),
             expert_map=getattr(layer, "expert_map", None),
-            w1_decode=getattr(layer, "w13_decode", None),
-            w2_decode=getattr(layer, "w2_decode", None),
             quant_config=self.moe_quant_config)
 
 

@@ -26,8 +26,9 @@ every worker, vllm/plugins/__init__.py:28-82; the function is idempotent, as vLL
 
 Options (keyword arguments of ``register`` or the environment variables in brackets, which is
 what a vLLM that loads the plug-in itself sees):
-  repack_decode  [AWQ_B200_REPACK_DECODE=1]  decode-layout copies of ``qweight`` for <= 8 tokens
-  decode_kmajor  [AWQ_B200_DECODE_KMAJOR=1]  K-major copies of the largest layers for 9..16 tokens
+  repack_decode  [AWQ_B200_REPACK_DECODE=1]  accepted, with a warning, and without effect: the kernels
+  decode_kmajor  [AWQ_B200_DECODE_KMAJOR=1]  on the checkpoint layout serve every token count, and a copy
+                 that no layer reads would only take memory from the KV cache
   dummy_fill     [AWQ_B200_DUMMY_FILL=seed]  after loading, overwrite the integer parameters and
                  scales from a seeded generator: ``--load-format dummy`` leaves integer
                  parameters uninitialised (model_loader/weight_utils.py:1484-1490) and draws
@@ -40,6 +41,7 @@ what a vLLM that loads the plug-in itself sees):
 from __future__ import annotations
 
 import os
+import warnings
 import zlib
 
 import torch
@@ -48,7 +50,7 @@ from . import ops
 
 _registered = False
 _lib_handle = None
-_options = {"repack_decode": False, "decode_kmajor": False, "dummy_fill": None}
+_options = {"dummy_fill": None}
 calls = {"linear": 0, "moe": 0, "awq_gemm_op": 0, "awq_dequantize_op": 0}
 
 
@@ -137,8 +139,10 @@ def register(full_gemm: bool = True, repack_decode: bool = False, decode_kmajor:
     the earlier signature: the linear method uses the fused kernels for every token count."""
     global _registered, _lib_handle
     env = os.environ.get
-    _options["repack_decode"] = repack_decode or env("AWQ_B200_REPACK_DECODE") == "1"
-    _options["decode_kmajor"] = decode_kmajor or env("AWQ_B200_DECODE_KMAJOR") == "1"
+    for name, asked in (("repack_decode", repack_decode), ("decode_kmajor", decode_kmajor)):
+        if asked or env("AWQ_B200_" + name.upper()) == "1":
+            warnings.warn(f"awq_b200: {name} makes no copies under vLLM, no layer would read them",
+                          stacklevel=2)
     if dummy_fill is None and env("AWQ_B200_DUMMY_FILL") not in (None, ""):
         dummy_fill = int(env("AWQ_B200_DUMMY_FILL"))
     _options["dummy_fill"] = dummy_fill

@@ -55,21 +55,21 @@ def test_vllm_awq_linear_method_runs_on_our_ops(built_library):
 
 
 def test_plugin_linear_method_with_layout_copies(built_library):
-    """register(repack_decode=True, decode_kmajor=True): the plug-in's linear method keeps the
-    decode-layout copy (and, for layers large enough, the K-major copy) after loading and serves
-    each token count from the layout made for it."""
+    """register(repack_decode=True, decode_kmajor=True): accepted with a warning, and the plug-in's linear
+    method, whose kernels read the checkpoint layout at every token count, holds no further copy."""
     try:
         import vllm._C  # noqa: F401
         from vllm.model_executor.layers.quantization import awq as vllm_awq
     except Exception as e:  # pragma: no cover
         pytest.skip(f"vllm not usable here: {e}")
     from awq_b200 import synth, vllm_plugin
-    vllm_plugin.register(repack_decode=True, decode_kmajor=True)
+    with pytest.warns(UserWarning, match="makes no copies"):
+        vllm_plugin.register(repack_decode=True, decode_kmajor=True)
     try:
         method_cls = vllm_plugin.classes["linear"]
         assert issubclass(method_cls, vllm_awq.AWQLinearMethod)
         cfg = vllm_awq.AWQConfig(weight_bits=4, group_size=128, zero_point=True)
-        for (k, n, want_kmajor) in ((2048, 1536, False), (8192, 59136, True)):
+        for (k, n) in ((2048, 1536), (8192, 59136)):
             qw, s, qz = synth.awq_linear_tensors(k, n, 128, seed=43)
             method = method_cls(cfg)
 
@@ -80,10 +80,9 @@ def test_plugin_linear_method_with_layout_copies(built_library):
             layer.qweight = torch.nn.Parameter(qw.cuda(), requires_grad=False)
             layer.scales = torch.nn.Parameter(s.cuda(), requires_grad=False)
             layer.qzeros = torch.nn.Parameter(qz.cuda(), requires_grad=False)
+            held = torch.cuda.memory_allocated()
             method.process_weights_after_loading(layer)
-            assert layer.qweight_decode is not None
-            assert layer.qweight_decode.shape == layer.qweight.shape
-            assert (layer.qweight_kmajor is not None) == want_kmajor
+            assert torch.cuda.memory_allocated() == held
             w = O.dequantize_fp32(qw.numpy(), s.numpy(), qz.numpy(), 128)
             for m in (1, 8, 9, 16, 300):
                 x = synth.activations(m, k, seed=m).cuda()
