@@ -178,37 +178,53 @@ def test_prefill_tiles_per_expert(A, counts, group):
     assert O.rel_err(y.cpu().numpy(), ref) < TOL
 
 
+# Groups of 128: gemm_ts; 64 and 32: the mma.sync kernels, whose down GEMM adds the slots itself unless its
+# counters do not fit (64 tokens of 8192).  Every case has at least twice as many experts as pairs, or is
+# not direct.
+@pytest.mark.parametrize("group", [128, 64, 32])
 @pytest.mark.parametrize("t,k,e,h,i", [(1, 8, 128, 2048, 768), (2, 8, 128, 2048, 768),
-                                       (3, 4, 16, 512, 256), (1, 2, 8, 256, 128),
+                                       (2, 4, 16, 512, 256), (1, 2, 8, 256, 128),
                                        (4, 8, 128, 2048, 768), (8, 8, 128, 2048, 768),
-                                       (5, 8, 16, 8192, 256), (64, 1, 64, 8192, 256),
-                                       (64, 1, 16, 512, 256)])
-def test_direct_mode_for_a_handful_of_pairs_equals_the_permuted_path(A, t, k, e, h, i, monkeypatch):
-    """A handful of (token, slot) pairs skip the permutation kernel (one row block per pair,
-    experts read from topk_ids) and the slot sum happens inside the down GEMM (or, when the
-    counters do not fit, in the sum kernel).  An identity expert_map forces the permuted path:
-    same bits."""
-    from awq_b200 import ops
-    monkeypatch.setattr(ops, "MOE_DIRECT_MAX_PAIRS", 64)     # the C ABI's limit
-    w1, w2, x, logits = _moe_case(e, h, i, t, k, seed=40 + t)
+                                       (5, 8, 128, 8192, 256), (64, 1, 128, 8192, 256),
+                                       (64, 1, 128, 512, 256)])
+def test_direct_mode_for_a_handful_of_pairs_equals_the_permuted_path(A, t, k, e, h, i, group, monkeypatch):
+    """A handful of (token, slot) pairs skip the permutation kernel (one row block per pair, experts read
+    from topk_ids): the same roundings as through the permutation, on the mma.sync kernels the same bits.
+    With an expert_map (here the identity) the direct mode reads the mapped ids."""
+    from awq_b200 import ops, synth
+    assert 2 * t * k <= e and t * k <= ops.MOE_DIRECT_MAX_PAIRS
+    w1, w2 = synth.moe_layer_tensors(e, h, i, group, seed=40 + t)
+    x, logits = synth.activations(t, h, seed=41 + t), synth.gating_logits(t, e, seed=42 + t)
     w1d = tuple(a.cuda() for a in w1)
     w2d = tuple(a.cuda() for a in w2)
     wts, ids, _ = A.fused_topk(x.cuda(), logits.cuda(), k, True)
-    direct = A.fused_experts(x.cuda(), w1d, w2d, wts, ids)
-    permuted = A.fused_experts(x.cuda(), w1d, w2d, wts, ids, global_num_experts=e,
-                               expert_map=torch.arange(e, dtype=torch.int32, device="cuda"))
-    assert torch.equal(direct, permuted)
+    emap = torch.arange(e, dtype=torch.int32, device="cuda")
+
+    def both(ids):
+        direct = A.fused_experts(x.cuda(), w1d, w2d, wts, ids, group_size=group)
+        mapped = A.fused_experts(x.cuda(), w1d, w2d, wts, ids, group_size=group, global_num_experts=e,
+                                 expert_map=emap)
+        with monkeypatch.context() as patch:
+            patch.setattr(ops, "MOE_DIRECT_MAX_PAIRS", 0)
+            permuted = A.fused_experts(x.cuda(), w1d, w2d, wts, ids, group_size=group)
+        assert torch.equal(direct, mapped)
+        if group != 128:
+            assert torch.equal(direct, permuted)
+        # gemm_ts cuts K by the number of tiles: fp32 sums in another order, which put some values on the
+        # other side of a rounding.  2^-11 each, fewer than one in six.
+        diff = (direct.double() - permuted.double()).norm() / permuted.double().norm()
+        assert diff < 2e-4
+        return direct
+
+    both(ids)
     # two slots of one token on the same expert: the pair blocks stay independent
     if k == 1:
         return
     ids2 = ids.clone()
     ids2[:, 1] = ids2[:, 0]
-    direct2 = A.fused_experts(x.cuda(), w1d, w2d, wts, ids2)
-    permuted2 = A.fused_experts(x.cuda(), w1d, w2d, wts, ids2, global_num_experts=e,
-                                expert_map=torch.arange(e, dtype=torch.int32, device="cuda"))
-    assert torch.equal(direct2, permuted2)
+    direct2 = both(ids2)
     ref = O.fused_experts_fp32(x.numpy(), *[a.numpy() for a in w1], *[a.numpy() for a in w2],
-                               wts.cpu().numpy(), ids2.cpu().numpy())
+                               wts.cpu().numpy(), ids2.cpu().numpy(), group)
     assert O.rel_err(direct2.float().cpu().numpy(), ref) < TOL
 
 
@@ -448,9 +464,9 @@ def test_fused_moe_full_size_rows_are_independent(A):
                                        (8, 256, 128, 50, 2), (40, 512, 256, 12, 2),
                                        (256, 2048, 768, 128, 8), (300, 512, 256, 4, 2)])
 def test_experts_on_decode_layout_copies_equal_checkpoint_layout(A, t, h, i, e, k):
-    """fused_experts with the decode-layout copies of the expert weights: bit-identical to the
-    checkpoint layout where the streaming kernels run (blocks of 8 / 16 rows), and the copies
-    are simply not used where the grouped tcgen05 GEMMs run (last case)."""
+    """Decode-layout copies of the expert weights.  fused_experts accepts them and reads the checkpoint
+    layout; the C ABI reads them when told so (flag bit 1): bit-identical to the same mma.sync kernels on
+    the checkpoint layout, which run when the scratch has no room for partial tiles."""
     from awq_b200 import synth
     w1, w2 = synth.moe_layer_tensors(e, h, i, 128, seed=t + e)
     w1 = tuple(a.cuda() for a in w1)
@@ -469,6 +485,40 @@ def test_experts_on_decode_layout_copies_equal_checkpoint_layout(A, t, h, i, e, 
     assert O.rel_err(y1.cpu().numpy(), ref) < TOL
     with pytest.raises(ValueError):
         A.fused_experts(x, w1, w2, w, ids, w1_decode=d1)
+
+    from awq_b200 import _lib
+    lib = _lib.load()
+    block = lib.awq_b200_moe_block_size(t, k, e, h, i, 128)
+    sorted_ids, expert_ids, post = A.moe_align_block_size(ids, block, e, None)
+    rows = -(-sorted_ids.numel() // block) * block
+
+    def experts(q1, q2, flags, tables, capacity, nbytes):
+        out = torch.full_like(x, float("nan"))
+        scratch = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+        rc = lib.awq_b200_moe_experts(
+            x.data_ptr(), q1.data_ptr(), w1[1].data_ptr(), w1[2].data_ptr(), q2.data_ptr(), w2[1].data_ptr(),
+            w2[2].data_ptr(), w.data_ptr(), *tables, out.data_ptr(), t, k, e, h, i, 128, block, flags,
+            capacity, scratch.data_ptr(), nbytes, torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        return rc, out
+
+    tables = (sorted_ids.data_ptr(), expert_ids.data_ptr(), post.data_ptr())
+    if block == 128:
+        full = lib.awq_b200_moe_workspace_bytes(t, k, e, h, i)
+        assert experts(d1, d2, 2, tables, sorted_ids.numel(), full)[0] == -2     # AWQ_B200_ERR_SHAPE
+        return
+    # activations of the permuted rows, rows by pair; the counters of the direct mode
+    layout = lambda rows: -(-rows * i * 2 // 256) * 256 + -(-t * k * h * 2 // 256) * 256   # noqa: E731
+    calls = [(0, tables, sorted_ids.numel(), layout(rows))]
+    if block == 8 and t * k <= 64:
+        calls.append((4, (None, ids.data_ptr(), None), t * k * 8, layout(t * k * 8) + 4096))
+    for flags, table, capacity, nbytes in calls:
+        rc, plain = experts(w1[0], w2[0], flags, table, capacity, nbytes)
+        assert rc == 0
+        rc, copies = experts(d1, d2, flags | 2, table, capacity, nbytes)
+        assert rc == 0
+        assert torch.equal(plain, copies)
+        assert O.rel_err(copies.float().cpu().numpy(), ref) < TOL
 
 
 # Batches of different sizes in turn, larger ones of NaN: nothing that an earlier call left in the

@@ -91,7 +91,9 @@ def test_linear_method_with_decode_copy(A):
         layers.append((method, layer))
     assert layers[0][1].qweight_decode is None
     assert layers[1][1].qweight_decode is not None
-    for m in (1, 8, 9, 40):     # 9 and 40 leave the decode copy unused
+    layer = layers[1][1]
+    # the layer reads the checkpoint layout with or without the copy, which serves callers that name its kernel
+    for m in (1, 8, 9, 40):
         x = synth.activations(m, k, seed=m).cuda()
         y0 = layers[0][0].apply(layers[0][1], x)
         y1 = layers[1][0].apply(layers[1][1], x)
@@ -99,3 +101,7 @@ def test_linear_method_with_decode_copy(A):
         assert O.rel_err(y1.cpu().numpy(), ref) < TOL
         if m > 8:
             assert torch.equal(y0, y1)
+        else:
+            y2 = A.awq_gemm(x, layer.qweight_decode, layer.scales, layer.qzeros, 8, kernel=A.KERNEL_STREAM_RP)
+            assert torch.equal(y2, A.awq_gemm(x, layer.qweight, layer.scales, layer.qzeros, 8,
+                                              kernel=A.KERNEL_STREAM))
