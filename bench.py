@@ -600,7 +600,6 @@ def run_sweep(dev, stream):
                 tq = graph_time(fns, stream, reps=10)
                 row["us_kmajor"] = round(tq * 1e6, 2)
                 row["weight_GBps_kmajor"] = round(wbytes / tq / 1e9, 1)
-            best = min(v for kk, v in row.items() if kk.startswith("us"))
             if V is None:
                 row["vllm"] = "compiled ops of the installed vLLM did not load"
             else:
@@ -616,7 +615,7 @@ def run_sweep(dev, stream):
                     tm = graph_time([(lambda mq=mq: V.marlin_gemm(x, mq)) for mq in marlin],
                                     stream, reps=max(2, reps // 2))
                     row["vllm_marlin_us"] = round(tm * 1e6, 2)
-                    row["speedup_vs_vllm_marlin"] = round(row["vllm_marlin_us"] / best, 2)
+                    row["speedup_vs_vllm_marlin"] = round(row["vllm_marlin_us"] / row["us"], 2)
                 except Exception as e:   # a vLLM op that refuses a shape is a missing column
                     row["vllm"] = f"{type(e).__name__}: {str(e)[:120]}"
             out.append(row)
@@ -646,15 +645,12 @@ def run_moe(dev, stream):
         w1, w2 = synth.moe_layer_tensors(e, h, i, GROUP, seed=seed)
         w1 = tuple(a.to(dev) for a in w1)
         w2 = tuple(a.to(dev) for a in w2)
-        layers.append((w1, w2, awq_b200.awq_repack(w1[0]), awq_b200.awq_repack(w2[0]),
-                       V.marlin_moe_prepare(w1, w2) if V is not None else None))
-    from awq_b200 import _lib
-    block_of = lambda t: _lib.load().awq_b200_moe_block_size(t, k, e, h, i, GROUP)  # noqa: E731
+        layers.append((w1, w2, V.marlin_moe_prepare(w1, w2) if V is not None else None))
     awq_b200.reserve_workspace(awq_b200.moe_workspace_bytes(max(synth.MOE_TOKENS), k, e, h, i), dev)
     out = []
     from awq_b200 import ops as awq_ops
     # the benchmark's token counts, plus the few-token decode points where the direct mode (no
-    # permutation kernel, slot sum inside the down GEMM) competes with the permuted chain
+    # permutation kernel) competes with the permuted chain
     for t in sorted(set(synth.MOE_TOKENS) | {2, 4, 8}):
         x = synth.activations(t, h).to(dev)
         logits = synth.gating_logits(t, e).to(dev)
@@ -679,25 +675,17 @@ def run_moe(dev, stream):
                 row[name] = round(sm * 1e6, 1)
             awq_ops.MOE_DIRECT_MAX_PAIRS = keep
             row["direct_by_default"] = t * k <= keep
-        if block_of(t) in (8, 16):
-            # the same layer with the optional decode-layout copies of the expert weights
-            def layer(L):
-                w, ids2, _ = awq_b200.fused_topk(x, logits, k, True)
-                return awq_b200.fused_experts(x, L[0], L[1], w, ids2, w1_decode=L[2], w2_decode=L[3])
-            sd = graph_time([(lambda L=L: layer(L)) for L in layers], stream, reps=reps)
-            row["us_decode_layout"] = round(sd * 1e6, 1)
         if V is None:
             row["vllm"] = "compiled ops of the installed vLLM did not load"
         else:
             try:
                 def theirs(L):
                     w, ids2 = V.topk_softmax(logits, k, True)
-                    return V.marlin_moe(x, L[4], w, ids2)
+                    return V.marlin_moe(x, L[2], w, ids2)
                 sv = graph_time([(lambda L=L: theirs(L)) for L in layers], stream,
                                 reps=max(2, reps // 2))
                 row["vllm_marlin_moe_us"] = round(sv * 1e6, 1)
-                best = min(v for kk, v in row.items() if kk.startswith("us"))
-                row["speedup_vs_vllm_marlin_moe"] = round(row["vllm_marlin_moe_us"] / best, 2)
+                row["speedup_vs_vllm_marlin_moe"] = round(row["vllm_marlin_moe_us"] / row["us"], 2)
             except Exception as ex:
                 row["vllm"] = f"{type(ex).__name__}: {str(ex)[:120]}"
         out.append(row)
