@@ -236,7 +236,6 @@ int ar_device_status(int* out, int clear);
 int launch_wna16_to_awq(const uint8_t* w, const __half* scales, const uint8_t* zeros,
                         uint32_t* qweight, __half* scales_out, uint32_t* qzeros, int E, int N,
                         int K, int group, cudaStream_t stream);
-bool moe_wt_supported(int H, int I, int group);
 int launch_wt_grouped(int mode, int tile_rows, const __half* a, int64_t a_rows, const uint32_t* w, int experts,
                       const __half* scales, const uint32_t* qzeros, const int4* tiles,
                       const int32_t* n_tiles, const float* row_weights, __half* out, int K, int N, int group,

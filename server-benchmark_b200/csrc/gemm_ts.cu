@@ -547,6 +547,8 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     if (lane == 0)
       for (int u = 0; u < NDB; ++u) mbar_arrive(unit_full(u));
     pdl_wait();  // orders this thread's writes after the kernel before this one
+    const unsigned long long token = p.flags.token;
+    unsigned long long* flag = p.flags.at(blockIdx.x, fold);  // this warp's
     bool ok = true;
     int u = 0;
     for (int seg = 0; seg < work.segs; ++seg) {
@@ -632,24 +634,26 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
           for (int m = 0; m < MT; ++m) part[m * kTsBN] = gate[m * 32];
         }
         __syncwarp();
-        if (lane == 0 && ok && !s_abort) p.flags.raise(blockIdx.x, fold);
+        if (lane == 0 && ok && !s_abort) handover::raise_flag(flag, token);
         continue;
       }
-      const int gather = work.helpers(seg);  // CTAs before this one that share the tile
-      if (gather > 0) {
-        if (ok)
-          for (int c = 1 + lane; c <= gather; c += 32) {
-            uint32_t polls = 0;
-            while (!p.flags.raised(blockIdx.x - c, fold)) {
-              if (++polls >= kSpinLimit || s_abort) {
-                s_abort = 1;
-                atomicCAS(&g_tc_status, 0, 29);
-                ok = false;
-                break;
-              }
+      int gather = 0;  // CTAs before this one that share the tile
+      if (kb > 0) {
+        gather = blockIdx.x - id * work.KT / work.chunk;
+        for (int c = 1 + lane; c <= gather; c += 32) {
+          unsigned long long* theirs = flag - c * handover::kMaxWarps;
+          uint32_t polls = 0;
+          while (handover::read_flag(theirs) != token) {
+            if (++polls >= kSpinLimit || s_abort) {
+              s_abort = 1;
+              atomicCAS(&g_tc_status, 0, 29);
+              ok = false;
+              linger();  // no replay must find what is raised meanwhile
+              break;
             }
-            p.flags.lower(blockIdx.x - c, fold);
           }
+          *theirs = 0;
+        }
         ok = __all_sync(0xffffffffu, ok);
         __syncwarp();  // what a lane acquired holds for the warp's reads of the partial tiles
       }
@@ -725,14 +729,8 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   __syncwarp();
   if (s_abort) {
     // a wait gave up: copies and MMAs may still be in flight towards this CTA's shared and tensor
-    // memory.  Let them land (a millisecond) before both are given back.
-    const long long t_end = clock64() + 2000000;
-    while (clock64() < t_end) {
-    }
-    // flags raised meanwhile: a replay of this launch must not find them
-    if (warp >= kTsFold0 && warp < kTsIssue && work.segs > 0)
-      for (int c = 1 + lane; c <= work.helpers(work.segs - 1); c += 32)
-        p.flags.lower(blockIdx.x - c, warp - kTsFold0);
+    // memory.  Let them land before both are given back.
+    linger();
   }
   tc_fence_before();
   __syncthreads();

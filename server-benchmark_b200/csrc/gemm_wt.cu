@@ -700,10 +700,8 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   __syncwarp();
   if (s_abort) {
     // a wait gave up: copies and MMAs may still be in flight towards this pair's shared and
-    // tensor memory.  Let them land (a millisecond) before both are given back.
-    const long long t_end = clock64() + 2000000;
-    while (clock64() < t_end) {
-    }
+    // tensor memory.  Let them land before both are given back.
+    linger();
     // flags raised meanwhile: a replay of this launch must not find them
     if (MODE == 0 && warp >= kWtEpiWarp0 && warp < kWtEpiWarp0 + kWtEpiWarps && work.segs > 0)
       for (int c = 1 + lane; c <= work.helpers(work.segs - 1); c += 32)
@@ -954,11 +952,6 @@ int launch_gemm_wt(const __half* x, const uint32_t* qweight, const __half* scale
   p.K = K;
   return group == 128 ? launch_wt_dense<128>(x, qweight, p, workspace, workspace_bytes, stream)
                       : launch_wt_dense<64>(x, qweight, p, workspace, workspace_bytes, stream);
-}
-
-bool moe_wt_supported(int H, int I, int group) {
-  // slabs: 128 gate + 128 up columns (I % 128), 256 hidden columns (H % 256); whole stages of K
-  return H % 256 == 0 && I % 128 == 0 && (group == 128 || group == 64);
 }
 
 namespace {

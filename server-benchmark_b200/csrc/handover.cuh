@@ -26,20 +26,22 @@ constexpr int kMaxCtas = 256;
 constexpr int kMaxWarps = 8;
 constexpr size_t kFlagBytes = (size_t)kMaxCtas * kMaxWarps * sizeof(unsigned long long);
 
+__device__ __forceinline__ void raise_flag(unsigned long long* flag, unsigned long long token) {
+  asm volatile("st.release.gpu.global.b64 [%0], %1;" ::"l"(flag), "l"(token) : "memory");
+}
+__device__ __forceinline__ unsigned long long read_flag(const unsigned long long* flag) {
+  unsigned long long v;
+  asm volatile("ld.acquire.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(flag) : "memory");
+  return v;
+}
 struct Flags {
   unsigned long long* base;  // [CTA][kMaxWarps]
   unsigned long long token;
   __device__ __forceinline__ unsigned long long* at(int cta, int warp) const {
     return base + cta * kMaxWarps + warp;
   }
-  __device__ __forceinline__ void raise(int cta, int warp) const {
-    asm volatile("st.release.gpu.global.b64 [%0], %1;" ::"l"(at(cta, warp)), "l"(token) : "memory");
-  }
-  __device__ __forceinline__ bool raised(int cta, int warp) const {
-    unsigned long long v;
-    asm volatile("ld.acquire.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(at(cta, warp)) : "memory");
-    return v == token;
-  }
+  __device__ __forceinline__ void raise(int cta, int warp) const { raise_flag(at(cta, warp), token); }
+  __device__ __forceinline__ bool raised(int cta, int warp) const { return read_flag(at(cta, warp)) == token; }
   __device__ __forceinline__ void lower(int cta, int warp) const { *at(cta, warp) = 0; }
 };
 

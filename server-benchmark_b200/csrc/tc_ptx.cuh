@@ -80,6 +80,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
                                           int code) {
   return mbar_wait_n(bar, parity, abort_flag, code, kSpinLimit);
 }
+// About a millisecond, after a wait that gave up.
+__device__ __forceinline__ void linger() {
+  const long long end = clock64() + 2000000;
+  while (clock64() < end) {
+  }
+}
 // True in exactly one lane of a fully active warp (always the same lane).  A tcgen05.mma or
 // tcgen05.commit issued this way from a converged warp costs its warp ~25-45 cycles; issued from
 // one lane that loops alone while the other 31 are parked elsewhere it was measured at ~150.
