@@ -71,11 +71,15 @@ int awq_b200_dequantize(const void* qweight, const void* scales, const void* qze
  * Replaces torch.ops._C.awq_gemm(input, qweight, scales, qzeros, split_k_iters)
  * (vllm/_custom_ops.py:576-587; called from quantization/awq.py:283) and the
  * awq_dequantize + torch.matmul pair used for >= 256 tokens (awq.py:276-281): one entry
- * point serves every M, picking a weight-streaming kernel or one of the tcgen05 kernels by M.
+ * point serves every M, picking one of the kernels by M, group and shape.
  * `kernel` selects the implementation: AWQ_B200_KERNEL_AUTO or one of the explicit ids (a
  * request the shape does not permit returns AWQ_B200_ERR_SHAPE).
- * Scratch: awq_b200_gemm_workspace_bytes(M, N, K, group, kernel) bytes, 256-byte aligned; may
- * be NULL when that size is 0.
+ * Scratch: awq_b200_gemm_workspace_bytes(M, N, K, group, kernel) bytes, 256-byte aligned, any
+ * content.  AWQ_B200_KERNEL_AUTO, _TS and _WT do without it where it is NULL, smaller or misaligned:
+ * AUTO then takes the streaming kernel at small M, TS and WT distribute whole slabs or tiles.  With it,
+ * CTAs hand partial tiles to each other there, announced by flags in the same buffer.  So calls that may
+ * overlap on the GPU need separate scratch buffers; this includes calls captured on one stream
+ * whose graphs are replayed on several.
  */
 #define AWQ_B200_KERNEL_AUTO 0
 #define AWQ_B200_KERNEL_GENERIC 1  /* CUDA-core reference kernel, any legal shape */
@@ -83,7 +87,7 @@ int awq_b200_dequantize(const void* qweight, const void* scales, const void* qze
 #define AWQ_B200_KERNEL_TCGEN05 3  /* large-M tcgen05/TMEM kernel with in-smem dequantisation */
 #define AWQ_B200_KERNEL_STREAM_EXACT 4 /* small-M kernel with the magic-number conversion */
 #define AWQ_B200_KERNEL_TS 5       /* M <= 16: registers -> TMEM weights, tcgen05.mma (A in TMEM) */
-#define AWQ_B200_KERNEL_TS_EXACT 6 /* the same with the magic-number conversion */
+#define AWQ_B200_KERNEL_TS_EXACT 6 /* shapes of TS: streaming kernel with the magic-number conversion */
 #define AWQ_B200_KERNEL_WT 7       /* any M: dequantised weights registers -> TMEM (A operand), x via TMA as B */
 #define AWQ_B200_KERNEL_STREAM_RP 8 /* M <= 8 streaming kernel; `qweight` is the output of awq_b200_repack_qweight */
 #define AWQ_B200_KERNEL_Q8 9 /* M <= 32: `qweight` is the output of awq_b200_repack_kmajor; nibbles widened by tcgen05.cp, int8 MMAs */
@@ -144,16 +148,16 @@ int awq_b200_gemm(const void* x, const void* qweight, const void* scales, const 
 
 /*
  * Health word of the tcgen05 kernel on the current device.  Its mbarrier waits are bounded;
- * a wait that ran out records which one (1 producer, 2-3 MMA issuer, 4 dequantisation,
- * 5 epilogue; 11-15 the M <= 16 kernel) and the kernel tears down instead of hanging.  0 = no wait ever ran out.
+ * a wait that ran out records which one (1-7 AWQ_B200_KERNEL_TCGEN05, 21-29 _TS and the expert GEMMs of
+ * small batches, 31-40 _WT and those of prefill, 31-35 also _Q8; 29, 39 and, for _Q8, 35: a partial tile of
+ * another CTA) and the kernel tears down instead of hanging.  0 = no wait ever ran out.
  * Synchronises the device (a plain device-to-host copy).  No counterpart in the reference.
  */
 int awq_b200_device_status(int* status);
 
 /*
  * The same, and the word is put back to 0 afterwards.  The word is sticky: it keeps the first
- * wait that ran out (31-35: the AWQ_B200_KERNEL_Q8 kernel; 35 = a CTA waited in vain for a
- * partial tile of another CTA) until it is cleared here, and a call during which a wait ran out
+ * wait that ran out until it is cleared here, and a call during which a wait ran out
  * still returns AWQ_B200_OK with an incomplete output.  No counterpart in the reference.
  */
 int awq_b200_device_status_clear(int* status);
@@ -259,9 +263,12 @@ int awq_b200_moe_align_block_size(const int32_t* topk_ids, int T, int topk, int 
  *   w2_q  int32 [E, I, H/8],  w2_s  fp16 [E, I/G, H],  w2_z  int32 [E, I/G, H/8]
  * (parameter layout: quantization/awq_marlin.py:549-623).  sorted_ids / expert_ids /
  * num_post_pad are the outputs of awq_b200_moe_align_block_size with block =
- * awq_b200_moe_block_size(T, topk, E, H, I, group): 8 or 16 (weight-streaming kernels; 8 while an
- * expert sees at most eight rows on average) for decode-size batches, 128 (tcgen05 grouped GEMMs)
- * once an expert sees 36 rows or more on average.
+ * awq_b200_moe_block_size(T, topk, E, H, I, group): 8 or 16 (8 while an expert sees at most eight
+ * rows on average) for decode-size batches, 128 (grouped GEMMs on tiles of up to 256 rows, weights rounded
+ * to fp16) once an expert sees 36 rows or more on average.
+ * Every (token, slot) row is rounded to fp16 after its routed weight, and a token's rows are added in fp32.
+ * Ids outside [0, E) are dropped by the permutation; with block 128 such a pair contributes zero, with
+ * the smaller blocks only if bit 0 below is set.
  * Replaces fused_experts / fused_experts_impl (fused_moe/fused_moe.py:1587-1631,1664-1869)
  * and the Marlin expert path (fused_moe/experts/marlin_moe.py:225-262).
  * E is the number of stacked (local) experts.  `expert_parallel` is a set of flags: bit 0 says
@@ -273,8 +280,7 @@ int awq_b200_moe_align_block_size(const int32_t* topk_ids, int T, int topk, int 
  * expert_map): no permutation is needed - expert_ids is the routed-id table topk_ids [T * topk]
  * itself, sorted_ids and num_post_pad are ignored (may be NULL), sorted_capacity must be
  * T * topk * 8 (one 8-row block per pair) - which takes awq_b200_moe_align_block_size out of the
- * chain for the decode of a few tokens; the down GEMM then also adds a token's slots itself, so the
- * chain is two launches; bit 3, only together with bit 2, says the table may hold negative ids
+ * chain for the decode of a few tokens; bit 3, only together with bit 2, says the table may hold negative ids
  * (experts of other ranks, awq_b200_moe_local_ids), whose pairs contribute zero.  Every other id must
  * be a valid expert index in this mode, and the scratch
  * need (one 8-row block per pair) exceeds the bound of awq_b200_moe_workspace_bytes once
@@ -286,7 +292,7 @@ int awq_b200_moe_align_block_size(const int32_t* topk_ids, int T, int topk, int 
  * was built for (the global count under expert parallelism, else E).  A buffer smaller than the
  * layout returns AWQ_B200_ERR_WORKSPACE before anything is launched; one of the full
  * awq_b200_moe_workspace_bytes also has room for the partial tiles of the faster expert kernels of
- * small batches (group 128, checkpoint layout).
+ * small batches (group 128, checkpoint layout).  Calls that may overlap need separate scratch buffers.
  * Requires H % 128 == 0, I % 128 == 0, group in {32, 64, 128}.
  */
 #define AWQ_B200_MOE_DIRECT_MAX_PAIRS 64

@@ -24,8 +24,8 @@ from . import _lib
 PACK_FACTOR = 8
 MOE_DIRECT_MAX_PAIRS = 64     # pairs up to which fused_experts goes direct, with at least twice as
                               # many experts (the limit of the C ABI, AWQ_B200_MOE_DIRECT_MAX_PAIRS;
-                              # measured on the Qwen3-30B-A3B layer: 18 / 21 / 28 / 40 us direct
-                              # against 24 / 27 / 37 / 50 us through the permutation at 1 / 2 / 4 / 8
+                              # experts of the Qwen3-30B-A3B layer: 17 / 20 / 29 / 42 us direct
+                              # against 21 / 25 / 33 / 46 us through the permutation at 1 / 2 / 4 / 8
                               # tokens)
 
 

@@ -49,7 +49,8 @@
 // Lane 32 q + 8 i + g of tile t holds column
 // 128 t + 32 q + 8 (g / 2) + 2 i + g % 2 of the slab.  Every wait is bounded (tc_ptx.cuh).
 //
-// Measured (B200, K x N; before: mma.sync streaming kernel up to M = 8, its decode-layout copy in
+// Measured (B200, K x N, first replays of a cool GPU; under the power limit of a long loop 8192 x 59136 takes 48 and
+// 52 us; before: mma.sync streaming kernel up to M = 8, its decode-layout copy in
 // brackets, an earlier form of this kernel above; K-major copy in brackets):
 //   8192 x 59136   M 4: 56.2 (50.6) -> 44.9 us, 5.4 TB/s of int4    M 16: 82.1 (64.1) -> 50.2 us
 //   29568 x 8192   M 4: 35.0 (30.2) -> 25.9 us                        M 16: 40.0 (43.7) -> 29.5 us
@@ -59,8 +60,8 @@
 //   8192 x 59136   M 4: 69.2 -> 52.9 us, M 16: 106.8 -> 65.5;  8192 x 1280   M 4: 11.1 -> 6.3 us
 // Bound by HBM on the long layers (a unit takes 718 cycles at M = 4, 712 is what 6.45 TB/s allows; 854
 // at M = 16), by start-up and hand-over (~5 us) on the short ones.
-// Expert GEMMs, 128 experts of 2048 x 768, 8 per token, both GEMMs (before: two mma.sync kernels on the
-// decode copies): T 1: 25 -> 18 us, T 16: 81 -> 67, T 64: 107 -> 87, T 128: 124 -> 109.  At T = 64 all
+// Experts without the router, 128 of 2048 x 768, 8 per token (before: mma.sync kernels on the decode copies;
+// replayed graph): T 1: 22.9 -> 17.4 us, T 16: 71.0 -> 62.1, T 64: 101.9 -> 79.9, T 128: 110.7 -> 104.0.  At T = 64 all
 // 302 MB of int4 words are read, 48 us at the HBM rate; a block of 8 rows costs the conversion of a
 // whole matrix, which is what bounds it.
 #include "common.cuh"

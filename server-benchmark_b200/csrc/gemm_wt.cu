@@ -51,11 +51,12 @@
 //   two against weights dequantised into shared memory; 1.24 PFLOP/s, where the 1 kW limit holds the
 //   clock near 1.4 GHz); 29568 x 8192   M 100: 70 -> 58 us; router + experts, 128 experts of
 //   2048 x 768, top-8, 2500 tokens: 510 -> 305 us.
-// What bounds it: at M >= 256 the tensor pipe under the power limit; below, the fp16x2 arithmetic of the
-// conversion.  add / mul / fma.f16x2 take two cycles a warp and scheduler here, so subtract and scale
-// of 128 weights per lane are 262 of the ~600 cycles a stage takes (without them: 83 -> 50 us on
-// 8192 x 59136 at M = 24); units of twice the K, more load warps and fewer shared-memory or TMEM
-// accesses changed nothing.
+// What bounds it: at M >= 256 the tensor pipe under the power limit; below, the conversion, without a full
+// pipe (ncu at M = 64: issue 56 %, ALU 41, FMA 24, tensor 34).  add / mul / fma.f16x2 take two cycles a warp
+// and scheduler here, so subtract and scale of 128 weights per lane are 262 of the ~600 cycles a stage takes,
+// and without them 8192 x 59136 at M = 24 falls from 83 to 50 us; that fits the chain of each of the four
+// conversion warps of a scheduler (words, arithmetic, A slot, tcgen05.wait::st) as well as the pipe.  Units
+// of twice the K, more load warps and fewer shared-memory or TMEM accesses changed nothing.
 #include "common.cuh"
 #include "handover.cuh"
 #include "tc_ptx.cuh"

@@ -402,11 +402,11 @@ PyObject* experts(PyObject*, PyObject* const* a, Py_ssize_t n) {
       const int block = awq_b200_moe_block_size(T, K, ng, H, I, G);
       const at::Tensor ws =
           workspace(x.device(), (int64_t)awq_b200_moe_workspace_bytes(T, K, ng, H, I));
-      // A handful of pairs: one row block per pair straight from topk_ids, no permutation (5 to 9 us
+      // A handful of pairs: one row block per pair straight from topk_ids, no permutation (3 to 5 us
       // less).  Up to half as many pairs as experts, where most pairs have their expert to themselves:
-      // beyond, the permutation pays because an expert's matrices are then read once for all of its
-      // rows.  64 experts of 4096 x 1536, direct / permuted: 43 / 52 us at 16 pairs, 64 / 67 at 32,
-      // 112 / 95 at 64; 128 of 2048 x 768: 40 / 50 at 64.  (The last condition: the scratch bound of
+      // the permutation makes an expert's matrices be read once for all of its rows.  64 experts of
+      // 4096 x 1536, direct / permuted: 20.5 / 25.0 us at 4 pairs, 41.9 / 46.5 at 16, 64.8 / 64.4 at 32;
+      // 128 of 2048 x 768: 17.3 / 21.1 at 8, 42.3 / 45.5 at 64.  (The last condition: the scratch bound of
       // awq_b200_moe_workspace_bytes covers one 8-row block per pair only while the pairs are few
       // compared with the experts.)
       const bool direct = block == 8 && pairs <= int_arg(a[11]) && 2 * pairs <= ng &&

@@ -1,12 +1,12 @@
 // AWQ fused-MoE layer: router, token -> expert permutation, grouped expert GEMMs.
 //
-//   topk_softmax_kernel   one warp per token: softmax over E logits, k rounds of warp arg-max
+//   topk_softmax_kernel   one warp per token: softmax over E logits, k rounds of two warp reductions
 //                         (ties -> lower expert id), optional renormalisation.
 //   moe_align_kernel      stable counting sort of the T*k (token, slot) pairs by expert with
-//                         every expert's run padded to the GEMM row block; one CTA per 256 pairs,
-//                         each CTA rebuilds the (cheap) histograms itself so a single launch
-//                         suffices; ranks come from warp match masks, in ascending flat index,
-//                         hence a deterministic order.
+//                         every expert's run padded to the GEMM row block, in a single launch; one CTA
+//                         per 256 pairs.  The histogram of all pairs is built by every CTA alone, of more
+//                         than 2048 pairs by clusters of eight; ranks come from warp match masks, in
+//                         ascending flat index, hence a deterministic order.
 //   moe_gemm1_kernel      per (row block, 128 gate + 128 up columns): x rows gathered through the
 //                         permutation, expert weights streamed (stream_core.cuh), epilogue
 //                         silu(gate) * up -> fp16 activation in permuted row order.
@@ -720,7 +720,10 @@ int launch_moe_align(const int32_t* topk_ids, int numel, int E, int block,
 // the shapes fit them.  They win from about 17 rows (128 experts of 2048 x 768, top-8: 128 against 146 us at
 // 20 rows, 135 against 204 at 35; 64 of 4096 x 1536, top-4: 222 against 319 at 32), but round (q - z) * s to
 // fp16, which the kernels of smaller blocks do not (error of the layer against 64 bits 5.0e-4 and 3.6e-4):
-// fewer rows stay with those.  8 up to eight rows per expert on average; else 16.
+// fewer rows stay with those.  8 up to eight rows per expert on average, else 16.  Blocks of 8 / 16, us, at 5, 6,
+// 7 and 8 rows: groups of 64, 128 experts 113 / 138, 118 / 138, 120 / 138, 132 / 138; 64 experts 193 / 244, 202 /
+// 245, 212 / 245, 239 / 248.  Groups of 128 (gemm_ts) cross at six: 83 / 89, 83 / 89, 94 / 89, 102 / 90; 134 /
+// 143, 145 / 143, 163 / 143, 180 / 144.  One limit for all groups, which callers of the C ABI see.
 int moe_block_size(int T, int topk, int E, int H, int I, int group) {
   const long long pairs = (long long)T * topk;
   if (pairs >= 36LL * E && moe_tc_supported(H, I, group)) return 128;
@@ -880,7 +883,7 @@ int launch_moe_experts_static(const MoeArgs& a, cudaStream_t stream) {
     }
     scratch = scratch_addr[dev];
   }
-  // The array still holds whatever the previous call left there.  Every row the kernels read is
+  // The array still holds whatever the previous call left there.  What the kernels use of it is
   // written earlier in the same call; the one region that must start at zero (per-pair outputs
   // under expert parallelism) is cleared inside launch_moe_experts.
   return launch_moe_experts(a, scratch, kMoeStaticScratchBytes, stream);

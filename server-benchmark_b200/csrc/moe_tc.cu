@@ -247,7 +247,8 @@ int launch_moe_experts_tc(const MoeArgs& a, void* workspace, size_t workspace_by
   }
   if (launch_pdl(moe_gather_kernel, dim3((unsigned)((rows + kGatherRows - 1) / kGatherRows + 1)),
                  dim3(kGatherThreads), 0, stream, a.x, a.sorted_ids, a.expert_ids, a.num_post_pad,
-                 a.topk_weights, x_perm, inverse, row_weights, tiles, n_tiles, a.sorted_capacity, numel, a.topk, a.H, a.block, max_rows) != cudaSuccess) {
+                 a.topk_weights, x_perm, inverse, row_weights, tiles, n_tiles, a.sorted_capacity, numel,
+                 a.topk, a.H, a.block, max_rows) != cudaSuccess) {
     cudaGetLastError();
     return AWQ_B200_ERR_LAUNCH;
   }
