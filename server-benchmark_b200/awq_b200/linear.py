@@ -10,8 +10,8 @@ kernel family serves every token count (the reference switches to dequantize + m
 tokens, awq.py:276-281).  ``AWQConfig(repack_decode=True)`` and ``decode_kmajor=True`` keep further
 copies of ``qweight`` in other layouts (ops.awq_repack, ops.awq_repack_kmajor) for callers that pass
 them to ``ops.awq_gemm`` themselves; ``apply`` reads the checkpoint layout, whose decode kernel is the
-faster one (K 8192 x N 59136: 45 us at 4 tokens against 51 on the decode-layout copy, 50 us at 16
-tokens against 64 on the K-major copy).
+faster one (K 8192 x N 59136: 47 us at 4 tokens against 53 on the decode-layout copy, 53 us at 16
+tokens against 65 on the K-major copy).
 """
 from __future__ import annotations
 

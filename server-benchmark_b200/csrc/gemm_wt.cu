@@ -47,10 +47,11 @@
 // All mbarrier and flag waits are bounded (tc_ptx.cuh).
 //
 // Measured (B200, K x N, against one CTA per tile with two A stages and 64 / 128 fixed tokens):
-//   8192 x 59136   M 100: 123.6 -> 99.8 us   M 1000: 888 -> 853 us   M 4096: 3542 -> 3209 us (the last
-//   two against weights dequantised into shared memory; 1.24 PFLOP/s, where the 1 kW limit holds the
-//   clock near 1.4 GHz); 29568 x 8192   M 100: 70 -> 58 us; router + experts, 128 experts of
-//   2048 x 768, top-8, 2500 tokens: 510 -> 305 us.
+//   8192 x 59136   M 100: 123.6 -> 99.8 us; 29568 x 8192   M 100: 70 -> 58 us; the four linears of a layer
+//   (8192 x 10240, 8192 x 8192, 8192 x 59136, 29568 x 8192) against weights dequantised into shared memory:
+//   M 1000 1694 -> 1482 us, M 4096 6522 -> 5885 (1.22 PFLOP/s in a long loop, where the 1 kW limit holds the
+//   clock near 1.3 GHz; 1.41 on 8192 x 59136 alone); router + experts, 128 experts of 2048 x 768, top-8, 2500
+//   tokens: 507 -> 298 us.
 // What bounds it: at M >= 256 the tensor pipe under the power limit; below, the conversion, without a full
 // pipe (ncu at M = 64: issue 56 %, ALU 41, FMA 24, tensor 34).  add / mul / fma.f16x2 take two cycles a warp
 // and scheduler here, so subtract and scale of 128 weights per lane are 262 of the ~600 cycles a stage takes,
