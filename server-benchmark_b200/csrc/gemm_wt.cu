@@ -51,7 +51,7 @@
 //   (8192 x 10240, 8192 x 8192, 8192 x 59136, 29568 x 8192) against weights dequantised into shared memory:
 //   M 1000 1694 -> 1482 us, M 4096 6522 -> 5885 (1.22 PFLOP/s in a long loop, where the 1 kW limit holds the
 //   clock near 1.3 GHz; 1.41 on 8192 x 59136 alone); router + experts, 128 experts of 2048 x 768, top-8, 2500
-//   tokens: 507 -> 298 us.
+//   tokens: 507 -> 296 us.
 // What bounds it: at M >= 256 the tensor pipe under the power limit; below, the conversion, without a full
 // pipe (ncu at M = 64: issue 56 %, ALU 41, FMA 24, tensor 34).  add / mul / fma.f16x2 take two cycles a warp
 // and scheduler here, so subtract and scale of 128 weights per lane are 262 of the ~600 cycles a stage takes,
@@ -202,14 +202,13 @@ __device__ __forceinline__ void wt_epilogue(const WtParams& p, const Work& work,
     const WtTile t = wt_tile<MODE, GROUP>(p, work.tile_id(seg));
     const int buf = seg & (p.nbuf - 1);
     const bool handover = MODE == 0 && work.k_end(seg) < p.KT;  // another pair holds the tile's last stage
-    // MODE 2: routed weights of tokens 8 k + 2 t4, + 1 of a chunk of 32, fetched a chunk ahead
-    float2 rw_next[4];
-    auto fetch_weights = [&](int c0) {
+    // MODE 2: lane l has the routed weights of tokens 32 i + l of the tile, all fetched ahead of the MMAs' end
+    // (the next 32 fetched under each chunk: 2500 tokens 305 us instead of 296)
+    float rw[MODE == 2 ? 8 : 1];
+    if (MODE == 2) {
 #pragma unroll
-      for (int k = 0; k < 4; ++k)
-        rw_next[k] = __ldcg(reinterpret_cast<const float2*>(p.row_weights + t.m0 + c0 + 8 * k + 2 * t4));
-    };
-    if (MODE == 2) fetch_weights(0);
+      for (int i = 0; i < 8; ++i) rw[i] = 32 * i < t.n ? __ldcg(p.row_weights + t.m0 + 32 * i + lane) : 0.f;
+    }
     // CTAs whose partial tiles are added: blockIdx.x - 2 gather .. blockIdx.x - 2
     const int gather = MODE == 0 ? work.helpers(seg) : 0;
     if (ok) ok = mbar_wait(d_full0 + 8 * buf, (uint32_t)(p.nbuf == 2 ? seg >> 1 : seg) & 1u, abort_flag,
@@ -334,12 +333,17 @@ __device__ __forceinline__ void wt_epilogue(const WtParams& p, const Work& work,
         }
       }
       if (MODE == 2) {
-        float2 rw[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) rw[k] = rw_next[k];
-        if (c0 + 32 < t.n) fetch_weights(c0 + 32);
+        for (int i = 0; i < 8; ++i) {  // token 8 (i / 2) + 2 t4 + i % 2 of the chunk
+          const float w = __shfl_sync(0xffffffffu, rw[0], 8 * (i >> 1) + 2 * t4 + (i & 1));
+          const int at = 4 * (i >> 1) + (i & 1);
+          d[0][at] *= w;
+          d[0][at + 2] *= w;
+          d[1][at] *= w;
+          d[1][at + 2] *= w;
+        }
 #pragma unroll
-        for (int i = 0; i < 32; ++i) d[i >> 4][i & 15] *= (i & 1) ? rw[(i & 15) >> 2].y : rw[(i & 15) >> 2].x;
+        for (int i = 0; i < 7; ++i) rw[i] = rw[i + 1];
       }
       wt_store<4>(d, dst + (size_t)c0 * pitch, pitch, ok ? rows - c0 : 0);
     }
