@@ -462,14 +462,11 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     const int q = warp & 3, team = warp >> 2;
     {
       const uint32_t lane_q = (uint32_t)(q * 32) << 16;
-      // ldmatrix: matrix m = lane / 8 of the four holds, of two 16-row steps (m / 2), the rows
-      // 4 t + {0, 1} (m even) or 4 t + {2, 3} (m odd) -- after the transposed load thread (g, t) has
-      // rows 4 t .. 4 t + 3 of halfword column g in two registers.  Rows of 128 B, 16-byte chunk c at
-      // position c ^ (row % 8).
-      const int mrow = lane & 7, m = lane >> 3;
-      const int krow = 16 * (m >> 1) + 4 * (mrow >> 1) + (mrow & 1) + 2 * (m & 1);
-      const uint32_t off0 = (uint32_t)(krow * 128 + ((q ^ (krow & 7)) << 4));
-      const uint32_t off1 = (uint32_t)(krow * 128 + (((q + 4) ^ (krow & 7)) << 4));
+      // ldmatrix: matrix m = lane / 8 of the four holds rows 8 m .. 8 m + 7 of 32; after the transposed load
+      // thread (g, t) has rows 2 t and 2 t + 1 of halfword column g in a register of each.  Rows of 128 B,
+      // 16-byte chunk c at position c ^ (row % 8).
+      const uint32_t off0 = (uint32_t)(lane * 128 + ((q ^ (lane & 7)) << 4));
+      const uint32_t off1 = (uint32_t)(lane * 128 + (((q + 4) ^ (lane & 7)) << 4));
       bool ok = true;
       int s = team;
       uint32_t phase = 0;
@@ -497,19 +494,17 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             // Logic and shifts take two cycles a warp and scheduler: 320 of them a unit are what
             // bounds the kernel beside HBM.  (The shift as a multiplication on the FMA pipe, which is
             // idle here, measured 7 % slower: mul.hi takes four cycles.)
-            uint32_t frag[2][16];  // [lane half of the quarter][4 * step + (i odd, k pair)]
+            uint32_t frag[2][16];  // [lane half of the quarter][2 * eight rows + i odd]
 #pragma unroll
-            for (int e = 0; e < 4; ++e)
+            for (int c = 0; c < 8; ++c) {
+              const uint32_t r = w[2 * h + (c >> 2)][c & 3], rh = r >> 8;
 #pragma unroll
-              for (int kp = 0; kp < 2; ++kp) {
-                const uint32_t r = w[2 * h + (e >> 1)][2 * (e & 1) + kp], rh = r >> 8;
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-                  frag[i >> 1][4 * e + 2 * (i & 1) + kp] =
-                      ((i & 2) ? rh : r) & ((i & 1) ? 0x00F000F0u : 0x000F000Fu);
-              }
-            tmem_st_16x256b_x4(a_slot + t * 64 + h * 32, frag[0]);
-            tmem_st_16x256b_x4(a_slot + (16u << 16) + t * 64 + h * 32, frag[1]);
+              for (int i = 0; i < 4; ++i)
+                frag[i >> 1][2 * c + (i & 1)] =
+                    ((i & 2) ? rh : r) & ((i & 1) ? 0x00F000F0u : 0x000F000Fu);
+            }
+            tmem_st_16x128b(a_slot + t * 64 + h * 32, frag[0]);
+            tmem_st_16x128b(a_slot + (16u << 16) + t * 64 + h * 32, frag[1]);
           }
         }
         if (!ok) break;

@@ -52,12 +52,15 @@
 //   M 1000 1694 -> 1482 us, M 4096 6522 -> 5885 (1.22 PFLOP/s in a long loop, where the 1 kW limit holds the
 //   clock near 1.3 GHz; 1.41 on 8192 x 59136 alone); router + experts, 128 experts of 2048 x 768, top-8, 2500
 //   tokens: 507 -> 296 us.
-// What bounds it: at M >= 256 the tensor pipe under the power limit; below, the conversion, without a full
-// pipe (ncu at M = 64: issue 56 %, ALU 41, FMA 24, tensor 34).  add / mul / fma.f16x2 take two cycles a warp
-// and scheduler here, so subtract and scale of 128 weights per lane are 262 of the ~600 cycles a stage takes,
-// and without them 8192 x 59136 at M = 24 falls from 83 to 50 us; that fits the chain of each of the four
-// conversion warps of a scheduler (words, arithmetic, A slot, tcgen05.wait::st) as well as the pipe.  Units
-// of twice the K, more load warps and fewer shared-memory or TMEM accesses changed nothing.
+// What bounds it: at M >= 256 the tensor pipe under the power limit; below, the conversion and, on the long layers,
+// the power limit.  A unit takes ~600 cycles at M = 24 and at M = 100.  The arithmetic is 270 of them (sub and mul
+// of f16x2 take two cycles a warp and scheduler; a loop of the conversion alone runs at 300), but a conversion warp
+// spends 2400 cycles on one of its own: half of that it waits for an instruction, a slot to issue, a branch or the
+// store port.  What helps is less of each: fragments of 32 rows at a time, one index for zero points and scales, so
+// that no register spills into the loop, and stores of the cheaper shape took
+// 8192 x 59136 from 87.8 to 84.5 us at M = 24 and 122.4 to 118.5 at M = 100, 8192 x 7680 at M = 24 from 17.9 to 17.3.
+// Units of twice the K, more load warps, a shorter loop (two halves in turn: 10 % slower) and longer suspended waits
+// changed nothing or lost.
 #include "common.cuh"
 #include "handover.cuh"
 #include "tc_ptx.cuh"
@@ -557,18 +560,15 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     const int g = lane >> 2;
     const int q = warp & 3, team = warp >> 2;
     const uint32_t lane_q = (uint32_t)(q * 32) << 16;
-    // ldmatrix: matrix m = lane / 8 of the four holds, of two 16-row steps (m / 2), the rows
-    // 4 t + {0, 1} (m even) or 4 t + {2, 3} (m odd) -- after the transposed load thread (g, t) has
-    // rows 4 t .. 4 t + 3 of halfword column g in two registers.
-    const int mrow = lane & 7, m = lane >> 3;
-    const int krow = 16 * (m >> 1) + 4 * (mrow >> 1) + (mrow & 1) + 2 * (m & 1);
+    // ldmatrix: matrix m = lane / 8 of the four holds rows 8 m .. 8 m + 7 of 32; after the transposed load
+    // thread (g, t) has rows 2 t and 2 t + 1 of halfword column g in a register of each.
     const uint32_t ld_off =
         MODE == 1
             // two boxes of [128 rows x 32 B], 32-byte swizzle
-            ? (uint32_t)((q >> 1) * (kWtRawBytes / 2) + krow * 32 + (((q & 1) ^ ((krow >> 2) & 1)) << 4))
+            ? (uint32_t)((q >> 1) * (kWtRawBytes / 2) + lane * 32 + (((q & 1) ^ ((lane >> 2) & 1)) << 4))
             // one box of [128 rows x 64 B], 64-byte swizzle
-            : (uint32_t)(krow * 64 + ((q ^ ((krow >> 1) & 3)) << 4));
-    constexpr uint32_t kPairBytes = 32 * (MODE == 1 ? 32 : 64);  // two steps further on
+            : (uint32_t)(lane * 64 + ((q ^ ((lane >> 1) & 3)) << 4));
+    constexpr uint32_t kPairBytes = 32 * (MODE == 1 ? 32 : 64);  // 32 rows further on
     const uint32_t half_sel = (g & 1) ? 0x3232u : 0x1010u;      // this lane's halfword, duplicated
     constexpr int kGroups = kWtBK / GROUP;                        // quantisation groups of a stage
     const uint32_t full_leader = map_rank(unit_full(0), 0);
@@ -584,14 +584,13 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       }
     };
     settle();
-    const uint32_t* zp = nullptr;
-    const uint4* sp = nullptr;
-    int zp_seg = -1;
+    uint32_t zs = 0;  // index of this lane's zero word and eight scales in the segment's first group
+    int zs_seg = -1;
     uint32_t zw_n[kGroups];
     uint4 sv_n[kGroups];
     auto fetch = [&]() {
-      if (seg != zp_seg) {
-        zp_seg = seg;
+      if (seg != zs_seg) {
+        zs_seg = seg;
         const WtTile t = wt_tile<MODE, GROUP>(p, work.tile_id(seg));
         int w;
         if (MODE == 1)
@@ -599,14 +598,13 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         else
           w = t.slab * (kWtBN / kPack) + rank * (kWtCols / kPack) + 4 * q + (g >> 1);
         w = min(w, words - 1);  // columns past the edge: any value, nothing of them is stored
-        zp = p.qzeros + (size_t)t.grp0 * words + w;
-        sp = reinterpret_cast<const uint4*>(p.scales) + (size_t)t.grp0 * words + w;
+        zs = (uint32_t)t.grp0 * words + w;
       }
 #pragma unroll
       for (int i = 0; i < kGroups; ++i) {
-        const size_t row = (size_t)(k * kGroups + i) * words;
-        zw_n[i] = __ldg(zp + row);
-        sv_n[i] = __ldg(sp + row);
+        const uint32_t at = zs + (uint32_t)(k * kGroups + i) * words;
+        zw_n[i] = __ldg(p.qzeros + at);
+        sv_n[i] = __ldg(reinterpret_cast<const uint4*>(p.scales) + at);
       }
     };
     if (team < work.count) fetch();
@@ -638,9 +636,9 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       // keep the nibble in place (1024 + 16 q): their zero is 1024 + 16 z, their scale s / 16.
       __half2 z[4], sc[4];
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {  // four 16-row steps each
-        if (h * 64 % GROUP == 0) {
-          const int gi = h * 64 / GROUP;
+      for (int h = 0; h < 4; ++h) {  // 32 rows each
+        if (h * 32 % GROUP == 0) {
+          const int gi = h * 32 / GROUP;
           const uint32_t zz = prmt(zw[gi], zw[gi], half_sel), zh = zz >> 8;
           z[0] = as_half2(lop3_and_or(zz, 0x000F000Fu, 0x64006400u));
           z[1] = as_half2(lop3_and_or(zz, 0x00F000F0u, 0x64006400u));
@@ -652,20 +650,18 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
           sc[2] = as_half2(prmt(sv[gi].z, sv[gi].z, half_sel));
           sc[3] = __hmul2(as_half2(prmt(sv[gi].w, sv[gi].w, half_sel)), r16);
         }
-        uint32_t frag[2][16];  // [lane half of the quarter][4 * step + (i odd, k pair)]
+        uint32_t frag[2][8];  // [lane half of the quarter][2 * eight rows + i odd]
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
+        for (int c = 0; c < 4; ++c) {
+          const uint32_t r = w[h][c], rh = r >> 8;
 #pragma unroll
-          for (int kp = 0; kp < 2; ++kp) {
-            const uint32_t r = w[2 * h + (e >> 1)][2 * (e & 1) + kp], rh = r >> 8;
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-              frag[i >> 1][4 * e + 2 * (i & 1) + kp] = as_u32(__hmul2(
-                  __hsub2(as_half2(lop3_and_or((i & 2) ? rh : r, (i & 1) ? 0x00F000F0u : 0x000F000Fu,
-                                               0x64006400u)),
-                          z[i]),
-                  sc[i]));
-          }
+          for (int i = 0; i < 4; ++i)
+            frag[i >> 1][2 * c + (i & 1)] = as_u32(__hmul2(
+                __hsub2(as_half2(lop3_and_or((i & 2) ? rh : r, (i & 1) ? 0x00F000F0u : 0x000F000Fu,
+                                             0x64006400u)),
+                        z[i]),
+                sc[i]));
+        }
         if (h == 0) {
           // the MMAs that read this A slot last must be complete
           if (u >= p.slots)
@@ -674,8 +670,8 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
           tc_fence_after();
         }
         if (!ok) break;
-        tmem_st_16x256b_x4(a_slot + h * 32, frag[0]);
-        tmem_st_16x256b_x4(a_slot + (16u << 16) + h * 32, frag[1]);
+        tmem_st_16x128b(a_slot + h * 16, frag[0]);
+        tmem_st_16x128b(a_slot + (16u << 16) + h * 16, frag[1]);
       }
       if (!ok) break;
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
