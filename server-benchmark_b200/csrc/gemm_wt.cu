@@ -40,6 +40,9 @@
 //   MODE 2  down: epilogue y[pos, c] = routed weight * D, in permuted order, so that a row is rounded once
 //           and what is rounded is the weighted row: D alone may lie outside the range of fp16.
 //
+// WIDE is the kernel of tiles with one accumulator, more than 128 tokens, that no pair shares: its epilogue goes
+// through shared memory (wt_epilogue_wide).
+//
 // TMEM columns: accumulators first (two of 64 or 128 tokens, one of 256), then A[slots][8 steps][8]: four
 // slots, six up to 64 tokens.  With as many slots as teams a team waits for the MMAs of its own last
 // unit; the two more take that wait out of its loop.
@@ -107,6 +110,7 @@ struct WtParams {
   int nbuf, dcols;             // accumulators in TMEM and the columns of one
   int slots, acol;             // A slots behind them (64 columns each) and the first one's column
   int xstage;                  // bytes of an x stage
+  int stage_bytes;             // WIDE: of a tile's way out through shared memory
   float* partial;              // [CTA][4][nt][32] partial tiles handed over
   handover::Flags flags;       // of the hand-over
   // grouped modes
@@ -151,10 +155,10 @@ __device__ __forceinline__ WtTile wt_tile(const WtParams& p, int id) {
   return t;
 }
 
-template <int MODE>
+template <int MODE, bool WIDE>
 __device__ __forceinline__ Work wt_work(const WtParams& p) {
   const int tiles = MODE == 0 ? p.slabs * p.mtiles : __ldcg(p.n_tiles) * p.slabs;
-  return Work(blockIdx.x >> 1, gridDim.x >> 1, tiles, p.KT, MODE == 0 ? p.chunk : 0);
+  return Work(blockIdx.x >> 1, gridDim.x >> 1, tiles, p.KT, MODE == 0 && !WIDE ? p.chunk : 0);
 }
 
 __device__ __forceinline__ float4 lds_float4(uint32_t addr) {
@@ -169,21 +173,184 @@ __device__ __forceinline__ void named_barrier(int off = 0) {
   asm volatile("bar.sync %0, %1;" ::"r"(ID + off), "n"(COUNT) : "memory");
 }
 
-// Stores 8 K8 tokens of a quarter's 32 columns: v[h][4 k + 2 e + j] is token 8 k + 2 t + j of the column in
-// TMEM lane 16 h + 8 e + g.  The four 8 x 8 matrices of eight tokens, transposed, leave thread (g, t)
-// columns 8 t .. 8 t + 7 of token g: one 16-byte store.  (Columns on lanes, neighbours paired by
-// shuffles and stored four bytes at a time, took twice the instructions: 1024 x 59136 at M 1024 144 ->
-// 132 us, router + experts of 128 x 2048 x 768, top-8, at 1000 tokens 171 -> 149.)
+// Rounds eight tokens of a quarter's 32 columns, k-th of the chunk: v[h][4 k + 2 e + j] is token 8 k + 2 t + j of the
+// column in TMEM lane 16 h + 8 e + g.  The four 8 x 8 matrices, transposed, leave thread (g, t) columns 8 t ..
+// 8 t + 7 of token g: one 16-byte store.  (Columns on lanes, neighbours paired by shuffles and stored four bytes
+// at a time, took twice the instructions: 1024 x 59136 at M 1024 144 -> 132 us, router + experts of 128 x 2048 x
+// 768, top-8, at 1000 tokens 171 -> 149.)
+template <int LEN>
+__device__ __forceinline__ uint4 wt_round(const float (&v)[2][LEN], int k) {
+  uint4 w;
+  w.x = movmatrix_trans(as_u32(__floats2half2_rn(v[0][4 * k], v[0][4 * k + 1])));
+  w.y = movmatrix_trans(as_u32(__floats2half2_rn(v[0][4 * k + 2], v[0][4 * k + 3])));
+  w.z = movmatrix_trans(as_u32(__floats2half2_rn(v[1][4 * k], v[1][4 * k + 1])));
+  w.w = movmatrix_trans(as_u32(__floats2half2_rn(v[1][4 * k + 2], v[1][4 * k + 3])));
+  return w;
+}
 template <int K8, int LEN>
 __device__ __forceinline__ void wt_store(const float (&v)[2][LEN], __half* dst, size_t pitch, int rows) {
 #pragma unroll
   for (int k = 0; k < K8; ++k) {
-    uint4 w;
-    w.x = movmatrix_trans(as_u32(__floats2half2_rn(v[0][4 * k], v[0][4 * k + 1])));
-    w.y = movmatrix_trans(as_u32(__floats2half2_rn(v[0][4 * k + 2], v[0][4 * k + 3])));
-    w.z = movmatrix_trans(as_u32(__floats2half2_rn(v[1][4 * k], v[1][4 * k + 1])));
-    w.w = movmatrix_trans(as_u32(__floats2half2_rn(v[1][4 * k + 2], v[1][4 * k + 3])));
+    const uint4 w = wt_round(v, k);
     if (8 * k < rows) *reinterpret_cast<uint4*>(dst + (size_t)(8 * k) * pitch) = w;
+  }
+}
+// Chunk of 32 tokens of a quarter of the accumulator.
+__device__ __forceinline__ void wt_load_chunk(uint32_t dcol, float (&d)[2][16]) {
+  tmem_ld_16x256b_x4(dcol, d[0]);
+  tmem_ld_16x256b_x4(dcol + (16u << 16), d[1]);
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+// Where an epilogue warp's part of a tile goes: this lane stores rows 0, 8, .. below `rows`.
+template <int MODE>
+struct WtOut {
+  __half* dst;
+  size_t pitch;
+  int rows;
+  bool inside;  // columns the output has
+  // columns: dense / down 32 q of the CTA's 128; gate_up 32 (q % 2) of its 64
+  __device__ __forceinline__ static int first_column(const WtTile& t, int rank, int q) {
+    return MODE == 1 ? t.slab * 128 + rank * 64 + 32 * (q & 1) : t.slab * kWtBN + rank * kWtCols + 32 * q;
+  }
+  __device__ __forceinline__ WtOut(const WtParams& p, const WtTile& t, int rank, int q, int lane) {
+    const int c = first_column(t, rank, q), width = MODE == 1 ? p.half_cols : p.N, g = lane >> 2;
+    inside = c < width;
+    rows = inside ? t.rows - g : 0;
+    pitch = (size_t)width;
+    dst = p.out + (size_t)(t.m0 + g) * width + c + 8 * (lane & 3);
+  }
+};
+// MODE 0: the columns in TMEM lanes 8 i + g of a quarter.
+__device__ __forceinline__ void wt_load_bias(const WtParams& p, int first_column, int g, float (&bias)[4]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    bias[i] = p.bias != nullptr && first_column < p.N
+                  ? __half2float(__ldg(p.bias + first_column + 8 * (g >> 1) + 2 * i + (g & 1)))
+                  : 0.f;
+}
+__device__ __forceinline__ void wt_add_bias(float (&d)[2][16], const float (&bias)[4]) {
+#pragma unroll
+  for (int i = 0; i < 32; ++i) d[i >> 4][i & 15] += bias[2 * (i >> 4) + ((i >> 1) & 1)];
+}
+// MODE 1: the gate warps (q 0, 1) finish the first 16 tokens of the chunk, the up warps (q 2, 3) the other 16; each
+// hands its partner through `box` the half it does not finish.
+__device__ __forceinline__ void wt_glu(const float (&d)[2][16], int q, int lane, float* box, float (&o)[2][8]) {
+  const bool up = q >= 2;
+  float4* give = reinterpret_cast<float4*>(box + (up ? 0 : kWtExFloats / 2) + lane * 20);
+  const float4* take = reinterpret_cast<const float4*>(box + (up ? kWtExFloats / 2 : 0) + lane * 20);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float* lo = &d[i >> 1][4 * (i & 1)];
+    give[i] = make_float4(up ? lo[0] : lo[8], up ? lo[1] : lo[9], up ? lo[2] : lo[10], up ? lo[3] : lo[11]);
+  }
+  named_barrier<2, 64>(q & 1);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float4 v = take[i];
+    const float got[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int at = 4 * (i & 1) + j;
+      const float mine = up ? d[i >> 1][8 + at] : d[i >> 1][at];
+      const float gt = up ? got[j] : mine, uv = up ? mine : got[j];
+      o[i >> 1][at] = __fdividef(gt, 1.f + __expf(-gt)) * uv;
+    }
+  }
+}
+// MODE 2: lane l has the routed weight of token l of the chunk.
+__device__ __forceinline__ void wt_weigh(float (&d)[2][16], float weight, int t4) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {  // token 8 (i / 2) + 2 t4 + i % 2
+    const float w = __shfl_sync(0xffffffffu, weight, 8 * (i >> 1) + 2 * t4 + (i & 1));
+    const int at = 4 * (i >> 1) + (i & 1);
+    d[0][at] *= w;
+    d[0][at + 2] *= w;
+    d[1][at] *= w;
+    d[1][at + 2] *= w;
+  }
+}
+__device__ __forceinline__ void sts_uint4(uint32_t addr, const uint4& v) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
+               : "memory");
+}
+__device__ __forceinline__ uint4 lds_uint4(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "r"(addr));
+  return v;
+}
+
+// Epilogue warp q of the WIDE kernel (one accumulator, whole tiles).  The next tile's MMAs wait for the accumulator,
+// so the warp first takes all of it, rounded, into shared memory and stores from there under those MMAs; a lane
+// reads back what it wrote.  What made this wait long were the stores: all CTAs finish their tiles at about the same
+// time, and 64 KB a CTA leave at 13 to 21 bytes a cycle and SM (256 tokens: 4900 cycles, 1900 without them).
+// 768 x 2048 at M 20480 77.0 -> 64.9 us, 8192 x 8192 at M 4096 454 -> 442, 8192 x 59136 at M 1000 807 -> 776; router +
+// experts of 128 x 2048 x 768, top-8, 2500 tokens 295 -> 282.  Through TMA stores, a proxy
+// fence and a store for each chunk, it was slower than without shared memory (82 us for the first); and with the
+// next chunk's load ahead of this one's rounding the kernel spilt registers (router + experts, 2500 tokens: 274 ->
+// 311 us).
+template <int MODE, int GROUP>
+__device__ __forceinline__ void wt_epilogue_wide(const WtParams& p, const Work& work, uint32_t tmem, int rank, int q,
+                                                 int lane, uint32_t d_full, uint32_t d_empty, float* ex,
+                                                 uint32_t stage, volatile int* abort_flag) {
+  const uint32_t dcol = tmem + ((uint32_t)(q * 32) << 16);
+  const int g = lane >> 2, t4 = lane & 3;
+  constexpr int K8 = MODE == 1 ? 2 : 4;  // eights of tokens that the warp finishes of a chunk
+  d_empty = map_rank(d_empty, 0);
+  stage += lane * 16;
+  pdl_wait();  // orders this thread's writes after the kernel before this one
+  // After a wait that gave up the loop still runs to its end, without waiting and without storing:
+  // every warp then passes the same named barriers.
+  bool ok = true;
+  int flip = 0;
+  for (int seg = 0; seg < work.segs; ++seg) {
+    const WtTile t = wt_tile<MODE, GROUP>(p, work.tile_id(seg));
+    float rw[MODE == 2 ? 8 : 1];  // lane l: routed weights of tokens 32 i + l
+    if (MODE == 2) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) rw[i] = 32 * i < t.n ? __ldcg(p.row_weights + t.m0 + 32 * i + lane) : 0.f;
+    }
+    float bias[4];
+    if (MODE == 0) wt_load_bias(p, WtOut<MODE>::first_column(t, rank, q), g, bias);
+    if (ok) ok = mbar_wait(d_full, (uint32_t)seg & 1u, abort_flag, 38);
+    ok = __all_sync(0xffffffffu, ok);
+    tc_fence_after();
+    uint32_t to = stage;
+    for (int c0 = 0; c0 < t.n; c0 += 32) {
+      float d[2][16];
+      wt_load_chunk(dcol + c0, d);
+      if (c0 + 32 >= t.n) {  // the accumulator is in registers: the next tile may start
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(d_empty);
+      }
+      if constexpr (MODE == 1) {
+        float o[2][8];
+        wt_glu(d, q, lane, ex + ((q & 1) * 2 + flip) * kWtExFloats, o);
+        flip ^= 1;
+#pragma unroll
+        for (int k = 0; k < K8; ++k) sts_uint4(to + k * 512, wt_round(o, k));
+      } else {
+        if (MODE == 0) wt_add_bias(d, bias);
+        if constexpr (MODE == 2) {
+          wt_weigh(d, rw[0], t4);
+#pragma unroll
+          for (int i = 0; i < 7; ++i) rw[i] = rw[i + 1];
+        }
+#pragma unroll
+        for (int k = 0; k < K8; ++k) sts_uint4(to + k * 512, wt_round(d, k));
+      }
+      to += K8 * 512;
+    }
+    const WtOut<MODE> out(p, t, rank, q, lane);
+    const int rows = ok ? out.rows : 0, pieces = (t.n + 31) / 32 * K8;
+#pragma unroll 4
+    for (int i = 0; i < pieces; ++i) {
+      const int m = MODE == 1 ? 32 * (i >> 1) + 16 * (q >> 1) + 8 * (i & 1) : 8 * i;
+      const uint4 v = lds_uint4(stage + i * 512);
+      if (m < rows) *reinterpret_cast<uint4*>(out.dst + (size_t)m * out.pitch) = v;
+    }
   }
 }
 
@@ -194,7 +361,7 @@ __device__ __forceinline__ void wt_epilogue(const WtParams& p, const Work& work,
                                             uint32_t d_empty0, float* ex, uint32_t part_ring,
                                             uint32_t part_full, volatile int* abort_flag) {
   const uint32_t lane_q = (uint32_t)(q * 32) << 16;
-  const int g = lane >> 2, t4 = lane & 3;  // row and column pair of the accumulator fragments
+  const int t4 = lane & 3;
   const uint32_t d_empty_leader = map_rank(d_empty0, 0);
   pdl_wait();  // orders this thread's writes after the kernel before this one
   // After a wait that gave up the loop still runs to its end, without waiting and without storing:
@@ -205,12 +372,12 @@ __device__ __forceinline__ void wt_epilogue(const WtParams& p, const Work& work,
     const WtTile t = wt_tile<MODE, GROUP>(p, work.tile_id(seg));
     const int buf = seg & (p.nbuf - 1);
     const bool handover = MODE == 0 && work.k_end(seg) < p.KT;  // another pair holds the tile's last stage
-    // MODE 2: lane l has the routed weights of tokens 32 i + l of the tile, all fetched ahead of the MMAs' end
-    // (the next 32 fetched under each chunk: 2500 tokens 305 us instead of 296)
-    float rw[MODE == 2 ? 8 : 1];
+    // MODE 2: lane l has the routed weights of tokens 32 i + l of the tile (128 at most), all fetched ahead of the
+    // MMAs' end
+    float rw[MODE == 2 ? 4 : 1];
     if (MODE == 2) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) rw[i] = 32 * i < t.n ? __ldcg(p.row_weights + t.m0 + 32 * i + lane) : 0.f;
+      for (int i = 0; i < 4; ++i) rw[i] = 32 * i < t.n ? __ldcg(p.row_weights + t.m0 + 32 * i + lane) : 0.f;
     }
     // CTAs whose partial tiles are added: blockIdx.x - 2 gather .. blockIdx.x - 2
     const int gather = MODE == 0 ? work.helpers(seg) : 0;
@@ -233,19 +400,10 @@ __device__ __forceinline__ void wt_epilogue(const WtParams& p, const Work& work,
     __syncwarp();  // what a lane acquired holds for the warp's reads of the partial tiles
     tc_fence_after();
     const uint32_t dcol = tmem + lane_q + buf * p.dcols;
-    // columns: dense / down 32 q of the CTA's 128; gate_up 32 (q % 2) of its 64
-    const int c_first = MODE == 1 ? t.slab * 128 + rank * 64 + 32 * (q & 1)
-                                  : t.slab * kWtBN + rank * kWtCols + 32 * q;
-    const int width = MODE == 1 ? p.half_cols : p.N;
-    const int rows = ok && c_first < width ? t.rows - g : 0;  // this lane stores rows 0, 8, .. below
-    __half* dst = p.out + (size_t)(t.m0 + g) * width + c_first + 8 * t4;
-    const size_t pitch = (size_t)width;
-    float bias[4] = {0.f, 0.f, 0.f, 0.f};  // of the columns in TMEM lanes 8 i + g
-    if (MODE == 0 && p.bias != nullptr && c_first < p.N) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-        bias[i] = __half2float(__ldg(p.bias + c_first + 8 * (g >> 1) + 2 * i + (g & 1)));
-    }
+    const WtOut<MODE> out(p, t, rank, q, lane);
+    const int rows = ok ? out.rows : 0;
+    float bias[4];
+    if (MODE == 0) wt_load_bias(p, WtOut<MODE>::first_column(t, rank, q), lane >> 2, bias);
     // Partial tiles handed over come through a ring in the packed words' and tokens' stages, which the
     // pair is done with (the tile it finishes for others is its last), 32 tokens of a CTA at a time: a
     // load that waits for L2 once per 32 tokens and CTA took 3.2 us per CTA at 128 tokens.
@@ -265,44 +423,18 @@ __device__ __forceinline__ void wt_epilogue(const WtParams& p, const Work& work,
     }
     for (int c0 = 0; c0 < t.n; c0 += 32) {
       float d[2][16];
-      tmem_ld_16x256b_x4(dcol + c0, d[0]);
-      tmem_ld_16x256b_x4(dcol + (16u << 16) + c0, d[1]);
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      wt_load_chunk(dcol + c0, d);
       if (c0 + 32 >= t.n) {  // the accumulator is in registers: the next tile may start
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(d_empty_leader + 8 * buf);
       }
       if (MODE == 1) {
-        // gate warps (q 0, 1) finish the first 16 tokens of the chunk, up warps (q 2, 3) the other
-        // 16: each hands its partner the half it does not finish
-        const bool up = q >= 2;
-        float* box = ex + ((q & 1) * 2 + flip) * kWtExFloats;
-        flip ^= 1;
-        float4* give = reinterpret_cast<float4*>(box + (up ? 0 : kWtExFloats / 2) + lane * 20);
-        const float4* take = reinterpret_cast<const float4*>(box + (up ? kWtExFloats / 2 : 0) + lane * 20);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float* lo = &d[i >> 1][4 * (i & 1)];
-          give[i] = make_float4(up ? lo[0] : lo[8], up ? lo[1] : lo[9], up ? lo[2] : lo[10],
-                                up ? lo[3] : lo[11]);
-        }
-        named_barrier<2, 64>(q & 1);
         float o[2][8];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float4 v = take[i];
-          const float got[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int at = 4 * (i & 1) + j;
-            const float mine = up ? d[i >> 1][8 + at] : d[i >> 1][at];
-            const float gt = up ? got[j] : mine, uv = up ? mine : got[j];
-            o[i >> 1][at] = __fdividef(gt, 1.f + __expf(-gt)) * uv;
-          }
-        }
-        const int m = c0 + (up ? 16 : 0);
-        wt_store<2>(o, dst + (size_t)m * pitch, pitch, rows - m);
+        wt_glu(d, q, lane, ex + ((q & 1) * 2 + flip) * kWtExFloats, o);
+        flip ^= 1;
+        const int m = c0 + 16 * (q >> 1);
+        wt_store<2>(o, out.dst + (size_t)m * out.pitch, out.pitch, rows - m);
         continue;
       }
       if (MODE == 0 && handover) {
@@ -315,8 +447,7 @@ __device__ __forceinline__ void wt_epilogue(const WtParams& p, const Work& work,
         continue;
       }
       if (MODE == 0) {
-#pragma unroll
-        for (int i = 0; i < 32; ++i) d[i >> 4][i & 15] += bias[2 * (i >> 4) + ((i >> 1) & 1)];
+        wt_add_bias(d, bias);
         for (int s = gather; s > 0; --s, ++piece) {
           const int slot = piece & (kWtPartRing - 1);
           if (ok) ok = mbar_wait(part_full + 8 * slot, (uint32_t)(piece / kWtPartRing) & 1u, abort_flag, 40);
@@ -336,19 +467,11 @@ __device__ __forceinline__ void wt_epilogue(const WtParams& p, const Work& work,
         }
       }
       if (MODE == 2) {
+        wt_weigh(d, rw[0], t4);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {  // token 8 (i / 2) + 2 t4 + i % 2 of the chunk
-          const float w = __shfl_sync(0xffffffffu, rw[0], 8 * (i >> 1) + 2 * t4 + (i & 1));
-          const int at = 4 * (i >> 1) + (i & 1);
-          d[0][at] *= w;
-          d[0][at + 2] *= w;
-          d[1][at] *= w;
-          d[1][at + 2] *= w;
-        }
-#pragma unroll
-        for (int i = 0; i < 7; ++i) rw[i] = rw[i + 1];
+        for (int i = 0; i < 3; ++i) rw[i] = rw[i + 1];
       }
-      wt_store<4>(d, dst + (size_t)c0 * pitch, pitch, ok ? rows - c0 : 0);
+      wt_store<4>(d, out.dst + (size_t)c0 * out.pitch, out.pitch, ok ? rows - c0 : 0);
     }
     if (MODE == 0 && handover) {
       fence_proxy_async_all();
@@ -358,7 +481,7 @@ __device__ __forceinline__ void wt_epilogue(const WtParams& p, const Work& work,
   }
 }
 
-template <int MODE, int GROUP>
+template <int MODE, int GROUP, bool WIDE>
 __global__ void __launch_bounds__(kWtThreads, 1)
 gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ WtXMaps<MODE> map_x,
                const WtParams p) {
@@ -390,7 +513,7 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 
   pdl_launch_dependents();
   if (MODE != 0) pdl_wait();  // the tile table comes from the kernel before this one
-  const Work work = wt_work<MODE>(p);
+  const Work work = wt_work<MODE, WIDE>(p);
   const int words = p.N / kPack;
 
   // Packed words, unit by unit: 128 rows x 16 words (MODE 1: 8 gate words and the matching 8 up
@@ -448,7 +571,7 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (MODE == 0 && warp >= kWtEpiWarp0 && warp < kWtEpiWarp0 + kWtEpiWarps && lane < kWtPartRing) {
+  if (MODE == 0 && !WIDE && warp >= kWtEpiWarp0 && warp < kWtEpiWarp0 + kWtEpiWarps && lane < kWtPartRing) {
     mbar_init(part_full(warp - kWtEpiWarp0) + 8 * lane, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -528,7 +651,7 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         const int n = __shfl_sync(0xffffffffu, t.n, 0);
         const uint32_t idesc = (1u << 4) | ((uint32_t)(n >> 3) << 17) | (16u << 24);
         const uint32_t half16 = (uint32_t)((n / 2 + 15) / 16) * (16 * 128 / 16);
-        const int buf = seg & (p.nbuf - 1), use = p.nbuf == 2 ? seg >> 1 : seg;
+        const int buf = WIDE ? 0 : seg & (p.nbuf - 1), use = !WIDE && p.nbuf == 2 ? seg >> 1 : seg;
         const uint32_t dcol = tmem_u + buf * p.dcols;
         const int u_end = u + work.k_end(seg) - work.k_begin(seg);
         // the accumulator's previous tile must have been read by both epilogues
@@ -691,11 +814,16 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     }
   } else {
     // ------------------------------------------------------------------ epilogue
-    wt_epilogue<MODE, GROUP>(p, work, tmem, rank, warp - kWtEpiWarp0, lane, d_full(0), d_empty(0),
-                             reinterpret_cast<float*>(smem_raw + (bar_base + kWtBarBytes -
-                                                                  smem_u32(smem_raw))),
-                             x_base + (warp - kWtEpiWarp0) * (kWtPartRing * kWtPartBytes),
-                             part_full(warp - kWtEpiWarp0), &s_abort);
+    const int e = warp - kWtEpiWarp0;
+    const uint32_t ex_base = bar_base + kWtBarBytes;
+    float* ex = reinterpret_cast<float*>(smem_raw + (ex_base - smem_u32(smem_raw)));
+    if constexpr (WIDE) {
+      const uint32_t stage = ex_base + (MODE == 1 ? kWtExBytes : 0) + e * (p.stage_bytes / kWtEpiWarps);
+      wt_epilogue_wide<MODE, GROUP>(p, work, tmem, rank, e, lane, d_full(0), d_empty(0), ex, stage, &s_abort);
+    } else {
+      wt_epilogue<MODE, GROUP>(p, work, tmem, rank, e, lane, d_full(0), d_empty(0), ex,
+                               x_base + e * (kWtPartRing * kWtPartBytes), part_full(e), &s_abort);
+    }
   }
 
   // ---- teardown ----
@@ -705,7 +833,7 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     // tensor memory.  Let them land before both are given back.
     linger();
     // flags raised meanwhile: a replay of this launch must not find them
-    if (MODE == 0 && warp >= kWtEpiWarp0 && warp < kWtEpiWarp0 + kWtEpiWarps && work.segs > 0)
+    if (MODE == 0 && !WIDE && warp >= kWtEpiWarp0 && warp < kWtEpiWarp0 + kWtEpiWarps && work.segs > 0)
       for (int c = 1 + lane; c <= work.helpers(work.segs - 1); c += 32)
         p.flags.lower(blockIdx.x - 2 * c, warp - kWtEpiWarp0);
   }
@@ -723,24 +851,24 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 // ---- host side -------------------------------------------------------------------------------
 
 // Pairs of CTAs the GPU holds at once (one CTA per SM).
-template <int MODE, int GROUP>
+template <int MODE, int GROUP, bool WIDE>
 int wt_pairs(int smem) {
   static std::atomic<int> cached[64][9];  // zero-initialised: not asked yet
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 1;
-  const int got = resident_clusters(gemm_wt_kernel<MODE, GROUP>, 2, kWtThreads, smem, cached[dev]);
+  const int got = resident_clusters(gemm_wt_kernel<MODE, GROUP, WIDE>, 2, kWtThreads, smem, cached[dev]);
   const int most = sm_count() / 2 < kWtMaxPairs ? sm_count() / 2 : kWtMaxPairs;
   return got < most ? got : most;
 }
 
-template <int MODE, int GROUP>
+template <int MODE, int GROUP, bool WIDE>
 int wt_prepare() {
   static std::atomic<bool> attr_done[64];  // zero-initialised; setting the attribute twice is harmless
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return AWQ_B200_ERR_DEVICE;
   if (!attr_done[dev]) {
-    if (cudaFuncSetAttribute(gemm_wt_kernel<MODE, GROUP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (cudaFuncSetAttribute(gemm_wt_kernel<MODE, GROUP, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              kWtSmemLimit) != cudaSuccess)
       return AWQ_B200_ERR_LAUNCH;
     attr_done[dev] = true;
@@ -753,22 +881,29 @@ int wt_prepare() {
 int wt_rings(WtParams* p, int mode) {
   const int rows = (p->nt / 2 + 15) / 16 * 16;
   p->xstage = rows * 256;
-  const int fixed = 1024 + kWtBarBytes + (mode == 1 ? kWtExBytes : 0);
   p->nx = p->xstage <= (16 << 10) ? 8 : 4;
   // Two accumulators while they fit beside four A slots, so that the next tile's MMAs run under the
   // epilogue; what TMEM is left over goes to A slots.
   p->nbuf = p->nt <= 128 ? 2 : 1;
+  // One accumulator and whole tiles: the WIDE kernel.
+  p->stage_bytes = p->nbuf == 2 || p->chunk > 0 ? 0 : (p->nt + 31) / 32 * 32 * kWtCols * (mode == 1 ? 1 : 2);
+  const int fixed = 1024 + kWtBarBytes + (mode == 1 ? kWtExBytes : 0) + p->stage_bytes;
   p->dcols = p->nt <= 64 ? 64 : 128;
   p->acol = p->nt <= 64 ? 128 : 256;
   p->slots = (kWtTmemCols - p->acol) / 64;
   p->nraw = (kWtSmemLimit - fixed - p->nx * p->xstage) / kWtRawBytes;
   if (p->nraw > kWtMaxRaw) p->nraw = kWtMaxRaw;
+  // A team waits for unit u in the stage that unit u - nraw had.  Either it read that one itself, or it has seen
+  // the MMAs of a later unit complete (u - 4 - slots, when it wrote unit u - 4); between the two, the parity of
+  // the filling before could pass for the one it waits for.
+  if (p->nraw < kWtTeams + p->slots) p->nraw = kWtTeams;
   return fixed + p->nx * p->xstage + p->nraw * kWtRawBytes;
 }
 
-template <int MODE, int GROUP>
+template <int MODE, int GROUP, bool WIDE>
 int launch_wt_kernel(const CUtensorMap& map_w, const WtXMaps<MODE>& map_x, const WtParams& p, int pairs,
                      int smem, cudaStream_t stream) {
+  if (int rc = wt_prepare<MODE, GROUP, WIDE>()) return rc;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * pairs, 1, 1);
   cfg.blockDim = dim3(kWtThreads, 1, 1);
@@ -781,7 +916,7 @@ int launch_wt_kernel(const CUtensorMap& map_w, const WtXMaps<MODE>& map_x, const
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = add_pdl_attribute(attr, 1);
-  if (cudaLaunchKernelEx(&cfg, gemm_wt_kernel<MODE, GROUP>, map_w, map_x, p) != cudaSuccess) {
+  if (cudaLaunchKernelEx(&cfg, gemm_wt_kernel<MODE, GROUP, WIDE>, map_w, map_x, p) != cudaSuccess) {
     cudaGetLastError();
     return AWQ_B200_ERR_LAUNCH;
   }
@@ -899,10 +1034,10 @@ WtPlan wt_plan(int M, int slabs, int KT, int most, bool split) {
 template <int GROUP>
 int launch_wt_dense(const __half* x, const uint32_t* qweight, WtParams p, void* workspace,
                     size_t workspace_bytes, cudaStream_t stream) {
-  if (int rc = wt_prepare<0, GROUP>()) return rc;
+  if (int rc = wt_prepare<0, GROUP, false>()) return rc;
   p.slabs = (p.N + kWtBN - 1) / kWtBN;
   p.KT = p.K / kWtBK;
-  const int most = wt_pairs<0, GROUP>(kWtSmemLimit);
+  const int most = wt_pairs<0, GROUP, false>(kWtSmemLimit);
   WtPlan plan = wt_plan(p.M, p.slabs, p.KT, most, true);
   if (plan.chunk > 0) {
     if (workspace != nullptr && workspace_bytes >= wt_scratch_bytes(plan.nt, plan.pairs)) {
@@ -924,7 +1059,8 @@ int launch_wt_dense(const __half* x, const uint32_t* qweight, WtParams p, void* 
     const int boxes = ((rows[i] + 15) / 16 * 8 + 15) / 16;
     if (int rc = encode_map_x(&map_x.map[i], x, p.M, p.K, boxes * 16)) return rc;
   }
-  return launch_wt_kernel<0, GROUP>(map_w, map_x, p, plan.pairs, smem, stream);
+  return p.stage_bytes > 0 ? launch_wt_kernel<0, GROUP, true>(map_w, map_x, p, plan.pairs, smem, stream)
+                           : launch_wt_kernel<0, GROUP, false>(map_w, map_x, p, plan.pairs, smem, stream);
 }
 
 }  // namespace
@@ -960,7 +1096,7 @@ namespace {
 template <int MODE, int GROUP>
 int launch_wt_moe(const __half* a, int64_t a_rows, const uint32_t* w, int experts, int tile_rows,
                   WtParams p, cudaStream_t stream) {
-  if (int rc = wt_prepare<MODE, GROUP>()) return rc;
+  if (int rc = wt_prepare<MODE, GROUP, false>()) return rc;
   p.KT = p.K / kWtBK;
   p.slabs = MODE == 1 ? p.half_cols / 128 : p.N / kWtBN;
   p.nt = tile_rows;
@@ -970,8 +1106,9 @@ int launch_wt_moe(const __half* a, int64_t a_rows, const uint32_t* w, int expert
   if (int rc = make_wt_map(&map_w, w, (int64_t)experts * p.K, p.N, MODE == 1 ? 8 : 16)) return rc;
   for (int boxes = 1; boxes <= 8; ++boxes)
     if (int rc = encode_map_x(&map_x.map[boxes - 1], a, a_rows, p.K, boxes * 16)) return rc;
-  return launch_wt_kernel<MODE, GROUP>(map_w, map_x, p, wt_pairs<MODE, GROUP>(kWtSmemLimit), smem,
-                                       stream);
+  const int pairs = wt_pairs<MODE, GROUP, false>(kWtSmemLimit);
+  return p.stage_bytes > 0 ? launch_wt_kernel<MODE, GROUP, true>(map_w, map_x, p, pairs, smem, stream)
+                           : launch_wt_kernel<MODE, GROUP, false>(map_w, map_x, p, pairs, smem, stream);
 }
 }  // namespace
 

@@ -153,3 +153,25 @@ def test_wt_collected_tiles(A, m, k, n, group):
     # fp16 weights and output: 2^-11 each, far inside TOL
     assert O.rel_err(y[0].cpu().numpy(), ref) < TOL
     assert O.elementwise_ok(y[0].cpu().numpy(), ref, TOL)
+
+
+# Whole tiles of more than 128 tokens, several per pair, whose epilogue goes through shared memory: every tile size
+# from 144 to 256 (4 to 13 stages of packed words), one to nine units a tile, a last tile of few tokens, a slab past N.
+@pytest.mark.parametrize("m,k,n,group", [
+    (400, 640, 9504, 128), (777, 384, 9504, 64), (500, 128, 9504, 128), (900, 640, 9504, 64), (777, 256, 8224, 128),
+    (430, 1152, 9472, 128), (900, 512, 8224, 64), (1000, 640, 8224, 128),
+])
+def test_wt_wide_tiles(A, m, k, n, group):
+    from awq_b200 import synth
+    qw, s, qz = synth.awq_linear_tensors(k, n, group, seed=m)
+    x = synth.activations(m, k, seed=n)
+    b = torch.randn(n, generator=torch.Generator().manual_seed(k)).half()
+    ref = O.awq_gemm_fp32_torch(x, qw, s, qz, group).numpy() + b.numpy().astype(np.float32)
+    dev = [a.cuda() for a in (x, qw, s, qz)]
+    y = [A.awq_gemm(*dev, 8, bias=b.cuda(), kernel=A.KERNEL_WT) for _ in range(3)]
+    torch.cuda.synchronize()
+    assert device_status() == 0, "a bounded wait ran out"
+    assert torch.equal(y[0], y[1]) and torch.equal(y[0], y[2])
+    # fp16 weights and output: 2^-11 each, far inside TOL
+    assert O.rel_err(y[0].cpu().numpy(), ref) < TOL
+    assert O.elementwise_ok(y[0].cpu().numpy(), ref, TOL)
