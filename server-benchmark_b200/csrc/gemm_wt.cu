@@ -60,8 +60,9 @@
 // of f16x2 take two cycles a warp and scheduler; a loop of the conversion alone runs at 300), but a conversion warp
 // spends 2400 cycles on one of its own: half of that it waits for an instruction, a slot to issue, a branch or the
 // store port.  What helps is less of each: fragments of 32 rows at a time, one index for zero points and scales, so
-// that no register spills into the loop, and stores of the cheaper shape took
-// 8192 x 59136 from 87.8 to 84.5 us at M = 24 and 122.4 to 118.5 at M = 100, 8192 x 7680 at M = 24 from 17.9 to 17.3.
+// that no register spills into the loop, and stores of the cheaper shape took 8192 x 59136 from 87.8 to 84.5 us at
+// M = 24 and 122.4 to 118.5 at M = 100; one wait per unit instead of two, arrivals without a branch and load warps
+// that stay converged to 80.7 and 114.8; router + experts of 128 x 2048 x 768, top-8, 1024 tokens 173 to 163.
 // Units of twice the K, more load warps, a shorter loop (two halves in turn: 10 % slower) and longer suspended waits
 // changed nothing or lost.
 #include "common.cuh"
@@ -520,7 +521,7 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   // words).  State of the raw producer's lane 0.
   int raw_u = 0, raw_seg = 0, raw_k = 0, raw_end = 0, raw_s = 0, raw_w0 = 0, raw_row0 = 0;
   uint32_t raw_phase = 0;
-  auto load_raw = [&]() {
+  auto load_raw = [&]() {  // returns whether the stage after this one is known to be empty
     if (raw_k == raw_end) {
       const WtTile t = wt_tile<MODE, GROUP>(p, work.tile_id(raw_seg));
       raw_k = work.k_begin(raw_seg);
@@ -531,29 +532,31 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     }
     const uint32_t dst = raw_base + raw_s * kWtRawBytes, bar = raw_full(raw_s);
     const int row = raw_row0 + raw_k * kWtBK;
-    mbar_arrive_expect_tx(bar, kWtRawBytes);
-    if (MODE == 1) {
-      tma_load_2d(dst, &map_w, raw_w0, row, bar);
-      tma_load_2d(dst + kWtRawBytes / 2, &map_w, p.half_cols / kPack + raw_w0, row, bar);
-    } else {
-      tma_load_2d(dst, &map_w, raw_w0, row, bar);
-    }
     ++raw_u;
     ++raw_k;
     if (++raw_s == p.nraw) {
       raw_s = 0;
       raw_phase ^= 1u;
     }
+    bool r = false;
+    if (elect_one()) {
+      r = mbar_test(raw_empty(raw_s), raw_phase ^ 1u);
+      mbar_arrive_expect_tx(bar, kWtRawBytes);
+      tma_load_2d(dst, &map_w, raw_w0, row, bar);
+      if (MODE == 1) tma_load_2d(dst + kWtRawBytes / 2, &map_w, p.half_cols / kPack + raw_w0, row, bar);
+    }
+    return __any_sync(0xffffffffu, r);
   };
 
-  if (warp == kWtRawWarp && lane == 0) {
-    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
-    for (int s = 0; s < p.nraw; ++s) {
-      mbar_init(raw_full(s), 1);
-      mbar_init(raw_empty(s), kWtCvWarps / kWtTeams);
+  if (warp == kWtRawWarp) {
+    if (lane == 0) asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
+    if (lane < p.nraw) {
+      mbar_init(raw_full(lane), 1);
+      mbar_init(raw_empty(lane), kWtCvWarps / kWtTeams);
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      fence_proxy_async();
     }
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    fence_proxy_async();
+    __syncwarp();
     // the first packed words are on their way before anyone else is through the prologue; no
     // kernel writes weights, so they need not wait for the kernel before this one
     for (int i = 0; i < kWtTeams && raw_u < work.count; ++i) load_raw();
@@ -591,46 +594,56 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 
   if (warp == kWtRawWarp) {
     // ------------------------------------------------------------------ packed words
-    if (lane == 0) {
-      bool ok = true;
-      while (raw_u < work.count && ok) {
-        // the first trip round the ring finds it empty
-        if (raw_u >= p.nraw) ok = mbar_wait(raw_empty(raw_s), raw_phase ^ 1u, &s_abort, 31);
-        if (ok) load_raw();
+    // Converged, an elected lane issues, and the next stage's barrier is probed ahead of this one's load: a lane
+    // that looped alone and waited for every stage took 444 cycles a unit whatever the rest of the kernel did.
+    // The same for the tokens.
+    bool ok = true, ready = false;
+    while (raw_u < work.count) {
+      if (raw_u >= p.nraw && !ready) {  // the first trip round the ring finds it empty
+        ok = mbar_wait(raw_empty(raw_s), raw_phase ^ 1u, &s_abort, 31);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
       }
+      ready = load_raw();
     }
   } else if (warp == kWtXWarp) {
     // ------------------------------------------------------------------ tokens
-    if (lane == 0) {
-      pdl_wait();  // the activations may be the output of the kernel before this one
-      bool ok = true;
-      int seg = 0, k = 0, k_end = 0, s = 0;
-      const CUtensorMap* map = nullptr;
-      uint32_t bytes = 0;
-      int row = 0;
-      const uint32_t full0 = map_rank(unit_full(0), 0);
-      for (int u = 0; u < work.count && ok; ++u) {
-        if (k == k_end) {
-          const WtTile t = wt_tile<MODE, GROUP>(p, work.tile_id(seg));
-          k = work.k_begin(seg);
-          k_end = work.k_end(seg++);
-          const int boxes = (t.n / 2 + 15) / 16;
-          map = &map_x.map[MODE == 0 ? (t.rows < p.nt ? 1 : 0) : boxes - 1];
-          bytes = (uint32_t)boxes * 16 * 256;
-          row = t.m0 + rank * (t.n / 2);
-        }
-        if (u >= p.nx) ok = mbar_wait(mma_done(u - p.nx), unit_phase(u - p.nx), &s_abort, 32);
+    pdl_wait();  // the activations may be the output of the kernel before this one
+    bool ok = true, ready = false;
+    int seg = 0, k = 0, k_end = 0, s = 0;
+    const CUtensorMap* map = nullptr;
+    uint32_t bytes = 0;
+    int row = 0;
+    const uint32_t full0 = map_rank(unit_full(0), 0);
+    for (int u = 0; u < work.count; ++u) {
+      if (k == k_end) {
+        const WtTile t = wt_tile<MODE, GROUP>(p, work.tile_id(seg));
+        k = work.k_begin(seg);
+        k_end = work.k_end(seg++);
+        const int boxes = (t.n / 2 + 15) / 16;
+        map = &map_x.map[MODE == 0 ? (t.rows < p.nt ? 1 : 0) : boxes - 1];
+        bytes = (uint32_t)boxes * 16 * 256;
+        row = t.m0 + rank * (t.n / 2);
+      }
+      if (u >= p.nx && !ready) {
+        ok = mbar_wait(mma_done(u - p.nx), unit_phase(u - p.nx), &s_abort, 32);
+        ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
+      }
+      bool r = false;
+      if (elect_one()) {
+        r = u + 1 >= p.nx && mbar_test(mma_done(u + 1 - p.nx), unit_phase(u + 1 - p.nx));
         if (rank == 0) mbar_arrive_expect_tx(unit_full(u), 2 * bytes);
         tma_load_3d_pair(x_base + s * p.xstage, map, 0, row, 2 * k, full0 + 8 * (u & (kWtMaxX - 1)));
-        ++k;
-        if (++s == p.nx) s = 0;
       }
-      // The commits of the last units arrive asynchronously and nobody else waits for all of
-      // them: see them land before the CTA may exit.
-      for (int u = work.count > kWtMaxX ? work.count - kWtMaxX : 0; u < work.count && ok; ++u)
-        ok = mbar_wait(mma_done(u), unit_phase(u), &s_abort, 32);
+      ready = __any_sync(0xffffffffu, r);
+      ++k;
+      if (++s == p.nx) s = 0;
     }
+    // The commits of the last units arrive asynchronously and nobody else waits for all of
+    // them: see them land before the CTA may exit.
+    for (int u = work.count > kWtMaxX ? work.count - kWtMaxX : 0; u < work.count && ok; ++u)
+      ok = mbar_wait(mma_done(u), unit_phase(u), &s_abort, 32);
   } else if (warp == kWtIssueWarp) {
     // ------------------------------------------------------------------ MMA issue (leader)
     if (rank == 0) {
@@ -707,30 +720,32 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       }
     };
     settle();
-    uint32_t zs = 0;  // index of this lane's zero word and eight scales in the segment's first group
-    int zs_seg = -1;
+    // index of this lane's zero word and eight scales of the next unit
+    const uint32_t zs_step = (uint32_t)(kWtTeams * kGroups * words);
+    auto locate = [&]() {
+      const WtTile t = wt_tile<MODE, GROUP>(p, work.tile_id(seg));
+      int w;
+      if (MODE == 1)
+        w = (q >> 1) * (p.half_cols / kPack) + t.slab * 16 + rank * 8 + 4 * (q & 1) + (g >> 1);
+      else
+        w = t.slab * (kWtBN / kPack) + rank * (kWtCols / kPack) + 4 * q + (g >> 1);
+      w = min(w, words - 1);  // columns past the edge: any value, nothing of them is stored
+      return (uint32_t)(t.grp0 + k * kGroups) * words + w;
+    };
+    uint32_t zs = 0;
     uint32_t zw_n[kGroups];
     uint4 sv_n[kGroups];
     auto fetch = [&]() {
-      if (seg != zs_seg) {
-        zs_seg = seg;
-        const WtTile t = wt_tile<MODE, GROUP>(p, work.tile_id(seg));
-        int w;
-        if (MODE == 1)
-          w = (q >> 1) * (p.half_cols / kPack) + t.slab * 16 + rank * 8 + 4 * (q & 1) + (g >> 1);
-        else
-          w = t.slab * (kWtBN / kPack) + rank * (kWtCols / kPack) + 4 * q + (g >> 1);
-        w = min(w, words - 1);  // columns past the edge: any value, nothing of them is stored
-        zs = (uint32_t)t.grp0 * words + w;
-      }
 #pragma unroll
       for (int i = 0; i < kGroups; ++i) {
-        const uint32_t at = zs + (uint32_t)(k * kGroups + i) * words;
-        zw_n[i] = __ldg(p.qzeros + at);
-        sv_n[i] = __ldg(reinterpret_cast<const uint4*>(p.scales) + at);
+        zw_n[i] = __ldg(p.qzeros + zs + i * words);
+        sv_n[i] = __ldg(reinterpret_cast<const uint4*>(p.scales) + zs + i * words);
       }
     };
-    if (team < work.count) fetch();
+    if (team < work.count) {
+      zs = locate();
+      fetch();
+    }
 
     bool ok = true;
     int s = team, slot = team;  // nraw, slots >= kWtTeams
@@ -743,13 +758,27 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         zw[i] = zw_n[i];
         sv[i] = sv_n[i];
       }
-      k += kWtTeams;
-      settle();
-      if (u + kWtTeams < work.count) fetch();
+      if (u + kWtTeams < work.count) {
+        k += kWtTeams;
+        zs += zs_step;
+        if (k >= k_end) {
+          settle();
+          zs = locate();
+        }
+        fetch();
+      }
 
-      ok = mbar_wait(raw_full(s), phase, &s_abort, 36);
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
+      // the unit's words, and the MMAs that read its A slot last; probed together, a wait of its own each took
+      // 100 to 150 cycles with nothing to wait for
+      const bool first = u < p.slots;
+      const uint32_t slot_bar = first ? raw_full(s) : mma_done(u - p.slots);
+      const uint32_t slot_phase = first ? phase : unit_phase(u - p.slots);
+      if (!__all_sync(0xffffffffu, mbar_try_wait2(raw_full(s), phase, slot_bar, slot_phase))) {
+        ok = mbar_wait(raw_full(s), phase, &s_abort, 36) && mbar_wait(slot_bar, slot_phase, &s_abort, 37);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+      }
+      tc_fence_after();
       const uint32_t raw = raw_base + s * kWtRawBytes + ld_off;
       uint32_t w[4][4];
 #pragma unroll
@@ -785,25 +814,13 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                         z[i]),
                 sc[i]));
         }
-        if (h == 0) {
-          // the MMAs that read this A slot last must be complete
-          if (u >= p.slots)
-            ok = mbar_wait(mma_done(u - p.slots), unit_phase(u - p.slots), &s_abort, 37);
-          ok = __all_sync(0xffffffffu, ok);
-          tc_fence_after();
-        }
-        if (!ok) break;
         tmem_st_16x128b(a_slot + h * 16, frag[0]);
         tmem_st_16x128b(a_slot + (16u << 16) + h * 16, frag[1]);
       }
-      if (!ok) break;
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) {
-        mbar_arrive_cluster(full_leader + 8 * (u & (kWtMaxX - 1)));
-        mbar_arrive(raw_empty(s));
-      }
+      mbar_arrive_both(full_leader + 8 * (u & (kWtMaxX - 1)), raw_empty(s), lane == 0);
       slot += kWtTeams;
       if (slot >= p.slots) slot -= p.slots;
       s += kWtTeams;

@@ -52,6 +52,20 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
+// Two barriers at once, whose latencies overlap.
+__device__ __forceinline__ bool mbar_try_wait2(uint32_t bar0, uint32_t parity0, uint32_t bar1, uint32_t parity1) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 q, [%3], %4;\n\t"
+      "and.pred p, p, q;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar0), "r"(parity0), "r"(bar1), "r"(parity1)
+      : "memory");
+  return ok != 0;
+}
 // Non-blocking probe of a phase.
 __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
   uint32_t ok;
@@ -321,6 +335,16 @@ __device__ __forceinline__ uint32_t map_rank(uint32_t saddr, uint32_t rank) {
 // at K 29568 x N 8192, M = 16.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
+// One lane's arrivals on a barrier given by its cluster address and on one of this CTA, without a branch.
+__device__ __forceinline__ void mbar_arrive_both(uint32_t cluster_bar, uint32_t bar, bool lane) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.u32 p, %2, 0;\n\t"
+      "@p mbarrier.arrive.shared::cluster.b64 _, [%0];\n\t"
+      "@p mbarrier.arrive.shared::cta.b64 _, [%1];\n\t}" ::"r"(cluster_bar),
+      "r"(bar), "r"((uint32_t)lane)
+      : "memory");
 }
 // TMA load into this CTA's shared memory that completes on a barrier of either CTA of the pair.
 __device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap* map, int c0, int c1,
