@@ -11,6 +11,8 @@
 //
 // Rows move in permuted order between the kernels, so the GEMM epilogues store whole row segments at
 // a fixed pitch; what is scattered is the last kernel's reads, 4 KB at a time.
+#include <cmath>
+
 #include "common.cuh"
 
 namespace awq {
@@ -20,11 +22,37 @@ namespace {
 constexpr int kMBM = 128;      // rows of a block of the permutation
 constexpr int kTileRows = 256;  // rows of a grouped GEMM's tile, at most
 
-// Rows of a tile: with up to 128 most experts are one tile, two accumulators fit beside the weights, and the
-// next tile's MMAs run under the epilogue of the last one.  Up to 100 rows per expert on average nearly all
-// experts fit: router + experts, 128 experts of 2048 x 768, top-8, 1600 tokens 184 -> 167 us.
-// `experts` counts those that the pairs are spread over, on all ranks.
-int tile_rows(long long pairs, long long experts) { return pairs <= 100 * experts ? 128 : kTileRows; }
+// Rows of a tile (a multiple of 16): those of the least expected cost, for experts whose row counts scatter about
+// the average by its root.  In SM cycles a (tile, slab) costs its units times max(500, 4 rows), the conversion or the
+// tensor pipe, and what its epilogue leaves uncovered: 400 with two accumulators (up to 128 rows), 400 + 12 rows with
+// one.  Fitted to tiles of 128, 160, 192 and 256 rows at 11 batches; the size it picks is at most 2 % from the best of
+// them.  Against 128 rows up to 100 per expert and 256 beyond, whatever the batch (router excluded, top-8, us):
+// 128 experts of 2048 x 768: 1800 tokens 237 -> 206, 4096 504 -> 428, others equal; 64 of 2048 x 768: 3000 327 -> 298;
+// 64 of 4096 x 1536: 4096 818 -> 723; 64 of 4096 x 1024: 3000 728 -> 689.
+int tile_rows(long long pairs, long long experts, int H, int I) {
+  const double mean = (double)pairs / experts, root = sqrt(mean);
+  const int slabs = I / 128 + H / 256;
+  const double units = (I / 128) * (H / 128.) + (H / 256) * (I / 128.);
+  int best = kMBM;
+  double best_cost = -1;
+  for (int rows = kMBM; rows <= kTileRows; rows += 16) {
+    auto tile = [&](double n) {
+      return units * (4 * n > 500 ? 4 * n : 500.) + slabs * (rows <= 128 ? 400. : 400 + 12 * n);
+    };
+    double cost = 0;
+    for (int z = -4; z <= 4; ++z) {  // half deviations, weighted by the normal density
+      constexpr double kWeight[5] = {0.399, 0.352, 0.242, 0.130, 0.054};
+      const double count = mean + 0.5 * z * root > 1 ? mean + 0.5 * z * root : 1;
+      const double whole = floor(count / rows), rest = count - whole * rows;
+      cost += kWeight[z < 0 ? -z : z] * (whole * tile(rows) + (rest > 0 ? tile(rest) : 0));
+    }
+    if (best_cost < 0 || cost < best_cost) {
+      best = rows;
+      best_cost = cost;
+    }
+  }
+  return best;
+}
 
 // Experts that the permutation was built for: those of all ranks under expert parallelism, where `E` counts
 // the local ones.  Read off the capacity of the permuted list, which has room for kMBM - 1 entries of padding
@@ -34,14 +62,13 @@ long long routed_experts(const MoeArgs& a) {
   return a.expert_parallel && from_capacity > a.E ? from_capacity : a.E;
 }
 
-// Tile table of the grouped GEMMs in gemm_wt.cu: up to `tile_rows` rows of one expert per entry, i.e.
-// every expert's run of row blocks cut into pieces of tile_rows / block blocks.  One CTA; blocks are scanned 256 at
-// a time.
+// Tile table of the grouped GEMMs in gemm_wt.cu: up to `tile_rows` rows of one expert per entry, i.e. every expert's
+// run of row blocks cut into pieces of that many rows.  One CTA; blocks are scanned 256 at a time, and the last
+// block of a run writes its tiles.
 constexpr int kGatherThreads = 256;
 __device__ void moe_tile_table(const int32_t* sorted_ids,
                                const int32_t* expert_ids, int used, int numel, int block,
                                int tile_rows, int4* __restrict__ tiles, int32_t* __restrict__ n_tiles) {
-  const int per_tile = tile_rows / block;
   __shared__ int s_max[kGatherThreads / 32], s_sum[kGatherThreads / 32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int start_carry = -1, count_carry = 0;
@@ -49,6 +76,7 @@ __device__ void moe_tile_table(const int32_t* sorted_ids,
     const int i = base + tid;
     const int e = i < used ? __ldcg(expert_ids + i) : -1;
     const bool begins = i < used && (i == 0 || __ldcg(expert_ids + i - 1) != e);
+    const bool ends = i < used && e >= 0 && (i + 1 == used || __ldcg(expert_ids + i + 1) != e);
     int start = begins ? i : -1;  // inclusive running maximum: first block of this block's run
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
@@ -63,33 +91,32 @@ __device__ void moe_tile_table(const int32_t* sorted_ids,
       all_max = max(all_max, s_max[w]);
     }
     start = max(start, start_carry);
-    const bool emit = i < used && e >= 0 && (i - start) % per_tile == 0;
-    const unsigned mask = __ballot_sync(0xffffffffu, emit);
-    if (lane == 0) s_sum[warp] = __popc(mask);
+    int rows = 0;
+    if (ends) {  // valid rows come first in the run's last block: find where its padding starts
+      int lo = 0, hi = block;
+      while (lo < hi) {
+        const int mid = (lo + hi) / 2;
+        if (__ldcg(sorted_ids + (int64_t)i * block + mid) < numel) lo = mid + 1;
+        else hi = mid;
+      }
+      rows = (i - start) * block + lo;
+    }
+    const int pieces = (rows + tile_rows - 1) / tile_rows;
+    int incl = pieces;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, d);
+      if (lane >= d) incl += v;
+    }
+    if (lane == 31) s_sum[warp] = incl;
     __syncthreads();
-    int pos = count_carry + __popc(mask & ((1u << lane) - 1u));
-    int all_sum = count_carry;
+    int pos = count_carry + incl - pieces, all_sum = count_carry;
     for (int w = 0; w < kGatherThreads / 32; ++w) {
       if (w < warp) pos += s_sum[w];
       all_sum += s_sum[w];
     }
-    if (emit) {
-      int blocks = 1;
-      while (blocks < per_tile && i + blocks < used && __ldcg(expert_ids + i + blocks) == e) ++blocks;
-      const int last = i + blocks - 1;
-      int rows = block;
-      if (!(last + 1 < used && __ldcg(expert_ids + last + 1) == e)) {
-        // the run's last block: its valid rows come first, find where the padding starts
-        int lo = 0, hi = block;
-        while (lo < hi) {
-          const int mid = (lo + hi) / 2;
-          if (__ldcg(sorted_ids + (int64_t)last * block + mid) < numel) lo = mid + 1;
-          else hi = mid;
-        }
-        rows = lo;
-      }
-      tiles[pos] = make_int4(e, i * block, (blocks - 1) * block + rows, 0);
-    }
+    for (int at = 0; at < rows; at += tile_rows)
+      tiles[pos++] = make_int4(e, start * block + at, min(tile_rows, rows - at), 0);
     start_carry = all_max;
     count_carry = all_sum;
     __syncthreads();
@@ -102,7 +129,7 @@ __device__ void moe_tile_table(const int32_t* sorted_ids,
 // One warp per row, eight rows per CTA; a lane keeps four 16-byte loads in flight.  The
 // first CTA writes the tile table instead of rows.
 constexpr int kGatherRows = kGatherThreads / 32;
-__global__ void __launch_bounds__(kGatherThreads)
+__global__ void __launch_bounds__(kGatherThreads, 8)
 moe_gather_kernel(const __half* x, const int32_t* sorted_ids,
                   const int32_t* expert_ids, const int32_t* num_post_pad, const float* weights,
                   __half* __restrict__ x_perm, int32_t* __restrict__ inverse, float* __restrict__ row_weights,
@@ -226,7 +253,7 @@ size_t moe_tc_layout_bytes(const MoeArgs& a) {
 int launch_moe_experts_tc(const MoeArgs& a, void* workspace, size_t workspace_bytes,
                           cudaStream_t stream) {
   if (a.block != kMBM || !moe_tc_supported(a.H, a.I, a.group)) return AWQ_B200_ERR_SHAPE;
-  const int numel = a.T * a.topk, max_rows = tile_rows(numel, routed_experts(a));
+  const int numel = a.T * a.topk, max_rows = tile_rows(numel, routed_experts(a), a.H, a.I);
   const int64_t rows = padded_rows(a.sorted_capacity);
   const TcScratch at(rows, numel, a.H, a.I);
   if (workspace == nullptr || workspace_bytes < at.bytes) return AWQ_B200_ERR_WORKSPACE;

@@ -178,6 +178,31 @@ def test_prefill_tiles_per_expert(A, counts, group):
     assert O.rel_err(y.cpu().numpy(), ref) < TOL
 
 
+# Averages of 128 to 190 rows per expert, for which the tiles have 160, 192, 208 and 224 rows: row counts at their
+# multiples, which do not fall on the 128-row blocks of the permutation.
+@pytest.mark.parametrize("group", [128, 64])
+@pytest.mark.parametrize("counts", [
+    (159, 160, 161, 17, 319, 1, 209, 0), (191, 192, 193, 17, 383, 1, 271, 0), (207, 208, 209, 415, 0, 321, 1, 16),
+    (223, 224, 225, 447, 0, 385, 1, 16),
+])
+def test_prefill_tiles_between_the_blocks(A, counts, group):
+    from awq_b200 import synth
+    e, h, i = len(counts), 1024, 1024
+    ids = torch.cat([torch.full((c,), x, dtype=torch.int32) for x, c in enumerate(counts)])
+    t = ids.numel()
+    ids = ids[torch.randperm(t, generator=torch.Generator().manual_seed(t))].reshape(t, 1)
+    w1, w2 = synth.moe_layer_tensors(e, h, i, group, seed=t + group)
+    x = synth.activations(t, h, seed=t)
+    w = torch.rand(t, 1, generator=torch.Generator().manual_seed(1)) + 0.5
+    ref = O.fused_experts_fp32(x.numpy(), *[a.numpy() for a in w1], *[a.numpy() for a in w2],
+                               w.numpy(), ids.numpy(), group)
+    y = A.fused_experts(x.cuda(), tuple(a.cuda() for a in w1), tuple(a.cuda() for a in w2), w.cuda(),
+                        ids.cuda(), group_size=group)
+    torch.cuda.synchronize()
+    # fp16 weights, intermediate activations, rows and output: 2^-11 each, far inside TOL
+    assert O.rel_err(y.cpu().numpy(), ref) < TOL
+
+
 # Groups of 128: gemm_ts; 64 and 32: the mma.sync kernels, whose down GEMM adds the slots itself unless its
 # counters do not fit (64 tokens of 8192).  Every case has at least twice as many experts as pairs, or is
 # not direct.
