@@ -58,6 +58,12 @@
 //   1024 x 8192    M 1: 7.6 -> 4.9 us
 //   groups of 64 (before: mma.sync streaming kernel)
 //   8192 x 59136   M 4: 69.2 -> 52.9 us, M 16: 106.8 -> 65.5;  8192 x 1280   M 4: 11.1 -> 6.3 us
+// The instructions of the some 36 waits a unit takes are a fifth of all, so a wait for a complete phase is one probe,
+// one vote and one branch (mbar_wait_warp): 8192 x 59136 at M 8 55.4 -> 53.3 us, 8192 x 10240 groups of 64 at M 8 13.27
+// -> 13.07, experts of 128 x 2048 x 768 at 64 tokens 83.2 -> 80.6.  Tried and taken back: a team per half unit, with two
+// halves of A slots each (the conversion warps then get in each other's way, 55 -> 59 us at M 16); all MMAs of a unit in
+// one asm block, predicated arrivals (no difference); the sum over a token's slots by the warp that stores the last
+// of its rows (fences and counters at the end of every tile: 80 -> 99 us at 64 tokens, 16.4 -> 17.0 at one).
 // Bound by HBM on the long layers (a unit takes 718 cycles at M = 4, 712 is what 6.45 TB/s allows; 854
 // at M = 16), by start-up and hand-over (~5 us) on the short ones.
 // Experts without the router, 128 of 2048 x 768, 8 per token (before: mma.sync kernels on the decode copies;
@@ -330,8 +336,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     bool ok = true;
     while (raw.u < work.count) {
       // the first trip round the ring finds it empty
-      if (raw.u >= NRAW) ok = mbar_wait(raw_empty(raw_s), raw_phase ^ 1u, &s_abort, 21);
-      ok = __all_sync(0xffffffffu, ok);
+      if (raw.u >= NRAW) ok = mbar_wait_warp(raw_empty(raw_s), raw_phase ^ 1u, &s_abort, 21);
       if (!ok) break;
       load_raw();
     }
@@ -362,8 +367,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         }
       }
       if (x.u >= kTsUnits)
-        ok = mbar_wait(mma_done(x.u - kTsUnits), unit_phase(x.u - kTsUnits), &s_abort, 22);
-      ok = __all_sync(0xffffffffu, ok);
+        ok = mbar_wait_warp(mma_done(x.u - kTsUnits), unit_phase(x.u - kTsUnits), &s_abort, 22);
       if (!ok) break;
       const uint32_t bar = unit_full(x.u), dst = x_base + (x.u & (kTsUnits - 1)) * kTsXBytes;
       const uint32_t zdst = sz_base + (x.u & (kTsSzRing - 1)) * kSz + kScales;
@@ -398,8 +402,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     const int row = (lane & 7) + 8 * ((lane >> 3) & 1), kc = lane >> 4;
     bool ok = true;
     for (int u = 0; u < work.count && ok; ++u) {
-      ok = mbar_wait(unit_full(u), unit_phase(u), &s_abort, 23);
-      ok = __all_sync(0xffffffffu, ok);
+      ok = mbar_wait_warp(unit_full(u), unit_phase(u), &s_abort, 23);
       if (!ok) break;
       const uint32_t xt = x_base + (u & (kTsUnits - 1)) * kTsXBytes;
 #pragma unroll
@@ -434,8 +437,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     int slot = 0;
     for (int u = 0; u < work.count; ++u) {
       if (!ready) {
-        ok = mbar_wait(unit_full(u), unit_phase(u), &s_abort, 24);
-        ok = __all_sync(0xffffffffu, ok);
+        ok = mbar_wait_warp(unit_full(u), unit_phase(u), &s_abort, 24);
         if (!ok) break;
       }
       tc_fence_after();
@@ -471,8 +473,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       int s = team;
       uint32_t phase = 0;
       for (int u = team; u < work.count; u += kTsTeams) {
-        ok = mbar_wait(raw_full(s), phase, &s_abort, 26);
-        ok = __all_sync(0xffffffffu, ok);
+        ok = mbar_wait_warp(raw_full(s), phase, &s_abort, 26);
         if (!ok) break;
         const uint32_t raw = raw_base + s * kTsRawBytes;
         const uint32_t a_slot = tmem + lane_q + kTsColA + team * 128;
@@ -484,8 +485,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
           if (t == 0) {
             // the MMAs that read this A slot last must be complete
             if (u >= kTsTeams)
-              ok = mbar_wait(mma_done(u - kTsTeams), unit_phase(u - kTsTeams), &s_abort, 27);
-            ok = __all_sync(0xffffffffu, ok);
+              ok = mbar_wait_warp(mma_done(u - kTsTeams), unit_phase(u - kTsTeams), &s_abort, 27);
             if (!ok) break;
             tc_fence_after();
           }
@@ -573,8 +573,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             tot[m] = 0ull;
           }
         }
-        if (ok) ok = mbar_wait(mma_done(u), unit_phase(u), &s_abort, 28);
-        ok = __all_sync(0xffffffffu, ok);
+        if (ok) ok = mbar_wait_warp(mma_done(u), unit_phase(u), &s_abort, 28);
         if (!ok) continue;
         tc_fence_after();
         const uint32_t dcol = d_addr + (uint32_t)(u & (NDB - 1)) * (G * 2 * NT);

@@ -94,6 +94,21 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
                                           int code) {
   return mbar_wait_n(bar, parity, abort_flag, code, kSpinLimit);
 }
+// The same for a converged warp, with one answer for all lanes.  The way through a complete phase is a probe, a vote
+// and a branch.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int code) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "vote.sync.all.pred q, p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  if (ok != 0) return true;
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, code));
+}
 // About a millisecond, after a wait that gave up.
 __device__ __forceinline__ void linger() {
   const long long end = clock64() + 2000000;
