@@ -56,9 +56,9 @@
 //   clock near 1.3 GHz; 1.41 on 8192 x 59136 alone); router + experts, 128 experts of 2048 x 768, top-8, 2500
 //   tokens: 507 -> 296 us.
 // What bounds it: at M >= 256 the tensor pipe under the power limit; below, the conversion and, on the long layers,
-// the power limit.  A unit takes ~600 cycles at M = 24 and at M = 100.  The arithmetic is 270 of them (sub and mul
+// the power limit.  A unit took 630 cycles at M = 24 and at M = 100, now ~510.  The arithmetic is 270 of them (sub and mul
 // of f16x2 take two cycles a warp and scheduler; a loop of the conversion alone runs at 300), but a conversion warp
-// spends 2400 cycles on one of its own: half of that it waits for an instruction, a slot to issue, a branch or the
+// spent 2500 cycles on one of its own: half of that it waited for an instruction, a slot to issue, a branch or the
 // store port.  What helps is less of each: fragments of 32 rows at a time, one index for zero points and scales, so
 // that no register spills into the loop, and stores of the cheaper shape took 8192 x 59136 from 87.8 to 84.5 us at
 // M = 24 and 122.4 to 118.5 at M = 100; one wait per unit instead of two, arrivals without a branch and load warps
