@@ -52,9 +52,8 @@
 // Measured (B200, K x N, against one CTA per tile with two A stages and 64 / 128 fixed tokens):
 //   8192 x 59136   M 100: 123.6 -> 99.8 us; 29568 x 8192   M 100: 70 -> 58 us; the four linears of a layer
 //   (8192 x 10240, 8192 x 8192, 8192 x 59136, 29568 x 8192) against weights dequantised into shared memory:
-//   M 1000 1694 -> 1482 us, M 4096 6522 -> 5885 (1.22 PFLOP/s in a long loop, where the 1 kW limit holds the
-//   clock near 1.3 GHz; 1.41 on 8192 x 59136 alone); router + experts, 128 experts of 2048 x 768, top-8, 2500
-//   tokens: 507 -> 296 us.
+//   M 1000 1694 -> 1443 us, M 4096 6522 -> 5794 (1.24 PFLOP/s in a long loop, where the 1 kW limit holds the
+//   clock near 1.2 GHz); router + experts, 128 experts of 2048 x 768, top-8, 2500 tokens: 507 -> 289 us.
 // What bounds it: at M >= 256 the tensor pipe under the power limit; below, the conversion and, on the long layers,
 // the power limit.  A unit took 630 cycles at M = 24 and at M = 100, now ~510.  The arithmetic is 270 of them (sub and mul
 // of f16x2 take two cycles a warp and scheduler; a loop of the conversion alone runs at 300), but a conversion warp
