@@ -545,6 +545,13 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     pdl_wait();  // orders this thread's writes after the kernel before this one
     const unsigned long long token = p.flags.token;
     unsigned long long* flag = p.flags.at(blockIdx.x, fold);  // this warp's
+    // After a wait that gave up nothing more is folded.  In which form the loop over the units says so decides how it
+    // compiles. The first figures are with one vote and going on.  Groups of 128 take one vote and leave (us): 8192 x
+    // 59136 at M 8 51.5 -> 50.2, M 16 56.2 -> 53.7; 2304 x 8288 at M 16 7.30 -> 6.74; 1152 x 2048 at M 1 4.22 -> 4.14;
+    // experts of 128 x 2048 x 768, top-8, 64 tokens 81.0 -> 79.3.  Groups of 64 differ by tokens: up to 4 a probe and a
+    // vote, then they leave (8192 x 59136 at M 1 49.0 -> 48.4; one vote 50.4); up to 8 as groups of 128 (52.8 at M 8; two
+    // 53.5); up to 16 a probe and a vote, and they go on (2304 x 8288 8.45 -> 7.99; leaving 8.20, with one vote 8.11).
+    constexpr bool kOneVote = GROUP == 128 || MT == 8, kStay = GROUP == 64 && MT == 16;
     bool ok = true;
     int u = 0;
     for (int seg = 0; seg < work.segs; ++seg) {
@@ -563,7 +570,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       uint64_t tot[MT / 2];
 #pragma unroll
       for (int m = 0; m < MT / 2; ++m) tot[m] = 0ull;
-      for (int k = kb; k < ke; ++k, ++u) {
+      for (int k = ok || kStay ? kb : ke; k < ke; ++k, ++u) {
         if (MODE == 1 && k == p.KT && kb < p.KT) {  // gate complete: park its sums, start on up
 #pragma unroll
           for (int m = 0; m < MT / 2; ++m) {
@@ -573,8 +580,16 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             tot[m] = 0ull;
           }
         }
-        if (ok) ok = mbar_wait_warp(mma_done(u), unit_phase(u), &s_abort, 28);
-        if (!ok) continue;
+        if constexpr (kOneVote) {
+          ok = mbar_wait_warp(mma_done(u), unit_phase(u), &s_abort, 28);
+        } else {
+          if (ok || !kStay) ok = mbar_wait(mma_done(u), unit_phase(u), &s_abort, 28);
+          ok = __all_sync(0xffffffffu, ok);
+        }
+        if (!ok) {
+          if constexpr (kStay) continue;
+          break;
+        }
         tc_fence_after();
         const uint32_t dcol = d_addr + (uint32_t)(u & (NDB - 1)) * (G * 2 * NT);
         const uint32_t ring = (uint32_t)(u & (kTsSzRing - 1));
