@@ -203,6 +203,32 @@ def test_prefill_tiles_between_the_blocks(A, counts, group):
     assert O.rel_err(y.cpu().numpy(), ref) < TOL
 
 
+# Runs of row blocks that begin, end or go on at the 32nd and the 256th block, where the tile table's scan changes
+# warps and starts again, and runs of one block there; 257 to 300 blocks in all.
+@pytest.mark.parametrize("counts", [
+    (31 * 128, 5, 1, 30 * 128 + 7, 128, 192 * 128, 1, 3, 129), (32 * 128 - 1, 224 * 128, 77, 0, 40 * 128 + 1),
+    (255 * 128, 128, 1), (257 * 128,),
+])
+def test_prefill_tile_table_of_many_blocks(A, counts):
+    from awq_b200 import synth
+    e, h, i = len(counts), 256, 128
+    ids = torch.cat([torch.full((c,), x, dtype=torch.int32) for x, c in enumerate(counts)])
+    t = ids.numel()
+    ids = ids[torch.randperm(t, generator=torch.Generator().manual_seed(t))].reshape(t, 1)
+    w1, w2 = synth.moe_layer_tensors(e, h, i, 128, seed=t)
+    x = synth.activations(t, h, seed=t)
+    w = torch.rand(t, 1, generator=torch.Generator().manual_seed(1)) + 0.5
+    ref = O.fused_experts_fp32(x.numpy(), *[a.numpy() for a in w1], *[a.numpy() for a in w2],
+                               w.numpy(), ids.numpy(), 128)
+    y = A.fused_experts(x.cuda(), tuple(a.cuda() for a in w1), tuple(a.cuda() for a in w2), w.cuda(), ids.cuda())
+    torch.cuda.synchronize()
+    # Row by row, as rows differ in size (silu(gate) * up has long tails).  Roundings of 2^-11 at most of the weights,
+    # the activation, the row and the output, independent over the 256 and 128 terms of a sum: some 2^-11 of the
+    # row's norm, 1 / 20 of TOL.  A row that no tile has, or another expert's tile, is off by all of itself.
+    err = np.linalg.norm(y.cpu().numpy().astype(np.float32) - ref, axis=1)
+    assert (err <= TOL * np.linalg.norm(ref, axis=1)).all()
+
+
 # Groups of 128: gemm_ts; 64 and 32: the mma.sync kernels, whose down GEMM adds the slots itself unless its
 # counters do not fit (64 tokens of 8192).  Every case has at least twice as many experts as pairs, or is
 # not direct.
