@@ -302,6 +302,14 @@ int awq_b200_moe_local_ids(const int32_t* topk_ids, int T, int topk, int E,
                            const int32_t* expert_map, int32_t* local_ids, void* stream);
 int awq_b200_moe_block_size(int T, int topk, int E, int H, int I, int group);
 
+/*
+ * Rows of a tile of the grouped GEMMs (a multiple of 16 from 128 to 256) that awq_b200_moe_experts takes with
+ * block 128: `E` experts the permutation was built for, `local` of them stacked here, on a GPU that holds `cta_pairs`
+ * pairs of CTAs (0: the current device's).  Host arithmetic, for tests that name a tile size.
+ * AWQ_B200_ERR_SHAPE where the block is another.  No counterpart in the reference.
+ */
+int awq_b200_moe_tile_rows(int T, int topk, int E, int local, int H, int I, int cta_pairs);
+
 size_t awq_b200_moe_workspace_bytes(int T, int topk, int E, int H, int I);
 
 int awq_b200_moe_experts(const void* x, const void* w13_q, const void* w13_s, const void* w13_z,

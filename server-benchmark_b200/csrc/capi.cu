@@ -390,6 +390,17 @@ int awq_b200_moe_block_size(int T, int topk, int E, int H, int I, int group) {
   return awq::moe_block_size(T, topk, E, H, I, group);
 }
 
+int awq_b200_moe_tile_rows(int T, int topk, int E, int local, int H, int I, int cta_pairs) {
+  if (T <= 0 || topk <= 0 || E <= 0 || local <= 0 || local > E || cta_pairs < 0 ||
+      awq::moe_block_size(T, topk, E, H, I, 128) != 128)
+    return AWQ_B200_ERR_SHAPE;
+  if (cta_pairs == 0) {
+    if (int rc = check_device()) return rc;
+    cta_pairs = awq::sm_count() / 2;
+  }
+  return awq::moe_tile_rows((long long)T * topk, E, local, H, I, cta_pairs);
+}
+
 size_t awq_b200_moe_workspace_bytes(int T, int topk, int E, int H, int I) {
   return awq::moe_workspace_bytes(T, topk, E, H, I);
 }

@@ -279,6 +279,7 @@ int launch_moe_local_ids(const int32_t* topk_ids, int n, const int32_t* expert_m
 bool moe_supported(int H, int I, int group, int block);
 size_t moe_workspace_bytes(int T, int topk, int E, int H, int I);
 int moe_block_size(int T, int topk, int E, int H, int I, int group);
+int moe_tile_rows(long long pairs, long long experts, int local, int H, int I, int cta_pairs);
 bool moe_tc_supported(int H, int I, int group);
 size_t moe_tc_workspace_bytes(int T, int topk, int E, int H, int I);
 size_t moe_tc_layout_bytes(const MoeArgs& a);

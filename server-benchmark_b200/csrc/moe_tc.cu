@@ -22,29 +22,44 @@ namespace {
 constexpr int kMBM = 128;      // rows of a block of the permutation
 constexpr int kTileRows = 256;  // rows of a grouped GEMM's tile, at most
 
+}  // namespace
+
 // Rows of a tile (a multiple of 16): those of the least expected cost, for experts whose row counts scatter about
-// the average by its root.  In SM cycles a (tile, slab) costs its units times max(500, 4 rows), the conversion or the
-// tensor pipe, and what its epilogue leaves uncovered: 400 with two accumulators (up to 128 rows), 400 + 12 rows with
-// one.  Fitted to tiles of 128, 160, 192 and 256 rows at 11 batches; the size it picks is at most 2 % from the best of
-// them.  Against 128 rows up to 100 per expert and 256 beyond, whatever the batch (router excluded, top-8, us):
-// 128 experts of 2048 x 768: 1800 tokens 237 -> 206, 4096 504 -> 428, others equal; 64 of 2048 x 768: 3000 327 -> 298;
-// 64 of 4096 x 1536: 4096 818 -> 723; 64 of 4096 x 1024: 3000 728 -> 689.
-int tile_rows(long long pairs, long long experts, int H, int I) {
+// the average by its root.  In SM cycles a (tile, slab) of n rows costs its units times max(460, 4 n), the conversion or
+// the tensor pipe, and what its epilogue leaves uncovered: 400 with two accumulators (up to 128 rows), 800 + 10 n with one.
+// A GEMM of `local` experts takes the average cost times the tiles of a pair, half way between their average and the
+// next whole number: with few experts some pairs have a tile more than the others.  Fitted to all tiles from 128 to 256
+// rows at 229 batches of 104 to 450 rows per expert, 15 shapes of 4 to 128 experts; the size it picks is 0.7 % from the
+// best on average, 14 % at worst, and 0.6 and 6 % at 90 batches of 11 other shapes.  Without the tiles of a pair (and 500,
+// 400 + 12 n) it was 1.8 %, 25 % at worst: 16 experts of 2048 x 1024, top-2, 960 tokens 128 rows, 49.9 us, 144 rows 46.3.
+// Routing that the host cannot know, experts drawn with a bias, prefers 128 rows by 10 %.
+// Against 128 rows up to 100 per expert and 256 beyond, whatever the batch (router excluded, top-8, us): 128 experts of
+// 2048 x 768: 1800 tokens 233 -> 200, 4096 492 -> 408; 64 of 4096 x 1536, top-4: 4096 814 -> 708.
+int moe_tile_rows(long long pairs, long long experts, int local, int H, int I, int cta_pairs) {
   const double mean = (double)pairs / experts, root = sqrt(mean);
-  const int slabs = I / 128 + H / 256;
-  const double units = (I / 128) * (H / 128.) + (H / 256) * (I / 128.);
+  const int slabs[2] = {I / 128, H / 256};
+  const double stages[2] = {H / 128., I / 128.};  // of a tile
   int best = kMBM;
   double best_cost = -1;
   for (int rows = kMBM; rows <= kTileRows; rows += 16) {
-    auto tile = [&](double n) {
-      return units * (4 * n > 500 ? 4 * n : 500.) + slabs * (rows <= 128 ? 400. : 400 + 12 * n);
+    double units = 0, epilogue = 0, tiles = 0;  // of one expert
+    auto add = [&](double count, double n) {
+      units += count * (4 * n > 460 ? 4 * n : 460.);
+      epilogue += count * (rows <= 128 ? 400. : 800 + 10 * n);
+      tiles += count;
     };
-    double cost = 0;
     for (int z = -4; z <= 4; ++z) {  // half deviations, weighted by the normal density
-      constexpr double kWeight[5] = {0.399, 0.352, 0.242, 0.130, 0.054};
+      constexpr double kWeight[5] = {0.2041, 0.1801, 0.1238, 0.0665, 0.0276};
+      const double weight = kWeight[z < 0 ? -z : z];
       const double count = mean + 0.5 * z * root > 1 ? mean + 0.5 * z * root : 1;
       const double whole = floor(count / rows), rest = count - whole * rows;
-      cost += kWeight[z < 0 ? -z : z] * (whole * tile(rows) + (rest > 0 ? tile(rest) : 0));
+      add(weight * whole, rows);
+      if (rest > 0) add(weight, rest);
+    }
+    double cost = 0;
+    for (int g = 0; g < 2; ++g) {
+      const double per_pair = tiles * local * slabs[g] / cta_pairs;
+      cost += (stages[g] * units + epilogue) / tiles * (per_pair + ceil(per_pair - 1e-3)) / 2;
     }
     if (best_cost < 0 || cost < best_cost) {
       best = rows;
@@ -53,6 +68,8 @@ int tile_rows(long long pairs, long long experts, int H, int I) {
   }
   return best;
 }
+
+namespace {
 
 // Experts that the permutation was built for: those of all ranks under expert parallelism, where `E` counts
 // the local ones.  Read off the capacity of the permuted list, which has room for kMBM - 1 entries of padding
@@ -258,7 +275,8 @@ size_t moe_tc_layout_bytes(const MoeArgs& a) {
 int launch_moe_experts_tc(const MoeArgs& a, void* workspace, size_t workspace_bytes,
                           cudaStream_t stream) {
   if (a.block != kMBM || !moe_tc_supported(a.H, a.I, a.group)) return AWQ_B200_ERR_SHAPE;
-  const int numel = a.T * a.topk, max_rows = tile_rows(numel, routed_experts(a), a.H, a.I);
+  const int numel = a.T * a.topk;
+  const int max_rows = moe_tile_rows(numel, routed_experts(a), a.E, a.H, a.I, sm_count() / 2);
   const int64_t rows = padded_rows(a.sorted_capacity);
   const TcScratch at(rows, numel, a.H, a.I);
   if (workspace == nullptr || workspace_bytes < at.bytes) return AWQ_B200_ERR_WORKSPACE;

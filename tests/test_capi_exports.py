@@ -218,3 +218,31 @@ def test_validation_of_the_newer_entry_points_without_gpu(built_library):
     assert lib.awq_b200_moe_experts(*many) == -2                                   # 128 pairs > 64
     # without the flag the permutation tables are required
     assert lib.awq_b200_moe_experts(*base, *tail(8, 0, T * topk * 8)) == -1
+
+
+# Batches at which the tiles of some sizes leave pairs of CTAs idle, and the sizes measured within 3 % of the best one
+# on 74 pairs.
+@pytest.mark.parametrize("t,topk,e,h,i,sizes", [
+    (960, 2, 16, 2048, 1024, range(144, 257, 16)),   # 128 rows: 8 % slower
+    (504, 1, 4, 2048, 1024, [128]), (800, 1, 4, 2048, 1024, [128]),  # 160 rows 13 %, 240 rows 25 %
+    (1320, 1, 4, 2048, 1024, [176, 192]), (856, 2, 8, 4096, 1536, [128]), (1776, 2, 12, 2048, 1408, [160]),
+    (879, 2, 6, 3072, 1024, [128]), (1520, 4, 16, 4096, 1536, [128]),
+    (2500, 8, 128, 2048, 768, range(176, 257, 16)), (4096, 8, 128, 2048, 768, [128]),
+])
+def test_prefill_tile_rows_count_idle_pairs(built_library, t, topk, e, h, i, sizes):
+    from awq_b200 import _lib
+    assert _lib.load().awq_b200_moe_tile_rows(t, topk, e, e, h, i, 74) in sizes
+
+
+def test_prefill_tile_rows_of_every_call(built_library):
+    from awq_b200 import _lib
+    rows = _lib.load().awq_b200_moe_tile_rows
+    for t, topk, e, local, h, i in [(36, 1, 1, 1, 256, 128), (4096, 8, 8, 8, 4096, 14336), (2500, 8, 128, 16, 2048, 768),
+                                    (100000, 8, 256, 1, 7168, 2048), (2000000, 8, 1024, 1024, 256, 128)]:
+        for pairs in (1, 66, 74):
+            got = rows(t, topk, e, local, h, i, pairs)
+            assert 128 <= got <= 256 and got % 16 == 0
+    assert rows(35, 1, 1, 1, 256, 128, 74) == -2          # smaller blocks: no tiles
+    assert rows(2500, 8, 128, 129, 2048, 768, 74) == -2
+    assert rows(2500, 8, 128, 128, 2048, 768, -1) == -2
+    assert rows(0, 8, 128, 128, 2048, 768, 74) == -2
