@@ -246,3 +246,14 @@ def test_prefill_tile_rows_of_every_call(built_library):
     assert rows(2500, 8, 128, 129, 2048, 768, 74) == -2
     assert rows(2500, 8, 128, 128, 2048, 768, -1) == -2
     assert rows(0, 8, 128, 128, 2048, 768, 74) == -2
+
+
+def test_grouped_tiles_of_every_size_are_tested(built_library):
+    """The GPU test of the grouped GEMMs' tiles names their sizes: on 74 pairs its shapes take them, and every size is
+    among them."""
+    from awq_b200 import _lib
+    from test_gpu_moe import TILE_CASES
+    rows = _lib.load().awq_b200_moe_tile_rows
+    for size, h, i, counts in TILE_CASES:
+        assert rows(sum(counts), 1, len(counts), len(counts), h, i, 74) == size
+    assert {c[0] for c in TILE_CASES} == set(range(128, 257, 16))

@@ -156,7 +156,7 @@ def test_fused_experts_vs_oracle(A, e, h, i, t, k):
 
 @pytest.mark.parametrize("group", [128, 64])
 @pytest.mark.parametrize("counts", [
-    (0, 1, 129, 256, 257, 128, 17, 300),     # around the 128-row blocks and 256-row tiles, a gap
+    (0, 1, 129, 256, 257, 128, 17, 300),     # around the multiples of 128 rows, a gap
     (513, 0, 0, 0, 0, 0, 0, 15),             # three tiles of one expert, experts without rows
 ])
 def test_prefill_tiles_per_expert(A, counts, group):
@@ -178,18 +178,30 @@ def test_prefill_tiles_per_expert(A, counts, group):
     assert O.rel_err(y.cpu().numpy(), ref) < TOL
 
 
-# Averages of 128 to 190 rows per expert, for which the tiles have 160, 192, 208 and 224 rows: row counts at their
-# multiples, which do not fall on the 128-row blocks of the permutation.
+# Every size of a tile above 128 rows, with row counts at its multiples, which do not fall on the 128-row blocks of
+# the permutation, and shapes for which that size is taken (asserted); then counts that leave 128 rows or 160.
+TILE_CASES = [
+    (144, 1024, 1024, (143, 144, 145, 287, 289, 432, 575, 17)),
+    (160, 768, 384, (159, 160, 161, 319, 321, 1, 17, 0, 119, 120, 121, 122, 123, 124, 125, 126)),
+    (176, 768, 384, (175, 176, 177, 351, 353, 1, 17, 0, 116, 117, 118, 119, 120, 121, 122, 123)),
+    (192, 768, 512, (191, 192, 193, 383, 385, 1, 17, 0, 132, 133, 134, 135, 136, 137, 139, 140)),
+    (208, 1024, 512, (207, 208, 209, 415, 417, 1, 17, 0, 148, 149, 150, 151, 152, 153, 154, 155)),
+    (224, 1792, 640, (223, 224, 225, 447, 449, 1, 17, 0, 150, 156)),
+    (240, 2048, 1536, (239, 240, 241, 481, 17, 10)),
+    (256, 4096, 2048, (255, 257, 241)), (256, 4096, 2048, (256, 511, 0)),
+    (160, 1024, 1024, (159, 160, 161, 17, 319, 1, 209, 0)), (128, 1024, 1024, (191, 192, 193, 17, 383, 1, 271, 0)),
+    (128, 1024, 1024, (207, 208, 209, 415, 0, 321, 1, 16)), (128, 1024, 1024, (223, 224, 225, 447, 0, 385, 1, 16)),
+]
+
+
 @pytest.mark.parametrize("group", [128, 64])
-@pytest.mark.parametrize("counts", [
-    (159, 160, 161, 17, 319, 1, 209, 0), (191, 192, 193, 17, 383, 1, 271, 0), (207, 208, 209, 415, 0, 321, 1, 16),
-    (223, 224, 225, 447, 0, 385, 1, 16),
-])
-def test_prefill_tiles_between_the_blocks(A, counts, group):
-    from awq_b200 import synth
-    e, h, i = len(counts), 1024, 1024
+@pytest.mark.parametrize("rows,h,i,counts", TILE_CASES)
+def test_prefill_tiles_between_the_blocks(A, rows, h, i, counts, group):
+    from awq_b200 import _lib, synth
+    e = len(counts)
     ids = torch.cat([torch.full((c,), x, dtype=torch.int32) for x, c in enumerate(counts)])
     t = ids.numel()
+    assert _lib.load().awq_b200_moe_tile_rows(t, 1, e, e, h, i, 0) == rows
     ids = ids[torch.randperm(t, generator=torch.Generator().manual_seed(t))].reshape(t, 1)
     w1, w2 = synth.moe_layer_tensors(e, h, i, group, seed=t + group)
     x = synth.activations(t, h, seed=t)
