@@ -150,6 +150,14 @@ size_t awq_b200_gemm_workspace_bytes(int M, int N, int K, int group, int kernel)
   return 0;
 }
 
+int awq_b200_gemm_wt_cut(int M, int N, int K, int group, int cta_pairs, int* tokens, int* chunk, int* wide) {
+  if (!tokens || !chunk || !wide) return AWQ_B200_ERR_NULL;
+  if (M <= 0 || N <= 0 || K <= 0 || cta_pairs < 0) return AWQ_B200_ERR_SHAPE;
+  if (cta_pairs == 0)
+    if (int rc = check_device()) return rc;
+  return awq::gemm_wt_cut(M, N, K, group, cta_pairs, tokens, chunk, wide);
+}
+
 int awq_b200_gemm(const void* x, const void* qweight, const void* scales, const void* qzeros,
                   const void* bias, void* out, int M, int N, int K, int group, int kernel,
                   void* workspace, size_t workspace_bytes, void* stream) {

@@ -1093,6 +1093,23 @@ size_t gemm_wt_workspace_bytes(int M, int N, int K, int group) {
   return plan.chunk > 0 ? wt_scratch_bytes(plan.nt, plan.pairs) : 0;
 }
 
+int gemm_wt_cut(int M, int N, int K, int group, int cta_pairs, int* tokens, int* chunk, int* wide) {
+  if (!gemm_wt_supported(M, N, K, group)) return AWQ_B200_ERR_SHAPE;
+  if (cta_pairs == 0) {
+    if (int rc = group == 128 ? wt_prepare<0, 128, false>() : wt_prepare<0, 64, false>()) return rc;
+    cta_pairs = group == 128 ? wt_pairs<0, 128, false>(kWtSmemLimit) : wt_pairs<0, 64, false>(kWtSmemLimit);
+  }
+  const WtPlan plan = wt_plan(M, (N + kWtBN - 1) / kWtBN, K / kWtBK, cta_pairs, true);
+  WtParams p = {};
+  p.nt = plan.nt;
+  p.chunk = plan.chunk;
+  wt_rings(&p, 0);
+  *tokens = plan.nt;
+  *chunk = plan.chunk;
+  *wide = p.stage_bytes > 0 ? 1 : 0;
+  return AWQ_B200_OK;
+}
+
 int launch_gemm_wt(const __half* x, const uint32_t* qweight, const __half* scales,
                    const uint32_t* qzeros, const __half* bias, __half* out, int M, int N, int K,
                    int group, void* workspace, size_t workspace_bytes, cudaStream_t stream) {

@@ -257,3 +257,23 @@ def test_grouped_tiles_of_every_size_are_tested(built_library):
     for size, h, i, counts in TILE_CASES:
         assert rows(sum(counts), 1, len(counts), len(counts), h, i, 74) == size
     assert {c[0] for c in TILE_CASES} == set(range(128, 257, 16))
+
+
+def test_wide_tiles_of_every_size_are_tested(built_library):
+    """The same for the dense tiles above 128 tokens, whole and split."""
+    from awq_b200 import _lib
+    from test_gpu_wt import CUT_CASES, cut
+    for m, k, n, group, tokens, split in CUT_CASES:
+        got = cut(m, k, n, group, 74)
+        assert (got[0], got[1] > 0, got[2]) == (tokens, split, 0 if split else 1)
+    assert {c[4] for c in CUT_CASES if not c[5]} == set(range(144, 257, 16))
+    assert any(-(-m // tokens) * -(-n // 256) > 74 for m, k, n, _, tokens, split in CUT_CASES if not split)
+    assert any(-(-m // tokens) * -(-n // 256) < 74 for m, k, n, _, tokens, split in CUT_CASES if not split)
+    lib = _lib.load()
+    v = [ctypes.c_int(-1) for _ in range(3)]
+    out = [ctypes.byref(x) for x in v]
+    assert lib.awq_b200_gemm_wt_cut(64, 8192, 1000, 128, 74, *out) == -2   # K no whole stages
+    assert lib.awq_b200_gemm_wt_cut(0, 8192, 1024, 128, 74, *out) == -2
+    assert lib.awq_b200_gemm_wt_cut(64, 8192, 1024, 128, -1, *out) == -2
+    assert lib.awq_b200_gemm_wt_cut(64, 8192, 1024, 128, 74, None, *out[:2]) == -1
+    assert [x.value for x in v] == [-1, -1, -1]

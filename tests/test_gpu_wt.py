@@ -155,13 +155,32 @@ def test_wt_collected_tiles(A, m, k, n, group):
     assert O.elementwise_ok(y[0].cpu().numpy(), ref, TOL)
 
 
-# Whole tiles of more than 128 tokens, several per pair, whose epilogue goes through shared memory: every tile size
-# from 144 to 256 (4 to 13 stages of packed words), one to nine units a tile, a last tile of few tokens, a slab past N.
-@pytest.mark.parametrize("m,k,n,group", [
-    (400, 640, 9504, 128), (777, 384, 9504, 64), (500, 128, 9504, 128), (900, 640, 9504, 64), (777, 256, 8224, 128),
-    (430, 1152, 9472, 128), (900, 512, 8224, 64), (1000, 640, 8224, 128),
-])
-def test_wt_wide_tiles(A, m, k, n, group):
+# Tiles of more than 128 tokens, one accumulator.  Whole ones, whose epilogue goes through shared memory: every tile size
+# from 144 to 256 (4 to 13 stages of packed words), one to nine units a tile, a last tile of few tokens, a slab past N,
+# first several tiles to a pair, then one.  Last, split ones, whose epilogue does not.  (m, k, n, group, tokens of a tile,
+# split): asserted, as the cut follows from a cost.
+CUT_CASES = [
+    (400, 640, 9504, 128, 144, False), (777, 384, 9504, 64, 160, False), (500, 128, 9504, 128, 176, False),
+    (900, 640, 9504, 64, 192, False), (777, 256, 8224, 128, 208, False), (430, 1152, 9472, 128, 224, False),
+    (900, 512, 8224, 64, 240, False), (1000, 640, 8224, 128, 256, False),
+    (264, 1024, 8192, 128, 144, False), (150, 4096, 11040, 64, 160, False), (400, 1024, 8192, 128, 208, False),
+    (511, 4096, 8192, 64, 256, False), (774, 8192, 544, 128, 144, True), (291, 7680, 3360, 64, 160, True),
+]
+
+
+def cut(m, k, n, group, cta_pairs):
+    """(tokens of a tile, units of a pair's range or 0, epilogue through shared memory)"""
+    from awq_b200 import _lib
+    v = [ctypes.c_int(-1) for _ in range(3)]
+    rc = _lib.load().awq_b200_gemm_wt_cut(m, n, k, group, cta_pairs, *[ctypes.byref(x) for x in v])
+    assert rc == 0
+    return tuple(x.value for x in v)
+
+
+@pytest.mark.parametrize("m,k,n,group,tokens,split", CUT_CASES)
+def test_wt_wide_tiles(A, m, k, n, group, tokens, split):
+    got = cut(m, k, n, group, 0)
+    assert (got[0], got[1] > 0, got[2]) == (tokens, split, 0 if split else 1)
     from awq_b200 import synth
     qw, s, qz = synth.awq_linear_tensors(k, n, group, seed=m)
     x = synth.activations(m, k, seed=n)
