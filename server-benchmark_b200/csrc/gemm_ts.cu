@@ -4,7 +4,7 @@
 //
 // The int4 weights are unpacked in registers (ldmatrix.trans pairs the rows k, k + 1 of a halfword
 // column in the load; one AND per pair, nibbles used as fp16 subnormals q * 2^-24, exact), written to
-// tensor memory with tcgen05.st.16x256b and are the A operand (128 weight columns x 16 k) of
+// tensor memory with tcgen05.st.16x128b and are the A operand (128 weight columns x 16 k) of
 // tcgen05.mma.kind::f16; the activations are the small B operand as TMA delivers them.  No arithmetic
 // is spent on a weight: zero point and scale are applied per quantisation group to the fp32
 // accumulators,  tot += scale * (acc - zero * sum_k x).
@@ -49,25 +49,26 @@
 // Lane 32 q + 8 i + g of tile t holds column
 // 128 t + 32 q + 8 (g / 2) + 2 i + g % 2 of the slab.  Every wait is bounded (tc_ptx.cuh).
 //
-// Measured (B200, K x N, first replays of a cool GPU; under the power limit of a long loop 8192 x 59136 takes 48 and
-// 52 us; before: mma.sync streaming kernel up to M = 8, its decode-layout copy in
+// Measured (B200, K x N, first replays of a cool GPU; under the power limit of a long loop 8192 x 59136 takes 47 and
+// 55 us; before: mma.sync streaming kernel up to M = 8, its decode-layout copy in
 // brackets, an earlier form of this kernel above; K-major copy in brackets):
-//   8192 x 59136   M 4: 56.2 (50.6) -> 44.9 us, 5.4 TB/s of int4    M 16: 82.1 (64.1) -> 50.2 us
-//   29568 x 8192   M 4: 35.0 (30.2) -> 25.9 us                        M 16: 40.0 (43.7) -> 29.5 us
-//   8192 x 10240   M 4: 17.2 (16.0) -> 12.8 us                        M 16: 20.0 (22.9) -> 14.8 us
-//   1024 x 8192    M 1: 7.6 -> 4.9 us
+//   8192 x 59136   M 4: 56.2 (50.6) -> 41.6 us, 5.8 TB/s of int4    M 16: 82.1 (64.1) -> 45.3 us
+//   29568 x 8192   M 4: 35.0 (30.2) -> 24.7 us                        M 16: 40.0 (43.7) -> 27.3 us
+//   8192 x 10240   M 4: 17.2 (16.0) -> 11.9 us                        M 16: 20.0 (22.9) -> 13.3 us
+//   1024 x 8192    M 1: 7.6 -> 4.6 us
 //   groups of 64 (before: mma.sync streaming kernel)
-//   8192 x 59136   M 4: 69.2 -> 52.9 us, M 16: 106.8 -> 65.5;  8192 x 1280   M 4: 11.1 -> 6.3 us
+//   8192 x 59136   M 4: 69.2 -> 43.2 us, M 16: 106.8 -> 59.7;  8192 x 1280   M 4: 11.1 -> 6.4 us
 // The instructions of the some 36 waits a unit takes are a fifth of all, so a wait for a complete phase is one probe,
 // one vote and one branch (mbar_wait_warp): 8192 x 59136 at M 8 55.4 -> 53.3 us, 8192 x 10240 groups of 64 at M 8 13.27
-// -> 13.07, experts of 128 x 2048 x 768 at 64 tokens 83.2 -> 80.6.  Tried and taken back: a team per half unit, with two
+// -> 13.07, experts of 128 x 2048 x 768 at 64 tokens 83.2 -> 80.6 (that step alone; the fold warps differ, see there).
+// Tried and taken back: a team per half unit, with two
 // halves of A slots each (the conversion warps then get in each other's way, 55 -> 59 us at M 16); all MMAs of a unit in
 // one asm block, predicated arrivals (no difference); the sum over a token's slots by the warp that stores the last
 // of its rows (fences and counters at the end of every tile: 80 -> 99 us at 64 tokens, 16.4 -> 17.0 at one).
-// Bound by HBM on the long layers (a unit takes 718 cycles at M = 4, 712 is what 6.45 TB/s allows; 854
-// at M = 16), by start-up and hand-over (~5 us) on the short ones.
+// Bound by HBM on the long layers (6.45 TB/s allow 712 cycles a unit; some 810 at M = 16, 46 300 of a CTA with 50 units,
+// ncu), by start-up and hand-over (~5 us) on the short ones.
 // Experts without the router, 128 of 2048 x 768, 8 per token (before: mma.sync kernels on the decode copies;
-// replayed graph): T 1: 22.9 -> 17.4 us, T 16: 71.0 -> 62.1, T 64: 101.9 -> 79.9, T 128: 110.7 -> 104.0.  At T = 64 all
+// replayed graph, cool): T 1: 22.9 -> 16.2 us, T 16: 71.0 -> 53.8, T 64: 101.9 -> 72.2, T 128: 110.7 -> 92.1.  At T = 64 all
 // 302 MB of int4 words are read, 48 us at the HBM rate; a block of 8 rows costs the conversion of a
 // whole matrix, which is what bounds it.
 #include "common.cuh"
@@ -490,7 +491,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             tc_fence_after();
           }
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {  // four 16-row steps each
+          for (int h = 0; h < 2; ++h) {  // 64 rows each, eight by eight
             // Logic and shifts take two cycles a warp and scheduler: 320 of them a unit are what
             // bounds the kernel beside HBM.  (The shift as a multiplication on the FMA pipe, which is
             // idle here, measured 7 % slower: mul.hi takes four cycles.)
@@ -546,7 +547,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     const unsigned long long token = p.flags.token;
     unsigned long long* flag = p.flags.at(blockIdx.x, fold);  // this warp's
     // After a wait that gave up nothing more is folded.  In which form the loop over the units says so decides how it
-    // compiles. The first figures are with one vote and going on.  Groups of 128 take one vote and leave (us): 8192 x
+    // compiles.  The first figures are with one vote and going on.  Groups of 128 take one vote and leave (us): 8192 x
     // 59136 at M 8 51.5 -> 50.2, M 16 56.2 -> 53.7; 2304 x 8288 at M 16 7.30 -> 6.74; 1152 x 2048 at M 1 4.22 -> 4.14;
     // experts of 128 x 2048 x 768, top-8, 64 tokens 81.0 -> 79.3.  Groups of 64 differ by tokens: up to 4 a probe and a
     // vote, then they leave (8192 x 59136 at M 1 49.0 -> 48.4; one vote 50.4); up to 8 as groups of 128 (52.8 at M 8; two

@@ -5,7 +5,7 @@
 // The weights are the A operand of tcgen05.mma.cta_group::2.kind::f16 (M = 256 weight columns, 128
 // per CTA, x K = 16) and live in TMEM: conversion warps take the packed words from shared memory
 // with ldmatrix.trans, dequantise them in registers to (q - z) * s in fp16 and write the fragments
-// with tcgen05.st.16x256b.  The activations are the B operand (up to 256 tokens, K-major, 128-byte
+// with tcgen05.st.16x128b.  The activations are the B operand (up to 256 tokens, K-major, 128-byte
 // swizzle) exactly as TMA delivers them, half of the tokens in each CTA's shared memory.
 //
 // Why this split: per 128-row stage a CTA moves 8 KB of packed words in and out of shared memory and
@@ -30,8 +30,8 @@
 // (handover.cuh).  The sum is taken in pair order: results do not depend on timing.
 // The cut of a call (tokens of a tile, units of a range) is the one of the least estimated time
 // (wt_cost).  Against tiles of up to 256 tokens that were always split, and partial tiles read with plain
-// loads: 8192 x 1280 at M 250 38.5 -> 15.5 us, 8192 x 7424 at M 250 50 -> 30, at M 100 26.5 -> 21.3,
-// 1024 x 8192 at M 24 8.1 -> 5.1, 1792 x 1984 at M 100 17.9 -> 6.9.
+// loads: 8192 x 1280 at M 250 38.5 -> 14.4 us, 8192 x 7424 at M 250 50 -> 28, at M 100 26.5 -> 20.6,
+// 1024 x 8192 at M 24 8.1 -> 4.6, 1792 x 1984 at M 100 17.9 -> 6.4.
 //
 // MODE 0 is the dense linear.  MODE 1 / 2 are the grouped expert GEMMs of a fused-MoE layer over the
 // tile table that moe_gather_kernel wrote: entry (expert, first row, rows) of the permuted list.
@@ -41,7 +41,10 @@
 //           and what is rounded is the weighted row: D alone may lie outside the range of fp16.
 //
 // WIDE is the kernel of tiles with one accumulator, more than 128 tokens, that no pair shares: its epilogue goes
-// through shared memory (wt_epilogue_wide).
+// through shared memory (wt_epilogue_wide).  That is the faster way also where a pair has one tile and no next tile hides
+// its stores, though the ring of packed words is down from 12 stages to 4 at 256 tokens; from registers with 12 stages:
+// 8192 x 8192 at M 264 31.4 us against 31.2, 4096 x 11040 at M 150 18.3 / 18.0, 1024 x 8192 at M 264 9.4 / 9.1, M 394 on
+// 1024 x 5120 9.15 / 8.8; 25 shapes, none the other way round by more than its runs differ.
 //
 // TMEM columns: accumulators first (two of 64 or 128 tokens, one of 256), then A[slots][8 steps][8]: four
 // slots, six up to 64 tokens.  With as many slots as teams a team waits for the MMAs of its own last
@@ -50,10 +53,10 @@
 // All mbarrier and flag waits are bounded (tc_ptx.cuh).
 //
 // Measured (B200, K x N, against one CTA per tile with two A stages and 64 / 128 fixed tokens):
-//   8192 x 59136   M 100: 123.6 -> 99.8 us; 29568 x 8192   M 100: 70 -> 58 us; the four linears of a layer
-//   (8192 x 10240, 8192 x 8192, 8192 x 59136, 29568 x 8192) against weights dequantised into shared memory:
-//   M 1000 1694 -> 1443 us, M 4096 6522 -> 5794 (1.24 PFLOP/s in a long loop, where the 1 kW limit holds the
-//   clock near 1.2 GHz); router + experts, 128 experts of 2048 x 768, top-8, 2500 tokens: 507 -> 289 us.
+//   8192 x 59136   M 100: 123.6 -> 94.9 us (cool; 115 in a long loop); 29568 x 8192   M 100: 70 -> 54 us; the four linears
+//   of a layer (8192 x 10240, 8192 x 8192, 8192 x 59136, 29568 x 8192) against weights dequantised into shared memory:
+//   M 1000 1694 -> 1448 us, M 4096 6522 -> 5749 (1.25 PFLOP/s in a long loop, where the 1 kW limit holds the
+//   clock near 1.2 GHz); router + experts, 128 experts of 2048 x 768, top-8, 2500 tokens: 507 -> 282 us.
 // What bounds it: at M >= 256 the tensor pipe under the power limit; below, the conversion and, on the long layers,
 // the power limit.  A unit took 630 cycles at M = 24 and at M = 100, now ~510.  The arithmetic is 270 of them (sub and mul
 // of f16x2 take two cycles a warp and scheduler; a loop of the conversion alone runs at 300), but a conversion warp
@@ -517,7 +520,7 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   const int words = p.N / kPack;
 
   // Packed words, unit by unit: 128 rows x 16 words (MODE 1: 8 gate words and the matching 8 up
-  // words).  State of the raw producer's lane 0.
+  // words).  State of the raw producer's warp.
   int raw_u = 0, raw_seg = 0, raw_k = 0, raw_end = 0, raw_s = 0, raw_w0 = 0, raw_row0 = 0;
   uint32_t raw_phase = 0;
   auto load_raw = [&]() {  // returns whether the stage after this one is known to be empty
@@ -957,8 +960,10 @@ struct WtPlan {
 };
 
 // Estimated time in ns of `tiles` tiles of `nt` tokens and KT units on `pairs` pairs (chunk as above).
-// Fitted to 7 shapes between 1024 x 8192 and 4096 x 11040 at 14 batch sizes from 17 to 1000, 1500 cuts
-// in all; the cut it picks is 0.5 % from the best one of each on average, 7 % at worst.
+// Fitted to 7 shapes between 1024 x 8192 and 4096 x 11040 at 14 batch sizes from 17 to 1000, 1500 cuts in all, when a
+// unit took 630 cycles and the epilogue of one accumulator 6600.  On the present kernel the cut it picks is 0.9 % from
+// the best one on average, 15 % at worst (1735 cuts of 174 batches, 12 shapes up to 8192 x 59136, 17 to 1000 tokens; 1024 x
+// 8192 at 160 tokens takes tiles of 80, 8.3 us, where 160 take 7.3).
 //   2400 + 18 nt            start, and the epilogue that nothing hides
 //   units x max(...)        315: the conversion arithmetic; 2.5 nt: the tensor pipe; 4.9 pairs: the words'
 //                           way from HBM through L2

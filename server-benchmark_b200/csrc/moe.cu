@@ -717,13 +717,14 @@ int launch_moe_align(const int32_t* topk_ids, int numel, int E, int block,
 }
 
 // Row block of the permutation.  128, the grouped tiles of gemm_wt.cu, from 36 rows per expert on average if
-// the shapes fit them.  They win from about 17 rows (128 experts of 2048 x 768, top-8: 128 against 146 us at
-// 20 rows, 135 against 204 at 35; 64 of 4096 x 1536, top-4: 222 against 319 at 32), but round (q - z) * s to
+// the shapes fit them.  They win from about 17 rows (128 experts of 2048 x 768, top-8: 117 against 132 us at
+// 20 rows, 130 against 202 at 35; 64 of 4096 x 1536, top-4: 234 against 326 at 32), but round (q - z) * s to
 // fp16, which the kernels of smaller blocks do not (error of the layer against 64 bits 5.0e-4 and 3.6e-4):
 // fewer rows stay with those.  8 up to eight rows per expert on average, else 16.  Blocks of 8 / 16, us, at 5, 6,
-// 7 and 8 rows: groups of 64, 128 experts 113 / 138, 118 / 138, 120 / 138, 132 / 138; 64 experts 193 / 244, 202 /
-// 245, 212 / 245, 239 / 248.  Groups of 128 (gemm_ts) cross at six: 83 / 89, 83 / 89, 94 / 89, 102 / 90; 134 /
-// 143, 145 / 143, 163 / 143, 180 / 144.  One limit for all groups, which callers of the C ABI see.
+// 7 and 8 rows: groups of 64, 128 experts 113 / 133, 112 / 133, 116 / 134, 127 / 133; 64 experts 189 / 241, 190 /
+// 241, 208 / 241, 231 / 242.  Groups of 128 (gemm_ts) cross between six and seven: 75 / 80, 76 / 81, 82 / 80, 92 / 82; 123 /
+// 142, 144 / 143, 162 / 147, 194 / 153.  The limit is that of groups of 64; one by group, which would serve groups of 128
+// at seven and eight rows, has not been made.
 int moe_block_size(int T, int topk, int E, int H, int I, int group) {
   const long long pairs = (long long)T * topk;
   if (pairs >= 36LL * E && moe_tc_supported(H, I, group)) return 128;
