@@ -35,27 +35,20 @@ int check_awq_shape(int N, int K, int group) {
 
 // Kernel choice for AWQ_B200_KERNEL_AUTO (measured crossovers on B200, Qwen2.5-72B shapes and their
 // tensor-parallel shards):
-//   M <= 16     unpacked weights in TMEM, zero point and scale applied to the accumulators (gemm_ts),
-//               groups of 128 and 64: faster than the mma.sync streaming kernel on every layer, 4.9
-//               against 7.6 us on K 1024 x N 8192 up to 45 against 56 us on K 8192 x N 59136.  Without the
-//               scratch it asks for it distributes whole slabs, and the streaming kernel's cluster split
-//               is the better one.
-//   M <= 32     groups of 64 and 32: kernels that apply the scales in fp32 (gemm_wt rounds (q - z) * s to
-//               fp16: error against 64 bits 2.9e-4 instead of 2.1e-4).  Groups of 64: gemm_ts, 16 rows of x
-//               at a time: M 24 12.5 (streaming kernel) and 12.6 us on K 2048 x N 5120, 25.1 -> 21.2 on
-//               4096 x 11040, 168 -> 113 on 8192 x 59136.  (gemm_wt: 7.4, 15.3, 77.)
+//   M <= 32     unpacked weights in TMEM, scales applied to the accumulators in fp32 (gemm_ts), groups of 128 and 64:
+//               faster than the mma.sync streaming kernel on every layer, 3.4 against 7.6 us on K 1024 x N 8192 up to 45
+//               against 56 us on K 8192 x N 59136 at M <= 16, and than gemm_wt, which also rounds (q - z) * s to fp16:
+//               M 24 on 1024 x 8192 4.6 -> 4.5 us, 2048 x 5120 6.9 -> 5.2, 8192 x 1280 9.9 -> 5.9, 8192 x 59136 76 -> 53.
+//               Without the scratch it asks for it may distribute whole slabs, and the streaming kernel's cluster split
+//               (groups of 128 above 16 rows: gemm_wt) is the better one.
 //   larger M    dequantised weights in TMEM, tiles of CTA pairs (gemm_wt): faster than weights
 //               dequantised into shared memory (gemm_tc) at every M measured, 128 to 4096, which is
 //               left with K that is not a multiple of 128
-constexpr int kTsRows = 16;  // of one gemm_ts launch
+constexpr int kTsNamedRows = 16;  // limit of a call that names gemm_ts
 int pick_gemm_kernel(int M, int N, int K, int group, bool scratch) {
-  if (M <= 16) {
-    const bool stream = awq::gemm_stream_supported(M, N, K, group);
-    if (awq::gemm_ts_supported(M, N, K, group) && (scratch || !stream)) return AWQ_B200_KERNEL_TS;
-    if (stream) return AWQ_B200_KERNEL_STREAM;
-  }
-  if (M <= 32 && group != 128 && awq::gemm_stream_supported(M, N, K, group))
-    return scratch && awq::gemm_ts_supported(kTsRows, N, K, group) ? AWQ_B200_KERNEL_TS : AWQ_B200_KERNEL_STREAM;
+  const bool stream = M <= (group == 128 ? 16 : 32) && awq::gemm_stream_supported(M, N, K, group);
+  if (awq::gemm_ts_supported(M, N, K, group) && (scratch || (M <= 16 && !stream))) return AWQ_B200_KERNEL_TS;
+  if (stream) return AWQ_B200_KERNEL_STREAM;
   if (awq::gemm_wt_supported(M, N, K, group)) return AWQ_B200_KERNEL_WT;
   if (awq::gemm_tc_supported(M, N, K, group)) return AWQ_B200_KERNEL_TCGEN05;
   return AWQ_B200_KERNEL_GENERIC;
@@ -145,7 +138,7 @@ size_t awq_b200_gemm_workspace_bytes(int M, int N, int K, int group, int kernel)
   if (automatic) kernel = pick_gemm_kernel(M, N, K, group, true);
   if (kernel == AWQ_B200_KERNEL_TCGEN05) return awq::gemm_tc_workspace_bytes(M, N, K, group);
   if (kernel == AWQ_B200_KERNEL_TS)
-    return awq::gemm_ts_workspace_bytes(automatic && M > kTsRows ? kTsRows : M, N, K, group);
+    return automatic || M <= kTsNamedRows ? awq::gemm_ts_workspace_bytes(M, N, K, group) : 0;
   if (kernel == AWQ_B200_KERNEL_WT) return awq::gemm_wt_workspace_bytes(M, N, K, group);
   return 0;
 }
@@ -193,17 +186,10 @@ int awq_b200_gemm(const void* x, const void* qweight, const void* scales, const 
       return awq::launch_gemm_stream(xh, qw, sc, qz, bh, oh, M, N, K, group,
                                      kernel == AWQ_B200_KERNEL_STREAM_EXACT, st);
     case AWQ_B200_KERNEL_TS:
-      if (!awq::gemm_ts_supported(automatic && M > kTsRows ? kTsRows : M, N, K, group))
-        return AWQ_B200_ERR_SHAPE;
+      if (!awq::gemm_ts_supported(M, N, K, group) || (!automatic && M > kTsNamedRows)) return AWQ_B200_ERR_SHAPE;
       // scratch is optional here: without it (or misaligned) whole slabs are distributed
       if ((reinterpret_cast<uintptr_t>(workspace) & 255u) != 0) workspace = nullptr;
-      for (int m = 0; m < M; m += kTsRows) {
-        const int rows = M - m < kTsRows ? M - m : kTsRows;
-        if (int rc = awq::launch_gemm_ts(xh + (size_t)m * K, qw, sc, qz, bh, oh + (size_t)m * N, rows, N, K,
-                                         group, workspace, workspace_bytes, st))
-          return rc;
-      }
-      return AWQ_B200_OK;
+      return awq::launch_gemm_ts(xh, qw, sc, qz, bh, oh, M, N, K, group, workspace, workspace_bytes, st);
     case AWQ_B200_KERNEL_TS_EXACT:
       // the magic-number conversion has one home, the streaming kernel
       if (M > 16 || !awq::gemm_ts_supported(M, N, K, group)) return AWQ_B200_ERR_SHAPE;

@@ -35,10 +35,11 @@ inline bool pdl_enabled() {
 // this runs in waves.  `cache` holds one answer per size (0 = not asked yet); an answer the
 // runtime cannot give counts as "enough".  The kernel's dynamic shared-memory limit must have
 // been raised before the first call.
+constexpr int kMaxCluster = 16;  // above 8 only kernels that allow it (a function attribute)
 template <typename Kernel>
 inline int resident_clusters(Kernel kernel, int S, int threads, size_t smem,
                              std::atomic<int>* cache) {
-  if (S < 1 || S > 8) return 1 << 30;
+  if (S < 1 || S > kMaxCluster) return 1 << 30;
   const int known = cache[S];
   if (known > 0) return known;
   cudaLaunchConfig_t cfg = {};
@@ -199,6 +200,7 @@ int launch_gemm_stream_rp(const __half* x, const uint32_t* qweight_rp, const __h
                           int K, int group, cudaStream_t stream);
 int launch_repack_qweight(const uint32_t* qweight, uint32_t* out, int K, int N,
                           cudaStream_t stream);
+constexpr int kTsMaxRows = 32;
 bool gemm_ts_supported(int M, int N, int K, int group);
 size_t gemm_ts_workspace_bytes(int M, int N, int K, int group);
 int launch_gemm_ts(const __half* x, const uint32_t* qweight, const __half* scales,

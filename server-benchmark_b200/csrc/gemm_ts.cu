@@ -1,4 +1,4 @@
-// Decode-size AWQ GEMM (M <= 16) on tcgen05 with the weights going registers -> TMEM.
+// Decode-size AWQ GEMM (M <= 32) on tcgen05 with the weights going registers -> TMEM.
 //
 //   D[n, m] = sum_k W[k, n] * x[m, k]          (the transposed product, as in stream_core.cuh)
 //
@@ -8,22 +8,44 @@
 // tcgen05.mma.kind::f16; the activations are the small B operand as TMA delivers them.  No arithmetic
 // is spent on a weight: zero point and scale are applied per quantisation group to the fp32
 // accumulators,  tot += scale * (acc - zero * sum_k x).
+// SUB forms subtract the zero point in the conversion (q - z is exact in the subnormals too) and need no token sums:
+// tot += scale * acc.  That costs the conversion 128 instructions a unit and scheduler, on the FMA pipe, and saves the
+// warp that sums tokens, whose chain of loads and mma.sync took 700 to 1200 cycles a unit and was the slowest role from
+// 16 tokens on, and half of the fold.  M 32 on 8192 x 59136: with token sums 74 us, with SUB and its second issuing warp
+// 56; M 16, groups of 64: 56.0 -> 50.5.  At M <= 16 and groups of 128 long layers keep the sums (SUB: 41.4 -> 43.6 us at
+// M 1, 47.4 -> 48.2 at 16), short ones go to clusters (below), which gain from a shorter chain: 2048 x 5120 at M 1 5.24 ->
+// 4.73 us from SUB alone.
 //
 // One CTA per SM; slab of 256 output columns = two A tiles of 128 lanes; unit = 128 weight rows = one
 // quantisation group (groups of 64: two, with accumulators and sums of their own): 16 KB of packed words,
 // 512 B of scales and 128 B of zero points per group, all by TMA.  The
 // (slab, unit) list is cut into one range per CTA and shared slabs are handed over (handover.cuh).
+// SPLIT is the form of short layers: a cluster of 2 to 16 CTAs shares each slab, and its sums go from CTA to CTA through
+// shared memory.  A CTA sums its share of the (32 columns, half of the tokens) pieces: every other CTA stores its
+// part of one there with st.async, counted by an mbarrier, and all warps that have nothing left to do add them up in the
+// CTAs' order.  A partial slab through global scratch costs its stores, a release, an acquire and the loads, 1.5 us at one
+// token and 4 to 8 at 32; this 0.8 us.  The barrier at the end is a relaxed one: as a release it waited 1000 cycles
+// for the stores of the output.  (Bulk copies between shared memories instead of st.async: 0.1 us slower.)
+//   us, ranges -> clusters (CTAs)   M 1                   M 16                  M 24 (ranges: gemm_wt)
+//   1024 x 8192                      4.6 -> 3.4 (2)        5.1 -> 3.8            4.6 -> 4.5
+//   2048 x 5120                      5.2 -> 4.1 (3)        6.6 -> 4.5            6.9 -> 5.2
+//   8192 x 1280                      6.2 -> 4.8 (16)       9.1 -> 5.3            9.9 -> 5.9
+//   8192 x 7424                     10.1 -> 10.1 (4)      12.0 -> 10.6          15.8 -> 11.4
+//   3712 x 8192                      6.9 -> 7.2 (3)        8.4 -> 7.7 (3)       11.0 -> 8.2 (4)
+// What is left of 1024 x 8192 at M 1, in cycles from the end of the kernel before: 860 the tokens' way through L2, 1400
+// the MMAs of four units (22 each), 350 the last fold, 900 the cluster's sum, 450 the exit.
 //
 // Warp roles (768 threads), joined by mbarrier rings:
 //   12      conversion   warp (q, team): chunk of 32 columns q of both tiles, units u = team (mod 3);
 //                        A slot = team                             raw_full -> unit_full, raw_empty
 //   8       fold         warp (q, tile): tcgen05.ld of the unit's sums, fold into registers; the
 //                        epilogue at the end of a segment          mma_done -> unit_full
-//   1       MMA issue    converged warp, elected lane              unit_full -> mma_done
-//   1       sums         sum_k x of every token with mma.sync against a constant operand
+//   1       MMA issue    converged warp, elected lane (SUB: two, units in turn)
 //                                                                  unit_full -> mma_done
-//   1       TMA          tokens; zero points but in MODE 1         mma_done -> unit_full
-//   1       TMA          packed words, scales; zero points in MODE 1
+//   1       sums         sum_k x of every token with mma.sync against a constant operand (not SUB)
+//                                                                  unit_full -> mma_done
+//   1       TMA          tokens; zero points but in MODE 1 and SUB mma_done -> unit_full
+//   1       TMA          packed words, scales; zero points in MODE 1 and SUB
 //                                                                  raw_empty -> raw_full
 // MODE 0 is the dense linear.  The other modes are the expert GEMMs of a fused-MoE layer with few rows
 // per expert; a tile is (row block, slab) and a block's rows belong to one expert:
@@ -37,7 +59,7 @@
 //           (negative id) gets a row of zeros.
 //
 // unit_full counts the conversion warps, the announcement of the tokens and the fold warps of the unit
-// four before, whose accumulators the MMAs overwrite.  mma_done counts the MMA warp's commit and the
+// NDB before, whose accumulators the MMAs overwrite.  mma_done counts the MMA warp's commit and the
 // sums warp: it frees the x stage and the A slot and hands accumulators and sums to the fold warps.
 //
 // Shared-memory rings without a barrier of their own: scales / zero points and token sums have 16
@@ -45,7 +67,7 @@
 // (the raw ring), which needs the MMAs of three units before, which need the folds of up to four before
 // that: unit u has long been folded.
 //
-// TMEM columns: D[4 buffers][2 tiles][16] at 0 .. 127, A[3 slots][2 tiles][8 steps][8] at 128 .. 511.
+// TMEM columns: D[buffers][2 tiles][16 or 32 tokens] at 0 .. 127, A[3 slots][2 tiles][8 steps][8] at 128 .. 511.
 // Lane 32 q + 8 i + g of tile t holds column
 // 128 t + 32 q + 8 (g / 2) + 2 i + g % 2 of the slab.  Every wait is bounded (tc_ptx.cuh).
 //
@@ -56,12 +78,14 @@
 //   29568 x 8192   M 4: 35.0 (30.2) -> 24.7 us                        M 16: 40.0 (43.7) -> 27.3 us
 //   8192 x 10240   M 4: 17.2 (16.0) -> 11.9 us                        M 16: 20.0 (22.9) -> 13.3 us
 //   1024 x 8192    M 1: 7.6 -> 4.6 us
-//   groups of 64 (before: mma.sync streaming kernel)
-//   8192 x 59136   M 4: 69.2 -> 43.2 us, M 16: 106.8 -> 59.7;  8192 x 1280   M 4: 11.1 -> 6.4 us
+//   M 24 and 32 (before: gemm_wt): 8192 x 59136 76 -> 53 and 76 -> 56 us; 29568 x 8192 M 32 41 -> 36
+//   groups of 64 (before: mma.sync streaming kernel; M 24: two calls of 16 rows)
+//   8192 x 59136   M 4: 69.2 -> 43.2 us, M 16: 106.8 -> 50.5, M 24: 113 -> 78;  4096 x 11040  M 20: 19.6 -> 13.2
 // The instructions of the some 36 waits a unit takes are a fifth of all, so a wait for a complete phase is one probe,
 // one vote and one branch (mbar_wait_warp): 8192 x 59136 at M 8 55.4 -> 53.3 us, 8192 x 10240 groups of 64 at M 8 13.27
 // -> 13.07, experts of 128 x 2048 x 768 at 64 tokens 83.2 -> 80.6 (that step alone; the fold warps differ, see there).
-// Tried and taken back: a team per half unit, with two
+// Tried and taken back: 16 fold warps of 16 tokens each for M 32 (64 registers a thread: 56 -> 64 us); two warps for the
+// token sums, or sums in four chains (nothing, or 1 % slower on short layers); a team per half unit, with two
 // halves of A slots each (the conversion warps then get in each other's way, 55 -> 59 us at M 16); all MMAs of a unit in
 // one asm block, predicated arrivals (no difference); the sum over a token's slots by the warp that stores the last
 // of its rows (fences and counters at the end of every tile: 80 -> 99 us at 64 tokens, 16.4 -> 17.0 at one).
@@ -89,32 +113,44 @@ constexpr int kTsSzRing = 16;
 constexpr int kTsUnits = 8;                            // x stages, unit barriers
 constexpr int kTsTmemCols = 512;
 
-// MT: tokens (4, 8, 16).
-constexpr int kTsNT = 16;                              // tokens of the B operand
-constexpr int kTsXBytes = kTsNT * kTsBK * 2;
+// MT: tokens (4, 8, 16, 32).
 constexpr int kTsTeams = 3;                            // sets of four conversion warps = A slots
-constexpr int kTsNDB = 4;                              // accumulator buffers, one per group
-constexpr int kTsCvWarps = 4 * kTsTeams, kTsFoldWarps = 8;
-constexpr int kTsFold0 = kTsCvWarps, kTsIssue = kTsFold0 + kTsFoldWarps;
-constexpr int kTsSum = kTsIssue + 1, kTsX = kTsSum + 1, kTsRaw = kTsX + 1;
-constexpr int kTsThreads = 32 * (kTsRaw + 1);          // 768
-constexpr int kTsColA = kTsNDB * 2 * kTsNT;
-// What depends on the quantisation group (128 or 64: one or two of a unit).
-template <int GROUP>
-struct TsGroup {
+constexpr int kTsColD = 128;                           // TMEM columns of the accumulators
+constexpr int kTsCvWarps = 4 * kTsTeams;
+static_assert(kTsColD + kTsTeams * 128 <= kTsTmemCols, "TMEM columns");
+// What depends on the quantisation group (128 or 64: one or two of a unit) and on the tokens.
+template <int MT, int GROUP, bool SPLIT = false>
+struct TsCfg {
   static constexpr int G = kTsBK / GROUP;              // groups of a unit
-  // Stages of packed words.  With 8 another team waits for a stage's next filling than read the last one;
-  // it cannot pass on the last one's parity, for it has seen the MMAs of two units later complete.
-  static constexpr int NRAW = G == 1 ? 9 : 8;
-  static constexpr int NDB = kTsNDB / G;               // units with accumulators of their own
+  static constexpr int NT = MT <= 16 ? 16 : 32;        // tokens of the B operand
+  static constexpr int kFoldWarps = 8;
+  static constexpr int kFold0 = kTsCvWarps, kIssue = kFold0 + kFoldWarps;
+  // the conversion subtracts the zero points: no token sums
+  static constexpr bool SUB = SPLIT || MT > 16 || (MT == 16 && GROUP == 64);
+  static constexpr int kIssueWarps = SUB ? 2 : 1;
+  static constexpr int kSum = kIssue + kIssueWarps, kXWarp = kSum + (SUB ? 0 : 1), kRaw = kXWarp + 1;
+  static constexpr int kThreads = 32 * (kRaw + 1);     // 768
+  static constexpr int kX = NT * kTsBK * 2;            // bytes of an x stage
+  // Stages of packed words.  A team must know that a stage's last filling has landed when it waits for the next one,
+  // or the parity of the filling before that could pass for it: it read the last one itself (a multiple of the teams), or
+  // has seen the MMAs of unit u - 6 complete, which had to wait for the folds up to unit u - 6 - NDB.
+  static constexpr int NRAW = SPLIT && MT > 16 ? 6 : G == 1 ? 9 : MT <= 16 ? 8 : 7;
+  static constexpr int NDB = kTsColD / (2 * G * NT);   // units with accumulators of their own
   static constexpr int kScales = G * kTsScaleBytes, kZeros = G * kTsZeroBytes;
   static constexpr int kSz = kScales + kZeros;         // scales, zero words
-  static constexpr int kSums = G * kTsNT * 4;
-  static constexpr int kSmem = 1024 + NRAW * kTsRawBytes + kTsUnits * kTsXBytes + kTsSzRing * (kSz + kSums) + 512;
-  static_assert(kSmem + kTsFoldWarps * 16 * 32 * 4 <= 232448 - 512, "shared memory");
+  static constexpr int kSums = SUB ? 0 : G * NT * 4;
+  // SPLIT: a fold warp's sums leave in pieces of up to half of the tokens, each summed by one CTA of the cluster
+  static constexpr int kHalves = MT >= 8 ? 2 : 1, kPieceTokens = MT / kHalves, kPieces = 8 * kHalves;
+  static constexpr int kPieceBytes = kPieceTokens * 32 * 4;
+  static constexpr int kRecvPieces = 20;  // (pieces that a CTA sums) x (CTAs of the cluster), at most
+  static constexpr int kRecv = SPLIT ? kRecvPieces * kPieceBytes : 0;
+  static constexpr int kSmem = 1024 + NRAW * kTsRawBytes + kTsUnits * kX + kTsSzRing * (kSz + kSums) + 512 + kRecv;
+  // MODE 1 parks the gate sums of 16 tokens at most in static shared memory
+  static_assert(kSmem + (MT <= 16 ? kFoldWarps * 16 * 32 * 4 : 0) <= 232448 - 512, "shared memory");
+  static_assert(8 * (2 * NRAW + 2 * kTsUnits + kPieces / 2) <= 512, "barriers");
+  static_assert(NRAW % kTsTeams == 0 || NRAW >= 2 * kTsTeams + NDB, "a stage's parity");
   static_assert(kTsSzRing >= NRAW + kTsTeams + NDB, "scale / sum ring too short");
 };
-static_assert(kTsColA + kTsTeams * 128 <= kTsTmemCols, "TMEM columns");
 
 struct TsParams {
   const __half* bias;
@@ -127,6 +163,7 @@ struct TsParams {
   const int32_t* num_post;     // permuted rows in use
   const float* topk_weights;
   int numel, topk, half_cols;
+  int split;                   // SPLIT: CTAs of a cluster
   int max_split;               // CTAs a tile is split over at most, about
   float* partial;          // [CTA][MT][256] partial tiles handed over (MODE 1: gate and up, [CTA][2])
   handover::Flags flags;
@@ -160,6 +197,16 @@ __device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t (&r)[4]) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                : "r"(addr)
+               : "memory");
+}
+// Four values into another CTA's shared memory, counted by a barrier there.
+__device__ __forceinline__ void st_async_v4(uint32_t dst, const float* v, uint32_t bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(dst),
+               "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void sts_float4(uint32_t addr, const float* v) {
+  asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3])
                : "memory");
 }
 template <int N>
@@ -241,13 +288,16 @@ struct TsWalk {
   __device__ __forceinline__ int column() const { return slab * kTsBN + (up() ? p.half_cols : 0); }
 };
 
-template <int MT, int MODE, int GROUP>
-__global__ void __launch_bounds__(kTsThreads, 1)
+template <int MT, int MODE, int GROUP, bool SPLIT>
+__global__ void __launch_bounds__((TsCfg<MT, GROUP, SPLIT>::kThreads), 1)
 gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_s,
                const __grid_constant__ CUtensorMap map_z, const __grid_constant__ CUtensorMap map_x,
                const TsParams p) {
-  using Cfg = TsGroup<GROUP>;
-  constexpr int NT = kTsNT, G = Cfg::G, NDB = Cfg::NDB, NRAW = Cfg::NRAW, kSz = Cfg::kSz;
+  using Cfg = TsCfg<MT, GROUP, SPLIT>;
+  constexpr int NT = Cfg::NT, G = Cfg::G, NDB = Cfg::NDB, NRAW = Cfg::NRAW, kSz = Cfg::kSz, kTsXBytes = Cfg::kX;
+  constexpr int kTsFoldWarps = Cfg::kFoldWarps, kTsFold0 = Cfg::kFold0, kTsIssue = Cfg::kIssue, kIssueWarps = Cfg::kIssueWarps;
+  constexpr bool SUB = Cfg::SUB, kRawZeros = MODE == 1 || SUB;  // zero points with the packed words
+  constexpr int kTsSum = Cfg::kSum, kTsX = Cfg::kXWarp, kTsRaw = Cfg::kRaw;
   constexpr int kScales = Cfg::kScales, kZeros = Cfg::kZeros, kSums = Cfg::kSums;
   extern __shared__ uint8_t smem_raw[];
   __shared__ volatile int s_abort;
@@ -272,7 +322,16 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   // every CTA here knows that the kernels that wrote the tables are complete.
   if (MODE == 1) pdl_wait();
   pdl_launch_dependents();
-  const Work work = ts_work<MT, MODE>(p);
+  const int rank = SPLIT ? blockIdx.x % p.split : 0;
+  const Work work = SPLIT ? Work::part(blockIdx.x / p.split, rank * p.KT / p.split, (rank + 1) * p.KT / p.split, p.KT)
+                          : ts_work<MT, MODE>(p);
+  // SPLIT: barrier and shared memory of the n-th piece that this CTA sums, partial sums of CTA `from`
+  auto recv_full = [&](int n) { return bar_base + 8 * (2 * NRAW + 2 * kTsUnits + n); };
+  auto recv_at = [&](int n, int from) { return bar_base + 512 + (n * p.split + from) * Cfg::kPieceBytes; };
+  // quads of tokens of a piece that the call has
+  auto piece_quads = [&](int half) {
+    return min(Cfg::kPieceTokens / 4, max(0, (p.M - half * Cfg::kPieceTokens + 3) / 4));
+  };
 
   // packed words, scales, MODE 1 also zero points (raw warp, converged: an elected lane issues; TMAs
   // of a lane that loops alone take it longer)
@@ -286,10 +345,10 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     const int column = raw.column(), row = raw.expert * p.K + raw.unit() * kTsBK;
     const int grp = (raw.expert * p.KT + raw.unit()) * G;
     if (elect_one()) {
-      mbar_arrive_expect_tx(bar, kTsRawBytes + kScales + (MODE == 1 ? kZeros : 0));
+      mbar_arrive_expect_tx(bar, kTsRawBytes + kScales + (kRawZeros ? kZeros : 0));
       tma_load_2d(dst, &map_w, column / kPack, row, bar);
       tma_load_2d(sz, &map_s, column, grp, bar);
-      if (MODE == 1) tma_load_2d(sz + kScales, &map_z, column / kPack, grp, bar);
+      if (kRawZeros) tma_load_2d(sz + kScales, &map_z, column / kPack, grp, bar);
     }
     raw.next();
     if (++raw_s == NRAW) {
@@ -315,8 +374,14 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     if (lane < kTsUnits) {
       // conversion warps, announcement of the tokens, fold warps (none before unit NDB)
       mbar_init(unit_full(lane), 4 + 1 + kTsFoldWarps);
-      mbar_init(mma_done(lane), 2);  // commit, sums warp
+      mbar_init(mma_done(lane), SUB ? 1 : 2);  // commit, sums warp
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (SPLIT && lane * p.split + rank < Cfg::kPieces) {  // piece lane * split + rank is this CTA's
+      const int quads = piece_quads((lane * p.split + rank) / 8);
+      mbar_init(recv_full(lane), 2);  // the bytes of the other CTAs, the warp here that has the piece
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      mbar_arrive_expect_tx(recv_full(lane), (p.split - 1) * quads * 512);
     }
   }
   __syncwarp();
@@ -330,6 +395,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  if (SPLIT) cluster_arrive();  // awaited ahead of the first store into another CTA
   const uint32_t tmem = s_tmem_base;
 
   if (warp == kTsRaw) {
@@ -384,9 +450,9 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 tma_gather4(dst + h * (kTsXBytes / 2) + m * 128, &map_x, unit * kTsBK + h * 64, rows[m],
                             rows[m + 1], rows[m + 2], rows[m + 3], bar);
         } else {
-          mbar_arrive_expect_tx(bar, (MODE == 1 ? 0 : kZeros) + kTsXBytes);
+          mbar_arrive_expect_tx(bar, (kRawZeros ? 0 : kZeros) + kTsXBytes);
           tma_load_3d(dst, &map_x, 0, row, 2 * unit, bar);
-          if (MODE != 1) tma_load_2d(zdst, &map_z, zcol, zrow, bar);
+          if (!kRawZeros) tma_load_2d(zdst, &map_z, zcol, zrow, bar);
         }
       }
       __syncwarp();
@@ -396,7 +462,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     // them land before the CTA may exit.
     for (int u = work.count > kTsUnits ? work.count - kTsUnits : 0; u < work.count && ok; ++u)
       ok = mbar_wait(mma_done(u), unit_phase(u), &s_abort, 22);
-  } else if (warp == kTsSum) {
+  } else if (!SUB && warp == kTsSum) {
     // ------------------------------------------------------------------ token sums
     // x tile as the A operand of mma.sync (16 tokens x 16 k), every B element 2^-24: each column of
     // the result is 2^-24 * sum_k x, in the scaling of the weight tiles' accumulators
@@ -425,18 +491,19 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       __syncwarp();
       if (lane == 0) mbar_arrive(mma_done(u));
     }
-  } else if (warp == kTsIssue) {
+  } else if (warp >= kTsIssue && warp < kTsIssue + kIssueWarps) {
     // ------------------------------------------------------------------ MMA issue
-    // One barrier per unit, the next unit's probed under this one's MMAs (a second issuing warp, one
-    // per tile, made it slower: 54 against 50 us on K 8192 x N 59136, M = 16).  D fp32, A / B fp16,
+    // One barrier per unit, the next unit's probed under this one's MMAs.  SUB: two warps issue units in turn, so that
+    // one's wait and loop run under the other's MMAs (M 32 on 8192 x 59136: 66.6 -> 64.4 us, with 16 fold warps then).  (A
+    // second issuing warp, one per tile, made it slower: 54 against 50 us at M = 16.)  D fp32, A / B fp16,
     // both K-major, N = NT tokens, M = 128 columns.
     constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(NT >> 3) << 17) | (8u << 24);
     constexpr uint32_t half = NT * 128 / 16;
     const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem, 0);
     const uint64_t desc0 = make_desc(__shfl_sync(0xffffffffu, x_base, 0), 16, 1024);
     bool ok = true, ready = false;
-    int slot = 0;
-    for (int u = 0; u < work.count; ++u) {
+    int slot = warp - kTsIssue;
+    for (int u = slot; u < work.count; u += kIssueWarps) {
       if (!ready) {
         ok = mbar_wait_warp(unit_full(u), unit_phase(u), &s_abort, 24);
         if (!ok) break;
@@ -444,10 +511,10 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       tc_fence_after();
       const uint64_t dx = desc0 + (uint32_t)(u & (kTsUnits - 1)) * (kTsXBytes / 16);
       const uint32_t dcol = tmem_u + (uint32_t)(u & (NDB - 1)) * (G * 2 * NT);
-      const uint32_t acol = tmem_u + kTsColA + slot * 128;
+      const uint32_t acol = tmem_u + kTsColD + slot * 128;
       bool r = false;
       if (elect_one()) {
-        r = mbar_test(unit_full(u + 1), unit_phase(u + 1));
+        r = mbar_test(unit_full(u + kIssueWarps), unit_phase(u + kIssueWarps));
 #pragma unroll
         for (int step = 0; step < 8; ++step) {
           const uint64_t db = dx + (step >> 2) * half + (step & 3) * 2;
@@ -457,7 +524,8 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         }
         umma_commit(mma_done(u));
       }
-      if (++slot == kTsTeams) slot = 0;
+      slot += kIssueWarps;
+      if (slot >= kTsTeams) slot -= kTsTeams;
       ready = __any_sync(0xffffffffu, r);
     }
   } else if (warp < kTsCvWarps) {
@@ -469,6 +537,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       // thread (g, t) has rows 2 t and 2 t + 1 of halfword column g in a register of each.  Rows of 128 B,
       // 16-byte chunk c at position c ^ (row % 8).
       const uint32_t off0 = (uint32_t)(lane * 128 + ((q ^ (lane & 7)) << 4));
+      const uint32_t z_addr = sz_base + kScales + (uint32_t)(4 * q + (lane >> 3)) * 4;
       const uint32_t off1 = (uint32_t)(lane * 128 + (((q + 4) ^ (lane & 7)) << 4));
       bool ok = true;
       int s = team;
@@ -477,7 +546,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         ok = mbar_wait_warp(raw_full(s), phase, &s_abort, 26);
         if (!ok) break;
         const uint32_t raw = raw_base + s * kTsRawBytes;
-        const uint32_t a_slot = tmem + lane_q + kTsColA + team * 128;
+        const uint32_t a_slot = tmem + lane_q + kTsColD + team * 128;
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
           uint32_t w[4][4];
@@ -490,6 +559,18 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             if (!ok) break;
             tc_fence_after();
           }
+          uint32_t zz[SUB ? G : 1][4];  // SUB: zero points of this lane's four columns, in place like the weights
+          if constexpr (SUB) {
+#pragma unroll
+            for (int gi = 0; gi < G; ++gi) {
+              const uint32_t zw = lds32(z_addr + (u & (kTsSzRing - 1)) * kSz + gi * kTsZeroBytes + t * (kTsZeroBytes / 2));
+              const uint32_t z2 = prmt(zw, zw, (lane & 4) ? 0x3232u : 0x1010u), zh = z2 >> 8;
+              zz[gi][0] = z2 & 0x000F000Fu;
+              zz[gi][1] = z2 & 0x00F000F0u;
+              zz[gi][2] = zh & 0x000F000Fu;
+              zz[gi][3] = zh & 0x00F000F0u;
+            }
+          }
 #pragma unroll
           for (int h = 0; h < 2; ++h) {  // 64 rows each, eight by eight
             // Logic and shifts take two cycles a warp and scheduler: 320 of them a unit are what
@@ -501,8 +582,11 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
               const uint32_t r = w[2 * h + (c >> 2)][c & 3], rh = r >> 8;
 #pragma unroll
               for (int i = 0; i < 4; ++i)
-                frag[i >> 1][2 * c + (i & 1)] =
-                    ((i & 2) ? rh : r) & ((i & 1) ? 0x00F000F0u : 0x000F000Fu);
+              {
+                uint32_t v = ((i & 2) ? rh : r) & ((i & 1) ? 0x00F000F0u : 0x000F000Fu);
+                if constexpr (SUB) v = as_u32(__hsub2(as_half2(v), as_half2(zz[h * G / 2][i])));
+                frag[i >> 1][2 * c + (i & 1)] = v;
+              }
             }
             tmem_st_16x128b(a_slot + t * 64 + h * 32, frag[0]);
             tmem_st_16x128b(a_slot + (16u << 16) + t * 64 + h * 32, frag[1]);
@@ -594,33 +678,57 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         tc_fence_after();
         const uint32_t dcol = d_addr + (uint32_t)(u & (NDB - 1)) * (G * 2 * NT);
         const uint32_t ring = (uint32_t)(u & (kTsSzRing - 1));
-        uint32_t d[G][MT];
-        uint64_t sc2[G], nz2[G];
-#pragma unroll
-        for (int h = 0; h < G; ++h) {
-          tmem_ld<MT>(dcol + h * 2 * NT, d[h]);
+        // scale of this lane's column in a group
+        auto scale = [&](int h) {
           uint16_t sh;
           asm volatile("ld.shared.u16 %0, [%1];" : "=h"(sh) : "r"(s_addr + ring * kSz + h * kTsScaleBytes));
-          const uint32_t zw = lds32(z_addr + ring * kSz + h * kTsZeroBytes);
           const float sc = __half2float(__ushort_as_half(sh));
-          const float nz = fmaf(__uint_as_float(((zw >> z_shift) & 0xFu) | 0x4B000000u), zf, zc);
-          sc2[h] = pack2(sc, sc);
-          nz2[h] = pack2(nz, nz);
-        }
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(unit_full(u + NDB));
+          return pack2(sc, sc);
+        };
+        auto release = [&]() {  // the accumulators are in registers
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(unit_full(u + NDB));
+        };
+        if constexpr (SUB) {  // sixteen tokens of a group at a time
+          constexpr int LD = MT <= 16 ? MT : 16;
 #pragma unroll
-        for (int h = 0; h < G; ++h) {
-          const uint32_t sx = sx_base + ring * kSums + h * (NT * 4);
+          for (int h = 0; h < G; ++h) {
+            const uint64_t sc2 = scale(h);
 #pragma unroll
-          for (int m = 0; m < MT; m += 4) {
-            uint64_t x01, x23;
-            lds_2x64(sx + m * 4, x01, x23);
-            tot[m / 2] = fma2(sc2[h], fma2(nz2[h], x01, pack2(d[h][m], d[h][m + 1])), tot[m / 2]);
-            tot[m / 2 + 1] =
-                fma2(sc2[h], fma2(nz2[h], x23, pack2(d[h][m + 2], d[h][m + 3])), tot[m / 2 + 1]);
+            for (int m0 = 0; m0 < MT; m0 += LD) {
+              uint32_t d[LD];
+              tmem_ld<LD>(dcol + h * 2 * NT + m0, d);
+              asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+              if (h == G - 1 && m0 + LD == MT) release();
+#pragma unroll
+              for (int m = 0; m < LD; m += 2) tot[(m0 + m) / 2] = fma2(sc2, pack2(d[m], d[m + 1]), tot[(m0 + m) / 2]);
+            }
+          }
+        } else {
+          uint32_t d[G][MT];
+          uint64_t sc2[G], nz2[G];
+#pragma unroll
+          for (int h = 0; h < G; ++h) {
+            tmem_ld<MT>(dcol + h * 2 * NT, d[h]);
+            sc2[h] = scale(h);
+            const uint32_t zw = lds32(z_addr + ring * kSz + h * kTsZeroBytes);
+            const float nz = fmaf(__uint_as_float(((zw >> z_shift) & 0xFu) | 0x4B000000u), zf, zc);
+            nz2[h] = pack2(nz, nz);
+          }
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          release();
+#pragma unroll
+          for (int h = 0; h < G; ++h) {
+            const uint32_t sx = sx_base + ring * kSums + h * (NT * 4);
+#pragma unroll
+            for (int m = 0; m < MT; m += 4) {
+              uint64_t x01, x23;
+              lds_2x64(sx + m * 4, x01, x23);
+              tot[m / 2] = fma2(sc2[h], fma2(nz2[h], x01, pack2(d[h][m], d[h][m + 1])), tot[m / 2]);
+              tot[m / 2 + 1] =
+                  fma2(sc2[h], fma2(nz2[h], x23, pack2(d[h][m + 2], d[h][m + 3])), tot[m / 2 + 1]);
+            }
           }
         }
       }
@@ -631,6 +739,27 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         const float2 t = unpack2(tot[m]);
         v[2 * m] = t.x;
         v[2 * m + 1] = t.y;
+      }
+      if constexpr (SPLIT) {
+        constexpr int T = Cfg::kPieceTokens, Q = T / 4;
+        cluster_wait();  // every CTA's barriers are set up
+#pragma unroll
+        for (int half = 0; half < Cfg::kHalves; ++half) {
+          const int piece = half * 8 + fold, owner = piece % p.split, n = piece / p.split, quads = piece_quads(half);
+          if (owner == rank) {
+#pragma unroll
+            for (int m = 0; m < Q; ++m)
+              if (m < quads) sts_float4(recv_at(n, rank) + lane * 16 + m * 512, &v[half * T + 4 * m]);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(recv_full(n));
+            continue;
+          }
+          const uint32_t dst = map_rank(recv_at(n, rank) + lane * 16, owner), bar = map_rank(recv_full(n), owner);
+#pragma unroll
+          for (int m = 0; m < Q; ++m)
+            if (m < quads) st_async_v4(dst + m * 512, &v[half * T + 4 * m], bar);
+        }
+        continue;
       }
       // partial tile of CTA c: [MT][256], MODE 1: gate, then up
       constexpr int kTile = MT * kTsBN, kTiles = MODE == 1 ? 2 : 1;
@@ -669,7 +798,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         __syncwarp();  // what a lane acquired holds for the warp's reads of the partial tiles
       }
       // sum of the partial tiles of CTAs [first, last] before this one, in CTA order, several in flight
-      constexpr int AHEAD = 32 / MT;
+      constexpr int AHEAD = MT > 16 ? 1 : 32 / MT;
       auto add_parts = [&](float (&sum)[MT], const float* src, int first, int last) {
         for (int c = first; c >= last; c -= AHEAD) {
           float w[AHEAD][MT];
@@ -736,6 +865,45 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     }
   }
 
+  if constexpr (SPLIT) {
+    // ------------------------------------------------------------------ sums over the cluster
+    // The quads of this CTA's pieces, shared out over the warps that convert and fold, are summed in the CTAs' order.
+    // Rolled loops: the code is cold.
+    constexpr int Q = Cfg::kPieceTokens / 4;
+    constexpr bool kAll = MT > 8;  // up to 8 tokens the fold warps have a quad each
+    constexpr int kWarps = kTsFoldWarps + (kAll ? kTsCvWarps : 0);
+    if (warp >= (kAll ? 0 : kTsFold0) && warp < kTsFold0 + kTsFoldWarps) {
+      __syncwarp();
+      if (kAll) pdl_wait();  // orders this thread's writes after the kernel before this one
+      const int own = (Cfg::kPieces - rank + p.split - 1) / p.split, g = lane & 7, i = lane >> 3;
+      const bool odd = (lane & 1) != 0;
+      const int first = odd ? 1 : 0, slab = blockIdx.x / p.split;
+      const float unscale = (i & 1) ? 1048576.f : 16777216.f;
+#pragma unroll 1
+      for (int task = warp >= kTsFold0 ? warp - kTsFold0 : warp + kTsFoldWarps; task < own * Q; task += kWarps) {
+        const int n = task / Q, piece = n * p.split + rank, token = (piece >> 3) * Cfg::kPieceTokens + 4 * (task % Q);
+        if (token >= p.M) continue;
+        const int n0 = slab * kTsBN + 32 * (piece & 7) + 8 * (g >> 1) + 2 * i;
+        const float bias = p.bias != nullptr && n0 < p.N ? __half2float(__ldg(p.bias + n0 + first)) : 0.f;
+        const bool ok = __all_sync(0xffffffffu, mbar_wait_cluster(recv_full(n), 0, &s_abort, 25));
+        const uint32_t src = recv_at(n, 0) + (task % Q) * 512 + lane * 16;
+        float y[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+        for (int r = 0; r < p.split; ++r) {
+          const float4 w = lds_float4(src + r * Cfg::kPieceBytes);
+          y[0] += w.x;
+          y[1] += w.y;
+          y[2] += w.z;
+          y[3] += w.w;
+        }
+#pragma unroll
+        for (int m = 0; m < 4; ++m) y[m] = y[m] * unscale + bias;
+        handover::store_rows<4>(y, p.out + (size_t)(token + first) * p.N + n0, (size_t)p.N, token + first,
+                                ok && !s_abort && n0 < p.N ? p.M : 0, odd);
+      }
+    }
+  }
+
   // ---- teardown ----
   __syncwarp();
   if (s_abort) {
@@ -744,6 +912,13 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     linger();
   }
   tc_fence_before();
+  if (SPLIT) {
+    // a CTA may go when nobody stores into it any more
+    __syncwarp();
+    if (warp < kTsFold0 || warp >= kTsFold0 + kTsFoldWarps || work.segs == 0) cluster_wait();
+    cluster_arrive_relaxed();
+    cluster_wait();
+  }
   __syncthreads();
   if (warp == kTsIssue) {
     tc_fence_after();
@@ -755,20 +930,25 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 
 // ---- host side -------------------------------------------------------------------------------
 
-// Units of a CTA's range: the cut of the least estimated time in ns, 0 for whole slabs.  Fitted to 12
-// shapes between 1024 x 1024 and 29568 x 8192 at 1, 4, 8 and 16 tokens, cut in up to 32 parts; the cut
-// it picks is 0.6 % from the best one on average, 6 % at worst.  (Always an eighth of a slab, or an even
-// share: 5.4 %.  1536 x 28672, M 4: 9.2 -> 7.8 us whole; 16384 x 1024, M 4: 9.9 -> 7.8 in 16 parts.)
+// How a dense call is cut: `split` CTAs of a cluster share a slab, or (0) `chunk` units of a CTA's range, 0: whole slabs.
+struct TsCut {
+  int split, chunk;
+  long cost;  // estimated time in ns
+};
+
+// Ranges: the cut of the least estimated time.  Fitted to 12 shapes between 1024 x 1024 and 29568 x 8192 at 1, 4, 8 and
+// 16 tokens, cut in up to 32 parts; the cut it picks is 0.6 % from the best one on average, 6 % at worst.  (Always an
+// eighth of a slab, or an even share: 5.4 %.  1536 x 28672, M 4: 9.2 -> 7.8 us whole; 16384 x 1024, M 4: 9.9 -> 7.8 in
+// 16 parts.)
 //   1700 + 47 tokens                start and end
 //   units x max(...)                352 + 3 tokens: conversion; 2.7 CTAs: the words' way from HBM
 //   1440 + 16 tokens (1 + CTAs)     a slab handed over, CTAs the last one collects from
 //   530                             a further slab
 //   580                             more than half of the GPU: the next kernel's start is not hidden
-int ts_chunk(int slabs, int KT, int tokens) {
+TsCut ts_ranges(int slabs, int KT, int tokens) {
   const long units = (long)slabs * KT;
   const int most = sm_count(), even = (int)((units + most - 1) / most);
-  long best_cost = -1;
-  int best = 0;
+  TsCut best = {0, 0, -1};
   for (const int parts : {1, 2, 3, 4, 6, 8, 12, 16}) {
     const int floor = (KT + parts - 1) / parts, chunk = parts == 1 ? 0 : (even > floor ? even : floor);
     int ctas, run, segs, gather = 0;
@@ -791,18 +971,89 @@ int ts_chunk(int slabs, int KT, int tokens) {
     long cost = 1700 + 47 * tokens + (long)run * unit + 530L * (segs - 1);
     if (gather > 0) cost += 1440 + 16 * tokens * (1 + gather);
     if (ctas > most / 2) cost += 580;
-    if (best_cost < 0 || cost < best_cost) {
-      best = chunk;
-      best_cost = cost;
-    }
+    if (best.cost < 0 || cost < best.cost) best = {0, chunk, cost};
     if (chunk == even) break;  // more parts: the same cut
   }
   return best;
 }
 
+// A slab to each cluster of `split` CTAs, in one wave: estimated time in ns, `resident` clusters of that size fit the
+// GPU.  With it the choice between ranges and clusters of 2, 3, 4, 5, 6, 8 and 16 is 0.3 % from the best one on average,
+// 5 % at worst (18 shapes from 1024 x 1024 to 14848 x 8192 at 1, 8, 16, 20 and 32 tokens, groups of 128 and 64).
+//   1950 + 23 tokens                start and end
+//   units x max(...)                355 + 2 tokens, groups of 64 15 + 2 tokens more: conversion, MMAs; 3.1 CTAs: words
+//   12 split                        the sum over the cluster
+//   780 + 1500 x (...)              no room for the next kernel's clusters beside these: its start is not hidden
+long ts_split_cost(int slabs, int KT, int tokens, int group, int split, int resident) {
+  const int arith = 355 + 2 * tokens + (group == 128 ? 0 : 15 + 2 * tokens), words = slabs * split * 31 / 10;
+  long cost = 1950 + 23 * tokens + (long)((KT + split - 1) / split) * (arith > words ? arith : words) + 12 * split;
+  if (2 * slabs > resident) cost += 780 + 1500L * (2 * slabs - resident) / resident;
+  return cost;
+}
+
 struct TsMaps {
   CUtensorMap w, s, z, x;
 };
+
+// Attributes of a SPLIT kernel, and how many of its clusters of every size the GPU holds at once.
+template <int MT, int GROUP>
+int ts_prepare_split() {
+  static std::atomic<bool> attr_done[64];  // as in launch_ts
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return AWQ_B200_ERR_DEVICE;
+  if (!attr_done[dev]) {
+    auto kernel = gemm_ts_kernel<MT, 0, GROUP, true>;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TsCfg<MT, GROUP, true>::kSmem) !=
+            cudaSuccess ||
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+      return AWQ_B200_ERR_LAUNCH;
+    attr_done[dev] = true;
+  }
+  return AWQ_B200_OK;
+}
+template <int MT, int GROUP>
+int ts_resident(int split) {
+  static std::atomic<int> cached[64][kMaxCluster + 1];  // zero-initialised: not asked yet
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  using Cfg = TsCfg<MT, GROUP, true>;
+  return resident_clusters(gemm_ts_kernel<MT, 0, GROUP, true>, split, Cfg::kThreads, Cfg::kSmem, cached[dev]);
+}
+
+template <int MT, int GROUP>
+TsCut ts_cut(int slabs, int KT) {
+  TsCut best = ts_ranges(slabs, KT, MT);
+  for (const int split : {2, 3, 4, 5, 6, 8, 16}) {
+    if (split > KT) break;
+    const int resident = ts_resident<MT, GROUP>(split);
+    if (slabs > resident) continue;
+    const long cost = ts_split_cost(slabs, KT, MT, GROUP, split, resident);
+    if (cost < best.cost) best = {split, 0, cost};
+  }
+  return best;
+}
+
+template <int MT, int GROUP>
+int launch_ts_split(const TsMaps& maps, const TsParams& p, cudaStream_t stream) {
+  using Cfg = TsCfg<MT, GROUP, true>;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(p.slabs * p.split, 1, 1);
+  cfg.blockDim = dim3(Cfg::kThreads, 1, 1);
+  cfg.dynamicSmemBytes = Cfg::kSmem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = p.split;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = add_pdl_attribute(attr, 1);
+  if (cudaLaunchKernelEx(&cfg, gemm_ts_kernel<MT, 0, GROUP, true>, maps.w, maps.s, maps.z, maps.x, p) != cudaSuccess) {
+    cudaGetLastError();
+    return AWQ_B200_ERR_LAUNCH;
+  }
+  return AWQ_B200_OK;
+}
 
 template <int MT, int MODE, int GROUP = 128>
 int launch_ts(const TsMaps& maps, const TsParams& p, int ctas, cudaStream_t stream) {
@@ -810,15 +1061,15 @@ int launch_ts(const TsMaps& maps, const TsParams& p, int ctas, cudaStream_t stre
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return AWQ_B200_ERR_DEVICE;
-  auto kernel = gemm_ts_kernel<MT, MODE, GROUP>;
-  constexpr int smem = TsGroup<GROUP>::kSmem;
+  auto kernel = gemm_ts_kernel<MT, MODE, GROUP, false>;
+  constexpr int smem = TsCfg<MT, GROUP>::kSmem;
   if (!attr_done[dev]) {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
         cudaSuccess)
       return AWQ_B200_ERR_LAUNCH;
     attr_done[dev] = true;
   }
-  if (launch_pdl(kernel, dim3(ctas), dim3(kTsThreads), smem, stream, maps.w, maps.s, maps.z,
+  if (launch_pdl(kernel, dim3(ctas), dim3(TsCfg<MT, GROUP>::kThreads), smem, stream, maps.w, maps.s, maps.z,
                  maps.x, p) != cudaSuccess) {
     cudaGetLastError();
     return AWQ_B200_ERR_LAUNCH;
@@ -855,18 +1106,20 @@ int launch_ts_dense(const __half* x, const uint32_t* qweight, const __half* scal
                     cudaStream_t stream) {
   p.KT = p.K / kTsBK;
   p.slabs = (p.N + kTsBN - 1) / kTsBN;
-  const long units = (long)p.slabs * p.KT;
+  if (int rc = ts_prepare_split<MT, GROUP>()) return rc;
+  const TsCut cut = ts_cut<MT, GROUP>(p.slabs, p.KT);
+  p.split = cut.split;
   int ctas = ts_ctas() < p.slabs ? ts_ctas() : p.slabs;
-  const int chunk = ts_chunk(p.slabs, p.KT, MT);
-  if (chunk > 0 && workspace != nullptr && workspace_bytes >= gemm_ts_workspace_bytes(p.M, p.N, p.K, GROUP)) {
-    p.chunk = chunk;
+  if (cut.chunk > 0 && workspace != nullptr && workspace_bytes >= gemm_ts_workspace_bytes(p.M, p.N, p.K, GROUP)) {
+    p.chunk = cut.chunk;
     p.partial = static_cast<float*>(workspace);
     p.flags = handover::make_flags(workspace, ts_partial_bytes(MT));
-    ctas = (int)((units + p.chunk - 1) / p.chunk);
+    ctas = (int)(((long)p.slabs * p.KT + p.chunk - 1) / p.chunk);
   }
   TsMaps maps;
   if (int rc = ts_weight_maps(&maps, qweight, scales, qzeros, (uint64_t)p.K, (uint64_t)p.N, GROUP)) return rc;
-  if (int rc = encode_map_x(&maps.x, x, (uint64_t)p.M, (uint64_t)p.K, kTsNT)) return rc;
+  if (int rc = encode_map_x(&maps.x, x, (uint64_t)p.M, (uint64_t)p.K, TsCfg<MT, GROUP>::NT)) return rc;
+  if (p.split > 1) return launch_ts_split<MT, GROUP>(maps, p, stream);
   return launch_ts<MT, 0, GROUP>(maps, p, ctas, stream);
 }
 
@@ -914,13 +1167,13 @@ int launch_ts_experts(const MoeArgs& a, __half* act, int64_t act_rows, __half* p
   return launch_ts<MT, 2>(maps, p, ctas, stream);
 }
 
-int ts_tokens(int M) { return M <= 4 ? 4 : (M <= 8 ? 8 : 16); }
+int ts_tokens(int M) { return M <= 4 ? 4 : (M <= 8 ? 8 : (M <= 16 ? 16 : 32)); }
 
 }  // namespace
 
 bool gemm_ts_supported(int M, int N, int K, int group) {
   // N % 32: 16-byte TMA row pitch of the packed weights; K % 128: whole stages
-  return M >= 1 && M <= 16 && N % 32 == 0 && K % kTsBK == 0 && (group == 128 || group == 64);
+  return M >= 1 && M <= kTsMaxRows && N % 32 == 0 && K % kTsBK == 0 && (group == 128 || group == 64);
 }
 
 size_t gemm_ts_workspace_bytes(int M, int N, int K, int group) {
@@ -938,9 +1191,10 @@ int launch_gemm_ts(const __half* x, const uint32_t* qweight, const __half* scale
   p.M = M;
   p.N = N;
   p.K = K;
-  auto launch = group == 128 ? launch_ts_dense<16, 128> : launch_ts_dense<16, 64>;
+  auto launch = group == 128 ? launch_ts_dense<32, 128> : launch_ts_dense<32, 64>;
   if (M <= 4) launch = group == 128 ? launch_ts_dense<4, 128> : launch_ts_dense<4, 64>;
   else if (M <= 8) launch = group == 128 ? launch_ts_dense<8, 128> : launch_ts_dense<8, 64>;
+  else if (M <= 16) launch = group == 128 ? launch_ts_dense<16, 128> : launch_ts_dense<16, 64>;
   return launch(x, qweight, scales, qzeros, p, workspace, workspace_bytes, stream);
 }
 

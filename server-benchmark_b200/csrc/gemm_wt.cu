@@ -164,13 +164,6 @@ __device__ __forceinline__ Work wt_work(const WtParams& p) {
   return Work(blockIdx.x >> 1, gridDim.x >> 1, tiles, p.KT, MODE == 0 && !WIDE ? p.chunk : 0);
 }
 
-__device__ __forceinline__ float4 lds_float4(uint32_t addr) {
-  float4 v;
-  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-               : "r"(addr));
-  return v;
-}
 template <int ID, int COUNT>
 __device__ __forceinline__ void named_barrier(int off = 0) {
   asm volatile("bar.sync %0, %1;" ::"r"(ID + off), "n"(COUNT) : "memory");

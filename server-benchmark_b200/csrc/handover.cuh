@@ -88,6 +88,8 @@ struct Work {
       end = KT;
     }
   }
+  // Stages [k0, k1) of one tile.
+  __device__ __forceinline__ static Work part(int tile, int k0, int k1, int KT) { return Work(tile, k0, k1, KT, true); }
   __device__ __forceinline__ int tile_id(int seg) const {
     return chunked ? tile0 + segs - 1 - seg : worker + seg * workers;
   }
@@ -99,6 +101,11 @@ struct Work {
   __device__ __forceinline__ int helpers(int seg) const {
     return k_begin(seg) > 0 && k_end(seg) == KT ? worker - tile_id(seg) * KT / chunk : 0;
   }
+
+ private:
+  __device__ __forceinline__ Work(int tile, int k0, int k1, int KT_, bool)
+      : worker(0), workers(1), KT(KT_), chunk(1), segs(k1 > k0 ? 1 : 0), count(k1 - k0), begin(k0), end(k1), tile0(tile),
+        chunked(true) {}
 };
 
 // Two tokens of 32 columns per step: this lane's column of tokens c, c + 1 packed to fp16, then

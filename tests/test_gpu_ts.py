@@ -234,3 +234,40 @@ def test_capture_on_a_new_stream_takes_calls_of_any_size(A):
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(y, want)
+
+
+# Slabs shared by clusters of 2, 3, 4, 5, 6, 8 and 16 CTAs (by the estimated cost of a B200's cuts), units that do not
+# divide by them, one unit a CTA, an edge of N inside a slab, the token variants at their ends; ranges over the whole
+# GPU with 17 to 32 tokens; one unit in all.
+@pytest.mark.parametrize("m,k,n,group", [
+    (1, 1024, 8192, 128), (30, 1024, 8192, 64), (3, 2176, 5120, 128), (32, 2176, 5152, 128), (17, 4096, 4064, 64),
+    (9, 640, 1312, 128), (25, 12288, 6176, 128), (24, 8192, 5120, 64), (12, 2048, 1024, 64), (16, 8192, 1280, 128),
+    (31, 8192, 1280, 128), (4, 16384, 992, 64), (5, 256, 256, 128), (20, 128, 32, 128), (23, 8192, 38176, 128),
+    (18, 4096, 28704, 64)])
+@pytest.mark.parametrize("bias", [False, True])
+def test_ts_clusters_and_up_to_32_tokens(A, m, k, n, group, bias):
+    """Nothing but the output is rounded to fp16, and the bits do not depend on timing."""
+    from awq_b200 import synth
+    qw, s, qz = synth.awq_linear_tensors(k, n, group, seed=m + n)
+    x = synth.activations(m, k, seed=k)
+    b = synth.activations(1, n, seed=3)[0] if bias else None
+    cols = torch.arange(n)[max(0, n - 1024):]  # of the oracle: the last ones, with the edge
+    ref = x.double() @ torch.from_numpy(O.dequantize_fp32(
+        qw[:, cols[0] // 8:].numpy(), s[:, cols].numpy(), qz[:, cols[0] // 8:].numpy(), group)).double()
+    if bias:
+        ref += b[cols].double()
+    outs = [A.awq_gemm(x.cuda(), qw.cuda(), s.cuda(), qz.cuda(), 8, bias=b.cuda() if bias else None)
+            for _ in range(3)]
+    torch.cuda.synchronize()
+    assert device_status() == 0, "a bounded wait ran out"
+    assert all(torch.equal(outs[0], y) for y in outs[1:])
+    error = (outs[0].cpu()[:, cols].double() - ref).norm()
+    # 5 %: the fp32 sums, K * 2^-24 of their terms' size at most, move few values to the other side
+    assert error < 1.05 * (ref.half().double() - ref).norm()
+
+
+def test_explicit_ts_takes_16_rows_at_most(A):
+    from awq_b200 import synth
+    dev = [t.cuda() for t in (synth.activations(17, 256, seed=2), *synth.awq_linear_tensors(256, 256, 128, seed=1))]
+    with pytest.raises(ValueError):
+        A.awq_gemm(*dev, 8, kernel=A.KERNEL_TS)
