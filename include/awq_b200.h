@@ -97,7 +97,8 @@ size_t awq_b200_gemm_workspace_bytes(int M, int N, int K, int group, int kernel)
 /*
  * How AWQ_B200_KERNEL_WT cuts a call that has its scratch, on a GPU that holds `cta_pairs` pairs of CTAs (0: the
  * current device's): tokens of a tile, (tile, K stage) units of a pair's range (0: whole tiles), and whether the
- * epilogue goes through shared memory (1) or from registers (0).  Host arithmetic, for tests that name a cut.
+ * epilogue goes through shared memory (1) or from registers (0).  Of a call that names AWQ_B200_KERNEL_WT: the
+ * automatic choice may let clusters of CTAs share tiles instead.  Host arithmetic, for tests that name a cut.
  * No counterpart in the reference.
  */
 int awq_b200_gemm_wt_cut(int M, int N, int K, int group, int cta_pairs, int* tokens, int* chunk, int* wide);

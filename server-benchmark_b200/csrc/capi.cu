@@ -201,8 +201,9 @@ int awq_b200_gemm(const void* x, const void* qweight, const void* scales, const 
       if (!awq::gemm_wt_supported(M, N, K, group)) return AWQ_B200_ERR_SHAPE;
       // scratch is optional here: without it (or misaligned) whole tiles are distributed
       if ((reinterpret_cast<uintptr_t>(workspace) & 255u) != 0) workspace = nullptr;
+      // a call that names the kernel gets the cut that awq_b200_gemm_wt_cut tells
       return awq::launch_gemm_wt(xh, qw, sc, qz, bh, oh, M, N, K, group, workspace, workspace_bytes,
-                                 st);
+                                 automatic, st);
     case AWQ_B200_KERNEL_Q8: {
       if (!awq::gemm_q8_supported(M, N, K, group)) return AWQ_B200_ERR_SHAPE;
       if ((reinterpret_cast<uintptr_t>(qweight) & 31u) != 0) return AWQ_B200_ERR_ALIGN;

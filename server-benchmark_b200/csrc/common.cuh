@@ -214,7 +214,7 @@ size_t gemm_wt_workspace_bytes(int M, int N, int K, int group);
 int gemm_wt_cut(int M, int N, int K, int group, int cta_pairs, int* tokens, int* chunk, int* wide);
 int launch_gemm_wt(const __half* x, const uint32_t* qweight, const __half* scales,
                    const uint32_t* qzeros, const __half* bias, __half* out, int M, int N, int K,
-                   int group, void* workspace, size_t workspace_bytes, cudaStream_t stream);
+                   int group, void* workspace, size_t workspace_bytes, bool clusters, cudaStream_t stream);
 int wt_device_status(int* out, int clear);
 
 // gemm_q8.cu: K-major nibble copy of the weights, widened to bytes by tcgen05.cp on the way into

@@ -199,12 +199,6 @@ __device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t (&r)[4]) {
                : "r"(addr)
                : "memory");
 }
-// Four values into another CTA's shared memory, counted by a barrier there.
-__device__ __forceinline__ void st_async_v4(uint32_t dst, const float* v, uint32_t bar) {
-  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(dst),
-               "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "r"(bar)
-               : "memory");
-}
 __device__ __forceinline__ void sts_float4(uint32_t addr, const float* v) {
   asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3])
                : "memory");
@@ -323,7 +317,8 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   if (MODE == 1) pdl_wait();
   pdl_launch_dependents();
   const int rank = SPLIT ? blockIdx.x % p.split : 0;
-  const Work work = SPLIT ? Work::part(blockIdx.x / p.split, rank * p.KT / p.split, (rank + 1) * p.KT / p.split, p.KT)
+  const Work work = SPLIT ? Work::range(blockIdx.x / p.split * p.KT + rank * p.KT / p.split,
+                                         blockIdx.x / p.split * p.KT + (rank + 1) * p.KT / p.split, p.KT)
                           : ts_work<MT, MODE>(p);
   // SPLIT: barrier and shared memory of the n-th piece that this CTA sums, partial sums of CTA `from`
   auto recv_full = [&](int n) { return bar_base + 8 * (2 * NRAW + 2 * kTsUnits + n); };

@@ -28,6 +28,20 @@
 // Work: tiles of 256 columns x `nt` tokens.  Strided: pair p takes the whole tiles p, p + P, ...
 // Chunked: one contiguous range of the (tile, stage) list per pair, shared tiles handed over
 // (handover.cuh).  The sum is taken in pair order: results do not depend on timing.
+// SPLIT: tiles few enough for one wave of clusters.  The 2 to 8 pairs of a cluster share a tile, or three pairs two
+// tiles, by even ranges of units; each pair sums some of the tile's eights of tokens, and the others store their parts of
+// those into its shared memory (st.async, counted by an mbarrier).  A tile handed over through scratch cost 12 500 cycles
+// from the MMAs' end at 112 tokens (helper: 4700 until its flag is up, finisher: 7000 for collection, sum and stores),
+// this 4600: 1400 to send, 700 under way, 2000 for the sum and the stores of a pair's share, 500 to the exit.  More warps do not
+// shorten it (the stores' path does not), nor does a rehearsal of the cold code.  us, ranges -> clusters (pairs):
+//   8192 x 1280 M 48 10.1 -> 6.1 (5), M 300 17.2 -> 12.4 (3); 8192 x 5120 M 100 19.1 -> 14.4 (3); 4096 x 4096 M 77
+//   groups of 64 12.1 -> 8.9 (2); 8192 x 8192 M 100 20.2 -> 16.9 (2), M 150 24.2 -> 21.1 (2); 8192 x 10240 M 100 23.4 ->
+//   21.8 (3 for two tiles); 16384 x 2048 M 64 16.6 -> 12.6 (5).
+// Prologue: tensor memory is asked for first, the warp of the packed words waits for nobody, a conversion warp's first
+// scales are on their way before anything is waited for, and the cluster barrier is awaited only where a CTA first reaches
+// into the other.  In a kernel that starts when the one before it has left the GPU the first MMAs wait for the first
+// conversion, 7400 cycles from the start before, some 1000 less now: 1024 x 8192 M 40 4.85 -> 4.5 us, router + experts of
+// 128 x 2048 x 768, top-8, 600 tokens 134.6 -> 123.0.
 // The cut of a call (tokens of a tile, units of a range) is the one of the least estimated time
 // (wt_cost).  Against tiles of up to 256 tokens that were always split, and partial tiles read with plain
 // loads: 8192 x 1280 at M 250 38.5 -> 14.4 us, 8192 x 7424 at M 250 50 -> 28, at M 100 26.5 -> 20.6,
@@ -98,6 +112,16 @@ constexpr int kWtExBytes = 2 * 2 * kWtExFloats * 4;
 constexpr int kWtSmemLimit = 232448 - 1024;   // dynamic shared memory less the static part
 constexpr int kWtMaxPairs = 128;
 
+// SPLIT: the tiles of a cluster and how its pairs share them.  A pair has at most two tiles, neighbours.
+constexpr int kWtMaxShare = 8, kWtMaxTiles = 4;
+struct WtShare {
+  int pairs, tiles;                      // of a cluster; pairs 0: no SPLIT
+  int recv;                              // bytes of partial sums that a CTA takes in for a tile
+  short bound[kWtMaxShare + 1];          // pair i has the units [bound[i], bound[i + 1]) of the cluster's list
+  signed char first[kWtMaxTiles], count[kWtMaxTiles];  // pairs that share a tile
+  int recip[kWtMaxTiles];                // ceil(2^16 / count)
+};
+
 struct WtParams {
   const __half* scales;
   const uint32_t* qzeros;
@@ -114,6 +138,7 @@ struct WtParams {
   int slots, acol;             // A slots behind them (64 columns each) and the first one's column
   int xstage;                  // bytes of an x stage
   int stage_bytes;             // WIDE: of a tile's way out through shared memory
+  WtShare share;               // SPLIT
   float* partial;              // [CTA][4][nt][32] partial tiles handed over
   handover::Flags flags;       // of the hand-over
   // grouped modes
@@ -158,8 +183,16 @@ __device__ __forceinline__ WtTile wt_tile(const WtParams& p, int id) {
   return t;
 }
 
-template <int MODE, bool WIDE>
+// SPLIT: of a tile's `eights` of tokens, those that sharer i of n sums are [first(i), first(i + 1)).
+__device__ __forceinline__ int wt_own_first(int eights, int n, int i) { return (i * eights + n - 1) / n; }
+
+template <int MODE, bool WIDE, bool SPLIT>
 __device__ __forceinline__ Work wt_work(const WtParams& p) {
+  if constexpr (SPLIT) {
+    const int cluster = blockIdx.x / (2 * p.share.pairs), pair = blockIdx.x % (2 * p.share.pairs) / 2;
+    const int base = cluster * p.share.tiles * p.KT;
+    return Work::range(base + p.share.bound[pair], base + p.share.bound[pair + 1], p.KT);
+  }
   const int tiles = MODE == 0 ? p.slabs * p.mtiles : __ldcg(p.n_tiles) * p.slabs;
   return Work(blockIdx.x >> 1, gridDim.x >> 1, tiles, p.KT, MODE == 0 && !WIDE ? p.chunk : 0);
 }
@@ -309,6 +342,7 @@ __device__ __forceinline__ void wt_epilogue_wide(const WtParams& p, const Work& 
     }
     float bias[4];
     if (MODE == 0) wt_load_bias(p, WtOut<MODE>::first_column(t, rank, q), g, bias);
+    const WtOut<MODE> out(p, t, rank, q, lane);
     if (ok) ok = mbar_wait(d_full, (uint32_t)seg & 1u, abort_flag, 38);
     ok = __all_sync(0xffffffffu, ok);
     tc_fence_after();
@@ -339,13 +373,141 @@ __device__ __forceinline__ void wt_epilogue_wide(const WtParams& p, const Work& 
       }
       to += K8 * 512;
     }
-    const WtOut<MODE> out(p, t, rank, q, lane);
     const int rows = ok ? out.rows : 0, pieces = (t.n + 31) / 32 * K8;
 #pragma unroll 4
     for (int i = 0; i < pieces; ++i) {
       const int m = MODE == 1 ? 32 * (i >> 1) + 16 * (q >> 1) + 8 * (i & 1) : 8 * i;
       const uint4 v = lds_uint4(stage + i * 512);
       if (m < rows) *reinterpret_cast<uint4*>(out.dst + (size_t)m * out.pitch) = v;
+    }
+  }
+}
+
+// Epilogue warp q of the SPLIT kernel: pairs of a cluster share a tile, and each sums some of its eights of tokens.  First
+// the parts that others sum are stored into their shared memory (the CTA of the same rank), for all segments; then the
+// own ones are added up in the pairs' order.  Every index is settled while the MMAs run: the warp has nothing else to do
+// then, and afterwards each division costs 200 cycles.
+struct WtSplitSegment {
+  uint32_t dcol;               // its accumulator
+  uint32_t base;               // partial sums that this warp takes in, or puts into another CTA at the same place:
+  int step;                    // [eights of the CTA that sums][other sharers], bytes of the inner dimension
+  uint32_t d_full, full;       // barriers
+  int first, n, me;            // sharers: the first pair, their number, this one
+  int eights, recip;
+  float bias[4];
+  __half* dst;
+  int rows;
+  __device__ __forceinline__ int own_first(int i) const { return ((i * eights + n - 1) * recip) >> 16; }
+};
+template <int GROUP>
+__device__ __forceinline__ WtSplitSegment wt_split_segment(const WtParams& p, const Work& work, int seg, uint32_t tmem,
+                                                           int rank, int q, int lane, uint32_t d_full0, uint32_t recv,
+                                                           uint32_t recv_full) {
+  WtSplitSegment f;
+  const int cluster = blockIdx.x / (2 * p.share.pairs), pair = blockIdx.x % (2 * p.share.pairs) / 2;
+  const int tile = work.tile_id(seg), lt = tile - cluster * p.share.tiles, buf = seg & (p.nbuf - 1);
+  const WtTile t = wt_tile<0, GROUP>(p, tile);
+  f.eights = t.n / 8;
+  f.first = p.share.first[lt];
+  f.n = p.share.count[lt];
+  f.recip = p.share.recip[lt];
+  f.me = pair - f.first;
+  f.step = (f.n - 1) * 1024;
+  f.base = recv + (lt & 1) * p.share.recv + q * f.own_first(1) * f.step + lane * 16;
+  f.full = recv_full + 8 * (lt & 1);
+  f.d_full = d_full0 + 8 * buf;
+  f.dcol = tmem + ((uint32_t)(q * 32) << 16) + buf * p.dcols;
+  wt_load_bias(p, WtOut<0>::first_column(t, rank, q), lane >> 2, f.bias);
+  const WtOut<0> out(p, t, rank, q, lane);
+  f.dst = out.dst;
+  f.rows = out.rows;
+  return f;
+}
+template <int GROUP>
+__device__ __forceinline__ void wt_epilogue_split(const WtParams& p, const Work& work, uint32_t tmem, int rank, int q,
+                                                  int lane, uint32_t d_full0, uint32_t recv, uint32_t recv_full,
+                                                  volatile int* abort_flag) {
+  const WtSplitSegment s0 = wt_split_segment<GROUP>(p, work, 0, tmem, rank, q, lane, d_full0, recv, recv_full);
+  WtSplitSegment s1 = s0;
+  if (work.segs > 1) s1 = wt_split_segment<GROUP>(p, work, 1, tmem, rank, q, lane, d_full0, recv, recv_full);
+  const size_t pitch = (size_t)p.N;
+  pdl_wait();  // orders this thread's writes after the kernel before this one
+  bool ok = true;
+#pragma unroll 1
+  for (int seg = 0; seg < work.segs; ++seg) {
+    const WtSplitSegment f = seg == 0 ? s0 : s1;
+    if (ok) ok = mbar_wait(f.d_full, 0, abort_flag, 38);
+    ok = __all_sync(0xffffffffu, ok);
+    tc_fence_after();
+    int e = 0;
+#pragma unroll 1
+    for (int to = 0; to < f.n; ++to) {
+      const int end = f.own_first(to + 1);
+      if (to != f.me) {
+        const uint32_t cta = 2 * (f.first + to) + rank, bar = map_rank(f.full, cta);
+        uint32_t dst = map_rank(f.base + (f.me - (f.me > to)) * 1024, cta);
+#pragma unroll 1
+        for (; e < end; e += 2) {
+          float d[2][8];
+          tmem_ld_16x256b_x2(f.dcol + 8 * e, d[0]);
+          tmem_ld_16x256b_x2(f.dcol + (16u << 16) + 8 * e, d[1]);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          st_async_v4(dst, &d[0][0], bar);
+          st_async_v4(dst + 512, &d[1][0], bar);
+          dst += f.step;
+          if (e + 1 < end) {
+            st_async_v4(dst, &d[0][4], bar);
+            st_async_v4(dst + 512, &d[1][4], bar);
+            dst += f.step;
+          }
+        }
+      }
+      e = end;
+    }
+  }
+#pragma unroll 1
+  for (int seg = 0; seg < work.segs; ++seg) {
+    const WtSplitSegment f = seg == 0 ? s0 : s1;
+    const int own0 = f.own_first(f.me), own1 = f.own_first(f.me + 1);
+    if (ok && f.n > 1 && own1 > own0) ok = mbar_wait_cluster(f.full, 0, abort_flag, 40);
+    ok = __all_sync(0xffffffffu, ok);
+    const int rows = ok ? f.rows : 0;
+    uint32_t src = f.base;
+    __half* dst = f.dst + (size_t)(8 * own0) * pitch;
+#pragma unroll 1
+    for (int e = own0; e < own1; e += 2) {
+      float d[2][8];
+      tmem_ld_16x256b_x2(f.dcol + 8 * e, d[0]);
+      tmem_ld_16x256b_x2(f.dcol + (16u << 16) + 8 * e, d[1]);
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        if (e + k >= own1) break;
+        float y[2][4] = {};
+#pragma unroll 1
+        for (int from = 0; from < f.n; ++from) {
+          float4 lo = make_float4(d[0][4 * k], d[0][4 * k + 1], d[0][4 * k + 2], d[0][4 * k + 3]);
+          float4 hi = make_float4(d[1][4 * k], d[1][4 * k + 1], d[1][4 * k + 2], d[1][4 * k + 3]);
+          if (from != f.me) {
+            lo = lds_float4(src);
+            hi = lds_float4(src + 512);
+            src += 1024;
+          }
+          y[0][0] += lo.x;
+          y[0][1] += lo.y;
+          y[0][2] += lo.z;
+          y[0][3] += lo.w;
+          y[1][0] += hi.x;
+          y[1][1] += hi.y;
+          y[1][2] += hi.z;
+          y[1][3] += hi.w;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) y[j >> 2][j & 3] += f.bias[2 * (j >> 2) + ((j >> 1) & 1)];
+        const uint4 w = wt_round(y, 0);
+        if (8 * (e + k) < rows) *reinterpret_cast<uint4*>(dst) = w;
+        dst += 8 * pitch;
+      }
     }
   }
 }
@@ -375,6 +537,10 @@ __device__ __forceinline__ void wt_epilogue(const WtParams& p, const Work& work,
 #pragma unroll
       for (int i = 0; i < 4; ++i) rw[i] = 32 * i < t.n ? __ldcg(p.row_weights + t.m0 + 32 * i + lane) : 0.f;
     }
+    // where the output goes: settled ahead of the MMAs' end as well
+    const WtOut<MODE> out(p, t, rank, q, lane);
+    float bias[4];
+    if (MODE == 0) wt_load_bias(p, WtOut<MODE>::first_column(t, rank, q), lane >> 2, bias);
     // CTAs whose partial tiles are added: blockIdx.x - 2 gather .. blockIdx.x - 2
     const int gather = MODE == 0 ? work.helpers(seg) : 0;
     if (ok) ok = mbar_wait(d_full0 + 8 * buf, (uint32_t)(p.nbuf == 2 ? seg >> 1 : seg) & 1u, abort_flag,
@@ -396,10 +562,7 @@ __device__ __forceinline__ void wt_epilogue(const WtParams& p, const Work& work,
     __syncwarp();  // what a lane acquired holds for the warp's reads of the partial tiles
     tc_fence_after();
     const uint32_t dcol = tmem + lane_q + buf * p.dcols;
-    const WtOut<MODE> out(p, t, rank, q, lane);
     const int rows = ok ? out.rows : 0;
-    float bias[4];
-    if (MODE == 0) wt_load_bias(p, WtOut<MODE>::first_column(t, rank, q), lane >> 2, bias);
     // Partial tiles handed over come through a ring in the packed words' and tokens' stages, which the
     // pair is done with (the tile it finishes for others is its last), 32 tokens of a CTA at a time: a
     // load that waits for L2 once per 32 tokens and CTA took 3.2 us per CTA at 128 tokens.
@@ -477,7 +640,66 @@ __device__ __forceinline__ void wt_epilogue(const WtParams& p, const Work& work,
   }
 }
 
-template <int MODE, int GROUP, bool WIDE>
+// Zero words and scales of a conversion warp's units, fetched one unit ahead; the warp's position in the work.
+template <int MODE, int GROUP>
+struct WtScales {
+  static constexpr int kGroups = kWtBK / GROUP;  // quantisation groups of a stage
+  const WtParams& p;
+  const Work& work;
+  const int rank, q, team, g, words;
+  int seg, k, k_end;
+  uint32_t zs;                 // index of this lane's zero word and eight scales of the next unit
+  uint32_t zw[kGroups];
+  uint4 sv[kGroups];
+  __device__ __forceinline__ WtScales(const WtParams& p_, const Work& work_, int rank_, int warp, int lane)
+      : p(p_), work(work_), rank(rank_), q(warp & 3), team(warp >> 2), g(lane >> 2), words(p_.N / kPack) {}
+  __device__ __forceinline__ void settle() {  // k past the end of its segment: into the next ones
+    while (k >= k_end && seg + 1 < work.segs) {
+      k -= k_end;
+      ++seg;
+      k += work.k_begin(seg);
+      k_end = work.k_end(seg);
+    }
+  }
+  __device__ __forceinline__ uint32_t locate() const {
+    const WtTile t = wt_tile<MODE, GROUP>(p, work.tile_id(seg));
+    int w;
+    if (MODE == 1)
+      w = (q >> 1) * (p.half_cols / kPack) + t.slab * 16 + rank * 8 + 4 * (q & 1) + (g >> 1);
+    else
+      w = t.slab * (kWtBN / kPack) + rank * (kWtCols / kPack) + 4 * q + (g >> 1);
+    w = min(w, words - 1);  // columns past the edge: any value, nothing of them is stored
+    return (uint32_t)(t.grp0 + k * kGroups) * words + w;
+  }
+  __device__ __forceinline__ void fetch() {
+#pragma unroll
+    for (int i = 0; i < kGroups; ++i) {
+      zw[i] = __ldg(p.qzeros + zs + i * words);
+      sv[i] = __ldg(reinterpret_cast<const uint4*>(p.scales) + zs + i * words);
+    }
+  }
+  __device__ __forceinline__ void start() {
+    seg = 0;
+    k = work.k_begin(0) + team;
+    k_end = work.k_end(0);
+    settle();
+    if (team < work.count) {
+      zs = locate();
+      fetch();
+    }
+  }
+  __device__ __forceinline__ void next() {
+    k += kWtTeams;
+    zs += (uint32_t)(kWtTeams * kGroups * words);
+    if (k >= k_end) {
+      settle();
+      zs = locate();
+    }
+    fetch();
+  }
+};
+
+template <int MODE, int GROUP, bool WIDE, bool SPLIT>
 __global__ void __launch_bounds__(kWtThreads, 1)
 gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ WtXMaps<MODE> map_x,
                const WtParams p) {
@@ -486,7 +708,9 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   __shared__ uint32_t s_tmem_base;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int rank = blockIdx.x & 1;  // cluster of two along x: rank 0 is the leader
+  const int rank = blockIdx.x & 1;  // of the pair: rank 0 is the leader
+  const int leader = SPLIT ? blockIdx.x % (2 * p.share.pairs) & ~1 : 0;  // its rank in the cluster
+  const uint16_t pair_mask = SPLIT ? (uint16_t)(3u << leader) : (uint16_t)3;
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t x_base = smem_base;
   const uint32_t raw_base = x_base + p.nx * p.xstage;
@@ -508,8 +732,15 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   };
 
   pdl_launch_dependents();
+  if (warp == kWtIssueWarp) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(&s_tmem_base)),
+                 "r"((uint32_t)kWtTmemCols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
   if (MODE != 0) pdl_wait();  // the tile table comes from the kernel before this one
-  const Work work = wt_work<MODE, WIDE>(p);
+  const Work work = wt_work<MODE, WIDE, SPLIT>(p);
   const int words = p.N / kPack;
 
   // Packed words, unit by unit: 128 rows x 16 words (MODE 1: 8 gate words and the matching 8 up
@@ -545,6 +776,7 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 
   if (warp == kWtRawWarp) {
     if (lane == 0) asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
+    if (lane == 0) s_abort = 0;
     if (lane < p.nraw) {
       mbar_init(raw_full(lane), 1);
       mbar_init(raw_empty(lane), kWtCvWarps / kWtTeams);
@@ -552,12 +784,13 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       fence_proxy_async();
     }
     __syncwarp();
+    asm volatile("bar.arrive 1, %0;" ::"n"(kWtThreads) : "memory");
+    cluster_arrive();
     // the first packed words are on their way before anyone else is through the prologue; no
     // kernel writes weights, so they need not wait for the kernel before this one
     for (int i = 0; i < kWtTeams && raw_u < work.count; ++i) load_raw();
   }
   if (warp == kWtXWarp && lane == 0) {
-    s_abort = 0;
     for (int u = 0; u < kWtMaxX; ++u) {
       // four conversion warps of each CTA, and the leader's announcement of the tokens' bytes
       mbar_init(unit_full(u), 2 * (kWtCvWarps / kWtTeams) + 1);
@@ -569,22 +802,30 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (MODE == 0 && !WIDE && warp >= kWtEpiWarp0 && warp < kWtEpiWarp0 + kWtEpiWarps && lane < kWtPartRing) {
+  if (MODE == 0 && !WIDE && !SPLIT && warp >= kWtEpiWarp0 && warp < kWtEpiWarp0 + kWtEpiWarps && lane < kWtPartRing) {
     mbar_init(part_full(warp - kWtEpiWarp0) + 8 * lane, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  __syncwarp();
-  if (warp == kWtIssueWarp) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     smem_u32(&s_tmem_base)),
-                 "r"((uint32_t)kWtTmemCols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  if (SPLIT && warp >= kWtEpiWarp0 && warp < kWtEpiWarp0 + kWtEpiWarps && lane < work.segs) {
+    // lane: segment.  What the tile's other pairs store into this CTA for this warp
+    const int tile = work.tile_id(lane), eights = wt_tile<MODE, GROUP>(p, tile).n / 8;
+    const int lt = tile % p.share.tiles, n = p.share.count[lt];
+    const int me = blockIdx.x % (2 * p.share.pairs) / 2 - p.share.first[lt];
+    const uint32_t bar = part_full(warp - kWtEpiWarp0) + 8 * (lt & 1);
+    mbar_init(bar, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    mbar_arrive_expect_tx(bar, (wt_own_first(eights, n, me + 1) - wt_own_first(eights, n, me)) * (n - 1) * 1024);
   }
+  // What a conversion warp needs for its first unit, on its way during the rest of the prologue: no kernel writes it.
+  WtScales<MODE, GROUP> scales(p, work, rank, warp, lane);
+  if (warp < kWtCvWarps) scales.start();
+  __syncwarp();
+  // Everyone but the warp of the packed words, which only tells that its barriers are set up, waits for the others'; the
+  // two CTAs' set-up is awaited where something first goes from one to the other.
   tc_fence_before();
-  __syncthreads();
-  cluster_barrier();  // both CTAs' barriers are initialised before anything arrives across
+  if (warp != kWtRawWarp) named_barrier<1, kWtThreads>();
   tc_fence_after();
+  if (warp != kWtRawWarp) cluster_arrive();
   const uint32_t tmem = s_tmem_base;
 
   if (warp == kWtRawWarp) {
@@ -601,15 +842,17 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       }
       ready = load_raw();
     }
+    cluster_wait();
   } else if (warp == kWtXWarp) {
     // ------------------------------------------------------------------ tokens
     pdl_wait();  // the activations may be the output of the kernel before this one
+    cluster_wait();
     bool ok = true, ready = false;
     int seg = 0, k = 0, k_end = 0, s = 0;
     const CUtensorMap* map = nullptr;
     uint32_t bytes = 0;
     int row = 0;
-    const uint32_t full0 = map_rank(unit_full(0), 0);
+    const uint32_t full0 = map_rank(unit_full(0), leader);
     for (int u = 0; u < work.count; ++u) {
       if (k == k_end) {
         const WtTile t = wt_tile<MODE, GROUP>(p, work.tile_id(seg));
@@ -642,6 +885,7 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         ok = mbar_wait(mma_done(u), unit_phase(u), &s_abort, 32);
   } else if (warp == kWtIssueWarp) {
     // ------------------------------------------------------------------ MMA issue (leader)
+    cluster_wait();
     if (rank == 0) {
       // What bounds this warp is its own serial chain: a barrier wait costs ~150 cycles even when
       // the phase is complete, an MMA ~25, every other instruction of the loop its full latency
@@ -679,8 +923,8 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
           bool r = false;
           if (elect_one()) {
             r = umma_unit_pair(dcol, acol, dx, half16, idesc, acc, done0 + 8 * (u & 7),
-                               full0 + 8 * ((u + 1) & 7), (uint32_t)((u + 1) >> 3) & 1u);
-            if (u == u_end - 1) umma_commit_pair(d_full(buf));
+                               full0 + 8 * ((u + 1) & 7), (uint32_t)((u + 1) >> 3) & 1u, pair_mask);
+            if (u == u_end - 1) umma_commit_pair(d_full(buf), pair_mask);
           }
           acc = 1;
           ready = __any_sync(0xffffffffu, r);
@@ -703,47 +947,9 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     constexpr uint32_t kPairBytes = 32 * (MODE == 1 ? 32 : 64);  // 32 rows further on
     const uint32_t half_sel = (g & 1) ? 0x3232u : 0x1010u;      // this lane's halfword, duplicated
     constexpr int kGroups = kWtBK / GROUP;                        // quantisation groups of a stage
-    const uint32_t full_leader = map_rank(unit_full(0), 0);
+    const uint32_t full_leader = map_rank(unit_full(0), leader);
 
-    // position of this team's next unit, and the scale / zero words of it (fetched one unit ahead)
-    int seg = 0, k = work.k_begin(0) + team, k_end = work.k_end(0);
-    auto settle = [&]() {  // k past the end of its segment: into the next ones
-      while (k >= k_end && seg + 1 < work.segs) {
-        k -= k_end;
-        ++seg;
-        k += work.k_begin(seg);
-        k_end = work.k_end(seg);
-      }
-    };
-    settle();
-    // index of this lane's zero word and eight scales of the next unit
-    const uint32_t zs_step = (uint32_t)(kWtTeams * kGroups * words);
-    auto locate = [&]() {
-      const WtTile t = wt_tile<MODE, GROUP>(p, work.tile_id(seg));
-      int w;
-      if (MODE == 1)
-        w = (q >> 1) * (p.half_cols / kPack) + t.slab * 16 + rank * 8 + 4 * (q & 1) + (g >> 1);
-      else
-        w = t.slab * (kWtBN / kPack) + rank * (kWtCols / kPack) + 4 * q + (g >> 1);
-      w = min(w, words - 1);  // columns past the edge: any value, nothing of them is stored
-      return (uint32_t)(t.grp0 + k * kGroups) * words + w;
-    };
-    uint32_t zs = 0;
-    uint32_t zw_n[kGroups];
-    uint4 sv_n[kGroups];
-    auto fetch = [&]() {
-#pragma unroll
-      for (int i = 0; i < kGroups; ++i) {
-        zw_n[i] = __ldg(p.qzeros + zs + i * words);
-        sv_n[i] = __ldg(reinterpret_cast<const uint4*>(p.scales) + zs + i * words);
-      }
-    };
-    if (team < work.count) {
-      zs = locate();
-      fetch();
-    }
-
-    bool ok = true;
+    bool ok = true, joined = false;
     int s = team, slot = team;  // nraw, slots >= kWtTeams
     uint32_t phase = 0;
     for (int u = team; u < work.count; u += kWtTeams) {
@@ -751,18 +957,10 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       uint4 sv[kGroups];
 #pragma unroll
       for (int i = 0; i < kGroups; ++i) {
-        zw[i] = zw_n[i];
-        sv[i] = sv_n[i];
+        zw[i] = scales.zw[i];
+        sv[i] = scales.sv[i];
       }
-      if (u + kWtTeams < work.count) {
-        k += kWtTeams;
-        zs += zs_step;
-        if (k >= k_end) {
-          settle();
-          zs = locate();
-        }
-        fetch();
-      }
+      if (u + kWtTeams < work.count) scales.next();
 
       // the unit's words, and the MMAs that read its A slot last; probed together, a wait of its own each took
       // 100 to 150 cycles with nothing to wait for
@@ -816,6 +1014,8 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       tc_fence_before();
       __syncwarp();
+      if (!joined) cluster_wait();  // the leader's barriers are set up
+      joined = true;
       mbar_arrive_both(full_leader + 8 * (u & (kWtMaxX - 1)), raw_empty(s), lane == 0);
       slot += kWtTeams;
       if (slot >= p.slots) slot -= p.slots;
@@ -825,14 +1025,18 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         phase ^= 1u;
       }
     }
+    if (!joined) cluster_wait();
   } else {
     // ------------------------------------------------------------------ epilogue
+    cluster_wait();
     const int e = warp - kWtEpiWarp0;
     const uint32_t ex_base = bar_base + kWtBarBytes;
     float* ex = reinterpret_cast<float*>(smem_raw + (ex_base - smem_u32(smem_raw)));
     if constexpr (WIDE) {
       const uint32_t stage = ex_base + (MODE == 1 ? kWtExBytes : 0) + e * (p.stage_bytes / kWtEpiWarps);
       wt_epilogue_wide<MODE, GROUP>(p, work, tmem, rank, e, lane, d_full(0), d_empty(0), ex, stage, &s_abort);
+    } else if constexpr (SPLIT) {
+      wt_epilogue_split<GROUP>(p, work, tmem, rank, e, lane, d_full(0), ex_base, part_full(e), &s_abort);
     } else {
       wt_epilogue<MODE, GROUP>(p, work, tmem, rank, e, lane, d_full(0), d_empty(0), ex,
                                x_base + e * (kWtPartRing * kWtPartBytes), part_full(e), &s_abort);
@@ -846,7 +1050,7 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     // tensor memory.  Let them land before both are given back.
     linger();
     // flags raised meanwhile: a replay of this launch must not find them
-    if (MODE == 0 && !WIDE && warp >= kWtEpiWarp0 && warp < kWtEpiWarp0 + kWtEpiWarps && work.segs > 0)
+    if (MODE == 0 && !WIDE && !SPLIT && warp >= kWtEpiWarp0 && warp < kWtEpiWarp0 + kWtEpiWarps && work.segs > 0)
       for (int c = 1 + lane; c <= work.helpers(work.segs - 1); c += 32)
         p.flags.lower(blockIdx.x - 2 * c, warp - kWtEpiWarp0);
   }
@@ -868,29 +1072,51 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 // ---- host side -------------------------------------------------------------------------------
 
 // Pairs of CTAs the GPU holds at once (one CTA per SM).
-template <int MODE, int GROUP, bool WIDE>
+template <int MODE, int GROUP, bool WIDE, bool SPLIT = false>
 int wt_pairs(int smem) {
   static std::atomic<int> cached[64][9];  // zero-initialised: not asked yet
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 1;
-  const int got = resident_clusters(gemm_wt_kernel<MODE, GROUP, WIDE>, 2, kWtThreads, smem, cached[dev]);
+  const int got = resident_clusters(gemm_wt_kernel<MODE, GROUP, WIDE, SPLIT>, 2, kWtThreads, smem, cached[dev]);
   const int most = sm_count() / 2 < kWtMaxPairs ? sm_count() / 2 : kWtMaxPairs;
   return got < most ? got : most;
 }
 
-template <int MODE, int GROUP, bool WIDE>
+template <int MODE, int GROUP, bool WIDE, bool SPLIT = false>
 int wt_prepare() {
   static std::atomic<bool> attr_done[64];  // zero-initialised; setting the attribute twice is harmless
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return AWQ_B200_ERR_DEVICE;
   if (!attr_done[dev]) {
-    if (cudaFuncSetAttribute(gemm_wt_kernel<MODE, GROUP, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (cudaFuncSetAttribute(gemm_wt_kernel<MODE, GROUP, WIDE, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              kWtSmemLimit) != cudaSuccess)
+      return AWQ_B200_ERR_LAUNCH;
+    if (SPLIT && cudaFuncSetAttribute(gemm_wt_kernel<MODE, GROUP, WIDE, SPLIT>,
+                                      cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
       return AWQ_B200_ERR_LAUNCH;
     attr_done[dev] = true;
   }
   return AWQ_B200_OK;
+}
+
+// How `pairs` pairs of a cluster share its `tiles` tiles of up to `nt` tokens: even ranges.
+WtShare wt_share(int pairs, int tiles, int KT, int nt) {
+  WtShare s = {};
+  s.pairs = pairs;
+  s.tiles = tiles;
+  for (int i = 0; i <= pairs; ++i) s.bound[i] = (short)((long)i * tiles * KT / pairs);
+  for (int t = 0; t < tiles; ++t) {
+    int a = 0, b = pairs - 1;
+    while (s.bound[a + 1] <= t * KT) ++a;
+    while (s.bound[b] >= (t + 1) * KT) --b;
+    const int n = b - a + 1, bytes = kWtEpiWarps * ((nt / 8 + n - 1) / n) * (n - 1) * 1024;
+    s.first[t] = (signed char)a;
+    s.count[t] = (signed char)n;
+    s.recip[t] = (65536 + n - 1) / n;
+    if (bytes > s.recv) s.recv = bytes;
+  }
+  return s;
 }
 
 // Ring depths for a tile of `nt` tokens; the rest of shared memory goes to the packed words, which
@@ -903,12 +1129,17 @@ int wt_rings(WtParams* p, int mode) {
   // epilogue; what TMEM is left over goes to A slots.
   p->nbuf = p->nt <= 128 ? 2 : 1;
   // One accumulator and whole tiles: the WIDE kernel.
-  p->stage_bytes = p->nbuf == 2 || p->chunk > 0 ? 0 : (p->nt + 31) / 32 * 32 * kWtCols * (mode == 1 ? 1 : 2);
-  const int fixed = 1024 + kWtBarBytes + (mode == 1 ? kWtExBytes : 0) + p->stage_bytes;
+  p->stage_bytes = p->nbuf == 2 || p->chunk > 0 || p->share.pairs > 0 ? 0 : (p->nt + 31) / 32 * 32 * kWtCols * (mode == 1 ? 1 : 2);
+  const int recv = p->share.pairs > 0 ? p->share.recv * (p->share.tiles > 1 ? 2 : 1) : 0;
+  const int fixed = 1024 + kWtBarBytes + (mode == 1 ? kWtExBytes : 0) + p->stage_bytes + recv;
   p->dcols = p->nt <= 64 ? 64 : 128;
   p->acol = p->nt <= 64 ? 128 : 256;
   p->slots = (kWtTmemCols - p->acol) / 64;
   p->nraw = (kWtSmemLimit - fixed - p->nx * p->xstage) / kWtRawBytes;
+  if (recv > 0 && p->nx == 8 && p->nraw < kWtTeams + p->slots) {
+    p->nx = 4;
+    p->nraw = (kWtSmemLimit - fixed - p->nx * p->xstage) / kWtRawBytes;
+  }
   if (p->nraw > kWtMaxRaw) p->nraw = kWtMaxRaw;
   // A team waits for unit u in the stage that unit u - nraw had.  Either it read that one itself, or it has seen
   // the MMAs of a later unit complete (u - 4 - slots, when it wrote unit u - 4); between the two, the parity of
@@ -917,10 +1148,10 @@ int wt_rings(WtParams* p, int mode) {
   return fixed + p->nx * p->xstage + p->nraw * kWtRawBytes;
 }
 
-template <int MODE, int GROUP, bool WIDE>
+template <int MODE, int GROUP, bool WIDE, bool SPLIT = false>
 int launch_wt_kernel(const CUtensorMap& map_w, const WtXMaps<MODE>& map_x, const WtParams& p, int pairs,
                      int smem, cudaStream_t stream) {
-  if (int rc = wt_prepare<MODE, GROUP, WIDE>()) return rc;
+  if (int rc = wt_prepare<MODE, GROUP, WIDE, SPLIT>()) return rc;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * pairs, 1, 1);
   cfg.blockDim = dim3(kWtThreads, 1, 1);
@@ -928,12 +1159,12 @@ int launch_wt_kernel(const CUtensorMap& map_w, const WtXMaps<MODE>& map_x, const
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.x = SPLIT ? 2 * p.share.pairs : 2;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = add_pdl_attribute(attr, 1);
-  if (cudaLaunchKernelEx(&cfg, gemm_wt_kernel<MODE, GROUP, WIDE>, map_w, map_x, p) != cudaSuccess) {
+  if (cudaLaunchKernelEx(&cfg, gemm_wt_kernel<MODE, GROUP, WIDE, SPLIT>, map_w, map_x, p) != cudaSuccess) {
     cudaGetLastError();
     return AWQ_B200_ERR_LAUNCH;
   }
@@ -951,9 +1182,12 @@ int make_wt_map(CUtensorMap* map_w, const uint32_t* qweight, int64_t wrows, int 
 size_t wt_partial_bytes(int nt, int pairs) { return (size_t)2 * pairs * nt * kWtCols * sizeof(float); }
 size_t wt_scratch_bytes(int nt, int pairs) { return wt_partial_bytes(nt, pairs) + handover::kFlagBytes; }
 
-// How a dense call is cut: tokens of a tile, and units of a pair's range (0: whole tiles, strided).
+// How a dense call is cut: tokens of a tile, and units of a pair's range (0: whole tiles, strided) or the pairs and
+// tiles of a cluster (SPLIT).
 struct WtPlan {
   int nt, chunk, pairs;
+  int share, share_tiles;
+  long cost;  // estimated time in ns
 };
 
 // Estimated time in ns of `tiles` tiles of `nt` tokens and KT units on `pairs` pairs (chunk as above).
@@ -996,16 +1230,12 @@ long wt_cost(int nt, int tiles, int KT, int chunk, int most, int pairs) {
 // fill the GPU the tiles stay whole and large, since the power limit then counts as well, and the waves of
 // tiles shall carry the fewest token columns in sequence.
 WtPlan wt_search(int M, int slabs, int KT, int most, bool split) {
-  WtPlan best = {0, 0, 1};
-  long best_cost = -1;
+  WtPlan best = {0, 0, 1, 0, 0, -1};
   const bool full = M > 256 && (long)slabs * ((M + 255) / 256) >= most;
   if (full) {
     for (int nt = 256; nt >= 128; nt -= 16) {
       const long tiles = (long)slabs * ((M + nt - 1) / nt), cost = (tiles + most - 1) / most * nt;
-      if (best_cost < 0 || cost < best_cost) {
-        best = {nt, 0, most};
-        best_cost = cost;
-      }
+      if (best.cost < 0 || cost < best.cost) best = {nt, 0, most, 0, 0, cost};
     }
     return best;
   }
@@ -1018,57 +1248,115 @@ WtPlan wt_search(int M, int slabs, int KT, int most, bool split) {
     const long units = (long)tiles * KT;
     const int even = (int)((units + most - 1) / most);
     for (int parts = 1; parts <= (split && units < (1 << 30) ? 6 : 1); ++parts) {
-      WtPlan plan = {nt, 0, tiles < most ? tiles : most};
+      WtPlan plan = {nt, 0, tiles < most ? tiles : most, 0, 0, 0};
       if (parts > 1) {
         const int floor = (KT + parts - 1) / parts;
         plan.chunk = even > floor ? even : floor;
         plan.pairs = (int)((units + plan.chunk - 1) / plan.chunk);
       }
-      const long cost = wt_cost(nt, tiles, KT, plan.chunk, most, plan.pairs);
-      if (best_cost < 0 || cost < best_cost) {
-        best = plan;
-        best_cost = cost;
-      }
+      plan.cost = wt_cost(nt, tiles, KT, plan.chunk, most, plan.pairs);
+      if (best.cost < 0 || plan.cost < best.cost) best = plan;
       if (plan.chunk == even) break;  // more parts: the same cut
     }
   }
   return best;
 }
 
-// The search takes a microsecond or two: a thread keeps the cuts it used last.
-WtPlan wt_plan(int M, int slabs, int KT, int most, bool split) {
+// Clusters of `pairs` pairs that share `tiles` tiles each, all in one wave: estimated time in ns; `resident` clusters
+// of that size fit the GPU.  Fitted to 550 cuts, 17 shapes from 1024 x 2048 to 14848 x 8192 at 11 batches from 33 to
+// 400 tokens, 4 % off on average.
+//   1170 + 25 nt + 144 pairs        start, the parts' way to the CTA that sums them, the sum
+//   units x max(...)                274: the conversion arithmetic; 2.3 nt: the tensor pipe; 5.1 pairs of the call: words
+//   1240 + 1510 x (...)             no room for the next kernel's clusters beside these: its start is not hidden
+//   18 nt - 600                     two tiles for three pairs: the middle pair sums parts of both
+long wt_cluster_cost(int nt, int pairs, int tiles, int clusters, int KT, int resident) {
+  long unit = 274;
+  if (unit < nt * 23 / 10) unit = nt * 23 / 10;
+  if (unit < (long)clusters * pairs * 51 / 10) unit = (long)clusters * pairs * 51 / 10;
+  long t = 1170 + 25 * nt + 144 * pairs + (tiles * KT + pairs - 1) / pairs * unit;
+  if (2 * clusters > resident) t += 1240 + 1510L * (2 * clusters - resident) / resident;
+  if (tiles > 1) t += 18 * nt - 600;
+  return t;
+}
+// The cheapest cut into clusters, if it is cheaper than `best` by more than the estimates are apart (400 ns: with it
+// the choice is 0.6 % from the best of all cuts on average; without 0.9 %, 24 % at worst).
+constexpr int kWtShares[][2] = {{2, 1}, {3, 1}, {4, 1}, {5, 1}, {6, 1}, {8, 1}, {3, 2}};  // pairs, tiles of a cluster
+template <typename Resident>
+WtPlan wt_cluster_search(WtPlan best, int M, int slabs, int KT, Resident resident) {
+  if (best.cost >= 0) best.cost -= 400;
+  for (int top = 256, last = 0; top >= 32; top -= 16) {
+    const int mtiles = (M + top - 1) / top, nt = ((M + mtiles - 1) / mtiles + 15) / 16 * 16;
+    if (nt == last) continue;
+    last = nt;
+    const int tiles = slabs * ((M + nt - 1) / nt);
+    for (const auto& s : kWtShares) {
+      const int pairs = s[0], per = s[1], clusters = tiles / per;
+      // two tiles in turn need two accumulators; every pair has a unit; WtShare counts in 16 bits
+      if (tiles % per != 0 || (long)per * KT > 32767 || (per > 1 && nt > 128) || KT < pairs || clusters > resident(pairs)) continue;
+      const long cost = wt_cluster_cost(nt, pairs, per, clusters, KT, resident(pairs));
+      if (best.cost >= 0 && cost >= best.cost) continue;
+      WtParams p = {};
+      p.nt = nt;
+      p.share = wt_share(pairs, per, KT, nt);
+      const int smem = wt_rings(&p, 0);
+      if (p.nraw >= kWtTeams && smem <= kWtSmemLimit) best = {nt, 0, clusters * pairs, pairs, per, cost};
+    }
+  }
+  return best;
+}
+
+// The search takes a few microseconds: a thread keeps the cuts it used last.  `resident`: nullptr for no clusters.
+WtPlan wt_plan(int M, int slabs, int KT, int most, bool split, int (*resident)(int pairs) = nullptr) {
   struct Entry {
     int M, slabs, KT, key;
+    int (*resident)(int);
     WtPlan plan;
   };
   static thread_local Entry seen[64];  // zero-initialised: M 0 is no call
   const unsigned hash = (unsigned)M * 2654435761u ^ (unsigned)slabs * 40503u ^ (unsigned)KT * 97u;
   Entry& e = seen[(hash >> 8) % 64];
   const int key = 2 * most + (split ? 1 : 0);
-  if (e.M != M || e.slabs != slabs || e.KT != KT || e.key != key)
-    e = Entry{M, slabs, KT, key, wt_search(M, slabs, KT, most, split)};
+  if (e.M != M || e.slabs != slabs || e.KT != KT || e.key != key || e.resident != resident) {
+    WtPlan plan = wt_search(M, slabs, KT, most, split);
+    // whole tiles that fill the GPU stay as they are
+    const bool full = M > 256 && (long)slabs * ((M + 255) / 256) >= most;
+    if (resident != nullptr && !full) plan = wt_cluster_search(plan, M, slabs, KT, resident);
+    e = Entry{M, slabs, KT, key, resident, plan};
+  }
   return e.plan;
+}
+
+// Clusters of that many pairs that the GPU holds at once.
+template <int GROUP>
+int wt_resident(int pairs) {
+  static std::atomic<int> cached[64][kMaxCluster + 1];  // zero-initialised: not asked yet
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  return resident_clusters(gemm_wt_kernel<0, GROUP, false, true>, 2 * pairs, kWtThreads, kWtSmemLimit, cached[dev]);
 }
 
 template <int GROUP>
 int launch_wt_dense(const __half* x, const uint32_t* qweight, WtParams p, void* workspace,
-                    size_t workspace_bytes, cudaStream_t stream) {
+                    size_t workspace_bytes, bool clusters, cudaStream_t stream) {
   if (int rc = wt_prepare<0, GROUP, false>()) return rc;
+  if (int rc = wt_prepare<0, GROUP, false, true>()) return rc;
   p.slabs = (p.N + kWtBN - 1) / kWtBN;
   p.KT = p.K / kWtBK;
   const int most = wt_pairs<0, GROUP, false>(kWtSmemLimit);
-  WtPlan plan = wt_plan(p.M, p.slabs, p.KT, most, true);
+  const auto resident = clusters ? wt_resident<GROUP> : nullptr;
+  WtPlan plan = wt_plan(p.M, p.slabs, p.KT, most, true, resident);
   if (plan.chunk > 0) {
     if (workspace != nullptr && workspace_bytes >= wt_scratch_bytes(plan.nt, plan.pairs)) {
       p.partial = static_cast<float*>(workspace);
       p.flags = handover::make_flags(workspace, wt_partial_bytes(plan.nt, plan.pairs));
     } else {
-      plan = wt_plan(p.M, p.slabs, p.KT, most, false);
+      plan = wt_plan(p.M, p.slabs, p.KT, most, false, resident);
     }
   }
   p.nt = plan.nt;
   p.chunk = plan.chunk;
   p.mtiles = (p.M + p.nt - 1) / p.nt;
+  if (plan.share > 0) p.share = wt_share(plan.share, plan.share_tiles, p.KT, p.nt);
   const int smem = wt_rings(&p, 0);
   CUtensorMap map_w;
   WtXMaps<0> map_x;
@@ -1078,6 +1366,7 @@ int launch_wt_dense(const __half* x, const uint32_t* qweight, WtParams p, void* 
     const int boxes = ((rows[i] + 15) / 16 * 8 + 15) / 16;
     if (int rc = encode_map_x(&map_x.map[i], x, p.M, p.K, boxes * 16)) return rc;
   }
+  if (plan.share > 0) return launch_wt_kernel<0, GROUP, false, true>(map_w, map_x, p, plan.pairs, smem, stream);
   return p.stage_bytes > 0 ? launch_wt_kernel<0, GROUP, true>(map_w, map_x, p, plan.pairs, smem, stream)
                            : launch_wt_kernel<0, GROUP, false>(map_w, map_x, p, plan.pairs, smem, stream);
 }
@@ -1114,7 +1403,7 @@ int gemm_wt_cut(int M, int N, int K, int group, int cta_pairs, int* tokens, int*
 
 int launch_gemm_wt(const __half* x, const uint32_t* qweight, const __half* scales,
                    const uint32_t* qzeros, const __half* bias, __half* out, int M, int N, int K,
-                   int group, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
+                   int group, void* workspace, size_t workspace_bytes, bool clusters, cudaStream_t stream) {
   if (!gemm_wt_supported(M, N, K, group)) return AWQ_B200_ERR_SHAPE;
   WtParams p = {};
   p.scales = scales;
@@ -1124,8 +1413,8 @@ int launch_gemm_wt(const __half* x, const uint32_t* qweight, const __half* scale
   p.M = M;
   p.N = N;
   p.K = K;
-  return group == 128 ? launch_wt_dense<128>(x, qweight, p, workspace, workspace_bytes, stream)
-                      : launch_wt_dense<64>(x, qweight, p, workspace, workspace_bytes, stream);
+  return group == 128 ? launch_wt_dense<128>(x, qweight, p, workspace, workspace_bytes, clusters, stream)
+                      : launch_wt_dense<64>(x, qweight, p, workspace, workspace_bytes, clusters, stream);
 }
 
 namespace {

@@ -88,8 +88,8 @@ struct Work {
       end = KT;
     }
   }
-  // Stages [k0, k1) of one tile.
-  __device__ __forceinline__ static Work part(int tile, int k0, int k1, int KT) { return Work(tile, k0, k1, KT, true); }
+  // Units [first, last) of the list, for workers that hand nothing over through scratch.
+  __device__ __forceinline__ static Work range(int first, int last, int KT) { return Work(first, last, KT); }
   __device__ __forceinline__ int tile_id(int seg) const {
     return chunked ? tile0 + segs - 1 - seg : worker + seg * workers;
   }
@@ -103,9 +103,14 @@ struct Work {
   }
 
  private:
-  __device__ __forceinline__ Work(int tile, int k0, int k1, int KT_, bool)
-      : worker(0), workers(1), KT(KT_), chunk(1), segs(k1 > k0 ? 1 : 0), count(k1 - k0), begin(k0), end(k1), tile0(tile),
-        chunked(true) {}
+  __device__ __forceinline__ Work(int first, int last, int KT_)
+      : worker(0), workers(1), KT(KT_), chunk(1), count(last - first), chunked(true) {
+    tile0 = first / KT;
+    const int top = (last - 1) / KT;
+    segs = count > 0 ? top - tile0 + 1 : 0;
+    begin = first - tile0 * KT;
+    end = last - top * KT;
+  }
 };
 
 // Two tokens of 32 columns per step: this lane's column of tokens c, c + 1 packed to fp16, then

@@ -320,6 +320,19 @@ __device__ __forceinline__ void tmem_ld_16x256b_x4(uint32_t taddr, float (&r)[16
 #pragma unroll
   for (int i = 0; i < 16; ++i) r[i] = __uint_as_float(v[i]);
 }
+// The same of 8 and 16 columns.
+__device__ __forceinline__ void tmem_ld_16x256b_x1(uint32_t taddr, float (&r)[4]) {
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x1.b32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3])
+               : "r"(taddr)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_ld_16x256b_x2(uint32_t taddr, float (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7])
+               : "r"(taddr)
+               : "memory");
+}
 // 8 x 8 fp16 matrix, two neighbouring values of row g per thread (g, t): transposed
 __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t v) {
   uint32_t r;
@@ -351,6 +364,12 @@ __device__ __forceinline__ uint32_t map_rank(uint32_t saddr, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
   return r;
 }
+// Four values into another CTA's shared memory, counted by a barrier there (both addresses as map_rank gives them).
+__device__ __forceinline__ void st_async_v4(uint32_t dst, const float* v, uint32_t bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(dst),
+               "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "r"(bar)
+               : "memory");
+}
 // Arrive on a barrier given by its cluster address (own or peer CTA).  What such arrivals hand over is
 // tensor memory, ordered by the tcgen05 fences around them, so the default CTA scope is enough; the
 // cluster-scope forms (release / acquire) add memory barriers: 65 against 55 us for the whole kernel
@@ -379,12 +398,13 @@ __device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap
 }
 // A 256-row MMA over the pair: rows 0-127 in the leader's tensor memory, 128-255 in the peer's; each
 // CTA holds half of B's rows at the same shared-memory offset.
-// Arrives on the barrier at this offset in both CTAs once the pair's MMAs so far are complete.
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
+// Arrives on the barrier at this offset in both CTAs (`mask`: their ranks in the cluster) once the pair's MMAs so far
+// are complete.
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar, uint16_t mask = 3) {
   asm volatile(
       "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 "
       "[%0], %1;" ::"r"(bar),
-      "h"((uint16_t)3)
+      "h"(mask)
       : "memory");
 }
 // One unit of a tile whose A operand lies in tensor memory: eight MMAs of K = 16 over the 128 k of an
@@ -394,7 +414,8 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
 // ~100 cycles).  Returns whether the next unit is ready.  One elected lane of the leader.
 __device__ __forceinline__ bool umma_unit_pair(uint32_t dcol, uint32_t acol, uint64_t dx,
                                                uint32_t half, uint32_t idesc, uint32_t acc,
-                                               uint32_t done, uint32_t next, uint32_t next_parity) {
+                                               uint32_t done, uint32_t next, uint32_t next_parity,
+                                               uint16_t mask = 3) {
   uint32_t ready;
   asm volatile(
       "{\n\t.reg .pred t, p, q;\n\t"
@@ -432,7 +453,7 @@ __device__ __forceinline__ bool umma_unit_pair(uint32_t dcol, uint32_t acol, uin
       "selp.u32 %0, 1, 0, t;\n\t}"
       : "=r"(ready)
       : "r"(dcol), "r"(acol), "l"(dx), "r"(half), "r"(idesc), "r"(acc), "r"(done), "r"(next),
-        "r"(next_parity), "h"((uint16_t)3)
+        "r"(next_parity), "h"(mask)
       : "memory");
   return ready != 0;
 }

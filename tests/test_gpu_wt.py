@@ -194,3 +194,34 @@ def test_wt_wide_tiles(A, m, k, n, group, tokens, split):
     # fp16 weights and output: 2^-11 each, far inside TOL
     assert O.rel_err(y[0].cpu().numpy(), ref) < TOL
     assert O.elementwise_ok(y[0].cpu().numpy(), ref, TOL)
+
+
+# Tiles shared by clusters (by the estimated cost of a B200's cuts): two to eight pairs a tile, two tiles for three
+# pairs, units that do not divide by the pairs, one unit a pair, an edge of N, several tiles of tokens with a shorter
+# last one, one accumulator (more than 128 tokens).
+@pytest.mark.parametrize("m,k,n,group", [
+    (40, 1024, 4096, 128), (130, 512, 2048, 64), (33, 384, 1056, 128), (97, 640, 2048, 128), (77, 4096, 4096, 64),
+    (100, 8192, 1280, 128), (300, 8192, 1312, 64), (150, 11008, 1536, 128), (60, 16384, 544, 128),
+    (100, 8192, 10240, 128), (48, 4352, 10208, 64), (250, 8192, 5120, 128), (500, 8192, 2080, 128)])
+@pytest.mark.parametrize("bias", [False, True])
+def test_wt_clusters_share_tiles(A, m, k, n, group, bias):
+    """Weights rounded to (q - z) * s and the output are all that is rounded to fp16; the bits do not depend on timing."""
+    from awq_b200 import synth
+    qw, s, qz = synth.awq_linear_tensors(k, n, group, seed=m + n)
+    x = synth.activations(m, k, seed=k)
+    b = synth.activations(1, n, seed=3)[0] if bias else None
+    c = max(0, n - 768)  # first column of the oracle: the last ones, with the edge
+    w = O.dequantize_fp32(qw[:, c // 8:].numpy(), s[:, c:].numpy(), qz[:, c // 8:].numpy(), group)
+    ref = x.double() @ torch.from_numpy(w).half().double()  # the fp32 product of 5 and 11 bits is exact
+    if bias:
+        ref += b[c:].double()
+    dev = [t.cuda() for t in (x, qw, s, qz)]
+    outs = [A.awq_gemm(*dev, 8, bias=b.cuda() if bias else None) for _ in range(3)]
+    named = A.awq_gemm(*dev, 8, bias=b.cuda() if bias else None, kernel=A.KERNEL_WT)
+    torch.cuda.synchronize()
+    assert device_status() == 0, "a bounded wait ran out"
+    assert all(torch.equal(outs[0], y) for y in outs[1:])
+    rounding = (ref.half().double() - ref).norm()
+    # 5 %: the fp32 sums, K * 2^-24 of their terms' size at most, move few values to the other side
+    for y in (outs[0], named):
+        assert (y.cpu()[:, c:].double() - ref).norm() < 1.05 * rounding
