@@ -275,7 +275,7 @@ constexpr int kMoeDirectTicketBytes = 4096;  // AWQ_B200_MOE_DIRECT_MAX_PAIRS to
 // gemm_ts.cu: expert GEMMs of small batches
 bool moe_ts_supported(const MoeArgs& a);
 size_t moe_ts_partial_bytes(int block);
-int launch_moe_ts(const MoeArgs& a, __half* act, int64_t act_rows, __half* pair_out, float* partial,
+int launch_moe_ts(const MoeArgs& a, __half* act, int64_t act_rows, __half* pair_out, float* partial, bool* summed,
                   cudaStream_t stream);
 int launch_moe_local_ids(const int32_t* topk_ids, int n, const int32_t* expert_map, int E,
                          int32_t* out, cudaStream_t stream);

@@ -57,6 +57,11 @@
 //   MODE 2  down: rows of act; epilogue pair_out[pair] = routed weight * D, rounded as in the other expert
 //           kernels, for a sum over the slots afterwards.  Direct form: a pair without an expert here
 //           (negative id) gets a row of zeros.
+// SPLIT, direct form: MODE 1 as a dense layer, every CTA with the same units of gate and up.  MODE 2: the CTAs of a
+// cluster have the slots of a token, each the whole matrix, and add the rounded rows in slot order, so that no kernel for
+// the sum follows.  Experts of 128 x 2048 x 768, one token, top-8 16.2 -> 14.45 us; 64 of 2048 x 1024 17.1 -> 15.4; two
+// tokens, top-4 15.5 -> 14.4.  (With zero points subtracted in the conversion 0.1 us slower, and other roundings than
+// through the permutation.)
 //
 // unit_full counts the conversion warps, the announcement of the tokens and the fold warps of the unit
 // NDB before, whose accumulators the MMAs overwrite.  mma_done counts the MMA warp's commit and the
@@ -119,14 +124,14 @@ constexpr int kTsColD = 128;                           // TMEM columns of the ac
 constexpr int kTsCvWarps = 4 * kTsTeams;
 static_assert(kTsColD + kTsTeams * 128 <= kTsTmemCols, "TMEM columns");
 // What depends on the quantisation group (128 or 64: one or two of a unit) and on the tokens.
-template <int MT, int GROUP, bool SPLIT = false>
+template <int MT, int MODE, int GROUP, bool SPLIT = false>
 struct TsCfg {
   static constexpr int G = kTsBK / GROUP;              // groups of a unit
   static constexpr int NT = MT <= 16 ? 16 : 32;        // tokens of the B operand
   static constexpr int kFoldWarps = 8;
   static constexpr int kFold0 = kTsCvWarps, kIssue = kFold0 + kFoldWarps;
   // the conversion subtracts the zero points: no token sums
-  static constexpr bool SUB = SPLIT || MT > 16 || (MT == 16 && GROUP == 64);
+  static constexpr bool SUB = (SPLIT && MODE == 0) || MT > 16 || (MT == 16 && GROUP == 64);
   static constexpr int kIssueWarps = SUB ? 2 : 1;
   static constexpr int kSum = kIssue + kIssueWarps, kXWarp = kSum + (SUB ? 0 : 1), kRaw = kXWarp + 1;
   static constexpr int kThreads = 32 * (kRaw + 1);     // 768
@@ -246,16 +251,29 @@ __device__ __forceinline__ Work ts_work(const TsParams& p) {
   return Work(blockIdx.x, gridDim.x, tiles, KT, max(1, max(even, least)));
 }
 
+// SPLIT: a cluster's tile.  MODE 2: the CTAs of a cluster have the slots of a token, whole.
+template <int MODE>
+__device__ __forceinline__ Work ts_split_work(const TsParams& p, int rank, int kt) {
+  const int cluster = blockIdx.x / p.split;
+  if (MODE == 0)
+    return Work::range(cluster * p.KT + rank * p.KT / p.split, cluster * p.KT + (rank + 1) * p.KT / p.split, p.KT);
+  if (MODE == 1) return Work::range(cluster * 2 * kt, (cluster + 1) * 2 * kt, 2 * kt);
+  const int token = cluster / p.slabs, tile = (token * p.split + rank) * p.slabs + cluster - token * p.slabs;
+  return Work::range(tile * p.KT, (tile + 1) * p.KT, p.KT);
+}
+
 // A load stream's walk over the CTA's units: the weight rows / group row of every unit, and the column
 // slab.  The expert of the next matrix is fetched while the current one is loaded.
 template <int MODE>
 struct TsWalk {
   const TsParams& p;
   const Work& work;
+  const int kt, unit0;  // units of a matrix that the walk has, and the first
   int u = 0, seg = 0, k = 0, k_end = 0, tile = 0, slab = 0;
   int expert = 0, expert_next = 0;
   bool fetched = false;
-  __device__ __forceinline__ TsWalk(const TsParams& p_, const Work& w_) : p(p_), work(w_) {}
+  __device__ __forceinline__ TsWalk(const TsParams& p_, const Work& w_, int kt_, int unit0_)
+      : p(p_), work(w_), kt(kt_), unit0(unit0_) {}
   // Positions on unit u; returns whether a new tile begins.  MODE 1: k counts gate units, then up.
   __device__ __forceinline__ bool settle() {
     if (k != k_end) return false;
@@ -277,17 +295,17 @@ struct TsWalk {
     ++u;
     ++k;
   }
-  __device__ __forceinline__ bool up() const { return MODE == 1 && k >= p.KT; }
-  __device__ __forceinline__ int unit() const { return up() ? k - p.KT : k; }  // inside the matrix
+  __device__ __forceinline__ bool up() const { return MODE == 1 && k >= kt; }
+  __device__ __forceinline__ int unit() const { return unit0 + (up() ? k - kt : k); }  // inside the matrix
   __device__ __forceinline__ int column() const { return slab * kTsBN + (up() ? p.half_cols : 0); }
 };
 
 template <int MT, int MODE, int GROUP, bool SPLIT>
-__global__ void __launch_bounds__((TsCfg<MT, GROUP, SPLIT>::kThreads), 1)
+__global__ void __launch_bounds__((TsCfg<MT, MODE, GROUP, SPLIT>::kThreads), 1)
 gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_s,
                const __grid_constant__ CUtensorMap map_z, const __grid_constant__ CUtensorMap map_x,
                const TsParams p) {
-  using Cfg = TsCfg<MT, GROUP, SPLIT>;
+  using Cfg = TsCfg<MT, MODE, GROUP, SPLIT>;
   constexpr int NT = Cfg::NT, G = Cfg::G, NDB = Cfg::NDB, NRAW = Cfg::NRAW, kSz = Cfg::kSz, kTsXBytes = Cfg::kX;
   constexpr int kTsFoldWarps = Cfg::kFoldWarps, kTsFold0 = Cfg::kFold0, kTsIssue = Cfg::kIssue, kIssueWarps = Cfg::kIssueWarps;
   constexpr bool SUB = Cfg::SUB, kRawZeros = MODE == 1 || SUB;  // zero points with the packed words
@@ -331,9 +349,10 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   if (MODE == 1) pdl_wait();
   pdl_launch_dependents();
   const int rank = SPLIT ? blockIdx.x % p.split : 0;
-  const Work work = SPLIT ? Work::range(blockIdx.x / p.split * p.KT + rank * p.KT / p.split,
-                                         blockIdx.x / p.split * p.KT + (rank + 1) * p.KT / p.split, p.KT)
-                          : ts_work<MT, MODE>(p);
+  // MODE 1, SPLIT: this CTA's units of gate, then the same of up
+  const int unit0 = SPLIT && MODE == 1 ? rank * p.KT / p.split : 0;
+  const int kt = SPLIT && MODE == 1 ? (rank + 1) * p.KT / p.split - unit0 : p.KT;
+  const Work work = SPLIT ? ts_split_work<MODE>(p, rank, kt) : ts_work<MT, MODE>(p);
   // SPLIT: barrier and shared memory of the n-th piece that this CTA sums, partial sums of CTA `from`
   auto recv_full = [&](int n) { return bar_base + 8 * (2 * NRAW + 2 * kTsUnits + n); };
   auto recv_at = [&](int n, int from) { return bar_base + 512 + (n * p.split + from) * Cfg::kPieceBytes; };
@@ -344,7 +363,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 
   // packed words, scales, MODE 1 also zero points (raw warp, converged: an elected lane issues; TMAs
   // of a lane that loops alone take it longer)
-  TsWalk<MODE> raw(p, work);
+  TsWalk<MODE> raw(p, work, kt, unit0);
   int raw_s = 0;
   uint32_t raw_phase = 0;
   auto load_raw = [&]() {
@@ -393,7 +412,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       const int quads = piece_quads((lane * p.split + rank) / 8);
       mbar_init(recv_full(lane), 2);  // the bytes of the other CTAs, the warp here that has the piece
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-      mbar_arrive_expect_tx(recv_full(lane), (p.split - 1) * quads * 512);
+      mbar_arrive_expect_tx(recv_full(lane), (p.split - 1) * (MODE == 0 ? quads * 512 : 256));
     }
   }
   __syncwarp();
@@ -417,7 +436,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   } else if (warp == kTsX) {
     // ------------------------------------------------------------------ tokens (zero points)
     pdl_wait();  // the activations may be the output of the kernel before this one
-    TsWalk<MODE> x(p, work);
+    TsWalk<MODE> x(p, work, kt, unit0);
     bool ok = true;
     int row = 0, fid_next = -1, quads = MT / 4;
     int rows[MODE == 1 ? MT : 1];  // MODE 1: the block's rows of x
@@ -663,7 +682,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 #pragma unroll
       for (int m = 0; m < MT / 2; ++m) tot[m] = 0ull;
       for (int k = ok || kStay ? kb : ke; k < ke; ++k, ++u) {
-        if (MODE == 1 && k == p.KT && kb < p.KT) {  // gate complete: park its sums, start on up
+        if (MODE == 1 && k == kt && kb < kt) {  // gate complete: park its sums, start on up
 #pragma unroll
           for (int m = 0; m < MT / 2; ++m) {
             const float2 v = unpack2(tot[m]);
@@ -746,6 +765,25 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         const float2 t = unpack2(tot[m]);
         v[2 * m] = t.x;
         v[2 * m + 1] = t.y;
+      }
+      if constexpr (SPLIT && MODE != 0) {
+        // direct form: one row.  MODE 1: gate and up; MODE 2: the pair's weighted row, rounded as ever
+        float a = gate[0], b = v[0];
+        if (MODE == 2) {
+          a = valid ? __half2float(__float2half_rn(v[0] * unscale * __shfl_sync(0xffffffffu, fw, 0))) : 0.f;
+          b = 0.f;
+        }
+        cluster_wait();
+        const int owner = fold % p.split, n = fold / p.split;
+        const uint32_t dst = recv_at(n, rank) + lane * 8;
+        if (owner == rank) {
+          asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(dst), "f"(a), "f"(b) : "memory");
+          __syncwarp();
+          if (lane == 0) mbar_arrive(recv_full(n));
+        } else {
+          st_async_v2(map_rank(dst, owner), a, b, map_rank(recv_full(n), owner));
+        }
+        continue;
       }
       if constexpr (SPLIT) {
         constexpr int T = Cfg::kPieceTokens, Q = T / 4;
@@ -872,7 +910,32 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     }
   }
 
-  if constexpr (SPLIT) {
+  if constexpr (SPLIT && MODE != 0) {
+    const int fold = warp - kTsFold0, piece = fold * p.split + rank;
+    if (fold >= 0 && piece < Cfg::kPieces) {
+      __syncwarp();
+      const int cluster = blockIdx.x / p.split, row = cluster / p.slabs, slab = cluster - row * p.slabs;
+      const int g = lane & 7, i = lane >> 3, width = MODE == 1 ? p.half_cols : p.N;
+      const int n0 = slab * kTsBN + 32 * piece + 8 * (g >> 1) + 2 * i;
+      const bool valid = MODE == 2 || __ldcg(p.expert_ids + row) >= 0;
+      const bool ok = __all_sync(0xffffffffu, mbar_wait_cluster(recv_full(fold), 0, &s_abort, 25));
+      float a = 0.f, b = 0.f;
+      for (int r = 0; r < p.split; ++r) {
+        float x, y;
+        asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(x), "=f"(y) : "r"(recv_at(fold, r) + lane * 8));
+        a += x;
+        b += y;
+      }
+      if (MODE == 1) {
+        const float unscale = (i & 1) ? 1048576.f : 16777216.f;
+        a *= unscale;
+        a = b * unscale * __fdividef(a, 1.f + __expf(-a));
+      }
+      const float other = __shfl_xor_sync(0xffffffffu, a, 1);
+      if (ok && !s_abort && valid && n0 < width && (lane & 1) == 0)
+        *reinterpret_cast<__half2*>(p.out + (size_t)row * width + n0) = __floats2half2_rn(a, other);
+    }
+  } else if constexpr (SPLIT) {
     // ------------------------------------------------------------------ sums over the cluster
     // The quads of this CTA's pieces, shared out over the warps that convert and fold, are summed in the CTAs' order.
     // Rolled loops: the code is cold.
@@ -998,19 +1061,27 @@ long ts_split_cost(int slabs, int KT, int tokens, int group, int split, int resi
   return cost;
 }
 
+// MODE 2, SPLIT: the CTAs of a cluster have a token's slots, whole, and add them up: estimated time, against ranges and
+// a kernel for the sum.
+constexpr long kTsSumKernel = 2200;
+long ts_slots_cost(int slabs, int clusters, int KT, int topk) {
+  const int arith = 363, words = clusters * topk * 31 / 10;
+  return 2050 + (long)KT * (arith > words ? arith : words) + 12 * topk;
+}
+
 struct TsMaps {
   CUtensorMap w, s, z, x;
 };
 
 // Attributes of a SPLIT kernel, and how many of its clusters of every size the GPU holds at once.
-template <int MT, int GROUP>
+template <int MT, int GROUP, int MODE = 0>
 int ts_prepare_split() {
   static std::atomic<bool> attr_done[64];  // as in launch_ts
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return AWQ_B200_ERR_DEVICE;
   if (!attr_done[dev]) {
-    auto kernel = gemm_ts_kernel<MT, 0, GROUP, true>;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TsCfg<MT, GROUP, true>::kSmem) !=
+    auto kernel = gemm_ts_kernel<MT, MODE, GROUP, true>;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TsCfg<MT, MODE, GROUP, true>::kSmem) !=
             cudaSuccess ||
         cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
       return AWQ_B200_ERR_LAUNCH;
@@ -1018,21 +1089,21 @@ int ts_prepare_split() {
   }
   return AWQ_B200_OK;
 }
-template <int MT, int GROUP>
+template <int MT, int GROUP, int MODE = 0>
 int ts_resident(int split) {
   static std::atomic<int> cached[64][kMaxCluster + 1];  // zero-initialised: not asked yet
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-  using Cfg = TsCfg<MT, GROUP, true>;
-  return resident_clusters(gemm_ts_kernel<MT, 0, GROUP, true>, split, Cfg::kThreads, Cfg::kSmem, cached[dev]);
+  using Cfg = TsCfg<MT, MODE, GROUP, true>;
+  return resident_clusters(gemm_ts_kernel<MT, MODE, GROUP, true>, split, Cfg::kThreads, Cfg::kSmem, cached[dev]);
 }
 
-template <int MT, int GROUP>
+template <int MT, int GROUP, int MODE = 0>
 TsCut ts_cut(int slabs, int KT) {
   TsCut best = ts_ranges(slabs, KT, MT);
   for (const int split : {2, 3, 4, 5, 6, 8, 16}) {
     if (split > KT) break;
-    const int resident = ts_resident<MT, GROUP>(split);
+    const int resident = ts_resident<MT, GROUP, MODE>(split);
     if (slabs > resident) continue;
     const long cost = ts_split_cost(slabs, KT, MT, GROUP, split, resident);
     if (cost < best.cost) best = {split, 0, cost};
@@ -1040,11 +1111,11 @@ TsCut ts_cut(int slabs, int KT) {
   return best;
 }
 
-template <int MT, int GROUP>
-int launch_ts_split(const TsMaps& maps, const TsParams& p, cudaStream_t stream) {
-  using Cfg = TsCfg<MT, GROUP, true>;
+template <int MT, int GROUP, int MODE = 0>
+int launch_ts_split(const TsMaps& maps, const TsParams& p, int clusters, cudaStream_t stream) {
+  using Cfg = TsCfg<MT, MODE, GROUP, true>;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(p.slabs * p.split, 1, 1);
+  cfg.gridDim = dim3(clusters * p.split, 1, 1);
   cfg.blockDim = dim3(Cfg::kThreads, 1, 1);
   cfg.dynamicSmemBytes = Cfg::kSmem;
   cfg.stream = stream;
@@ -1055,7 +1126,7 @@ int launch_ts_split(const TsMaps& maps, const TsParams& p, cudaStream_t stream) 
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = add_pdl_attribute(attr, 1);
-  if (cudaLaunchKernelEx(&cfg, gemm_ts_kernel<MT, 0, GROUP, true>, maps.w, maps.s, maps.z, maps.x, p) != cudaSuccess) {
+  if (cudaLaunchKernelEx(&cfg, gemm_ts_kernel<MT, MODE, GROUP, true>, maps.w, maps.s, maps.z, maps.x, p) != cudaSuccess) {
     cudaGetLastError();
     return AWQ_B200_ERR_LAUNCH;
   }
@@ -1069,14 +1140,14 @@ int launch_ts(const TsMaps& maps, const TsParams& p, int ctas, cudaStream_t stre
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return AWQ_B200_ERR_DEVICE;
   auto kernel = gemm_ts_kernel<MT, MODE, GROUP, false>;
-  constexpr int smem = TsCfg<MT, GROUP>::kSmem;
+  constexpr int smem = TsCfg<MT, MODE, GROUP>::kSmem;
   if (!attr_done[dev]) {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
         cudaSuccess)
       return AWQ_B200_ERR_LAUNCH;
     attr_done[dev] = true;
   }
-  if (launch_pdl(kernel, dim3(ctas), dim3(TsCfg<MT, GROUP>::kThreads), smem, stream, maps.w, maps.s, maps.z,
+  if (launch_pdl(kernel, dim3(ctas), dim3(TsCfg<MT, MODE, GROUP>::kThreads), smem, stream, maps.w, maps.s, maps.z,
                  maps.x, p) != cudaSuccess) {
     cudaGetLastError();
     return AWQ_B200_ERR_LAUNCH;
@@ -1125,16 +1196,18 @@ int launch_ts_dense(const __half* x, const uint32_t* qweight, const __half* scal
   }
   TsMaps maps;
   if (int rc = ts_weight_maps(&maps, qweight, scales, qzeros, (uint64_t)p.K, (uint64_t)p.N, GROUP)) return rc;
-  if (int rc = encode_map_x(&maps.x, x, (uint64_t)p.M, (uint64_t)p.K, TsCfg<MT, GROUP>::NT)) return rc;
-  if (p.split > 1) return launch_ts_split<MT, GROUP>(maps, p, stream);
+  if (int rc = encode_map_x(&maps.x, x, (uint64_t)p.M, (uint64_t)p.K, TsCfg<MT, 0, GROUP>::NT)) return rc;
+  if (p.split > 1) return launch_ts_split<MT, GROUP>(maps, p, p.slabs, stream);
   return launch_ts<MT, 0, GROUP>(maps, p, ctas, stream);
 }
 
 // Expert GEMMs: gate_up, then down.
+// *summed: whether the sum over a token's slots is done as well (MODE 2, SPLIT).
 template <int MT>
-int launch_ts_experts(const MoeArgs& a, __half* act, int64_t act_rows, __half* pair_out, TsParams p,
+int launch_ts_experts(const MoeArgs& a, __half* act, int64_t act_rows, __half* pair_out, TsParams p, bool* summed,
                       cudaStream_t stream) {
   const int ctas = ts_ctas();
+  *summed = false;
   p.flags = handover::make_flags(p.partial, 2 * ts_partial_bytes(MT));
   p.sorted_ids = a.sorted_ids;
   p.expert_ids = a.expert_ids;
@@ -1159,7 +1232,17 @@ int launch_ts_experts(const MoeArgs& a, __half* act, int64_t act_rows, __half* p
                                        CU_TENSOR_MAP_SWIZZLE_128B)
                        : encode_map_x(&maps.x, a.x, (uint64_t)a.T, (uint64_t)a.H, 16);
     if (rc) return rc;
-    if (int rc2 = launch_ts<MT, 1>(maps, p, ctas, stream)) return rc2;
+    bool split = false;
+    if constexpr (MT == 4) {
+      // Direct form, the number of tiles is known: clusters as for a dense layer of that many slabs and twice the units
+      if (int rc2 = ts_prepare_split<MT, 128, 1>()) return rc2;
+      if (p.sorted_ids == nullptr) p.split = ts_cut<MT, 128, 1>(p.numel * p.slabs, 2 * p.KT).split;
+      split = p.split > 1 && p.split <= 8 && p.split <= p.KT;
+      if (split)
+        if (int rc2 = launch_ts_split<MT, 128, 1>(maps, p, p.numel * p.slabs, stream)) return rc2;
+    }
+    if (!split)
+      if (int rc2 = launch_ts<MT, 1>(maps, p, ctas, stream)) return rc2;
   }
   p.K = a.I;
   p.N = a.H;
@@ -1171,6 +1254,19 @@ int launch_ts_experts(const MoeArgs& a, __half* act, int64_t act_rows, __half* p
   if (int rc = ts_weight_maps(&maps, a.w2_q, a.w2_s, a.w2_z, (uint64_t)a.E * a.I, (uint64_t)a.H))
     return rc;
   if (int rc = encode_map_x(&maps.x, act, (uint64_t)act_rows, I, 16)) return rc;
+  if constexpr (MT == 4) {
+    if (int rc = ts_prepare_split<MT, 128, 2>()) return rc;
+    if (p.sorted_ids == nullptr && a.topk > 1 && a.topk <= 8) {
+      const int clusters = a.T * p.slabs, resident = ts_resident<MT, 128, 2>(a.topk);
+      if (clusters <= resident && ts_slots_cost(p.slabs, clusters, p.KT, a.topk) <
+                                      ts_ranges(p.numel * p.slabs, p.KT, MT).cost + kTsSumKernel) {
+        *summed = true;
+        p.split = a.topk;
+        p.out = a.out;
+        return launch_ts_split<MT, 128, 2>(maps, p, clusters, stream);
+      }
+    }
+  }
   return launch_ts<MT, 2>(maps, p, ctas, stream);
 }
 
@@ -1215,13 +1311,13 @@ size_t moe_ts_partial_bytes(int block) { return 2 * ts_partial_bytes(block) + ha
 
 // Both expert GEMMs of a small batch, pair_out by pair.  Rows of act by position, direct (no
 // permutation) by pair.
-int launch_moe_ts(const MoeArgs& a, __half* act, int64_t act_rows, __half* pair_out, float* partial,
+int launch_moe_ts(const MoeArgs& a, __half* act, int64_t act_rows, __half* pair_out, float* partial, bool* summed,
                   cudaStream_t stream) {
   TsParams p = {};
   p.partial = partial;
-  if (a.direct) return launch_ts_experts<4>(a, act, act_rows, pair_out, p, stream);
-  return a.block == 8 ? launch_ts_experts<8>(a, act, act_rows, pair_out, p, stream)
-                      : launch_ts_experts<16>(a, act, act_rows, pair_out, p, stream);
+  if (a.direct) return launch_ts_experts<4>(a, act, act_rows, pair_out, p, summed, stream);
+  return a.block == 8 ? launch_ts_experts<8>(a, act, act_rows, pair_out, p, summed, stream)
+                      : launch_ts_experts<16>(a, act, act_rows, pair_out, p, summed, stream);
 }
 
 int ts_device_status(int* out, int clear) { return read_tc_status(out, clear); }

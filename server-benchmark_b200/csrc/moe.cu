@@ -830,8 +830,9 @@ int launch_moe_experts(const MoeArgs& a, void* workspace, size_t workspace_bytes
       return AWQ_B200_ERR_LAUNCH;
   }
   int rc;
+  bool summed = tickets != nullptr;  // the sum over a token's slots is part of the down GEMM
   if (ts)
-    rc = launch_moe_ts(a, act, rows, pair_out, ts_partial, stream);
+    rc = launch_moe_ts(a, act, rows, pair_out, ts_partial, &summed, stream);
   else if (a.decode_layout)
     rc = a.block == 8 ? launch_moe_gemms<1, 128, true>(a, act, pair_out, tickets, numel, nblk, stream)
                       : launch_moe_gemms<2, 128, true>(a, act, pair_out, tickets, numel, nblk, stream);
@@ -842,7 +843,7 @@ int launch_moe_experts(const MoeArgs& a, void* workspace, size_t workspace_bytes
     rc = a.block == 8 ? launch_moe_gemms<1, 0, false>(a, act, pair_out, tickets, numel, nblk, stream)
                       : launch_moe_gemms<2, 0, false>(a, act, pair_out, tickets, numel, nblk, stream);
   if (rc) return rc;
-  if (tickets == nullptr) {
+  if (!summed) {
     const long long work = (long long)a.T * (a.H / 8);
     if (launch_pdl(moe_sum_kernel, dim3((unsigned)((work + 255) / 256)), dim3(256), 0, stream,
                    (const __half*)pair_out, a.out, a.T, a.topk, a.H) != cudaSuccess) {

@@ -370,6 +370,11 @@ __device__ __forceinline__ void st_async_v4(uint32_t dst, const float* v, uint32
                "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "r"(bar)
                : "memory");
 }
+__device__ __forceinline__ void st_async_v2(uint32_t dst, float a, float b, uint32_t bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];" ::"r"(dst), "f"(a),
+               "f"(b), "r"(bar)
+               : "memory");
+}
 // Arrive on a barrier given by its cluster address (own or peer CTA).  What such arrivals hand over is
 // tensor memory, ordered by the tcgen05 fences around them, so the default CTA scope is enough; the
 // cluster-scope forms (release / acquire) add memory barriers: 65 against 55 us for the whole kernel

@@ -322,6 +322,32 @@ def test_small_batch_experts_edges(A, t, k, e, h, i, parallel):
         assert O.rel_err(y, ref) < TOL
 
 
+# One or two tokens: gate_up on clusters (units of gate and up that do not divide by them, an edge of the columns inside
+# a slab, one unit in all), down on clusters of a token's slots; every number of slots; a third of the experts absent.
+@pytest.mark.parametrize("t,k,h,i", [(1, 2, 256, 128), (1, 3, 1152, 384), (1, 4, 4096, 1536), (1, 5, 640, 640),
+                                     (1, 6, 2048, 768), (1, 7, 896, 896), (1, 8, 2048, 1024), (2, 4, 2048, 768),
+                                     (2, 3, 512, 128)])
+@pytest.mark.parametrize("parallel", [False, True])
+def test_direct_clusters_round_like_the_permuted_path(A, t, k, h, i, parallel, monkeypatch):
+    from awq_b200 import ops
+    e = 64
+    w1, w2, x, logits = _moe_case(e, h, i, t, k, seed=t + k)
+    w, ids, _ = A.fused_topk(x.cuda(), logits.cuda(), k, True)
+    here = torch.tensor([n for n in range(e) if not parallel or n % 3 != 1])
+    emap = torch.full((e,), -1, dtype=torch.int32)
+    emap[here] = torch.arange(len(here), dtype=torch.int32)
+    local = [tuple(a[here].contiguous().cuda() for a in ws) for ws in (w1, w2)]
+    kwargs = dict(global_num_experts=e, expert_map=emap.cuda() if parallel else None)
+    y = [A.fused_experts(x.cuda(), *local, w, ids, **kwargs) for _ in range(3)]
+    with monkeypatch.context() as patch:
+        patch.setattr(ops, "MOE_DIRECT_MAX_PAIRS", 0)
+        permuted = A.fused_experts(x.cuda(), *local, w, ids, **kwargs)
+    torch.cuda.synchronize()
+    assert torch.equal(y[0], y[1]) and torch.equal(y[0], y[2])
+    # fp32 sums in another order put some values on the other side of a rounding: 2^-11 each, fewer than one in six
+    assert (y[0].double() - permuted.double()).norm() <= 2e-4 * permuted.double().norm()
+
+
 # Tokens of one expert each: whole prompts (grouped tiles), a server's batch (a tile per row block).
 @pytest.mark.parametrize("t,e", [(300, 4), (40, 8)])
 def test_rows_leave_the_range_of_fp16_only_before_their_weight(A, t, e):
