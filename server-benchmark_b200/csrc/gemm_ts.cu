@@ -132,6 +132,9 @@ struct TsCfg {
   static constexpr int kFold0 = kTsCvWarps, kIssue = kFold0 + kFoldWarps;
   // the conversion subtracts the zero points: no token sums
   static constexpr bool SUB = (SPLIT && MODE == 0) || MT > 16 || (MT == 16 && GROUP == 64);
+  // Scales and zero points by plain bulk copies (TsRow).  Groups of 64 need twice as many: up to 16 tokens 4096 x 11040 at
+  // M 16 took 10.4 -> 10.7 us with them, at M 24 12.4 -> 11.5.
+  static constexpr bool BULK = SPLIT && MODE == 0 && (GROUP == 128 || MT > 16);
   static constexpr int kIssueWarps = SUB ? 2 : 1;
   static constexpr int kSum = kIssue + kIssueWarps, kXWarp = kSum + (SUB ? 0 : 1), kRaw = kXWarp + 1;
   static constexpr int kThreads = 32 * (kRaw + 1);     // 768
@@ -163,8 +166,14 @@ struct TsParams {
   int M, N, K, KT, slabs;  // KT: units of one matrix (K / 128)
   int chunk;               // dense: units per CTA, 0: whole slabs strided
   // grouped modes
-  const int32_t* sorted_ids;   // permuted flat pair ids, padding = numel; nullptr: direct form
-  const int32_t* expert_ids;   // expert of every row block (direct: of every pair)
+  union {
+    const int32_t* sorted_ids;  // permuted flat pair ids, padding = numel; nullptr: direct form
+    const __half* scales;       // BULK: [groups][N]
+  };
+  union {
+    const int32_t* expert_ids;  // expert of every row block (direct: of every pair)
+    const uint32_t* qzeros;     // BULK: [groups][N / 8]
+  };
   const int32_t* num_post;     // permuted rows in use
   const float* topk_weights;
   int numel, topk, half_cols;
@@ -262,6 +271,20 @@ __device__ __forceinline__ Work ts_split_work(const TsParams& p, int rank, int k
   return Work::range(tile * p.KT, (tile + 1) * p.KT, p.KT);
 }
 
+// BULK: scales and zero words of 256 columns of a group, of which `cols` exist, for plain bulk copies.  They are
+// contiguous, and a tensor map costs the host 0.2 us of a call, which is what bounds an eager call of a short layer (2048 x
+// 5120 at M 1: 5.1 -> 4.7 us; replayed 4.16 -> 4.2).  What a copy leaves as it is belongs to columns that are not stored.
+// Long layers keep their maps: bulk copies took 55 -> 58 us on 8192 x 59136 at M 32.
+struct TsRow {
+  const __half* scales;
+  const uint32_t* zeros;
+  uint32_t cols;
+  __device__ __forceinline__ TsRow(const TsParams& p, int column, int group)
+      : scales(p.scales + (size_t)group * p.N + column),
+        zeros(p.qzeros + (size_t)group * (p.N / kPack) + column / kPack),
+        cols((uint32_t)min(kTsBN, p.N - column)) {}
+};
+
 // A load stream's walk over the CTA's units: the weight rows / group row of every unit, and the column
 // slab.  The expert of the next matrix is fetched while the current one is loaded.
 template <int MODE>
@@ -302,6 +325,7 @@ struct TsWalk {
 
 template <int MT, int MODE, int GROUP, bool SPLIT>
 __global__ void __launch_bounds__((TsCfg<MT, MODE, GROUP, SPLIT>::kThreads), 1)
+// map_s, map_z: not read where BULK
 gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_s,
                const __grid_constant__ CUtensorMap map_z, const __grid_constant__ CUtensorMap map_x,
                const TsParams p) {
@@ -372,7 +396,19 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     const uint32_t sz = sz_base + (raw.u & (kTsSzRing - 1)) * kSz;
     const int column = raw.column(), row = raw.expert * p.K + raw.unit() * kTsBK;
     const int grp = (raw.expert * p.KT + raw.unit()) * G;
-    if (elect_one()) {
+    if constexpr (Cfg::BULK) {
+      const TsRow of(p, column, grp);
+      if (elect_one()) {
+        mbar_arrive_expect_tx(bar, kTsRawBytes + G * (of.cols * 2 + (kRawZeros ? of.cols / 2 : 0)));
+        tma_load_2d(dst, &map_w, column / kPack, row, bar);
+#pragma unroll
+        for (int h = 0; h < G; ++h) {
+          bulk_load(sz + h * kTsScaleBytes, of.scales + (size_t)h * p.N, of.cols * 2, bar);
+          if (kRawZeros)
+            bulk_load(sz + kScales + h * kTsZeroBytes, of.zeros + (size_t)h * (p.N / kPack), of.cols / 2, bar);
+        }
+      }
+    } else if (elect_one()) {
       mbar_arrive_expect_tx(bar, kTsRawBytes + kScales + (kRawZeros ? kZeros : 0));
       tma_load_2d(dst, &map_w, column / kPack, row, bar);
       tma_load_2d(sz, &map_s, column, grp, bar);
@@ -1157,15 +1193,18 @@ int launch_ts(const TsMaps& maps, const TsParams& p, int ctas, cudaStream_t stre
 
 int ts_ctas() { return sm_count() < handover::kMaxCtas ? sm_count() : handover::kMaxCtas; }
 
-// packed words [rows][words], box [128 rows x 32 words], 128-byte swizzle; scales and zero points, one
-// row per group
+// packed words [rows][words], box [128 rows x 32 words], 128-byte swizzle
+int ts_word_map(TsMaps* m, const uint32_t* w, uint64_t rows, uint64_t N) {
+  const uint64_t words = N / kPack;
+  return encode_map_2d(&m->w, CU_TENSOR_MAP_DATA_TYPE_INT32, w, words, rows, words * 4, kTsBN / kPack, kTsBK,
+                       CU_TENSOR_MAP_SWIZZLE_128B);
+}
+// The same, and scales and zero points, one row per group.
 int ts_weight_maps(TsMaps* m, const uint32_t* w, const __half* scales, const uint32_t* qzeros,
                    uint64_t rows, uint64_t N, int group = kTsBK) {
   const uint64_t words = N / kPack, groups = rows / group;
   const uint32_t box = kTsBK / group;  // groups of a unit
-  if (int rc = encode_map_2d(&m->w, CU_TENSOR_MAP_DATA_TYPE_INT32, w, words, rows, words * 4,
-                             kTsBN / kPack, kTsBK, CU_TENSOR_MAP_SWIZZLE_128B))
-    return rc;
+  if (int rc = ts_word_map(m, w, rows, N)) return rc;
   if (int rc = encode_map_2d(&m->s, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, scales, N, groups, N * 2,
                              kTsBN, box, CU_TENSOR_MAP_SWIZZLE_NONE))
     return rc;
@@ -1195,7 +1234,14 @@ int launch_ts_dense(const __half* x, const uint32_t* qweight, const __half* scal
     ctas = (int)(((long)p.slabs * p.KT + p.chunk - 1) / p.chunk);
   }
   TsMaps maps;
-  if (int rc = ts_weight_maps(&maps, qweight, scales, qzeros, (uint64_t)p.K, (uint64_t)p.N, GROUP)) return rc;
+  if (p.split > 1 && TsCfg<MT, 0, GROUP, true>::BULK) {
+    p.scales = scales;
+    p.qzeros = qzeros;
+    if (int rc = ts_word_map(&maps, qweight, (uint64_t)p.K, (uint64_t)p.N)) return rc;
+    maps.s = maps.z = maps.w;  // the kernel does not read them
+  } else if (int rc = ts_weight_maps(&maps, qweight, scales, qzeros, (uint64_t)p.K, (uint64_t)p.N, GROUP)) {
+    return rc;
+  }
   if (int rc = encode_map_x(&maps.x, x, (uint64_t)p.M, (uint64_t)p.K, TsCfg<MT, 0, GROUP>::NT)) return rc;
   if (p.split > 1) return launch_ts_split<MT, GROUP>(maps, p, p.slabs, stream);
   return launch_ts<MT, 0, GROUP>(maps, p, ctas, stream);
