@@ -135,6 +135,8 @@ struct TsCfg {
   // Scales and zero points by plain bulk copies (TsRow).  Groups of 64 need twice as many: up to 16 tokens 4096 x 11040 at
   // M 16 took 10.4 -> 10.7 us with them, at M 24 12.4 -> 11.5.
   static constexpr bool BULK = SPLIT && MODE == 0 && (GROUP == 128 || MT > 16);
+  // Partial tiles handed over with a token beside every two sums, without flags
+  static constexpr bool MARKS = MODE != 0 && MT <= 8;
   static constexpr int kIssueWarps = SUB ? 2 : 1;
   static constexpr int kSum = kIssue + kIssueWarps, kXWarp = kSum + (SUB ? 0 : 1), kRaw = kXWarp + 1;
   static constexpr int kThreads = 32 * (kRaw + 1);     // 768
@@ -701,18 +703,36 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     constexpr bool kOneVote = GROUP == 128 || MT == 8, kStay = GROUP == 64 && MT == 16;
     bool ok = true;
     int u = 0;
+    // MODE 2: tiles are walked down one by one, so a segment's block and slab need no division, and pairs are fetched a
+    // segment ahead: the address of their weights waits for them.  Experts of 128 x 2048 x 768, top-8, 128 tokens 94.5 ->
+    // 93.1 us, 500 tokens 189 -> 184.
+    int block_next = 0, slab_next = 0, fid_next = p.numel;
+    auto pair_of = [&](int block) {  // lane m: pair in row m
+      if (lane >= MT) return p.numel;
+      return p.sorted_ids != nullptr ? __ldcg(p.sorted_ids + block * MT + lane) : (lane == 0 ? block : p.numel);
+    };
+    if (MODE == 2 && work.segs > 0) {
+      block_next = work.tile_id(0) / p.slabs;
+      slab_next = work.tile_id(0) - block_next * p.slabs;
+      fid_next = pair_of(block_next);
+    }
     for (int seg = 0; seg < work.segs; ++seg) {
       const int id = work.tile_id(seg), kb = work.k_begin(seg), ke = work.k_end(seg);
-      const int block = MODE == 0 ? 0 : id / p.slabs, slab = MODE == 0 ? id : id - block * p.slabs;
+      const int block = MODE == 0 ? 0 : MODE == 2 ? block_next : id / p.slabs;
+      const int slab = MODE == 0 ? id : MODE == 2 ? slab_next : id - block * p.slabs;
       // What the end of the segment needs, fetched ahead of its units.  MODE 2: lane m knows pair and
       // routed weight of row m.
-      int fid = p.numel;
+      const int fid = fid_next;
       float fw = 0.f;
-      bool valid = true;  // false: an expert of another rank
-      if (MODE == 1 || MODE == 2) valid = __ldcg(p.expert_ids + block) >= 0;
-      if (MODE == 2 && lane < MT) {
-        fid = p.sorted_ids != nullptr ? __ldcg(p.sorted_ids + block * MT + lane) : (lane == 0 ? block : p.numel);
-        fw = fid < p.numel ? __ldcg(p.topk_weights + fid) : 0.f;
+      int expert = 0;  // negative: an expert of another rank
+      if (MODE == 1 || MODE == 2) expert = __ldcg(p.expert_ids + block);
+      if (MODE == 2) {
+        if (fid < p.numel) fw = __ldcg(p.topk_weights + fid);
+        if (--slab_next < 0) {
+          slab_next = p.slabs - 1;
+          --block_next;
+        }
+        if (seg + 1 < work.segs) fid_next = pair_of(block_next);
       }
       uint64_t tot[MT / 2];
 #pragma unroll
@@ -795,6 +815,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         }
       }
       // ---- end of the segment ----
+      const bool valid = expert >= 0;
       float v[MT];
 #pragma unroll
       for (int m = 0; m < MT / 2; ++m) {
@@ -845,7 +866,27 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       // partial tile of CTA c: [MT][256], MODE 1: gate, then up
       constexpr int kTile = MT * kTsBN, kTiles = MODE == 1 ? 2 : 1;
       float* part = p.partial + (size_t)blockIdx.x * (kTiles * kTile) + chunk_col + lane;
-      if (ke < work.KT) {  // another CTA holds the tile's last unit
+      // MARKS: [MT / 2][256] pairs of sums with the launch's token beside each.  Whoever adds them reads until it sees the
+      // token.  A release took a fold warp 2000 to 5000 cycles under the words' stream, also long after its stores, and the
+      // next tile's folds waited for it: experts of 128 x 2048 x 768, top-8, 16 tokens 54.2 -> 51.4 us, 64 tokens 72.2 -> 70.0,
+      // 128 tokens 95 -> 90.  Reading costs more (16-byte strong loads, 2500 cycles for eight), so dense layers, where
+      // more CTAs share a slab, and blocks of 16 rows keep the flags: 29568 x 8192 at M 16 28 -> 37 us with marks, 8192 x
+      // 59136 at M 1 41.4 -> 43.3, 500 tokens 171 -> 175.
+      constexpr int P = MT / 2, kMarked = P * kTsBN;
+      uint4* marked = reinterpret_cast<uint4*>(p.partial) + (size_t)blockIdx.x * (kTiles * kMarked) + chunk_col + lane;
+      if (Cfg::MARKS && ke < work.KT) {
+        uint4* dst = marked + (MODE == 1 && ke > p.KT ? kMarked : 0);
+        const unsigned long long mark = ok && !s_abort ? token : 0ull;
+#pragma unroll
+        for (int m = 0; m < P; ++m) handover::store_marked(dst + m * kTsBN, pack2(v[2 * m], v[2 * m + 1]), mark);
+        if (MODE == 1 && ke > p.KT && kb < p.KT) {
+#pragma unroll
+          for (int m = 0; m < P; ++m)
+            handover::store_marked(marked + m * kTsBN, pack2(gate[2 * m * 32], gate[(2 * m + 1) * 32]), mark);
+        }
+        continue;
+      }
+      if (!Cfg::MARKS && ke < work.KT) {  // another CTA holds the tile's last unit
         float* dst = part + (MODE == 1 && ke > p.KT ? kTile : 0);
 #pragma unroll
         for (int m = 0; m < MT; ++m)
@@ -861,7 +902,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       int gather = 0;  // CTAs before this one that share the tile
       if (kb > 0) {
         gather = blockIdx.x - id * work.KT / work.chunk;
-        for (int c = 1 + lane; c <= gather; c += 32) {
+        for (int c = 1 + lane; !Cfg::MARKS && c <= gather; c += 32) {
           unsigned long long* theirs = flag - c * handover::kMaxWarps;
           uint32_t polls = 0;
           while (handover::read_flag(theirs) != token) {
@@ -896,6 +937,42 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             for (int m = 0; m < MT; ++m) sum[m] += w[a][m];
         }
       };
+      // MARKS: the same
+      constexpr int M_AHEAD = 8 / P > 0 ? 8 / P : 1;
+      auto add_marked = [&](float (&sum)[MT], uint4* src, int first, int last) {
+        for (int c = first; c >= last; c -= M_AHEAD) {
+          uint64_t w[M_AHEAD][P];
+          const auto at = [&](int a, int m) { return src - (size_t)(c - a) * (kTiles * kMarked) + m * kTsBN; };
+          for (uint32_t polls = 0;;) {
+            bool got = true;
+#pragma unroll
+            for (int a = 0; a < M_AHEAD; ++a)
+#pragma unroll
+              for (int m = 0; m < P; ++m) {
+                w[a][m] = 0ull;
+                if (c - a >= last) got &= handover::load_marked(at(a, m), w[a][m]) == token;
+              }
+            if (__all_sync(0xffffffffu, got)) break;
+            if (!ok || ++polls >= kSpinLimit || s_abort) {
+              s_abort = 1;
+              atomicCAS(&g_tc_status, 0, 29);
+              ok = false;
+              linger();  // no replay must find what arrives meanwhile
+              break;
+            }
+          }
+          ok = __all_sync(0xffffffffu, ok);
+#pragma unroll
+          for (int a = 0; a < M_AHEAD; ++a)
+#pragma unroll
+            for (int m = 0; m < P; ++m) {
+              if (c - a >= last) handover::take_mark(at(a, m));
+              const float2 x = unpack2(w[a][m]);
+              sum[2 * m] += x.x;
+              sum[2 * m + 1] += x.y;
+            }
+        }
+      };
       // MODE 1: CTA blockIdx.x - c has units of up if its range ends past unit KT of the tile, of gate
       // if it begins before
       int up_first = gather, gate_last = 1;
@@ -904,7 +981,8 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         while (up_first > 0 && ((int)blockIdx.x - up_first + 1) * work.chunk <= split) --up_first;
         while (gate_last <= gather && ((int)blockIdx.x - gate_last) * work.chunk >= split) ++gate_last;
       }
-      add_parts(v, part + (MODE == 1 ? kTile : 0), up_first, 1);
+      if constexpr (Cfg::MARKS) add_marked(v, marked + (MODE == 1 ? kMarked : 0), up_first, 1);
+      else add_parts(v, part + (MODE == 1 ? kTile : 0), up_first, 1);
 #pragma unroll
       for (int m = 0; m < MT; ++m) v[m] *= unscale;
       const int first = odd ? 1 : 0;
@@ -919,7 +997,8 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         float gt[MT];
 #pragma unroll
         for (int m = 0; m < MT; ++m) gt[m] = kb < p.KT ? gate[m * 32] : 0.f;
-        add_parts(gt, part, gather, gate_last);
+        if constexpr (Cfg::MARKS) add_marked(gt, marked, gather, gate_last);
+        else add_parts(gt, part, gather, gate_last);
 #pragma unroll
         for (int m = 0; m < MT; ++m) {
           const float x = gt[m] * unscale;
@@ -1254,7 +1333,7 @@ int launch_ts_experts(const MoeArgs& a, __half* act, int64_t act_rows, __half* p
                       cudaStream_t stream) {
   const int ctas = ts_ctas();
   *summed = false;
-  p.flags = handover::make_flags(p.partial, 2 * ts_partial_bytes(MT));
+  p.flags = handover::make_flags(p.partial, 2 * ts_partial_bytes(MT));  // flags: blocks of 16 rows
   p.sorted_ids = a.sorted_ids;
   p.expert_ids = a.expert_ids;
   p.num_post = a.num_post_pad;
@@ -1353,7 +1432,11 @@ bool moe_ts_supported(const MoeArgs& a) {
 }
 
 // Partial tiles of gate and up, rows of the largest block, and the flags.
-size_t moe_ts_partial_bytes(int block) { return 2 * ts_partial_bytes(block) + handover::kFlagBytes; }
+size_t moe_ts_partial_bytes(int block) {
+  // blocks of 8 rows and the direct form: a token beside every two sums
+  if (block <= 8) return (size_t)2 * ts_ctas() * block * kTsBN * 8;
+  return 2 * ts_partial_bytes(block) + handover::kFlagBytes;
+}
 
 // Both expert GEMMs of a small batch, pair_out by pair.  Rows of act by position, direct (no
 // permutation) by pair.

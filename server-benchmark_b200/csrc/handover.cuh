@@ -45,6 +45,32 @@ struct Flags {
   __device__ __forceinline__ void lower(int cta, int warp) const { *at(cta, warp) = 0; }
 };
 
+// Two sums and the token of their launch in 16 bytes that are written and read as one, so that they need no flag.  Who
+// reads them takes the token away again.
+__device__ __forceinline__ void store_marked(uint4* at, unsigned long long value, unsigned long long token) {
+  asm volatile(
+      "{\n\t.reg .b128 t;\n\t"
+      "mov.b128 t, {%1, %2};\n\t"
+      "st.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(at),
+      "l"(value), "l"(token)
+      : "memory");
+}
+__device__ __forceinline__ unsigned long long load_marked(const uint4* at, uint64_t& value) {
+  unsigned long long token;
+  asm volatile(
+      "{\n\t.reg .b128 t;\n\t"
+      "ld.relaxed.gpu.global.b128 t, [%2];\n\t"
+      "mov.b128 {%0, %1}, t;\n\t}"
+      : "=l"(value), "=l"(token)
+      : "l"(at)
+      : "memory");
+  return token;
+}
+__device__ __forceinline__ void take_mark(uint4* at) {
+  asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(reinterpret_cast<unsigned long long*>(at) + 1), "l"(0ull)
+               : "memory");
+}
+
 // Token of a launch: a counter, started by the clock and spread over 64 bits by an odd factor.
 inline unsigned long long next_token() {
   static std::atomic<unsigned long long> counter{

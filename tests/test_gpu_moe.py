@@ -623,3 +623,44 @@ def test_batches_in_turn_do_not_see_each_other(A, e, h, i, t, k):
     for _ in range(30):
         A.fused_experts(nan, w1d, w2d, *other)
         assert torch.equal(A.fused_experts(xd, w1d, w2d, weights, ids), first)
+
+
+def test_partial_tiles_of_experts_with_any_scratch_and_replays(A):
+    """Sums with a token beside them: scratch full of other data, one buffer again and again, and replays of one graph
+    whose token is the same every time."""
+    from awq_b200 import _lib, ops
+    t, k, e, h, i = 24, 4, 16, 2048, 768
+    w1, w2, x, logits = _moe_case(e, h, i, t, k, seed=5)
+    w1d, w2d = (tuple(a.cuda() for a in ws) for ws in (w1, w2))
+    xd = x.cuda()
+    w, ids, _ = A.fused_topk(xd, logits.cuda(), k, True)
+    block = _lib.load().awq_b200_moe_block_size(t, k, e, h, i, 128)
+    assert block == 8
+    want = A.fused_experts(xd, w1d, w2d, w, ids)
+    sid, eid, npp = ops.moe_align_block_size(ids, block, e)
+    need = _lib.load().awq_b200_moe_workspace_bytes(t, k, e, h, i)
+    out = torch.empty_like(want)
+    gen = torch.Generator(device="cuda").manual_seed(3)
+
+    def call(scratch):
+        rc = _lib.load().awq_b200_moe_experts(
+            xd.data_ptr(), *[v.data_ptr() for v in (*w1d, *w2d)], w.data_ptr(), sid.data_ptr(), eid.data_ptr(),
+            npp.data_ptr(), out.data_ptr(), t, k, e, h, i, 128, block, 0, sid.numel(), scratch.data_ptr(),
+            scratch.numel(), torch.cuda.current_stream().cuda_stream)
+        assert rc == 0
+    for n in range(12):
+        scratch = torch.randint(0, 256, (need,), dtype=torch.uint8, device="cuda", generator=gen)
+        for _ in range(4):
+            out.fill_(float("nan"))
+            call(scratch)
+            assert torch.equal(out, want), n
+    graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        call(scratch)
+        call(scratch)
+    for _ in range(10):
+        out.fill_(float("nan"))
+        graph.replay()
+        assert torch.equal(out, want)
+    torch.cuda.synchronize()
