@@ -664,3 +664,52 @@ def test_partial_tiles_of_experts_with_any_scratch_and_replays(A):
         graph.replay()
         assert torch.equal(out, want)
     torch.cuda.synchronize()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("t,k,e,h,i", [(300, 2, 8, 512, 256), (160, 2, 4, 2048, 128)])
+def test_prefill_calls_back_to_back_read_their_own_routing(A, t, k, e, h, i):
+    """The down GEMM reads the tile table ahead of its wait for gate_up: calls with other routing right behind one
+    another, in one buffer, give the bits that they give alone."""
+    from awq_b200 import _lib, ops
+    w1, w2, x, logits = _moe_case(e, h, i, t, k, seed=7)
+    w1d, w2d = (tuple(a.cuda() for a in ws) for ws in (w1, w2))
+    xd = x.cuda()
+    assert _lib.load().awq_b200_moe_block_size(t, k, e, h, i, 128) == 128
+    # most tokens on one expert, on another one, and spread out
+    skews = [(0, 8.0), (e - 1, 8.0), (0, 0.0)]
+    routed, want = [], []
+    for expert, by in skews:
+        ld = logits.cuda().clone()
+        ld[:, expert] += by
+        w, ids, _ = A.fused_topk(xd, ld, k, True)
+        routed.append((w, *ops.moe_align_block_size(ids, 128, e)))
+        want.append(A.fused_experts(xd, w1d, w2d, w, ids))
+        torch.cuda.synchronize()
+    need = _lib.load().awq_b200_moe_workspace_bytes(t, k, e, h, i)
+    scratch = torch.empty(need, dtype=torch.uint8, device="cuda")
+    order = [0, 1, 2, 1, 0, 2, 2, 0, 1] * 2
+    outs = [torch.empty_like(want[0]) for _ in order]
+
+    def calls():
+        for n, out in zip(order, outs):
+            w, sid, eid, npp = routed[n]
+            rc = _lib.load().awq_b200_moe_experts(
+                xd.data_ptr(), *[v.data_ptr() for v in (*w1d, *w2d)], w.data_ptr(), sid.data_ptr(), eid.data_ptr(),
+                npp.data_ptr(), out.data_ptr(), t, k, e, h, i, 128, 128, 0, sid.numel(), scratch.data_ptr(),
+                scratch.numel(), torch.cuda.current_stream().cuda_stream)
+            assert rc == 0
+    calls()
+    for n, out in zip(order, outs):
+        assert torch.equal(out, want[n]), n
+    graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        calls()
+    for _ in range(5):
+        for out in outs:
+            out.fill_(float("nan"))
+        graph.replay()
+        for n, out in zip(order, outs):
+            assert torch.equal(out, want[n]), n
+    torch.cuda.synchronize()
