@@ -60,9 +60,14 @@
 // 8192 x 8192 at M 264 31.4 us against 31.2, 4096 x 11040 at M 150 18.3 / 18.0, 1024 x 8192 at M 264 9.4 / 9.1, M 394 on
 // 1024 x 5120 9.15 / 8.8; 25 shapes, none the other way round by more than its runs differ.
 //
-// TMEM columns: accumulators first (two of 64 or 128 tokens, one of 256), then A[slots][8 steps][8]: four
-// slots, six up to 64 tokens.  With as many slots as teams a team waits for the MMAs of its own last
-// unit; the two more take that wait out of its loop.
+// TMEM columns: accumulators first, then A[slots][8 steps][8], 64 columns a slot.  With as many slots as teams a team waits
+// for the MMAs of its own last unit; two more take that wait out of its loop.  Up to 64 tokens there are two accumulators and
+// six slots.  Up to 128, two accumulators leave four slots; where a CTA ends few tiles for its units it has one accumulator
+// and six slots instead, and the conversion fills them under the epilogue.  That is in clusters with one tile (4096 x 4096
+// M 77 7.8 -> 7.3 us) and in ranges with K from 7168 up: 29568 x 8192 M 100 54.8 -> 53.7 us, in groups of 64 56.4 -> 55.0,
+// 8192 x 10240 M 100 23.8 -> 23.2, 14336 x 4096 26.4 -> 25.9, 7168 x 14336 M 80 28.8 -> 28.7, the four linears of a layer
+// M 100 229 -> 224.5.  With smaller K it loses: 6144 x 28672 M 128 41.4 -> 41.9, 4096 x 22016 M 100 22.75 -> 23.05, 3072 x
+// 22016 M 120 19.4 -> 20.0.  Whole tiles in turn, the grouped ones too, keep two.
 // Lane 32 q + 8 i + g holds column 8 (4 q + g / 2) + 2 i + g % 2 of the CTA's 128.
 // All mbarrier and flag waits are bounded (tc_ptx.cuh).
 //
@@ -107,6 +112,7 @@ constexpr int kWtMaxRaw = 16, kWtMaxX = 8;    // ring depths the barrier block h
 constexpr int kWtPartRing = 8, kWtPartBytes = 32 * 32 * 4;  // per epilogue warp: 32 tokens x 32 columns
 constexpr int kWtBarBytes = 1024;
 static_assert(8 * (2 * kWtMaxRaw + 2 * kWtMaxX + 4 + kWtEpiWarps * kWtPartRing) <= kWtBarBytes, "barriers");
+constexpr int kWtOneStages = 56;              // K stages from which ranges of 65 to 128 tokens have one accumulator
 constexpr int kWtExFloats = 2 * 32 * 20;      // MODE 1: gate / up exchange of two epilogue warps
 constexpr int kWtExBytes = 2 * 2 * kWtExFloats * 4;
 constexpr int kWtSmemLimit = 232448 - 1024;   // dynamic shared memory less the static part
@@ -1132,26 +1138,29 @@ int wt_rings(WtParams* p, int mode) {
   const int rows = (p->nt / 2 + 15) / 16 * 16;
   p->xstage = rows * 256;
   p->nx = p->xstage <= (16 << 10) ? 8 : 4;
-  // Two accumulators while they fit beside four A slots, so that the next tile's MMAs run under the
-  // epilogue; what TMEM is left over goes to A slots.
-  p->nbuf = p->nt <= 128 ? 2 : 1;
+  // Two accumulators, so that the next tile's MMAs run under the epilogue, while they fit beside six A slots, or beside four
+  // where a CTA has many tiles; what TMEM is left over goes to A slots.
+  const bool one = p->nt > 128 || (p->nt > 64 && (p->share.tiles == 1 || (p->chunk > 0 && p->KT >= kWtOneStages)));
+  p->nbuf = one ? 1 : 2;
   // One accumulator and whole tiles: the WIDE kernel.
   p->stage_bytes = p->nbuf == 2 || p->chunk > 0 || p->share.pairs > 0 ? 0 : (p->nt + 31) / 32 * 32 * kWtCols * (mode == 1 ? 1 : 2);
   const int recv = p->share.pairs > 0 ? p->share.recv * (p->share.tiles > 1 ? 2 : 1) : 0;
   const int fixed = 1024 + kWtBarBytes + (mode == 1 ? kWtExBytes : 0) + p->stage_bytes + recv;
   p->dcols = p->nt <= 64 ? 64 : 128;
-  p->acol = p->nt <= 64 ? 128 : 256;
+  p->acol = p->nbuf == 2 ? 2 * p->dcols : (p->nt + 63) / 64 * 64;
   p->slots = (kWtTmemCols - p->acol) / 64;
   p->nraw = (kWtSmemLimit - fixed - p->nx * p->xstage) / kWtRawBytes;
-  if (recv > 0 && p->nx == 8 && p->nraw < kWtTeams + p->slots) {
+  if (recv > 0 && p->nx == 8 && p->nraw < 2 * kWtTeams) {
     p->nx = 4;
     p->nraw = (kWtSmemLimit - fixed - p->nx * p->xstage) / kWtRawBytes;
   }
   if (p->nraw > kWtMaxRaw) p->nraw = kWtMaxRaw;
   // A team waits for unit u in the stage that unit u - nraw had.  Either it read that one itself, or it has seen
   // the MMAs of a later unit complete (u - 4 - slots, when it wrote unit u - 4); between the two, the parity of
-  // the filling before could pass for the one it waits for.
-  if (p->nraw < kWtTeams + p->slots) p->nraw = kWtTeams;
+  // the filling before could pass for the one it waits for.  Fewer slots rather than fewer x stages: with four of those 8192 x
+  // 8192 at M 100 took 17.3 us, with eight 17.0.
+  if (p->nraw < 2 * kWtTeams) p->nraw = kWtTeams;
+  else if (p->slots > p->nraw - kWtTeams) p->slots = p->nraw - kWtTeams;
   return fixed + p->nx * p->xstage + p->nraw * kWtRawBytes;
 }
 
@@ -1401,6 +1410,7 @@ int gemm_wt_cut(int M, int N, int K, int group, int cta_pairs, int* tokens, int*
   WtParams p = {};
   p.nt = plan.nt;
   p.chunk = plan.chunk;
+  p.KT = K / kWtBK;
   wt_rings(&p, 0);
   *tokens = plan.nt;
   *chunk = plan.chunk;

@@ -225,3 +225,12 @@ def test_wt_clusters_share_tiles(A, m, k, n, group, bias):
     # 5 %: the fp32 sums, K * 2^-24 of their terms' size at most, move few values to the other side
     for y in (outs[0], named):
         assert (y.cpu()[:, c:].double() - ref).norm() < 1.05 * rounding
+
+
+# Ranges of 65 to 128 tokens on either side of the K from which they have one accumulator and six A slots: a tile shared by
+# pairs, three tiles in a range, tiles of 80 and 128 tokens, a slab past N.
+@pytest.mark.parametrize("m,k,n,group", [
+    (100, 7168, 8224, 64), (100, 7040, 8224, 128), (72, 7168, 20512, 128), (128, 7296, 1568, 128),
+])
+def test_wt_ranges_with_one_or_two_accumulators(A, m, k, n, group):
+    test_wt_work_split_edges(A, m, k, n, group)
