@@ -1300,6 +1300,8 @@ constexpr int kWtShares[][2] = {{2, 1}, {3, 1}, {4, 1}, {5, 1}, {6, 1}, {8, 1}, 
 template <typename Resident>
 WtPlan wt_cluster_search(WtPlan best, int M, int slabs, int KT, Resident resident) {
   if (best.cost >= 0) best.cost -= 400;
+  int room[kMaxCluster + 1] = {};
+  for (const auto& s : kWtShares) room[s[0]] = resident(s[0]);
   for (int top = 256, last = 0; top >= 32; top -= 16) {
     const int mtiles = (M + top - 1) / top, nt = ((M + mtiles - 1) / mtiles + 15) / 16 * 16;
     if (nt == last) continue;
@@ -1308,8 +1310,8 @@ WtPlan wt_cluster_search(WtPlan best, int M, int slabs, int KT, Resident residen
     for (const auto& s : kWtShares) {
       const int pairs = s[0], per = s[1], clusters = tiles / per;
       // two tiles in turn need two accumulators; every pair has a unit; WtShare counts in 16 bits
-      if (tiles % per != 0 || (long)per * KT > 32767 || (per > 1 && nt > 128) || KT < pairs || clusters > resident(pairs)) continue;
-      const long cost = wt_cluster_cost(nt, pairs, per, clusters, KT, resident(pairs));
+      if (tiles % per != 0 || (long)per * KT > 32767 || (per > 1 && nt > 128) || KT < pairs || clusters > room[pairs]) continue;
+      const long cost = wt_cluster_cost(nt, pairs, per, clusters, KT, room[pairs]);
       if (best.cost >= 0 && cost >= best.cost) continue;
       WtParams p = {};
       p.nt = nt;
