@@ -335,7 +335,6 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   constexpr int NT = Cfg::NT, G = Cfg::G, NDB = Cfg::NDB, NRAW = Cfg::NRAW, kSz = Cfg::kSz, kTsXBytes = Cfg::kX;
   constexpr int kTsFoldWarps = Cfg::kFoldWarps, kTsFold0 = Cfg::kFold0, kTsIssue = Cfg::kIssue, kIssueWarps = Cfg::kIssueWarps;
   constexpr bool SUB = Cfg::SUB, kRawZeros = MODE == 1 || SUB;  // zero points with the packed words
-  constexpr bool kTells = MODE == 0 && !SPLIT && MT <= 16;  // the token warp raises the flags of partial tiles
   constexpr int kTsSum = Cfg::kSum, kTsX = Cfg::kXWarp, kTsRaw = Cfg::kRaw;
   constexpr int kScales = Cfg::kScales, kZeros = Cfg::kZeros, kSums = Cfg::kSums;
   extern __shared__ uint8_t smem_raw[];
@@ -355,8 +354,6 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   // fold warps have read unit u - NDB)
   auto unit_full = [&](int u) { return bar_base + 8 * (2 * NRAW + (u & (kTsUnits - 1))); };
   auto mma_done = [&](int u) { return bar_base + 8 * (2 * NRAW + kTsUnits + (u & (kTsUnits - 1))); };
-  // ranges of dense layers: the fold warps have stored the partial tile of the first segment
-  auto handed = [&]() { return bar_base + 8 * (2 * NRAW + 2 * kTsUnits); };
   auto unit_phase = [&](int u) { return (uint32_t)((u / kTsUnits) & 1); };
 
   // With 32 tokens tensor memory is asked for first and the warp of the packed words, which only tells that its barriers
@@ -449,10 +446,6 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       mbar_init(mma_done(lane), SUB ? 1 : 2);  // commit, sums warp
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (kTells && lane == 0) {
-      mbar_init(handed(), kTsFoldWarps);
-      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
     if (SPLIT && lane * p.split + rank < Cfg::kPieces) {  // piece lane * split + rank is this CTA's
       const int quads = piece_quads((lane * p.split + rank) / 8);
       mbar_init(recv_full(lane), 2);  // the bytes of the other CTAs, the warp here that has the piece
@@ -482,17 +475,6 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     // ------------------------------------------------------------------ tokens (zero points)
     pdl_wait();  // the activations may be the output of the kernel before this one
     TsWalk<MODE> x(p, work, kt, unit0);
-    // The first segment's partial tile, if it is one, is announced from here: a release takes 2000 to 5000 cycles under the
-    // words' stream, which would hold up the folds of the next slab, and this warp is eight units ahead. Announced by the
-    // fold warps -> from here, us: 8192x10240 11.71 -> 11.35 at 1 token, 11.84 -> 11.46 at 4; 29568x8192 24.5 -> 24.2 at 1,
-    // 27.7 -> 26.5 at 16. With 32 tokens (65.6 -> 68.9 at 8192x59136) and in MoE blocks of 16 (200 tokens, 128 experts:
-    // 86.1 -> 88.7, registers spilled) the fold warps' own way is the faster.
-    int tell_from = kTells && work.segs > 0 && work.k_end(0) < work.KT ? work.k_end(0) - work.k_begin(0) + 10 : 1 << 30;
-    auto tell = [&]() {
-      if (lane < kTsFoldWarps) p.flags.raise(blockIdx.x, lane);
-      __syncwarp();
-      tell_from = 1 << 30;
-    };
     bool ok = true;
     int row = 0, fid_next = -1, quads = MT / 4;
     int rows[MODE == 1 ? MT : 1];  // MODE 1: the block's rows of x
@@ -515,7 +497,6 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
           quads = max(1, (__popc(__ballot_sync(0xffffffffu, fid < p.numel)) + 3) / 4);
         }
       }
-      if (kTells && x.u >= tell_from && __all_sync(0xffffffffu, mbar_test(handed(), 0))) tell();
       if (x.u >= kTsUnits)
         ok = mbar_wait_warp(mma_done(x.u - kTsUnits), unit_phase(x.u - kTsUnits), &s_abort, 22);
       if (!ok) break;
@@ -545,7 +526,6 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     // them land before the CTA may exit.
     for (int u = work.count > kTsUnits ? work.count - kTsUnits : 0; u < work.count && ok; ++u)
       ok = mbar_wait(mma_done(u), unit_phase(u), &s_abort, 22);
-    if (kTells && tell_from < 1 << 30 && __all_sync(0xffffffffu, ok && mbar_wait(handed(), 0, &s_abort, 30))) tell();
   } else if (!SUB && warp == kTsSum) {
     // ------------------------------------------------------------------ token sums
     // x tile as the A operand of mma.sync (16 tokens x 16 k), every B element 2^-24: each column of
@@ -916,10 +896,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
           for (int m = 0; m < MT; ++m) part[m * kTsBN] = gate[m * 32];
         }
         __syncwarp();
-        if (lane == 0 && ok && !s_abort) {
-          if (kTells) mbar_arrive(handed());
-          else handover::raise_flag(flag, token);
-        }
+        if (lane == 0 && ok && !s_abort) handover::raise_flag(flag, token);
         continue;
       }
       int gather = 0;  // CTAs before this one that share the tile
