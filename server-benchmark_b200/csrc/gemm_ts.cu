@@ -1227,14 +1227,14 @@ TsCut ts_cut(int slabs, int KT) {
     best = {split, 0, cost};
     hidden = 2 * slabs <= resident;
   }
-  // The two estimates were fitted apart, and up to 16 tokens the ranges have become faster since.  What brings them
-  // together was fitted to 57 shapes from 1024 to 16128 rows at 1, 4, 8 and 16 tokens: 200 of it keeps clusters to where they
-  // gain: none of the 228 calls is slower than with ranges (without all this 30 were, 3712 x 8192 at M 1 6.8 -> 7.4 us, 1280 x
-  // 14752 5.3 -> 6.0, 8192 x 14848 at M 16 15.9 -> 16.6), 0.6 % from the better of the two on average.
+  // The two estimates were fitted apart.  What brings them together up to 16 tokens was fitted to 95 shapes from 1024 to 29440
+  // rows at 1, 4, 8 and 16 tokens, ranges and every cluster timed: none of the 380 calls is slower in clusters than it is in
+  // ranges, 1.0 % from the best of all on average.  With the bare estimates 34 were (3712 x 8192 at M 1 6.8 -> 7.4 us, 1280 x
+  // 14752 5.3 -> 6.0, 4864 x 11456 groups of 64 a quarter slower at M 8), 1.1 %.
   long margin = 0;
   if (MODE == 0 && MT <= 16) {
     const int run = ranges.chunk > 0 ? ranges.chunk : KT;
-    margin = 850 + 15 * MT - 52 * run + (hidden ? 0 : 490);
+    margin = 600 + 25 * MT + (GROUP == 128 ? 0 : 200) - 45 * (run < 30 ? run : 30) + (hidden ? 0 : 300);
   }
   return best.cost >= 0 && best.cost + margin < ranges.cost ? best : ranges;
 }
