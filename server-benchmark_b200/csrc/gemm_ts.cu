@@ -32,6 +32,7 @@
 //   8192 x 1280                      6.2 -> 4.8 (16)       9.1 -> 5.3            9.9 -> 5.9
 //   8192 x 7424                     10.1 -> 10.1 (4)      12.0 -> 10.6          15.8 -> 11.4
 //   3712 x 8192                      6.9 -> 7.2 (3)        8.4 -> 7.7 (3)       11.0 -> 8.2 (4)
+// The last two stay in ranges at one token (ts_cut).
 // What is left of 1024 x 8192 at M 1, in cycles from the end of the kernel before: 860 the tokens' way through L2, 1400
 // the MMAs of four units (22 each), 350 the last fold, 900 the cluster's sum, 450 the exit.
 //
@@ -1163,8 +1164,8 @@ TsCut ts_ranges(int slabs, int KT, int tokens) {
 }
 
 // A slab to each cluster of `split` CTAs, in one wave: estimated time in ns, `resident` clusters of that size fit the
-// GPU.  With it the choice between ranges and clusters of 2, 3, 4, 5, 6, 8 and 16 is 0.3 % from the best one on average,
-// 5 % at worst (18 shapes from 1024 x 1024 to 14848 x 8192 at 1, 8, 16, 20 and 32 tokens, groups of 128 and 64).
+// GPU.  Fitted to 18 shapes from 1024 x 1024 to 14848 x 8192 at 1, 8, 16, 20 and 32 tokens, groups of 128 and 64, clusters
+// of 2, 3, 4, 5, 6, 8 and 16.
 //   1950 + 23 tokens                start and end
 //   units x max(...)                355 + 2 tokens, groups of 64 15 + 2 tokens more: conversion, MMAs; 3.1 CTAs: words
 //   12 split                        the sum over the cluster
