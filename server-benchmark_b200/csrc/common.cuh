@@ -26,6 +26,10 @@ __device__ __forceinline__ void pdl_launch_dependents() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// An element of the bias, which may be the output of the kernel before this one: after pdl_wait.
+__device__ __forceinline__ float load_bias(const __half* at) {
+  return __half2float(__ushort_as_half(__ldcg(reinterpret_cast<const unsigned short*>(at))));
+}
 inline bool pdl_enabled() {
   static const bool on = getenv("AWQ_B200_NO_PDL") == nullptr;
   return on;

@@ -615,7 +615,7 @@ gemm_q8_kernel(const __grid_constant__ CUtensorMap map_w, const Q8Params p) {
             for (int sub = 0; sub < 2; ++sub) {
               const int n = slab * kQ8BN + sub * 128 + nl;
               if (n < p.N) {
-                const float bv = p.bias != nullptr ? __half2float(__ldg(p.bias + n)) : 0.f;
+                const float bv = p.bias != nullptr ? load_bias(p.bias + n) : 0.f;
 #pragma unroll
                 for (int m = 0; m < MT; ++m)
                   if (m < p.M)

@@ -114,7 +114,7 @@ gemm_stream_kernel(const StreamParams p) {
         }
       }
       if (p.bias != nullptr) {
-        const uint4 bv = __ldg(reinterpret_cast<const uint4*>(p.bias + n));
+        const uint4 bv = __ldcg(reinterpret_cast<const uint4*>(p.bias + n));
         const __half* bh = reinterpret_cast<const __half*>(&bv);
 #pragma unroll
         for (int j = 0; j < 8; ++j) v[j] += __half2float(bh[j]);

@@ -989,7 +989,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       const int first = odd ? 1 : 0;
       const int n0 = slab * kTsBN + (col & ~1);
       if (MODE == 0) {
-        const float bias = p.bias != nullptr && n0 < p.N ? __half2float(__ldg(p.bias + n0 + first)) : 0.f;
+        const float bias = p.bias != nullptr && n0 < p.N ? load_bias(p.bias + n0 + first) : 0.f;
 #pragma unroll
         for (int m = 0; m < MT; ++m) v[m] += bias;
         handover::store_rows<MT>(v, p.out + (size_t)first * p.N + n0, (size_t)p.N, first,
@@ -1070,7 +1070,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         const int n = task / Q, piece = n * p.split + rank, token = (piece >> 3) * Cfg::kPieceTokens + 4 * (task % Q);
         if (token >= p.M) continue;
         const int n0 = slab * kTsBN + 32 * (piece & 7) + 8 * (g >> 1) + 2 * i;
-        const float bias = p.bias != nullptr && n0 < p.N ? __half2float(__ldg(p.bias + n0 + first)) : 0.f;
+        const float bias = p.bias != nullptr && n0 < p.N ? load_bias(p.bias + n0 + first) : 0.f;
         const bool ok = __all_sync(0xffffffffu, mbar_wait_cluster(recv_full(n), 0, &s_abort, 25));
         const uint32_t src = recv_at(n, 0) + (task % Q) * 512 + lane * 16;
         float y[4] = {0.f, 0.f, 0.f, 0.f};

@@ -260,7 +260,7 @@ __device__ __forceinline__ void wt_load_bias(const WtParams& p, int first_column
 #pragma unroll
   for (int i = 0; i < 4; ++i)
     bias[i] = p.bias != nullptr && first_column < p.N
-                  ? __half2float(__ldg(p.bias + first_column + 8 * (g >> 1) + 2 * i + (g & 1)))
+                  ? load_bias(p.bias + first_column + 8 * (g >> 1) + 2 * i + (g & 1))
                   : 0.f;
 }
 __device__ __forceinline__ void wt_add_bias(float (&d)[2][16], const float (&bias)[4]) {
@@ -391,8 +391,8 @@ __device__ __forceinline__ void wt_epilogue_wide(const WtParams& p, const Work& 
 
 // Epilogue warp q of the SPLIT kernel: pairs of a cluster share a tile, and each sums some of its eights of tokens.  First
 // the parts that others sum are stored into their shared memory (the CTA of the same rank), for all segments; then the
-// own ones are added up in the pairs' order.  Every index is settled while the MMAs run: the warp has nothing else to do
-// then, and afterwards each division costs 200 cycles.
+// own ones are added up in the pairs' order.  Every index is settled, and the bias fetched, while the MMAs run: the warp
+// has nothing else to do then, and afterwards each division costs 200 cycles.
 struct WtSplitSegment {
   uint32_t dcol;               // its accumulator
   uint32_t base;               // partial sums that this warp takes in, or puts into another CTA at the same place:
@@ -400,7 +400,8 @@ struct WtSplitSegment {
   uint32_t d_full, full;       // barriers
   int first, n, me;            // sharers: the first pair, their number, this one
   int eights, recip;
-  float bias[4];
+  int column;                  // first one of the warp
+  float bias[4];               // loaded after pdl_wait
   __half* dst;
   int rows;
   __device__ __forceinline__ int own_first(int i) const { return ((i * eights + n - 1) * recip) >> 16; }
@@ -423,7 +424,7 @@ __device__ __forceinline__ WtSplitSegment wt_split_segment(const WtParams& p, co
   f.full = recv_full + 8 * (lt & 1);
   f.d_full = d_full0 + 8 * buf;
   f.dcol = tmem + ((uint32_t)(q * 32) << 16) + buf * p.dcols;
-  wt_load_bias(p, WtOut<0>::first_column(t, rank, q), lane >> 2, f.bias);
+  f.column = WtOut<0>::first_column(t, rank, q);
   const WtOut<0> out(p, t, rank, q, lane);
   f.dst = out.dst;
   f.rows = out.rows;
@@ -433,11 +434,13 @@ template <int GROUP>
 __device__ __forceinline__ void wt_epilogue_split(const WtParams& p, const Work& work, uint32_t tmem, int rank, int q,
                                                   int lane, uint32_t d_full0, uint32_t recv, uint32_t recv_full,
                                                   volatile int* abort_flag) {
-  const WtSplitSegment s0 = wt_split_segment<GROUP>(p, work, 0, tmem, rank, q, lane, d_full0, recv, recv_full);
+  WtSplitSegment s0 = wt_split_segment<GROUP>(p, work, 0, tmem, rank, q, lane, d_full0, recv, recv_full);
   WtSplitSegment s1 = s0;
   if (work.segs > 1) s1 = wt_split_segment<GROUP>(p, work, 1, tmem, rank, q, lane, d_full0, recv, recv_full);
   const size_t pitch = (size_t)p.N;
-  pdl_wait();  // orders this thread's writes after the kernel before this one
+  pdl_wait();  // orders this thread's writes after the kernel before this one, which may have written the bias
+  wt_load_bias(p, s0.column, lane >> 2, s0.bias);
+  wt_load_bias(p, s1.column, lane >> 2, s1.bias);
   bool ok = true;
 #pragma unroll 1
   for (int seg = 0; seg < work.segs; ++seg) {

@@ -215,6 +215,43 @@ def test_back_to_back_layers_see_each_others_outputs(A, m):
             assert torch.equal(ref, o)
 
 
+# Every kernel that adds a bias, each of its forms: clusters and ranges, whole tiles through shared memory.
+@pytest.mark.parametrize("kernel,m,k,n,group", [
+    ("KERNEL_AUTO", 100, 8192, 5120, 128), ("KERNEL_AUTO", 60, 4096, 4096, 64), ("KERNEL_AUTO", 300, 8192, 1312, 128),
+    ("KERNEL_AUTO", 100, 8192, 10240, 128), ("KERNEL_WT", 40, 8192, 1312, 128), ("KERNEL_WT", 500, 128, 9504, 128),
+    ("KERNEL_AUTO", 3, 2048, 5120, 128), ("KERNEL_AUTO", 24, 8192, 1280, 128), ("KERNEL_AUTO", 4, 8192, 10240, 128),
+    ("KERNEL_STREAM", 8, 4096, 1536, 128), ("KERNEL_AUTO", 8, 4096, 1536, 32), ("KERNEL_Q8", 8, 4096, 1536, 128)])
+def test_bias_may_be_the_output_of_the_call_before(A, kernel, m, k, n, group):
+    """A kernel runs ahead of the end of the one before it, and reads the bias only after that end."""
+    from awq_b200 import synth
+    maker = [t.cuda() for t in synth.awq_linear_tensors(8192, n, 128, seed=5)]
+    qw, s, qz = (t.cuda() for t in synth.awq_linear_tensors(k, n, group, seed=6))
+    if kernel == "KERNEL_Q8":
+        qw = A.awq_repack_kmajor(qw)
+    x = synth.activations(m, k, seed=7).cuda()
+    makers = [synth.activations(1, 8192, seed=8 + i).cuda() for i in range(3)]
+    bias = torch.zeros(1, n, dtype=torch.float16, device="cuda")
+
+    def calls(sync):
+        ys = []
+        for i in range(12):
+            A.awq_gemm(makers[i % 3], *maker, 8, out=bias)
+            if sync:
+                torch.cuda.synchronize()
+            ys.append(A.awq_gemm(x, qw, s, qz, 8, bias=bias[0], kernel=getattr(A, kernel)))
+            if sync:
+                torch.cuda.synchronize()
+        return ys
+
+    want = calls(True)
+    assert not torch.equal(want[0], want[1]) and torch.equal(want[0], want[3])
+    for _ in range(3):
+        bias.fill_(float("nan"))
+        got = calls(False)
+        torch.cuda.synchronize()
+        assert all(torch.equal(y, ref) for y, ref in zip(got, want))
+
+
 @pytest.mark.parametrize("m,group", [(8, 128), (16, 128), (16, 64), (17, 64), (24, 64), (32, 64), (32, 32)])
 def test_small_batches_apply_the_scales_in_fp32(A, m, group):
     """Up to 16 tokens, and 32 with the finer groups, nothing but the output is rounded to fp16: its error
