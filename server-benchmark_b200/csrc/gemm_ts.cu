@@ -832,6 +832,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
           b = 0.f;
         }
         cluster_wait();
+        if (!ok) continue;  // a CTA that gave up sends nothing: who sums waits in vain, and stores nothing
         const int owner = fold % p.split, n = fold / p.split;
         const uint32_t dst = recv_at(n, rank) + lane * 8;
         if (owner == rank) {
@@ -846,6 +847,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       if constexpr (SPLIT) {
         constexpr int T = Cfg::kPieceTokens, Q = T / 4;
         cluster_wait();  // every CTA's barriers are set up
+        if (!ok) continue;  // as above
 #pragma unroll
         for (int half = 0; half < Cfg::kHalves; ++half) {
           const int piece = half * 8 + fold, owner = piece % p.split, n = piece / p.split, quads = piece_quads(half);

@@ -449,8 +449,9 @@ __device__ __forceinline__ void wt_epilogue_split(const WtParams& p, const Work&
     ok = __all_sync(0xffffffffu, ok);
     tc_fence_after();
     int e = 0;
+    // a CTA that gave up sends nothing: who sums waits in vain, and stores nothing
 #pragma unroll 1
-    for (int to = 0; to < f.n; ++to) {
+    for (int to = ok ? 0 : f.n; to < f.n; ++to) {
       const int end = f.own_first(to + 1);
       if (to != f.me) {
         const uint32_t cta = 2 * (f.first + to) + rank, bar = map_rank(f.full, cta);
