@@ -1094,11 +1094,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 
   // ---- teardown ----
   __syncwarp();
-  if (s_abort) {
-    // a wait gave up: copies and MMAs may still be in flight towards this CTA's shared and tensor
-    // memory.  Let them land before both are given back.
-    linger();
-  }
+  const bool gave_up = s_abort != 0;
   tc_fence_before();
   if (SPLIT) {
     // a CTA may go when nobody stores into it any more
@@ -1106,6 +1102,11 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     if (warp < kTsFold0 || warp >= kTsFold0 + kTsFoldWarps || work.segs == 0) cluster_wait();
     cluster_arrive_relaxed();
     cluster_wait();
+  }
+  if (gave_up) {
+    // copies, MMAs and what other CTAs stored until the barrier above may still be in flight
+    // towards this CTA's shared and tensor memory.  Let them land before both are given back.
+    linger();
   }
   __syncthreads();
   if (warp == kTsIssue) {
