@@ -36,16 +36,17 @@ inline bool pdl_enabled() {
 }
 // How many clusters of `S` CTAs (x dimension) of `kernel` the GPU holds at once.  A cluster must
 // find all its SMs free inside one GPC, so odd sizes pack badly: a grid with more clusters than
-// this runs in waves.  `cache` holds one answer per size (0 = not asked yet); an answer the
-// runtime cannot give counts as "enough".  The kernel's dynamic shared-memory limit must have
-// been raised before the first call.
+// this runs in waves.  `cache` holds one answer per size (0 = not asked yet, -1 = none fits); 0 also
+// where the runtime gives no answer, which is not kept: who chooses a size by it must not choose one that
+// a part of a GPU may not have.  The kernel's dynamic shared-memory limit must have been raised before the
+// first call.
 constexpr int kMaxCluster = 16;  // above 8 only kernels that allow it (a function attribute)
 template <typename Kernel>
 inline int resident_clusters(Kernel kernel, int S, int threads, size_t smem,
                              std::atomic<int>* cache) {
-  if (S < 1 || S > kMaxCluster) return 1 << 30;
+  if (S < 1 || S > kMaxCluster) return 0;
   const int known = cache[S];
-  if (known > 0) return known;
+  if (known != 0) return known < 0 ? 0 : known;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(S, 1024, 1);
   cfg.blockDim = dim3(threads, 1, 1);
@@ -58,12 +59,12 @@ inline int resident_clusters(Kernel kernel, int S, int threads, size_t smem,
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   int got = 0;
-  if (cudaOccupancyMaxActiveClusters(&got, kernel, &cfg) != cudaSuccess || got <= 0) {
+  if (cudaOccupancyMaxActiveClusters(&got, kernel, &cfg) != cudaSuccess) {
     (void)cudaGetLastError();
-    got = 1 << 30;
+    return 0;
   }
-  cache[S] = got;
-  return got;
+  cache[S] = got > 0 ? got : -1;
+  return got > 0 ? got : 0;
 }
 
 // Plain (non-cluster) launch with the attribute.  The kernel must execute pdl_wait before it

@@ -1090,7 +1090,7 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 
 // ---- host side -------------------------------------------------------------------------------
 
-// Pairs of CTAs the GPU holds at once (one CTA per SM).
+// Pairs of CTAs the GPU holds at once (one CTA per SM): how wide the work is spread, every GPU has room for one.
 template <int MODE, int GROUP, bool WIDE, bool SPLIT = false>
 int wt_pairs(int smem) {
   static std::atomic<int> cached[64][9];  // zero-initialised: not asked yet
@@ -1098,7 +1098,7 @@ int wt_pairs(int smem) {
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 1;
   const int got = resident_clusters(gemm_wt_kernel<MODE, GROUP, WIDE, SPLIT>, 2, kWtThreads, smem, cached[dev]);
   const int most = sm_count() / 2 < kWtMaxPairs ? sm_count() / 2 : kWtMaxPairs;
-  return got < most ? got : most;
+  return got > 0 && got < most ? got : most;
 }
 
 template <int MODE, int GROUP, bool WIDE, bool SPLIT = false>
