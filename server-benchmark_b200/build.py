@@ -55,7 +55,7 @@ def _run(cmd: list[str], out: str, verbose: bool) -> None:
 def build(force: bool = False, verbose: bool = False) -> str:
     """Compile every .cu under csrc/ into one shared library, then the host path that links to
     it; returns the library's path."""
-    if force or _stale(OUT, sources() + glob.glob(os.path.join(CSRC, "*.cuh")) + _headers()):
+    if force or _stale(OUT, sources() + glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(CSRC, "*.h")) + _headers()):
         nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
         if not os.path.exists(nvcc):
             raise RuntimeError("nvcc not found: cannot build libawq_b200.so")

@@ -87,6 +87,7 @@
 // Units of twice the K, more load warps, a shorter loop (two halves in turn: 10 % slower) and longer suspended waits
 // changed nothing or lost.
 #include "common.cuh"
+#include "cut_cache.h"
 #include "handover.cuh"
 #include "tc_ptx.cuh"
 
@@ -1329,25 +1330,22 @@ WtPlan wt_cluster_search(WtPlan best, int M, int slabs, int KT, Resident residen
   return best;
 }
 
-// The search takes a few microseconds: a thread keeps the cuts it used last.  `resident`: nullptr for no clusters.
-WtPlan wt_plan(int M, int slabs, int KT, int most, bool split, int (*resident)(int pairs) = nullptr) {
-  struct Entry {
-    int M, slabs, KT, key;
-    int (*resident)(int);
-    WtPlan plan;
-  };
-  static thread_local Entry seen[64];  // zero-initialised: M 0 is no call
-  const unsigned hash = (unsigned)M * 2654435761u ^ (unsigned)slabs * 40503u ^ (unsigned)KT * 97u;
-  Entry& e = seen[(hash >> 8) % 64];
-  const int key = 2 * most + (split ? 1 : 0);
-  if (e.M != M || e.slabs != slabs || e.KT != KT || e.key != key || e.resident != resident) {
+int current_device() {
+  int dev = -1;
+  return cudaGetDevice(&dev) == cudaSuccess ? dev : -1;
+}
+
+// `resident`: nullptr for no clusters.  A call asks for the ranges (how much scratch) and for the clusters of one shape.
+WtPlan wt_plan(int M, int slabs, int KT, int most, bool split, int group, int (*resident)(int pairs) = nullptr) {
+  static thread_local CutCache<WtPlan> cuts;
+  const CutKey key = {M, slabs, KT, most, current_device(), group, (split ? 1 : 0) + (resident != nullptr ? 2 : 0)};
+  return cuts.get(key, [&] {
     WtPlan plan = wt_search(M, slabs, KT, most, split);
     // whole tiles that fill the GPU stay as they are
     const bool full = M > 256 && (long)slabs * ((M + 255) / 256) >= most;
     if (resident != nullptr && !full) plan = wt_cluster_search(plan, M, slabs, KT, resident);
-    e = Entry{M, slabs, KT, key, resident, plan};
-  }
-  return e.plan;
+    return plan;
+  });
 }
 
 // Clusters of that many pairs that the GPU holds at once.
@@ -1368,13 +1366,13 @@ int launch_wt_dense(const __half* x, const uint32_t* qweight, WtParams p, void* 
   p.KT = p.K / kWtBK;
   const int most = wt_pairs<0, GROUP, false>(kWtSmemLimit);
   const auto resident = clusters ? wt_resident<GROUP> : nullptr;
-  WtPlan plan = wt_plan(p.M, p.slabs, p.KT, most, true, resident);
+  WtPlan plan = wt_plan(p.M, p.slabs, p.KT, most, true, GROUP, resident);
   if (plan.chunk > 0) {
     if (workspace != nullptr && workspace_bytes >= wt_scratch_bytes(plan.nt, plan.pairs)) {
       p.partial = static_cast<float*>(workspace);
       p.flags = handover::make_flags(workspace, wt_partial_bytes(plan.nt, plan.pairs));
     } else {
-      plan = wt_plan(p.M, p.slabs, p.KT, most, false, resident);
+      plan = wt_plan(p.M, p.slabs, p.KT, most, false, GROUP, resident);
     }
   }
   p.nt = plan.nt;
@@ -1404,7 +1402,7 @@ bool gemm_wt_supported(int M, int N, int K, int group) {
 
 size_t gemm_wt_workspace_bytes(int M, int N, int K, int group) {
   if (!gemm_wt_supported(M, N, K, group)) return 0;
-  const WtPlan plan = wt_plan(M, (N + kWtBN - 1) / kWtBN, K / kWtBK, sm_count() / 2, true);
+  const WtPlan plan = wt_plan(M, (N + kWtBN - 1) / kWtBN, K / kWtBK, sm_count() / 2, true, group);
   return plan.chunk > 0 ? wt_scratch_bytes(plan.nt, plan.pairs) : 0;
 }
 
@@ -1414,7 +1412,7 @@ int gemm_wt_cut(int M, int N, int K, int group, int cta_pairs, int* tokens, int*
     if (int rc = group == 128 ? wt_prepare<0, 128, false>() : wt_prepare<0, 64, false>()) return rc;
     cta_pairs = group == 128 ? wt_pairs<0, 128, false>(kWtSmemLimit) : wt_pairs<0, 64, false>(kWtSmemLimit);
   }
-  const WtPlan plan = wt_plan(M, (N + kWtBN - 1) / kWtBN, K / kWtBK, cta_pairs, true);
+  const WtPlan plan = wt_plan(M, (N + kWtBN - 1) / kWtBN, K / kWtBK, cta_pairs, true, group);
   WtParams p = {};
   p.nt = plan.nt;
   p.chunk = plan.chunk;
