@@ -104,6 +104,16 @@ size_t awq_b200_gemm_workspace_bytes(int M, int N, int K, int group, int kernel)
 int awq_b200_gemm_wt_cut(int M, int N, int K, int group, int cta_pairs, int* tokens, int* chunk, int* wide);
 
 /*
+ * How a call of awq_b200_gemm that has its scratch is cut, in cut[6]: the kernel (what AWQ_B200_KERNEL_AUTO takes);
+ * and of AWQ_B200_KERNEL_TS and AWQ_B200_KERNEL_WT, otherwise 0: tokens of a tile; units of 128 rows in a CTA's (WT: a
+ * pair's) range (0: whole tiles, or clusters); CTAs of a cluster that share tiles through distributed shared memory (0:
+ * none do), and how many tiles; accumulators of WT.  A call that names the kernel is never cut into clusters.
+ * room[i], i up to 16: clusters of i CTAs of such a kernel (one CTA per SM) that the GPU holds at once, room[1] its SMs;
+ * NULL: the current device's.  Host arithmetic, for tests that name a cut.  No counterpart in the reference.
+ */
+int awq_b200_gemm_cut(int M, int N, int K, int group, int kernel, const int* room, int* cut);
+
+/*
  * Optional load-time repack of qweight for the decode kernel (AWQ_B200_KERNEL_STREAM_RP):
  * out int32 [K/4, N/8, 4] holds, for every quad of rows and packed word column, the four
  * row-pair registers the in-kernel unpack otherwise builds with byte permutes -- a pure

@@ -32,6 +32,7 @@ PROTOTYPES = {
                                     c_void_p]),
     "awq_b200_gemm_workspace_bytes": (c_size_t, [c_int, c_int, c_int, c_int, c_int]),
     "awq_b200_gemm_wt_cut": (c_int, [c_int] * 5 + [POINTER(c_int)] * 3),
+    "awq_b200_gemm_cut": (c_int, [c_int] * 5 + [POINTER(c_int)] * 2),
     "awq_b200_repack_qweight": (c_int, [c_void_p, c_void_p, c_int, c_int, c_void_p]),
     "awq_b200_gemm": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
                               c_int, c_int, c_int, c_int, c_void_p, c_size_t, c_void_p]),

@@ -151,6 +151,26 @@ int awq_b200_gemm_wt_cut(int M, int N, int K, int group, int cta_pairs, int* tok
   return awq::gemm_wt_cut(M, N, K, group, cta_pairs, tokens, chunk, wide);
 }
 
+int awq_b200_gemm_cut(int M, int N, int K, int group, int kernel, const int* room, int* cut) {
+  if (!cut) return AWQ_B200_ERR_NULL;
+  if (M <= 0 || (room != nullptr && (room[1] < 1 || room[2] < 1))) return AWQ_B200_ERR_SHAPE;
+  if (int rc = check_awq_shape(N, K, group)) return rc;
+  if (room == nullptr)
+    if (int rc = check_device()) return rc;
+  const bool automatic = kernel == AWQ_B200_KERNEL_AUTO;
+  if (automatic) kernel = pick_gemm_kernel(M, N, K, group, true);
+  awq::GemmCut c = {};
+  if (kernel == AWQ_B200_KERNEL_TS) {
+    if (!automatic && M > kTsNamedRows) return AWQ_B200_ERR_SHAPE;
+    if (int rc = awq::gemm_ts_cut(M, N, K, group, automatic, room, &c)) return rc;
+  } else if (kernel == AWQ_B200_KERNEL_WT) {
+    if (int rc = awq::gemm_wt_cut(M, N, K, group, automatic, room, &c)) return rc;
+  }
+  const int told[6] = {kernel, c.tokens, c.chunk, c.cluster, c.tiles, c.accumulators};
+  for (int i = 0; i < 6; ++i) cut[i] = told[i];
+  return AWQ_B200_OK;
+}
+
 int awq_b200_gemm(const void* x, const void* qweight, const void* scales, const void* qzeros,
                   const void* bias, void* out, int M, int N, int K, int group, int kernel,
                   void* workspace, size_t workspace_bytes, void* stream) {
@@ -189,7 +209,8 @@ int awq_b200_gemm(const void* x, const void* qweight, const void* scales, const 
       if (!awq::gemm_ts_supported(M, N, K, group) || (!automatic && M > kTsNamedRows)) return AWQ_B200_ERR_SHAPE;
       // scratch is optional here: without it (or misaligned) whole slabs are distributed
       if ((reinterpret_cast<uintptr_t>(workspace) & 255u) != 0) workspace = nullptr;
-      return awq::launch_gemm_ts(xh, qw, sc, qz, bh, oh, M, N, K, group, workspace, workspace_bytes, st);
+      // a call that names the kernel keeps the ranges, of this kernel and of gemm_wt
+      return awq::launch_gemm_ts(xh, qw, sc, qz, bh, oh, M, N, K, group, workspace, workspace_bytes, automatic, st);
     case AWQ_B200_KERNEL_TS_EXACT:
       // the magic-number conversion has one home, the streaming kernel
       if (M > 16 || !awq::gemm_ts_supported(M, N, K, group)) return AWQ_B200_ERR_SHAPE;
@@ -201,7 +222,6 @@ int awq_b200_gemm(const void* x, const void* qweight, const void* scales, const 
       if (!awq::gemm_wt_supported(M, N, K, group)) return AWQ_B200_ERR_SHAPE;
       // scratch is optional here: without it (or misaligned) whole tiles are distributed
       if ((reinterpret_cast<uintptr_t>(workspace) & 255u) != 0) workspace = nullptr;
-      // a call that names the kernel gets the cut that awq_b200_gemm_wt_cut tells
       return awq::launch_gemm_wt(xh, qw, sc, qz, bh, oh, M, N, K, group, workspace, workspace_bytes,
                                  automatic, st);
     case AWQ_B200_KERNEL_Q8: {

@@ -210,13 +210,19 @@ bool gemm_ts_supported(int M, int N, int K, int group);
 size_t gemm_ts_workspace_bytes(int M, int N, int K, int group);
 int launch_gemm_ts(const __half* x, const uint32_t* qweight, const __half* scales,
                    const uint32_t* qzeros, const __half* bias, __half* out, int M, int N, int K,
-                   int group, void* workspace, size_t workspace_bytes, cudaStream_t stream);
+                   int group, void* workspace, size_t workspace_bytes, bool clusters, cudaStream_t stream);
+// How a dense call with its scratch is cut (awq_b200_gemm_cut).
+struct GemmCut {
+  int tokens, chunk, cluster, tiles, accumulators;
+};
+int gemm_ts_cut(int M, int N, int K, int group, bool clusters, const int* room, GemmCut* cut);
 int ts_device_status(int* out, int clear);
 
 // gemm_wt.cu: dequantised weights in tensor memory as the A operand, activations as B
 bool gemm_wt_supported(int M, int N, int K, int group);
 size_t gemm_wt_workspace_bytes(int M, int N, int K, int group);
 int gemm_wt_cut(int M, int N, int K, int group, int cta_pairs, int* tokens, int* chunk, int* wide);
+int gemm_wt_cut(int M, int N, int K, int group, bool clusters, const int* room, GemmCut* cut);
 int launch_gemm_wt(const __half* x, const uint32_t* qweight, const __half* scales,
                    const uint32_t* qzeros, const __half* bias, __half* out, int M, int N, int K,
                    int group, void* workspace, size_t workspace_bytes, bool clusters, cudaStream_t stream);

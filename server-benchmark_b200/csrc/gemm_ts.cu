@@ -1133,10 +1133,10 @@ struct TsCut {
 //   units x max(...)                352 + 3 tokens: conversion; 2.7 CTAs: the words' way from HBM
 //   1440 + 16 tokens (1 + CTAs)     a slab handed over, CTAs the last one collects from
 //   530                             a further slab
-//   580                             more than half of the GPU: the next kernel's start is not hidden
-TsCut ts_ranges(int slabs, int KT, int tokens) {
+//   580                             more than half of the GPU (of `most` SMs): the next kernel's start is not hidden
+TsCut ts_ranges(int slabs, int KT, int tokens, int most) {
   const long units = (long)slabs * KT;
-  const int most = sm_count(), even = (int)((units + most - 1) / most);
+  const int even = (int)((units + most - 1) / most);
   TsCut best = {0, 0, -1};
   for (const int parts : {1, 2, 3, 4, 6, 8, 12, 16}) {
     const int floor = (KT + parts - 1) / parts, chunk = parts == 1 ? 0 : (even > floor ? even : floor);
@@ -1217,14 +1217,15 @@ int ts_resident(int split) {
   return resident_clusters(gemm_ts_kernel<MT, MODE, GROUP, true>, split, Cfg::kThreads, Cfg::kSmem, cached[dev]);
 }
 
+// `room`: clusters of every size that the GPU holds at once, the first its SMs; nullptr: of this GPU.
 template <int MT, int GROUP, int MODE = 0>
-TsCut ts_cut(int slabs, int KT) {
-  const TsCut ranges = ts_ranges(slabs, KT, MT);
+TsCut ts_cut(int slabs, int KT, const int* room = nullptr) {
+  const TsCut ranges = ts_ranges(slabs, KT, MT, room != nullptr ? room[1] : sm_count());
   TsCut best = {0, 0, -1};
   bool hidden = true;  // the next kernel's start
   for (const int split : {2, 3, 4, 5, 6, 8, 16}) {
     if (split > KT) break;
-    const int resident = ts_resident<MT, GROUP, MODE>(split);
+    const int resident = room != nullptr ? room[split] : ts_resident<MT, GROUP, MODE>(split);
     if (slabs > resident) continue;
     const long cost = ts_split_cost(slabs, KT, MT, GROUP, split, resident);
     if (best.cost >= 0 && cost >= best.cost) continue;
@@ -1316,11 +1317,11 @@ constexpr size_t ts_partial_bytes(int tokens) {
 template <int MT, int GROUP>
 int launch_ts_dense(const __half* x, const uint32_t* qweight, const __half* scales,
                     const uint32_t* qzeros, TsParams p, void* workspace, size_t workspace_bytes,
-                    cudaStream_t stream) {
+                    bool clusters, cudaStream_t stream) {
   p.KT = p.K / kTsBK;
   p.slabs = (p.N + kTsBN - 1) / kTsBN;
   if (int rc = ts_prepare_split<MT, GROUP>()) return rc;
-  const TsCut cut = ts_cut<MT, GROUP>(p.slabs, p.KT);
+  const TsCut cut = clusters ? ts_cut<MT, GROUP>(p.slabs, p.KT) : ts_ranges(p.slabs, p.KT, MT, sm_count());
   p.split = cut.split;
   int ctas = ts_ctas() < p.slabs ? ts_ctas() : p.slabs;
   if (cut.chunk > 0 && workspace != nullptr && workspace_bytes >= gemm_ts_workspace_bytes(p.M, p.N, p.K, GROUP)) {
@@ -1401,7 +1402,7 @@ int launch_ts_experts(const MoeArgs& a, __half* act, int64_t act_rows, __half* p
     if (p.sorted_ids == nullptr && a.topk > 1 && a.topk <= 8) {
       const int clusters = a.T * p.slabs, resident = ts_resident<MT, 128, 2>(a.topk);
       if (clusters <= resident && ts_slots_cost(p.slabs, clusters, p.KT, a.topk) <
-                                      ts_ranges(p.numel * p.slabs, p.KT, MT).cost + kTsSumKernel) {
+                                      ts_ranges(p.numel * p.slabs, p.KT, MT, sm_count()).cost + kTsSumKernel) {
         *summed = true;
         p.split = a.topk;
         p.out = a.out;
@@ -1428,7 +1429,7 @@ size_t gemm_ts_workspace_bytes(int M, int N, int K, int group) {
 
 int launch_gemm_ts(const __half* x, const uint32_t* qweight, const __half* scales,
                    const uint32_t* qzeros, const __half* bias, __half* out, int M, int N, int K,
-                   int group, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
+                   int group, void* workspace, size_t workspace_bytes, bool clusters, cudaStream_t stream) {
   if (!gemm_ts_supported(M, N, K, group)) return AWQ_B200_ERR_SHAPE;
   TsParams p = {};
   p.bias = bias;
@@ -1440,7 +1441,30 @@ int launch_gemm_ts(const __half* x, const uint32_t* qweight, const __half* scale
   if (M <= 4) launch = group == 128 ? launch_ts_dense<4, 128> : launch_ts_dense<4, 64>;
   else if (M <= 8) launch = group == 128 ? launch_ts_dense<8, 128> : launch_ts_dense<8, 64>;
   else if (M <= 16) launch = group == 128 ? launch_ts_dense<16, 128> : launch_ts_dense<16, 64>;
-  return launch(x, qweight, scales, qzeros, p, workspace, workspace_bytes, stream);
+  return launch(x, qweight, scales, qzeros, p, workspace, workspace_bytes, clusters, stream);
+}
+
+namespace {
+template <int MT, int GROUP>
+int ts_tell_cut(int slabs, int KT, bool clusters, const int* room, TsCut* cut) {
+  if (room == nullptr)
+    if (int rc = ts_prepare_split<MT, GROUP>()) return rc;
+  *cut = clusters ? ts_cut<MT, GROUP>(slabs, KT, room)
+                  : ts_ranges(slabs, KT, MT, room != nullptr ? room[1] : sm_count());
+  return AWQ_B200_OK;
+}
+}  // namespace
+
+int gemm_ts_cut(int M, int N, int K, int group, bool clusters, const int* room, GemmCut* out) {
+  if (!gemm_ts_supported(M, N, K, group)) return AWQ_B200_ERR_SHAPE;
+  auto tell = group == 128 ? ts_tell_cut<32, 128> : ts_tell_cut<32, 64>;
+  if (M <= 4) tell = group == 128 ? ts_tell_cut<4, 128> : ts_tell_cut<4, 64>;
+  else if (M <= 8) tell = group == 128 ? ts_tell_cut<8, 128> : ts_tell_cut<8, 64>;
+  else if (M <= 16) tell = group == 128 ? ts_tell_cut<16, 128> : ts_tell_cut<16, 64>;
+  TsCut cut;
+  if (int rc = tell((N + kTsBN - 1) / kTsBN, K / kTsBK, clusters, room, &cut)) return rc;
+  *out = {ts_tokens(M), cut.chunk, cut.split, cut.split > 0 ? 1 : 0, 0};
+  return AWQ_B200_OK;
 }
 
 bool moe_ts_supported(const MoeArgs& a) {

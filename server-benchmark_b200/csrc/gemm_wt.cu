@@ -1330,6 +1330,14 @@ WtPlan wt_cluster_search(WtPlan best, int M, int slabs, int KT, Resident residen
   return best;
 }
 
+template <typename Resident>
+WtPlan wt_find(int M, int slabs, int KT, int most, bool split, bool clusters, Resident resident) {
+  const WtPlan plan = wt_search(M, slabs, KT, most, split);
+  // whole tiles that fill the GPU stay as they are
+  const bool full = M > 256 && (long)slabs * ((M + 255) / 256) >= most;
+  return clusters && !full ? wt_cluster_search(plan, M, slabs, KT, resident) : plan;
+}
+
 int current_device() {
   int dev = -1;
   return cudaGetDevice(&dev) == cudaSuccess ? dev : -1;
@@ -1339,13 +1347,7 @@ int current_device() {
 WtPlan wt_plan(int M, int slabs, int KT, int most, bool split, int group, int (*resident)(int pairs) = nullptr) {
   static thread_local CutCache<WtPlan> cuts;
   const CutKey key = {M, slabs, KT, most, current_device(), group, (split ? 1 : 0) + (resident != nullptr ? 2 : 0)};
-  return cuts.get(key, [&] {
-    WtPlan plan = wt_search(M, slabs, KT, most, split);
-    // whole tiles that fill the GPU stay as they are
-    const bool full = M > 256 && (long)slabs * ((M + 255) / 256) >= most;
-    if (resident != nullptr && !full) plan = wt_cluster_search(plan, M, slabs, KT, resident);
-    return plan;
-  });
+  return cuts.get(key, [&] { return wt_find(M, slabs, KT, most, split, resident != nullptr, resident); });
 }
 
 // Clusters of that many pairs that the GPU holds at once.
@@ -1421,6 +1423,29 @@ int gemm_wt_cut(int M, int N, int K, int group, int cta_pairs, int* tokens, int*
   *tokens = plan.nt;
   *chunk = plan.chunk;
   *wide = p.stage_bytes > 0 ? 1 : 0;
+  return AWQ_B200_OK;
+}
+
+int gemm_wt_cut(int M, int N, int K, int group, bool clusters, const int* room, GemmCut* out) {
+  if (!gemm_wt_supported(M, N, K, group)) return AWQ_B200_ERR_SHAPE;
+  const int slabs = (N + kWtBN - 1) / kWtBN, KT = K / kWtBK;
+  WtPlan plan;
+  if (room == nullptr) {
+    int rc = group == 128 ? wt_prepare<0, 128, false>() : wt_prepare<0, 64, false>();
+    if (rc == AWQ_B200_OK) rc = group == 128 ? wt_prepare<0, 128, false, true>() : wt_prepare<0, 64, false, true>();
+    if (rc) return rc;
+    const int most = group == 128 ? wt_pairs<0, 128, false>(kWtSmemLimit) : wt_pairs<0, 64, false>(kWtSmemLimit);
+    plan = wt_plan(M, slabs, KT, most, true, group, !clusters ? nullptr : group == 128 ? wt_resident<128> : wt_resident<64>);
+  } else {
+    plan = wt_find(M, slabs, KT, room[2], true, clusters, [room](int pairs) { return room[2 * pairs]; });
+  }
+  WtParams p = {};
+  p.nt = plan.nt;
+  p.chunk = plan.chunk;
+  p.KT = KT;
+  if (plan.share > 0) p.share = wt_share(plan.share, plan.share_tiles, KT, plan.nt);
+  wt_rings(&p, 0);
+  *out = {plan.nt, plan.chunk, 2 * plan.share, plan.share_tiles, p.nbuf};
   return AWQ_B200_OK;
 }
 

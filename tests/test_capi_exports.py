@@ -259,6 +259,53 @@ def test_grouped_tiles_of_every_size_are_tested(built_library):
     assert {c[0] for c in TILE_CASES} == set(range(128, 257, 16))
 
 
+def test_clusters_of_every_size_and_ranges_are_tested(built_library):
+    """The cuts that the GPU tests of the dense kernels are for, by the room that a B200 has for clusters."""
+    import test_gpu_ts
+    import test_gpu_wt
+    from awq_b200 import _lib
+    from cuts import B200, cut
+    ts, wt = _lib.KERNEL_TS, _lib.KERNEL_WT
+    for call, (ctas, units) in test_gpu_ts.CLUSTERS.items():
+        assert cut(*call, room=B200)[2:5] == (units, ctas, 1 if ctas else 0), call
+    assert {c for c, _ in test_gpu_ts.CLUSTERS.values()} == {0, 2, 3, 4, 5, 6, 8, 16}
+    assert any(c * 128 == k for (_, k, _, _), (c, _) in test_gpu_ts.CLUSTERS.items())
+    for group, ranges in ((128, test_gpu_ts.RANGES), (64, test_gpu_ts.RANGES_64)):
+        for call, units in ranges.items():
+            assert cut(*call, group, ts, B200)[2:4] == (units, 0), call
+    for call, shared in test_gpu_wt.CLUSTERS.items():
+        got = cut(*call, room=B200)
+        assert (got.kernel, got[3:5]) == (wt, shared), call
+        assert cut(*call, wt, B200).cluster == 0
+    assert set(test_gpu_wt.CLUSTERS.values()) == {(c, 1) for c in (4, 6, 8, 10, 12, 16)} | {(6, 2)}
+
+
+def test_calls_whose_clusters_do_not_fit_take_ranges(built_library):
+    """A GPU, or a part of one, without room for a size of clusters: the next best cut, never that size."""
+    import test_gpu_ts
+    import test_gpu_wt
+    from cuts import B200, cut
+    for call in list(test_gpu_ts.CLUSTERS) + list(test_gpu_wt.CLUSTERS):
+        for most in (2, 4, 8):
+            got = cut(*call, room=[n if i <= most else 0 for i, n in enumerate(B200)])
+            assert got.cluster <= most, call
+            rooms = B200[:3] + [min(n, most) for n in B200[3:]]
+            few = cut(*call, room=rooms)
+            slabs, tiles = -(-call[2] // 256), -(-call[0] // few.tokens)
+            assert few.cluster == 0 or slabs * tiles <= rooms[few.cluster] * few.tiles, call
+    from awq_b200 import _lib
+    lib = _lib.load()
+    told = (ctypes.c_int * 6)(*[-1] * 6)
+    room = (ctypes.c_int * 17)(*B200)
+    assert lib.awq_b200_gemm_cut(0, 8192, 1024, 128, 0, room, told) == -2
+    assert lib.awq_b200_gemm_cut(8, 8200, 1024, 128, 5, room, told) == -2   # N % 32
+    assert lib.awq_b200_gemm_cut(17, 8192, 1024, 128, 5, room, told) == -2  # the kernel by name: 16 rows
+    assert lib.awq_b200_gemm_cut(8, 8192, 1024, 128, 0, room, None) == -1
+    assert lib.awq_b200_gemm_cut(8, 8192, 1024, 128, 0, (ctypes.c_int * 17)(0, 148), told) == -2
+    assert list(told) == [-1] * 6
+    assert lib.awq_b200_gemm_cut(8, 8192, 1024, 32, 0, room, told) == 0 and list(told) == [2, 0, 0, 0, 0, 0]
+
+
 def test_wide_tiles_of_every_size_are_tested(built_library):
     """The same for the dense tiles above 128 tokens, whole and split."""
     from awq_b200 import _lib

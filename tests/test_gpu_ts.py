@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 import torch
 
+from cuts import cut
 from oracle import awq_oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -80,12 +81,14 @@ def test_ts_bias_determinism_and_agreement_with_stream_kernel(A):
 
 # Sizes at which the work split and the token variants change: fewer units than CTAs, slabs shared by
 # several CTAs, ranges that end on a slab, whole slabs only, N edge inside a slab, every token variant
-# at its ends.
-@pytest.mark.parametrize("m,k,n", [
-    (1, 128, 32), (4, 8192, 1280), (5, 384, 4768), (8, 2432, 8192), (12, 1024, 38144),
-    (16, 29568, 288), (9, 3712, 2592), (13, 4096, 1056),
-])
+# at its ends.  Units of a CTA's range (0: whole slabs): asserted, as the cut follows from a cost.
+RANGES = {(1, 128, 32): 0, (4, 8192, 1280): 4, (5, 384, 4768): 0, (8, 2432, 8192): 5, (12, 1024, 38144): 9,
+          (16, 29568, 288): 15, (9, 3712, 2592): 5, (13, 4096, 1056): 4}
+
+
+@pytest.mark.parametrize("m,k,n", list(RANGES))
 def test_ts_work_split_edges(A, m, k, n):
+    assert cut(m, k, n, 128, A.KERNEL_TS)[1:4] == (next(t for t in (4, 8, 16) if m <= t), RANGES[m, k, n], 0)
     run_case(A, A.KERNEL_TS, m, k, n, seed=m + n, bias=m % 2 == 1)
 
     # replays of one captured launch interleaved with another shape on the same scratch, and a call
@@ -121,11 +124,15 @@ def test_ts_work_split_edges(A, m, k, n):
 
 # Two quantisation groups of 64 in a unit: one unit in all, shared and whole slabs, the token counts of
 # every variant at their edges, a slab past N, bias.
-@pytest.mark.parametrize("m,k,n", [(1, 128, 32), (4, 8192, 1280), (5, 384, 2080), (8, 4096, 4768),
-                                   (9, 15360, 544), (16, 1536, 28704)])
+RANGES_64 = {(1, 128, 32): 0, (4, 8192, 1280): 4, (5, 384, 2080): 0, (8, 4096, 4768): 5, (9, 15360, 544): 8,
+             (16, 1536, 28704): 0}
+
+
+@pytest.mark.parametrize("m,k,n", list(RANGES_64))
 @pytest.mark.parametrize("bias", [False, True])
 def test_ts_groups_of_64(A, m, k, n, bias):
     from awq_b200 import synth
+    assert cut(m, k, n, 64, A.KERNEL_TS)[2:4] == (RANGES_64[m, k, n], 0)
     qw, s, qz = synth.awq_linear_tensors(k, n, 64, seed=m + n)
     x = synth.activations(m, k, seed=k)
     b = synth.activations(1, n, seed=3)[0] if bias else None
@@ -139,7 +146,9 @@ def test_ts_groups_of_64(A, m, k, n, bias):
     assert O.rel_err(y[0].cpu().numpy(), ref) < TOL
 
 
-@pytest.mark.parametrize("kernel,m,k,n", [("KERNEL_TS", 5, 8192, 1280), ("KERNEL_WT", 40, 8192, 1312)])
+@pytest.mark.parametrize("kernel,m,k,n", [("KERNEL_TS", 5, 8192, 1280), ("KERNEL_WT", 40, 8192, 1312),
+                                          ("KERNEL_TS", 3, 8192, 1280), ("KERNEL_TS", 14, 8192, 1280),
+                                          ("KERNEL_AUTO", 12, 1024, 38144), ("KERNEL_AUTO", 20, 2048, 38144)])
 def test_scratch_may_be_any_buffer_with_any_content(A, kernel, m, k, n):
     """Shared slabs and tiles with more scratch buffers, one after the other, than a table of them could hold,
     each full of other data, and one buffer again and again: always the same bits."""
@@ -147,6 +156,7 @@ def test_scratch_may_be_any_buffer_with_any_content(A, kernel, m, k, n):
     qw, s, qz = (t.cuda() for t in synth.awq_linear_tensors(k, n, 128, seed=1))
     x = synth.activations(m, k, seed=2).cuda()
     lib, kernel = _lib.load(), getattr(A, kernel)
+    assert cut(m, k, n, 128, kernel).chunk > 0  # handed over through the scratch
     need = lib.awq_b200_gemm_workspace_bytes(m, n, k, 128, kernel)
     assert need > 0
     step = -(-need // 256) * 256
@@ -186,12 +196,15 @@ def test_automatic_choice_without_enough_scratch_takes_the_streaming_kernel(A, m
 
 
 def _layers(A, m):
+    """A linear as the automatic choice cuts it (clusters), one that is handed over through the scratch, a MoE layer."""
     from awq_b200 import synth
+    ranges = A.KERNEL_TS if m <= 16 else A.KERNEL_WT
+    assert cut(m, 8192, 1280, 128).cluster > 0 and cut(m, 8192, 1280, 128, ranges).chunk > 0
     dense = [t.cuda() for t in (synth.activations(m, 8192, seed=m), *synth.awq_linear_tensors(8192, 1280, 128, seed=1))]
     e, h, i, k = 16, 1024, 256, 4
     w1, w2 = (tuple(t.cuda() for t in w) for w in synth.moe_layer_tensors(e, h, i, 128, seed=2))
     x, logits = synth.activations(m, h, seed=m).cuda(), synth.gating_logits(m, e, seed=m).cuda()
-    return lambda: (A.awq_gemm(*dense, 8), A.fused_moe(x, w1, w2, logits, k, True))
+    return lambda: (A.awq_gemm(*dense, 8), A.awq_gemm(*dense, 8, kernel=ranges), A.fused_moe(x, w1, w2, logits, k, True))
 
 
 def test_graphs_captured_on_one_stream_run_side_by_side(A):
@@ -236,18 +249,26 @@ def test_capture_on_a_new_stream_takes_calls_of_any_size(A):
     assert torch.equal(y, want)
 
 
-# Slabs shared by clusters of 2, 3, 4, 5, 6, 8 and 16 CTAs (by the estimated cost of a B200's cuts), units that do not
-# divide by them, one unit a CTA, an edge of N inside a slab, the token variants at their ends; ranges over the whole
-# GPU with 17 to 32 tokens; one unit in all.
-@pytest.mark.parametrize("m,k,n,group", [
-    (1, 1024, 8192, 128), (30, 1024, 8192, 64), (3, 2176, 5120, 128), (32, 2176, 5152, 128), (17, 4096, 4064, 64),
-    (9, 640, 1312, 128), (25, 12288, 6176, 128), (24, 8192, 5120, 64), (12, 2048, 1024, 64), (16, 8192, 1280, 128),
-    (31, 8192, 1280, 128), (4, 16384, 992, 64), (5, 256, 256, 128), (20, 128, 32, 128), (23, 8192, 38176, 128),
-    (18, 4096, 28704, 64)])
+# Slabs shared by clusters of 2, 3, 4, 5, 6, 8 and 16 CTAs, units that do not divide by them, one unit a CTA, an edge of N
+# inside a slab, the token variants at their ends; ranges over the whole GPU with 17 to 32 tokens, whole slabs, one unit in
+# all.  CTAs of a cluster on a B200, or units of a range: which of the two is asserted on the GPU, which number on the CPU.
+CLUSTERS = {
+    (1, 1024, 8192, 128): (2, 0), (30, 1024, 8192, 64): (2, 0), (3, 2176, 5120, 128): (3, 0),
+    (32, 2176, 5152, 128): (3, 0), (17, 4096, 4064, 64): (4, 0), (9, 640, 1312, 128): (5, 0),
+    (25, 12288, 6176, 128): (5, 0), (24, 8192, 5120, 64): (6, 0), (12, 2048, 1024, 64): (8, 0),
+    (16, 8192, 1280, 128): (16, 0), (31, 8192, 1280, 128): (16, 0), (4, 16384, 992, 64): (16, 0),
+    (5, 256, 256, 128): (0, 0), (20, 128, 32, 128): (0, 0), (23, 8192, 38176, 128): (0, 65),
+    (18, 4096, 28704, 64): (0, 0), (20, 256, 2080, 128): (2, 0), (2, 512, 1056, 128): (4, 0),
+    (7, 768, 544, 128): (6, 0), (27, 4096, 20512, 64): (0, 18), (32, 2048, 38144, 128): (0, 17)}
+
+
+@pytest.mark.parametrize("m,k,n,group", list(CLUSTERS))
 @pytest.mark.parametrize("bias", [False, True])
 def test_ts_clusters_and_up_to_32_tokens(A, m, k, n, group, bias):
     """Nothing but the output is rounded to fp16, and the bits do not depend on timing."""
     from awq_b200 import synth
+    got, (ctas, units) = cut(m, k, n, group), CLUSTERS[m, k, n, group]
+    assert (got.kernel, got.cluster > 0, got.chunk > 0) == (A.KERNEL_TS, ctas > 0, units > 0)
     qw, s, qz = synth.awq_linear_tensors(k, n, group, seed=m + n)
     x = synth.activations(m, k, seed=k)
     b = synth.activations(1, n, seed=3)[0] if bias else None
