@@ -1217,14 +1217,15 @@ int ts_resident(int split) {
   return resident_clusters(gemm_ts_kernel<MT, MODE, GROUP, true>, split, Cfg::kThreads, Cfg::kSmem, cached[dev]);
 }
 
-// `room`: clusters of every size that the GPU holds at once, the first its SMs; nullptr: of this GPU.
+// `room`: clusters of every size that the GPU holds at once, the first its SMs; nullptr: of this GPU.  `most`: CTAs of a
+// cluster that the caller takes.
 template <int MT, int GROUP, int MODE = 0>
-TsCut ts_cut(int slabs, int KT, const int* room = nullptr) {
+TsCut ts_cut(int slabs, int KT, const int* room = nullptr, int most = kMaxCluster) {
   const TsCut ranges = ts_ranges(slabs, KT, MT, room != nullptr ? room[1] : sm_count());
   TsCut best = {0, 0, -1};
   bool hidden = true;  // the next kernel's start
   for (const int split : {2, 3, 4, 5, 6, 8, 16}) {
-    if (split > KT) break;
+    if (split > KT || split > most) break;
     const int resident = room != nullptr ? room[split] : ts_resident<MT, GROUP, MODE>(split);
     if (slabs > resident) continue;
     const long cost = ts_split_cost(slabs, KT, MT, GROUP, split, resident);
@@ -1379,8 +1380,9 @@ int launch_ts_experts(const MoeArgs& a, __half* act, int64_t act_rows, __half* p
     if constexpr (MT == 4) {
       // Direct form, the number of tiles is known: clusters as for a dense layer of that many slabs and twice the units
       if (int rc2 = ts_prepare_split<MT, 128, 1>()) return rc2;
-      if (p.sorted_ids == nullptr) p.split = ts_cut<MT, 128, 1>(p.numel * p.slabs, 2 * p.KT).split;
-      split = p.split > 1 && p.split <= 8 && p.split <= p.KT;
+      if (p.sorted_ids == nullptr)
+        p.split = ts_cut<MT, 128, 1>(p.numel * p.slabs, 2 * p.KT, nullptr, p.KT < 8 ? p.KT : 8).split;
+      split = p.split > 1;
       if (split)
         if (int rc2 = launch_ts_split<MT, 128, 1>(maps, p, p.numel * p.slabs, stream)) return rc2;
     }

@@ -326,7 +326,7 @@ def test_small_batch_experts_edges(A, t, k, e, h, i, parallel):
 # a slab, one unit in all), down on clusters of a token's slots; every number of slots; a third of the experts absent.
 @pytest.mark.parametrize("t,k,h,i", [(1, 2, 256, 128), (1, 3, 1152, 384), (1, 4, 4096, 1536), (1, 5, 640, 640),
                                      (1, 6, 2048, 768), (1, 7, 896, 896), (1, 8, 2048, 1024), (2, 4, 2048, 768),
-                                     (2, 3, 512, 128)])
+                                     (2, 3, 512, 128), (1, 1, 2048, 768), (1, 2, 2048, 256), (2, 1, 256, 128)])
 @pytest.mark.parametrize("parallel", [False, True])
 def test_direct_clusters_round_like_the_permuted_path(A, t, k, h, i, parallel, monkeypatch):
     from awq_b200 import ops
@@ -532,6 +532,29 @@ def test_expert_parallel_batch_takes_the_kernels_of_its_rows_per_expert(A):
         pytest.skip("the profiler sees no kernels here")
     assert any("gemm_ts_kernel" in n for n in names), names
     assert not any("gemm_wt_kernel" in n for n in names), names
+
+
+# Up to three tiles, for which clusters of more than eight CTAs would be estimated best, and more.
+@pytest.mark.parametrize("k,h,i", [(1, 2048, 768), (2, 2048, 256), (1, 1024, 384), (8, 2048, 768)])
+def test_one_token_runs_gate_up_on_clusters(A, k, h, i):
+    import re
+    from torch.profiler import ProfilerActivity, profile
+    w1, w2, x, logits = _moe_case(16, h, i, 1, k, seed=3)
+    w1d, w2d, xd = tuple(a.cuda() for a in w1), tuple(a.cuda() for a in w2), x.cuda()
+    w, ids, _ = A.fused_topk(xd, logits.cuda(), k, True)
+    A.fused_experts(xd, w1d, w2d, w, ids)
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as prof:
+        A.fused_experts(xd, w1d, w2d, w, ids)
+        torch.cuda.synchronize()
+    names = [event.key for event in prof.key_averages() if "awq::" in event.key]
+    if not names:
+        pytest.skip("the profiler sees no kernels here")
+    # tokens, mode, group, clusters
+    forms = [re.sub(r"\(\w+\)", "", m.group(1)).replace(" ", "").split(",") for m in
+             (re.search(r"gemm_ts_kernel<([^>]*)>", n) for n in names) if m]
+    assert ["4", "1", "128"] in [f[:3] for f in forms], names
+    assert all(f[3] in ("true", "1") for f in forms if f[1] == "1"), names
 
 
 def test_fused_moe_full_size_rows_are_independent(A):
