@@ -28,7 +28,10 @@ namespace cg = cooperative_groups;
 // Scratch for awq_b200_moe_experts_static: 16 MiB of device memory per GPU, reserved when the
 // library is loaded on that GPU and kept until the process ends.
 constexpr size_t kMoeStaticScratchBytes = 16u << 20;
-static __device__ __align__(256) unsigned char g_moe_static_scratch[kMoeStaticScratchBytes];
+// Room beside it for the tokens that row blocks of 8 keep beside their partial sums (gemm_ts.cu): with as much scratch as
+// the layout alone may take they keep the kernels that they had with flags.
+constexpr size_t kMoeStaticMarkBytes = 640u << 10;
+static __device__ __align__(256) unsigned char g_moe_static_scratch[kMoeStaticScratchBytes + kMoeStaticMarkBytes];
 
 namespace awq {
 
@@ -888,7 +891,7 @@ int launch_moe_experts_static(const MoeArgs& a, cudaStream_t stream) {
   // The array still holds whatever the previous call left there.  What the kernels use of it is
   // written earlier in the same call; the one region that must start at zero (per-pair outputs
   // under expert parallelism) is cleared inside launch_moe_experts.
-  return launch_moe_experts(a, scratch, kMoeStaticScratchBytes, stream);
+  return launch_moe_experts(a, scratch, kMoeStaticScratchBytes + (a.block == 8 ? kMoeStaticMarkBytes : 0), stream);
 }
 
 size_t moe_static_scratch_bytes() { return kMoeStaticScratchBytes; }

@@ -78,6 +78,21 @@ def test_static_scratch_entry_point_matches_caller_scratch_twice(built_library):
         assert O.rel_err(out_new.cpu().numpy(), ref) < 1e-2
 
 
+def test_static_scratch_takes_the_same_kernels_near_its_limit(built_library):
+    """Row blocks of 8 whose partial tiles just fit: other kernels would sum in another order."""
+    from awq_b200 import _lib
+    lib = _lib.load()
+    e, h, i, t, k = 64, 128, 6272, 64, 8
+    assert lib.awq_b200_moe_block_size(t, k, e, h, i, 128) == 8
+    p = _problem(lib, e, h, i, t, k, 5)
+    rows = -(-p["sorted_ids"].numel() // 8) * 8
+    partial = 2 * 256 * 8 * 256 * 4 + 256 * 64  # sums of 256 CTAs, two tiles of 8 x 256, and flags
+    assert (15 << 20) < rows * i * 2 + t * k * h * 2 + partial < (16 << 20)
+    out_ref, out_new = _run_both(lib, p)
+    assert torch.isfinite(out_new.float()).all()
+    assert torch.equal(out_ref, out_new)
+
+
 def test_static_scratch_entry_point_refuses_oversized_problems(built_library):
     from awq_b200 import _lib
     lib = _lib.load()
