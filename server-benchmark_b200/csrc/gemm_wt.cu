@@ -62,12 +62,10 @@
 //
 // TMEM columns: accumulators first, then A[slots][8 steps][8], 64 columns a slot.  With as many slots as teams a team waits
 // for the MMAs of its own last unit; two more take that wait out of its loop.  Up to 64 tokens there are two accumulators and
-// six slots.  Up to 128, two accumulators leave four slots; where a CTA ends few tiles for its units it has one accumulator
-// and six slots instead, and the conversion fills them under the epilogue.  That is in clusters with one tile (4096 x 4096
-// M 77 7.8 -> 7.3 us) and in ranges with K from 7168 up: 29568 x 8192 M 100 54.8 -> 53.7 us, in groups of 64 56.4 -> 55.0,
-// 8192 x 10240 M 100 23.8 -> 23.2, 14336 x 4096 26.4 -> 25.9, 7168 x 14336 M 80 28.8 -> 28.7, the four linears of a layer
-// M 100 229 -> 224.5.  With smaller K it loses: 6144 x 28672 M 128 41.4 -> 41.9, 4096 x 22016 M 100 22.75 -> 23.05, 3072 x
-// 22016 M 120 19.4 -> 20.0.  Whole tiles in turn, the grouped ones too, keep two.
+// six slots.  Up to 128, two accumulators leave four slots; one accumulator and six slots gain on every unit, and lose at
+// every tile that a CTA ends before another one, whose MMAs wait for the epilogue (wt_one_accumulator).  They are taken in
+// clusters with one tile (4096 x 4096 M 77 7.8 -> 7.3 us) and in ranges with enough units between two ends of tiles.  Whole
+// tiles in turn, the grouped ones too, keep two.
 // Lane 32 q + 8 i + g holds column 8 (4 q + g / 2) + 2 i + g % 2 of the CTA's 128.
 // All mbarrier and flag waits are bounded (tc_ptx.cuh).
 //
@@ -113,7 +111,6 @@ constexpr int kWtMaxRaw = 16, kWtMaxX = 8;    // ring depths the barrier block h
 constexpr int kWtPartRing = 8, kWtPartBytes = 32 * 32 * 4;  // per epilogue warp: 32 tokens x 32 columns
 constexpr int kWtBarBytes = 1024;
 static_assert(8 * (2 * kWtMaxRaw + 2 * kWtMaxX + 4 + kWtEpiWarps * kWtPartRing) <= kWtBarBytes, "barriers");
-constexpr int kWtOneStages = 56;              // K stages from which ranges of 65 to 128 tokens have one accumulator
 constexpr int kWtExFloats = 2 * 32 * 20;      // MODE 1: gate / up exchange of two epilogue warps
 constexpr int kWtExBytes = 2 * 2 * kWtExFloats * 4;
 constexpr int kWtSmemLimit = 232448 - 1024;   // dynamic shared memory less the static part
@@ -1139,15 +1136,29 @@ WtShare wt_share(int pairs, int tiles, int KT, int nt) {
   return s;
 }
 
+// Ranges of `chunk` units, tiles of KT units and 65 to 128 tokens: whether one accumulator and six A slots are faster than
+// two and four.  The epilogue that nothing hides is paid for once a tile of KT units, unless the range is shorter than a
+// tile and ends one at most.  At 128 tokens the MMAs take as long as the conversion, and a unit gains less, but in groups
+// of 64, whose conversion is longer.  Two -> one, us: 29568 x 8192 M 100 54.8 -> 53.7, groups of 64 56.4 -> 55.0; 14336 x
+// 28672 M 100 87.3 -> 85.6; 7168 x 22016 M 100 36.2 -> 36.0, M 128 42.3 -> 43.1; 8192 x 28672 M 128 58.3 -> 59.2, groups
+// of 64 62.3 -> 61.8; 11008 x 57344 M 128 98.3 -> 98.0, x 28672 no difference; 14336 x 28672 M 128 105.1 -> 104.3; 8192
+// x 12288 M 112 34.9 -> 33.9 and 10240 x 11008 M 128 34.5 -> 33.8 (less than a tile a range); 4096 x 22016 M 100 22.7 ->
+// 22.9.
+constexpr int kWtOneStages = 56, kWtOneStagesFull = 80;
+bool wt_one_accumulator(int nt, int chunk, int KT, int group) {
+  if (chunk == 0 || KT < kWtOneStages) return false;
+  return nt < 128 || group == 64 || chunk < KT || KT >= kWtOneStagesFull;
+}
+
 // Ring depths for a tile of `nt` tokens; the rest of shared memory goes to the packed words, which
-// come from HBM (8 KB a stage).
-int wt_rings(WtParams* p, int mode) {
+// come from HBM (8 KB a stage).  `group`: of a dense call.
+int wt_rings(WtParams* p, int mode, int group) {
   const int rows = (p->nt / 2 + 15) / 16 * 16;
   p->xstage = rows * 256;
   p->nx = p->xstage <= (16 << 10) ? 8 : 4;
   // Two accumulators, so that the next tile's MMAs run under the epilogue, while they fit beside six A slots, or beside four
   // where a CTA has many tiles; what TMEM is left over goes to A slots.
-  const bool one = p->nt > 128 || (p->nt > 64 && (p->share.tiles == 1 || (p->chunk > 0 && p->KT >= kWtOneStages)));
+  const bool one = p->nt > 128 || (p->nt > 64 && (p->share.tiles == 1 || wt_one_accumulator(p->nt, p->chunk, p->KT, group)));
   p->nbuf = one ? 1 : 2;
   // One accumulator and whole tiles: the WIDE kernel.
   p->stage_bytes = p->nbuf == 2 || p->chunk > 0 || p->share.pairs > 0 ? 0 : (p->nt + 31) / 32 * 32 * kWtCols * (mode == 1 ? 1 : 2);
@@ -1323,7 +1334,7 @@ WtPlan wt_cluster_search(WtPlan best, int M, int slabs, int KT, Resident residen
       WtParams p = {};
       p.nt = nt;
       p.share = wt_share(pairs, per, KT, nt);
-      const int smem = wt_rings(&p, 0);
+      const int smem = wt_rings(&p, 0, kWtBK);
       if (p.nraw >= kWtTeams && smem <= kWtSmemLimit) best = {nt, 0, clusters * pairs, pairs, per, cost};
     }
   }
@@ -1381,7 +1392,7 @@ int launch_wt_dense(const __half* x, const uint32_t* qweight, WtParams p, void* 
   p.chunk = plan.chunk;
   p.mtiles = (p.M + p.nt - 1) / p.nt;
   if (plan.share > 0) p.share = wt_share(plan.share, plan.share_tiles, p.KT, p.nt);
-  const int smem = wt_rings(&p, 0);
+  const int smem = wt_rings(&p, 0, GROUP);
   CUtensorMap map_w;
   WtXMaps<0> map_x;
   if (int rc = make_wt_map(&map_w, qweight, p.K, p.N, 16)) return rc;
@@ -1419,7 +1430,7 @@ int gemm_wt_cut(int M, int N, int K, int group, int cta_pairs, int* tokens, int*
   p.nt = plan.nt;
   p.chunk = plan.chunk;
   p.KT = K / kWtBK;
-  wt_rings(&p, 0);
+  wt_rings(&p, 0, group);
   *tokens = plan.nt;
   *chunk = plan.chunk;
   *wide = p.stage_bytes > 0 ? 1 : 0;
@@ -1444,7 +1455,7 @@ int gemm_wt_cut(int M, int N, int K, int group, bool clusters, const int* room, 
   p.chunk = plan.chunk;
   p.KT = KT;
   if (plan.share > 0) p.share = wt_share(plan.share, plan.share_tiles, KT, plan.nt);
-  wt_rings(&p, 0);
+  wt_rings(&p, 0, group);
   *out = {plan.nt, plan.chunk, 2 * plan.share, plan.share_tiles, p.nbuf};
   return AWQ_B200_OK;
 }
@@ -1473,7 +1484,7 @@ int launch_wt_moe(const __half* a, int64_t a_rows, const uint32_t* w, int expert
   p.KT = p.K / kWtBK;
   p.slabs = MODE == 1 ? p.half_cols / 128 : p.N / kWtBN;
   p.nt = tile_rows;
-  const int smem = wt_rings(&p, MODE);
+  const int smem = wt_rings(&p, MODE, GROUP);
   CUtensorMap map_w;
   WtXMaps<MODE> map_x;
   if (int rc = make_wt_map(&map_w, w, (int64_t)experts * p.K, p.N, MODE == 1 ? 8 : 16)) return rc;

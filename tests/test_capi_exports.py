@@ -277,6 +277,9 @@ def test_clusters_of_every_size_and_ranges_are_tested(built_library):
         got = cut(*call, room=B200)
         assert (got.kernel, got[3:5]) == (wt, shared), call
         assert cut(*call, wt, B200).cluster == 0
+    for call, accumulators in test_gpu_wt.ACCUMULATORS.items():
+        got = cut(*call, wt, B200)
+        assert got.chunk > 0 and got.accumulators == accumulators, call
     assert set(test_gpu_wt.CLUSTERS.values()) == {(c, 1) for c in (4, 6, 8, 10, 12, 16)} | {(6, 2)}
 
 

@@ -234,10 +234,16 @@ def test_wt_clusters_share_tiles(A, m, k, n, group, bias):
         assert (y.cpu()[:, c:].double() - ref).norm() < 1.05 * rounding
 
 
-# Ranges of 65 to 128 tokens on either side of the K from which they have one accumulator and six A slots: a tile shared by
-# pairs, three tiles in a range, tiles of 80 and 128 tokens, a slab past N.
-@pytest.mark.parametrize("m,k,n,group", [
-    (100, 7168, 8224, 64), (100, 7040, 8224, 128), (72, 7168, 20512, 128), (128, 7296, 1568, 128),
-])
+# Ranges of 65 to 128 tokens on either side of the K from which they have one accumulator and six A slots, which is larger
+# for 128 tokens in groups of 128 and ranges of more than a tile: a tile shared by pairs, three tiles in a range, tiles of
+# 48, 80, 112 and 128 tokens, a slab past N.
+ACCUMULATORS = {(100, 7168, 8224, 64): 1, (100, 7040, 8224, 128): 2, (72, 7168, 20512, 128): 1, (128, 7296, 1568, 128): 2,
+                (128, 8192, 10784, 128): 1, (128, 7168, 20512, 128): 2, (128, 11264, 20512, 128): 1,
+                (128, 7168, 20512, 64): 1}
+
+
+@pytest.mark.parametrize("m,k,n,group", list(ACCUMULATORS))
 def test_wt_ranges_with_one_or_two_accumulators(A, m, k, n, group):
+    got = cuts.cut(m, k, n, group, A.KERNEL_WT)
+    assert got.chunk > 0 and got.accumulators == ACCUMULATORS[m, k, n, group]
     test_wt_work_split_edges(A, m, k, n, group)
