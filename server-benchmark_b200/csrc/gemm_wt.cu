@@ -117,7 +117,7 @@ constexpr int kWtSmemLimit = 232448 - 1024;   // dynamic shared memory less the 
 constexpr int kWtMaxPairs = 128;
 
 // SPLIT: the tiles of a cluster and how its pairs share them.  A pair has at most two tiles, neighbours.
-constexpr int kWtMaxShare = 8, kWtMaxTiles = 4;
+constexpr int kWtMaxShare = 8, kWtMaxTiles = 2;
 struct WtShare {
   int pairs, tiles;                      // of a cluster; pairs 0: no SPLIT
   int recv;                              // bytes of partial sums that a CTA takes in for a tile
@@ -756,7 +756,6 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     pdl_launch_dependents();
   }
   const Work work = wt_work<MODE, WIDE, SPLIT>(p);
-  const int words = p.N / kPack;
 
   // Packed words, unit by unit: 128 rows x 16 words (MODE 1: 8 gate words and the matching 8 up
   // words).  State of the raw producer's warp.

@@ -320,13 +320,7 @@ __device__ __forceinline__ void tmem_ld_16x256b_x4(uint32_t taddr, float (&r)[16
 #pragma unroll
   for (int i = 0; i < 16; ++i) r[i] = __uint_as_float(v[i]);
 }
-// The same of 8 and 16 columns.
-__device__ __forceinline__ void tmem_ld_16x256b_x1(uint32_t taddr, float (&r)[4]) {
-  asm volatile("tcgen05.ld.sync.aligned.16x256b.x1.b32 {%0, %1, %2, %3}, [%4];"
-               : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3])
-               : "r"(taddr)
-               : "memory");
-}
+// The same of 16 columns.
 __device__ __forceinline__ void tmem_ld_16x256b_x2(uint32_t taddr, float (&r)[8]) {
   asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7])
@@ -468,10 +462,6 @@ __device__ __forceinline__ void cluster_arrive_relaxed() {
   asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_barrier() {
-  cluster_arrive();
-  cluster_wait();
-}
 // Bounded wait for what other CTAs of the cluster stored into this one (st.async).
 __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, volatile int* abort_flag, int code) {
   for (uint32_t i = 0; i < kSpinLimit; ++i) {

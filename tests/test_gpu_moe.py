@@ -689,7 +689,6 @@ def test_partial_tiles_of_experts_with_any_scratch_and_replays(A):
     torch.cuda.synchronize()
 
 
-@pytest.mark.gpu
 @pytest.mark.parametrize("t,k,e,h,i", [(300, 2, 8, 512, 256), (160, 2, 4, 2048, 128)])
 def test_prefill_calls_back_to_back_read_their_own_routing(A, t, k, e, h, i):
     """The down GEMM reads the tile table ahead of its wait for gate_up: calls with other routing right behind one
