@@ -1070,14 +1070,13 @@ gemm_wt_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   }
   tc_fence_before();
   __syncthreads();
-  const bool gave_up = s_abort != 0;
   // Nothing of another CTA is on its way to this one any more: whatever one sent another has been waited for there, but
   // after a wait that gave up.  So the barrier orders no memory: a release waits for this CTA's stores of the output, 1000
   // cycles.  1024 x 8192 at M 40 5.00 -> 4.85 us, 3712 x 8192 at M 200 15.0 -> 14.4, 2048 x 5120 at M 300 10.9 -> 10.3.
   cluster_arrive_relaxed();
   cluster_wait();
   if (warp == kWtIssueWarp) {
-    if (gave_up) linger();  // what was sent until the barrier lands
+    if (s_abort) linger();  // what was sent until the barrier lands
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem),
                  "r"((uint32_t)kWtTmemCols)
