@@ -1310,12 +1310,16 @@ long wt_cluster_cost(int nt, int pairs, int tiles, int clusters, int KT, int res
   if (tiles > 1) t += 18 * nt - 600;
   return t;
 }
-// The cheapest cut into clusters, if it is cheaper than `best` by more than the estimates are apart (400 ns: with it
-// the choice is 0.6 % from the best of all cuts on average; without 0.9 %, 24 % at worst).
+// The cheapest cut into clusters, if it is cheaper than the ranges by more than the estimates are apart: wt_cost was fitted
+// to a kernel whose start took longer.  Of 1300 calls of 33 to 700 tokens that went to clusters with a margin of 400 ns, 135
+// were slower there than in ranges by more than 1 %, most of them with K up to 1024 (896 x 3232 at M 109 4.3 -> 5.3 us);
+// now 14, 5 % at most, and 0.1 % from the better of the two on average, which was 0.8 %.
+constexpr long kWtMargin = 1300, kWtMarginTwo = 200;  // two tiles for three pairs: more
 constexpr int kWtShares[][2] = {{2, 1}, {3, 1}, {4, 1}, {5, 1}, {6, 1}, {8, 1}, {3, 2}};  // pairs, tiles of a cluster
 template <typename Resident>
 WtPlan wt_cluster_search(WtPlan best, int M, int slabs, int KT, Resident resident) {
-  if (best.cost >= 0) best.cost -= 400;
+  const WtPlan ranges = best;
+  best.cost = -1;
   int room[kMaxCluster + 1] = {};
   for (const auto& s : kWtShares) room[s[0]] = resident(s[0]);
   for (int top = 256, last = 0; top >= 32; top -= 16) {
@@ -1336,7 +1340,9 @@ WtPlan wt_cluster_search(WtPlan best, int M, int slabs, int KT, Resident residen
       if (p.nraw >= kWtTeams && smem <= kWtSmemLimit) best = {nt, 0, clusters * pairs, pairs, per, cost};
     }
   }
-  return best;
+  if (best.cost < 0) return ranges;
+  const long margin = kWtMargin + (best.share_tiles > 1 ? kWtMarginTwo : 0);
+  return best.cost + margin < ranges.cost ? best : ranges;
 }
 
 template <typename Resident>

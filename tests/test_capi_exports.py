@@ -280,7 +280,7 @@ def test_clusters_of_every_size_and_ranges_are_tested(built_library):
     for call, accumulators in test_gpu_wt.ACCUMULATORS.items():
         got = cut(*call, wt, B200)
         assert got.chunk > 0 and got.accumulators == accumulators, call
-    assert set(test_gpu_wt.CLUSTERS.values()) == {(c, 1) for c in (4, 6, 8, 10, 12, 16)} | {(6, 2)}
+    assert set(test_gpu_wt.CLUSTERS.values()) == {(c, 1) for c in (4, 6, 8, 10, 12, 16)} | {(6, 2), (0, 0)}
 
 
 def test_calls_whose_clusters_do_not_fit_take_ranges(built_library):
