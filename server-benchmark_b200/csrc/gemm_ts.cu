@@ -1226,19 +1226,29 @@ TsCut ts_cut(int slabs, int KT, const int* room = nullptr, int most = kMaxCluste
     if (split > KT || split > most) break;
     const int resident = room != nullptr ? room[split] : ts_resident<MT, GROUP, MODE>(split);
     if (slabs > resident) continue;
-    const long cost = ts_split_cost(slabs, KT, MT, GROUP, split, resident);
+    long cost = ts_split_cost(slabs, KT, MT, GROUP, split, resident);
+    // Every cluster taken: odd sizes leave SMs of a GPC idle until the last one is done, and with few tokens 112 CTAs load
+    // the words more slowly than 148.
+    if (MODE == 0 && slabs == resident) cost += split % 2 != 0 ? 1000 : (split == 16 && MT <= 4 ? 700 : 0);
     if (best.cost >= 0 && cost >= best.cost) continue;
     best = {split, 0, cost};
     hidden = 2 * slabs <= resident;
   }
-  // The two estimates were fitted apart.  What brings them together up to 16 tokens was fitted to 95 shapes from 1024 to 29440
-  // rows at 1, 4, 8 and 16 tokens, ranges and every cluster timed: none of the 380 calls is slower in clusters than it is in
-  // ranges, 1.0 % from the best of all on average.  With the bare estimates 34 were (3712 x 8192 at M 1 6.8 -> 7.4 us, 1280 x
-  // 14752 5.3 -> 6.0, 4864 x 11456 groups of 64 a quarter slower at M 8), 1.1 %.
+  // The two estimates were fitted apart.  What brings them together up to 16 tokens was fitted to 95 shapes at 1, 4, 8 and 16
+  // tokens, ranges and every cluster timed, and then, with the terms for all clusters taken, whole slabs and short K, to 2500
+  // calls of 256 to 32768 rows that went to clusters, timed in ranges too: 113 of them were slower in clusters by more than
+  // 1 % (15488 x 1696 at M 2 6.9 -> 7.5 us, 4864 x 11360 at M 15 11.2 -> 12.4, 384 x 576 at M 10 2.8 -> 3.0); now 32, 5 % at
+  // most, and 5 gain more than 3 % less than they could.  In clusters instead of ranges a call takes 0.71 of the time on
+  // average.  From 17 tokens whole slabs take less time than estimated: of 1000 calls that went to clusters 125 were slower
+  // there (1152 x 9088 at M 32 5.8 -> 7.3 us, 256 x 5120 at M 24 2.9 -> 3.7), now 16.
   long margin = 0;
-  if (MODE == 0 && MT <= 16) {
+  if (MODE == 0 && MT > 16) {
+    if (ranges.chunk == 0) margin = GROUP == 128 || KT <= 3 ? 1600 : 1000;
+  } else if (MODE == 0) {
     const int run = ranges.chunk > 0 ? ranges.chunk : KT;
     margin = 600 + 25 * MT + (GROUP == 128 ? 0 : 200) - 45 * (run < 30 ? run : 30) + (hidden ? 0 : 300);
+    if (ranges.chunk == 0) margin += 60;
+    if (!hidden && GROUP == 128 && KT <= 32) margin += 100;
   }
   return best.cost >= 0 && best.cost + margin < ranges.cost ? best : ranges;
 }

@@ -258,7 +258,7 @@ CLUSTERS = {
     (25, 12288, 6176, 128): (5, 0), (24, 8192, 5120, 64): (6, 0), (12, 2048, 1024, 64): (8, 0),
     (16, 8192, 1280, 128): (16, 0), (31, 8192, 1280, 128): (16, 0), (4, 16384, 992, 64): (16, 0),
     (5, 256, 256, 128): (0, 0), (20, 128, 32, 128): (0, 0), (23, 8192, 38176, 128): (0, 65),
-    (18, 4096, 28704, 64): (0, 0), (20, 256, 2080, 128): (2, 0), (2, 512, 1056, 128): (4, 0),
+    (18, 4096, 28704, 64): (0, 0), (20, 256, 2080, 128): (0, 0), (20, 512, 1056, 128): (4, 0), (2, 512, 1056, 128): (4, 0),
     (7, 768, 544, 128): (6, 0), (27, 4096, 20512, 64): (0, 18), (32, 2048, 38144, 128): (0, 17)}
 
 
