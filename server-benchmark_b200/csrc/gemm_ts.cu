@@ -101,6 +101,8 @@
 // replayed graph, cool): T 1: 22.9 -> 16.2 us, T 16: 71.0 -> 53.8, T 64: 101.9 -> 72.2, T 128: 110.7 -> 92.1.  At T = 64 all
 // 302 MB of int4 words are read, 48 us at the HBM rate; a block of 8 rows costs the conversion of a
 // whole matrix, which is what bounds it.
+#include <cmath>
+
 #include "common.cuh"
 #include "handover.cuh"
 #include "tc_ptx.cuh"
@@ -136,8 +138,6 @@ struct TsCfg {
   // Scales and zero points by plain bulk copies (TsRow).  Groups of 64 need twice as many: up to 16 tokens 4096 x 11040 at
   // M 16 took 10.4 -> 10.7 us with them, at M 24 12.4 -> 11.5.
   static constexpr bool BULK = SPLIT && MODE == 0 && (GROUP == 128 || MT > 16);
-  // Partial tiles handed over with a token beside every two sums, without flags
-  static constexpr bool MARKS = MODE != 0 && MT <= 8;
   static constexpr int kIssueWarps = SUB ? 2 : 1;
   static constexpr int kSum = kIssue + kIssueWarps, kXWarp = kSum + (SUB ? 0 : 1), kRaw = kXWarp + 1;
   static constexpr int kThreads = 32 * (kRaw + 1);     // 768
@@ -326,7 +326,8 @@ struct TsWalk {
   __device__ __forceinline__ int column() const { return slab * kTsBN + (up() ? p.half_cols : 0); }
 };
 
-template <int MT, int MODE, int GROUP, bool SPLIT>
+// MARKS: partial tiles are handed over with a token beside every two sums, without flags (ts_marks).
+template <int MT, int MODE, int GROUP, bool SPLIT, bool MARKS = false>
 __global__ void __launch_bounds__((TsCfg<MT, MODE, GROUP, SPLIT>::kThreads), 1)
 // map_s, map_z: not read where BULK
 gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_s,
@@ -870,14 +871,10 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       constexpr int kTile = MT * kTsBN, kTiles = MODE == 1 ? 2 : 1;
       float* part = p.partial + (size_t)blockIdx.x * (kTiles * kTile) + chunk_col + lane;
       // MARKS: [MT / 2][256] pairs of sums with the launch's token beside each.  Whoever adds them reads until it sees the
-      // token.  A release took a fold warp 2000 to 5000 cycles under the words' stream, also long after its stores, and the
-      // next tile's folds waited for it: experts of 128 x 2048 x 768, top-8, 16 tokens 54.2 -> 51.4 us, 64 tokens 72.2 -> 70.0,
-      // 128 tokens 95 -> 90.  Reading costs more (16-byte strong loads, 2500 cycles for eight), so dense layers, where
-      // more CTAs share a slab, and blocks of 16 rows keep the flags: 29568 x 8192 at M 16 28 -> 37 us with marks, 8192 x
-      // 59136 at M 1 41.4 -> 43.3, 500 tokens 171 -> 175.
+      // token.
       constexpr int P = MT / 2, kMarked = P * kTsBN;
       uint4* marked = reinterpret_cast<uint4*>(p.partial) + (size_t)blockIdx.x * (kTiles * kMarked) + chunk_col + lane;
-      if (Cfg::MARKS && ke < work.KT) {
+      if (MARKS && ke < work.KT) {
         uint4* dst = marked + (MODE == 1 && ke > p.KT ? kMarked : 0);
         const unsigned long long mark = ok && !s_abort ? token : 0ull;
 #pragma unroll
@@ -889,7 +886,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         }
         continue;
       }
-      if (!Cfg::MARKS && ke < work.KT) {  // another CTA holds the tile's last unit
+      if (!MARKS && ke < work.KT) {  // another CTA holds the tile's last unit
         float* dst = part + (MODE == 1 && ke > p.KT ? kTile : 0);
 #pragma unroll
         for (int m = 0; m < MT; ++m)
@@ -905,7 +902,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
       int gather = 0;  // CTAs before this one that share the tile
       if (kb > 0) {
         gather = blockIdx.x - id * work.KT / work.chunk;
-        for (int c = 1 + lane; !Cfg::MARKS && c <= gather; c += 32) {
+        for (int c = 1 + lane; !MARKS && c <= gather; c += 32) {
           unsigned long long* theirs = flag - c * handover::kMaxWarps;
           uint32_t polls = 0;
           while (handover::read_flag(theirs) != token) {
@@ -984,7 +981,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         while (up_first > 0 && ((int)blockIdx.x - up_first + 1) * work.chunk <= split) --up_first;
         while (gate_last <= gather && ((int)blockIdx.x - gate_last) * work.chunk >= split) ++gate_last;
       }
-      if constexpr (Cfg::MARKS) add_marked(v, marked + (MODE == 1 ? kMarked : 0), up_first, 1);
+      if constexpr (MARKS) add_marked(v, marked + (MODE == 1 ? kMarked : 0), up_first, 1);
       else add_parts(v, part + (MODE == 1 ? kTile : 0), up_first, 1);
 #pragma unroll
       for (int m = 0; m < MT; ++m) v[m] *= unscale;
@@ -1000,7 +997,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         float gt[MT];
 #pragma unroll
         for (int m = 0; m < MT; ++m) gt[m] = kb < p.KT ? gate[m * 32] : 0.f;
-        if constexpr (Cfg::MARKS) add_marked(gt, marked, gather, gate_last);
+        if constexpr (MARKS) add_marked(gt, marked, gather, gate_last);
         else add_parts(gt, part, gather, gate_last);
 #pragma unroll
         for (int m = 0; m < MT; ++m) {
@@ -1275,13 +1272,13 @@ int launch_ts_split(const TsMaps& maps, const TsParams& p, int clusters, cudaStr
   return AWQ_B200_OK;
 }
 
-template <int MT, int MODE, int GROUP = 128>
+template <int MT, int MODE, int GROUP = 128, bool MARKS = false>
 int launch_ts(const TsMaps& maps, const TsParams& p, int ctas, cudaStream_t stream) {
   static std::atomic<bool> attr_done[64];  // zero-initialised; setting the attribute twice is harmless
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return AWQ_B200_ERR_DEVICE;
-  auto kernel = gemm_ts_kernel<MT, MODE, GROUP, false>;
+  auto kernel = gemm_ts_kernel<MT, MODE, GROUP, false, MARKS>;
   constexpr int smem = TsCfg<MT, MODE, GROUP>::kSmem;
   if (!attr_done[dev]) {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
@@ -1353,6 +1350,38 @@ int launch_ts_dense(const __half* x, const uint32_t* qweight, const __half* scal
   return launch_ts<MT, 0, GROUP>(maps, p, ctas, stream);
 }
 
+// Expert GEMMs, blocks of up to 8 rows: whether partial tiles carry a token beside every two sums instead of a flag each.  A
+// release takes a fold warp 2000 to 5000 cycles under the words' stream, also long after its stores, and the next tile's
+// folds wait for it; but reading takes longer (16-byte strong loads, 2500 cycles for eight), and for every CTA that shares
+// the tile.  So flags where many share it: in gate_up, which has twice the sums, more than about two, in down more than
+// three, and in both more than six with one row.  `tiles` are expected ones.  Without the router, flags -> tokens, us: 128
+// experts of 2048 x 768, top-8, 4 tokens 27.5 -> 25.6, 16 55.8 -> 53.6, 64 75.0 -> 73.4 (runs differ by 1.5); 16 of 2048 x
+// 256, top-6, 2 tokens 19.9 -> 24.1 (gate_up 16 CTAs a tile; down alone 19.9); 16 of 896 x 128, top-2, 15 tokens 16.0 ->
+// 17.2 (down alone 15.5).  Dense layers, where many CTAs share a slab, and blocks of 16 rows have flags: 29568 x 8192 at M
+// 16 28 us, with tokens 37, 8192 x 59136 at M 1 41.4 and 43.3, 500 tokens 171 and 175.
+template <int MT, int MODE>
+bool ts_marks(double tiles, int KT, int max_split, int ctas) {
+  const double even = tiles * KT / ctas, least = (double)KT / max_split, chunk = even > least ? even : least;
+  return KT <= (MT == 4 ? 6.0 : MODE == 1 ? 1.25 : 3.0) * (chunk > 1.0 ? chunk : 1.0);
+}
+// Row blocks to expect: one for every expert that any pair has, and more if they do not hold the rows.
+double ts_expected_blocks(const MoeArgs& a) {
+  const double numel = (double)a.T * a.topk;
+  if (a.direct) return numel;  // a block for a pair
+  // a permutation's capacity tells over how many experts the pairs are spread, of which E are here
+  const double all = a.expert_parallel ? (a.sorted_capacity - numel) / (a.block - 1) : 0.0;
+  const double experts = all > a.E ? all : a.E, here = a.E / experts;
+  const double hit = a.E * (1.0 - std::pow(1.0 - 1.0 / experts, numel)), full = numel * here / a.block;
+  return hit > full ? hit : full;
+}
+template <int MT, int MODE>
+int launch_ts_grouped(const TsMaps& maps, const TsParams& p, double blocks, int ctas, cudaStream_t stream) {
+  if constexpr (MT <= 8)
+    if (ts_marks<MT, MODE>(blocks * p.slabs, MODE == 1 ? 2 * p.KT : p.KT, p.max_split, ctas))
+      return launch_ts<MT, MODE, 128, true>(maps, p, ctas, stream);
+  return launch_ts<MT, MODE>(maps, p, ctas, stream);
+}
+
 // Expert GEMMs: gate_up, then down.
 // *summed: whether the sum over a token's slots is done as well (MODE 2, SPLIT).
 template <int MT>
@@ -1360,7 +1389,7 @@ int launch_ts_experts(const MoeArgs& a, __half* act, int64_t act_rows, __half* p
                       cudaStream_t stream) {
   const int ctas = ts_ctas();
   *summed = false;
-  p.flags = handover::make_flags(p.partial, 2 * ts_partial_bytes(MT));  // flags: blocks of 16 rows
+  p.flags = handover::make_flags(p.partial, 2 * ts_partial_bytes(MT));
   p.sorted_ids = a.sorted_ids;
   p.expert_ids = a.expert_ids;
   p.num_post = a.num_post_pad;
@@ -1369,6 +1398,7 @@ int launch_ts_experts(const MoeArgs& a, __half* act, int64_t act_rows, __half* p
   p.topk = a.topk;
   p.half_cols = a.I;
   p.max_split = 16;
+  const double blocks = ts_expected_blocks(a);
   const uint64_t I = (uint64_t)a.I;
   {
     p.K = a.H;
@@ -1395,7 +1425,7 @@ int launch_ts_experts(const MoeArgs& a, __half* act, int64_t act_rows, __half* p
         if (int rc2 = launch_ts_split<MT, 128, 1>(maps, p, p.numel * p.slabs, stream)) return rc2;
     }
     if (!split)
-      if (int rc2 = launch_ts<MT, 1>(maps, p, ctas, stream)) return rc2;
+      if (int rc2 = launch_ts_grouped<MT, 1>(maps, p, blocks, ctas, stream)) return rc2;
   }
   p.K = a.I;
   p.N = a.H;
@@ -1420,7 +1450,7 @@ int launch_ts_experts(const MoeArgs& a, __half* act, int64_t act_rows, __half* p
       }
     }
   }
-  return launch_ts<MT, 2>(maps, p, ctas, stream);
+  return launch_ts_grouped<MT, 2>(maps, p, blocks, ctas, stream);
 }
 
 int ts_tokens(int M) { return M <= 4 ? 4 : (M <= 8 ? 8 : (M <= 16 ? 16 : 32)); }
@@ -1484,9 +1514,10 @@ bool moe_ts_supported(const MoeArgs& a) {
 
 // Partial tiles of gate and up, rows of the largest block, and the flags.
 size_t moe_ts_partial_bytes(int block) {
-  // blocks of 8 rows and the direct form: a token beside every two sums
-  if (block <= 8) return (size_t)2 * ts_ctas() * block * kTsBN * 8;
-  return 2 * ts_partial_bytes(block) + handover::kFlagBytes;
+  const size_t flagged = 2 * ts_partial_bytes(block) + handover::kFlagBytes;
+  // blocks of 8 rows and the direct form may have a token beside every two sums
+  const size_t marked = block <= 8 ? (size_t)2 * ts_ctas() * block * kTsBN * 8 : 0;
+  return marked > flagged ? marked : flagged;
 }
 
 // Both expert GEMMs of a small batch, pair_out by pair.  Rows of act by position, direct (no
