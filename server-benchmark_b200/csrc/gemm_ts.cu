@@ -1247,6 +1247,9 @@ TsCut ts_cut(int slabs, int KT, const int* room = nullptr, int most = kMaxCluste
     if (ranges.chunk == 0) margin += 60;
     if (!hidden && GROUP == 128 && KT <= 32) margin += 100;
   }
+  // gate_up of one or two tokens: of 85 calls on clusters 19 were slower there than in ranges by more than 1 %, most with
+  // eight units a CTA or more (128 experts of 3712 x 256, top-4, 3 tokens 15.9 -> 17.7 us with the down GEMM).
+  if (MODE == 1 && best.split > 0 && KT >= 8 * best.split) margin = 800;
   return best.cost >= 0 && best.cost + margin < ranges.cost ? best : ranges;
 }
 
