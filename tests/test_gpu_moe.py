@@ -323,7 +323,7 @@ def test_small_batch_experts_edges(A, t, k, e, h, i, parallel):
 
 
 # One or two tokens: gate_up on clusters (units of gate and up that do not divide by them, an edge of the columns inside
-# a slab, one unit in all), down on clusters of a token's slots; every number of slots; a third of the experts absent.
+# a slab, one unit in all) or in ranges, down on clusters of a token's slots; every number of slots; a third of the experts absent.
 @pytest.mark.parametrize("t,k,h,i", [(1, 2, 256, 128), (1, 3, 1152, 384), (1, 4, 4096, 1536), (1, 5, 640, 640),
                                      (1, 6, 2048, 768), (1, 7, 896, 896), (1, 8, 2048, 1024), (2, 4, 2048, 768),
                                      (2, 3, 512, 128), (1, 1, 2048, 768), (1, 2, 2048, 256), (2, 1, 256, 128)])
@@ -534,27 +534,19 @@ def test_expert_parallel_batch_takes_the_kernels_of_its_rows_per_expert(A):
     assert not any("gemm_wt_kernel" in n for n in names), names
 
 
-# Up to three tiles, for which clusters of more than eight CTAs would be estimated best, and more.
-@pytest.mark.parametrize("k,h,i", [(1, 2048, 768), (2, 2048, 256), (1, 1024, 384), (8, 2048, 768)])
-def test_one_token_runs_gate_up_on_clusters(A, k, h, i):
-    import re
-    from torch.profiler import ProfilerActivity, profile
+# Up to three tiles, for which clusters of more than eight CTAs would be estimated best, and more; ranges with many units.
+@pytest.mark.parametrize("k,h,i,clusters", [(1, 2048, 768, 1), (2, 2048, 256, 1), (1, 1024, 384, 1), (8, 640, 640, 1),
+                                            (8, 2048, 768, 0)])
+def test_one_token_runs_gate_up_on_clusters(A, k, h, i, clusters):
     w1, w2, x, logits = _moe_case(16, h, i, 1, k, seed=3)
     w1d, w2d, xd = tuple(a.cuda() for a in w1), tuple(a.cuda() for a in w2), x.cuda()
     w, ids, _ = A.fused_topk(xd, logits.cuda(), k, True)
     A.fused_experts(xd, w1d, w2d, w, ids)
     torch.cuda.synchronize()
-    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as prof:
-        A.fused_experts(xd, w1d, w2d, w, ids)
-        torch.cuda.synchronize()
-    names = [event.key for event in prof.key_averages() if "awq::" in event.key]
-    if not names:
+    forms = _ts_forms(lambda: A.fused_experts(xd, w1d, w2d, w, ids))
+    if not forms:
         pytest.skip("the profiler sees no kernels here")
-    # tokens, mode, group, clusters
-    forms = [re.sub(r"\(\w+\)", "", m.group(1)).replace(" ", "").split(",") for m in
-             (re.search(r"gemm_ts_kernel<([^>]*)>", n) for n in names) if m]
-    assert ["4", "1", "128"] in [f[:3] for f in forms], names
-    assert all(f[3] in ("true", "1") for f in forms if f[1] == "1"), names
+    assert [f[3] for f in forms if f[:3] == (4, 1, 128)] == [clusters], forms
 
 
 def test_fused_moe_full_size_rows_are_independent(A):
@@ -648,9 +640,50 @@ def test_batches_in_turn_do_not_see_each_other(A, e, h, i, t, k):
         assert torch.equal(A.fused_experts(xd, w1d, w2d, weights, ids), first)
 
 
+def _ts_forms(call):
+    """(rows, mode, group, clusters, tokens beside the sums) of every gemm_ts kernel that a call launches, or nothing
+    where the profiler sees no kernels."""
+    import re
+    from torch.profiler import ProfilerActivity, profile
+    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as prof:
+        call()
+        torch.cuda.synchronize()
+    found = [re.search(r"gemm_ts_kernel<([^>]*)>", event.key) for event in prof.key_averages()]
+    args = [re.sub(r"\(\w+\)", "", m.group(1)).replace(" ", "").split(",") for m in found if m]
+    return [tuple(int(v) if v.isdigit() else int(v == "true") for v in a) for a in args]
+
+
+# Blocks of 8 rows, then without a permutation: flags in both GEMMs, in gate_up alone, in none; flags and tokens in down.
+@pytest.mark.parametrize("t,k,e,h,i,gate,down", [
+    (5, 2, 8, 384, 640, 0, 0), (2, 6, 16, 2048, 256, 0, 1), (64, 4, 32, 512, 1024, 1, 1), (3, 1, 16, 512, 1152, None, 0),
+    (9, 1, 32, 1024, 256, None, 1)])
+def test_partial_tiles_of_experts_with_flags_and_with_tokens(A, t, k, e, h, i, gate, down):
+    w1, w2, x, logits = _moe_case(e, h, i, t, k, seed=t)
+    w1d, w2d, xd = tuple(a.cuda() for a in w1), tuple(a.cuda() for a in w2), x.cuda()
+    w, ids, _ = A.fused_topk(xd, logits.cuda(), k, True)
+    want = A.fused_experts(xd, w1d, w2d, w, ids)
+    forms = {f[1]: f for f in _ts_forms(lambda: A.fused_experts(xd, w1d, w2d, w, ids))}
+    if forms:
+        assert gate is None or forms[1][3:] == (0, gate)  # None: on clusters or not
+        assert forms[2][3:] == (0, down)
+    ref = O.fused_experts_fp32(x.numpy(), *[a.numpy() for a in w1], *[a.numpy() for a in w2], w.cpu().numpy(),
+                               ids.cpu().numpy())
+    assert O.rel_err(want.cpu().numpy(), ref) < TOL
+    graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        out = [A.fused_experts(xd, w1d, w2d, w, ids) for _ in range(3)]
+    for _ in range(20):
+        for y in out:
+            y.fill_(float("nan"))
+        graph.replay()
+        assert all(torch.equal(y, want) for y in out)
+    torch.cuda.synchronize()
+
+
 def test_partial_tiles_of_experts_with_any_scratch_and_replays(A):
-    """Sums with a token beside them: scratch full of other data, one buffer again and again, and replays of one graph
-    whose token is the same every time."""
+    """Flags in gate_up, a token beside the sums in down: scratch full of other data, one buffer again and again, and
+    replays of one graph whose tokens are the same every time."""
     from awq_b200 import _lib, ops
     t, k, e, h, i = 24, 4, 16, 2048, 768
     w1, w2, x, logits = _moe_case(e, h, i, t, k, seed=5)
