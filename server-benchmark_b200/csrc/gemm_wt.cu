@@ -1311,13 +1311,18 @@ long wt_cluster_cost(int nt, int pairs, int tiles, int clusters, int KT, int res
   return t;
 }
 // The cheapest cut into clusters, if it is cheaper than the ranges by more than the estimates are apart: wt_cost was fitted
-// to a kernel whose start took longer.  Of 1300 calls of 33 to 700 tokens that went to clusters with a margin of 400 ns, 135
-// were slower there than in ranges by more than 1 %, most of them with K up to 1024 (896 x 3232 at M 109 4.3 -> 5.3 us);
-// now 14, 5 % at most, and 0.1 % from the better of the two on average, which was 0.8 %.
-constexpr long kWtMargin = 1300, kWtMarginTwo = 200;  // two tiles for three pairs: more
+// to a kernel whose start took longer, and says too little of whole tiles on more than half of the GPU, beside which the next
+// kernel's do not start.  Fitted to 1540 calls of 33 to 700 tokens, near the line most of them, timed as clusters and as
+// ranges; `most` pairs fit the GPU.  With a margin of 400 ns 271 were slower in clusters than in ranges by more than 1 %, most
+// of them with K up to 1024 (896 x 3232 at M 109 4.3 -> 5.3 us); now 40, 8 % at worst, and 0.2 % from the better of the two
+// on average, which was 1.3 %.
+long wt_cluster_margin(bool two_tiles, const WtPlan& ranges, int KT, int most) {
+  const bool over_half = ranges.chunk == 0 && 2 * ranges.pairs > most;
+  return 1200 + (two_tiles ? 200 : 0) - (over_half ? 30 * (KT < 30 ? KT : 30) : 0);
+}
 constexpr int kWtShares[][2] = {{2, 1}, {3, 1}, {4, 1}, {5, 1}, {6, 1}, {8, 1}, {3, 2}};  // pairs, tiles of a cluster
 template <typename Resident>
-WtPlan wt_cluster_search(WtPlan best, int M, int slabs, int KT, Resident resident) {
+WtPlan wt_cluster_search(WtPlan best, int M, int slabs, int KT, int most, Resident resident) {
   const WtPlan ranges = best;
   best.cost = -1;
   int room[kMaxCluster + 1] = {};
@@ -1341,8 +1346,7 @@ WtPlan wt_cluster_search(WtPlan best, int M, int slabs, int KT, Resident residen
     }
   }
   if (best.cost < 0) return ranges;
-  const long margin = kWtMargin + (best.share_tiles > 1 ? kWtMarginTwo : 0);
-  return best.cost + margin < ranges.cost ? best : ranges;
+  return best.cost + wt_cluster_margin(best.share_tiles > 1, ranges, KT, most) < ranges.cost ? best : ranges;
 }
 
 template <typename Resident>
@@ -1350,7 +1354,7 @@ WtPlan wt_find(int M, int slabs, int KT, int most, bool split, bool clusters, Re
   const WtPlan plan = wt_search(M, slabs, KT, most, split);
   // whole tiles that fill the GPU stay as they are
   const bool full = M > 256 && (long)slabs * ((M + 255) / 256) >= most;
-  return clusters && !full ? wt_cluster_search(plan, M, slabs, KT, resident) : plan;
+  return clusters && !full ? wt_cluster_search(plan, M, slabs, KT, most, resident) : plan;
 }
 
 int current_device() {

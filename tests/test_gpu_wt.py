@@ -197,12 +197,12 @@ def test_wt_wide_tiles(A, m, k, n, group, tokens, split):
     assert O.elementwise_ok(y[0].cpu().numpy(), ref, TOL)
 
 
-# Tiles shared by clusters: two to eight pairs a tile, two tiles for three pairs, units that do not divide by the pairs, a
-# pair with one unit, an edge of N, several tiles of tokens with a shorter last one, one accumulator (tiles above 64
+# Tiles shared by clusters: two to eight pairs a tile, two tiles for three pairs, units that do not divide by the pairs, one
+# unit a pair, an edge of N, several tiles of tokens with a shorter last one, one accumulator (tiles above 64
 # tokens, and above 128); and, (0, 0), calls near them that are faster in ranges.  CTAs and tiles of a cluster on a B200:
 # asserted on the CPU, on the GPU whether there are clusters.
 CLUSTERS = {
-    (40, 1024, 4096, 128): (4, 1), (130, 512, 2048, 64): (0, 0), (33, 384, 1056, 128): (0, 0),
+    (40, 1024, 4096, 128): (4, 1), (130, 512, 2048, 64): (0, 0), (33, 384, 1056, 128): (6, 1),
     (97, 640, 2048, 128): (0, 0), (77, 4096, 4096, 64): (4, 1), (100, 8192, 1280, 128): (10, 1),
     (300, 8192, 1312, 64): (6, 1), (150, 11008, 1536, 128): (8, 1), (60, 16384, 544, 128): (16, 1),
     (100, 8192, 10240, 128): (6, 2), (48, 4352, 10208, 64): (6, 2), (250, 8192, 5120, 128): (6, 2),
