@@ -1090,7 +1090,12 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   }
 
   // ---- teardown ----
+  // After a wait that gave up: copies, MMAs and, until the barrier below, what other CTAs of the cluster store may still be
+  // in flight towards this CTA's shared and tensor memory.  Let them land before both are given back.  In ranges every warp
+  // asks (one warp at the end: 6656 x 2464 in groups of 64 at M 1 6.2 -> 6.5 us), in clusters the last one (every warp: 2304
+  // x 3168 at M 2 3.7 -> 4.3).
   __syncwarp();
+  if (!SPLIT && s_abort) linger();
   tc_fence_before();
   if (SPLIT) {
     // a CTA may go when nobody stores into it any more
@@ -1101,10 +1106,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
   }
   __syncthreads();
   if (warp == kTsIssue) {
-    // After a wait that gave up: copies, MMAs and what other CTAs stored until the barrier above may still be in flight
-    // towards this CTA's shared and tensor memory.  Let them land before both are given back.  (Asked by every warp ahead of
-    // the barrier, 2304 x 3168 at M 2 in clusters of 5 took 3.7 -> 4.3 us.)
-    if (s_abort) linger();
+    if (SPLIT && s_abort) linger();
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
                  "r"((uint32_t)kTsTmemCols)
