@@ -86,7 +86,7 @@ int awq_b200_dequantize(const void* qweight, const void* scales, const void* qze
 #define AWQ_B200_KERNEL_STREAM 2   /* small-M weight-streaming kernel (mma.sync, cluster split-K) */
 #define AWQ_B200_KERNEL_TCGEN05 3  /* large-M tcgen05/TMEM kernel with in-smem dequantisation */
 #define AWQ_B200_KERNEL_STREAM_EXACT 4 /* small-M kernel with the magic-number conversion */
-#define AWQ_B200_KERNEL_TS 5       /* M <= 16: registers -> TMEM weights, tcgen05.mma (A in TMEM) */
+#define AWQ_B200_KERNEL_TS 5       /* by name M <= 16: registers -> TMEM weights, tcgen05.mma (A in TMEM) */
 #define AWQ_B200_KERNEL_TS_EXACT 6 /* shapes of TS: streaming kernel with the magic-number conversion */
 #define AWQ_B200_KERNEL_WT 7       /* any M: dequantised weights registers -> TMEM (A operand), x via TMA as B */
 #define AWQ_B200_KERNEL_STREAM_RP 8 /* M <= 8 streaming kernel; `qweight` is the output of awq_b200_repack_qweight */

@@ -30,8 +30,8 @@
 //   1024 x 8192                      4.6 -> 3.4 (2)        5.1 -> 3.8            4.6 -> 4.5
 //   2048 x 5120                      5.2 -> 4.1 (3)        6.6 -> 4.5            6.9 -> 5.2
 //   8192 x 1280                      6.2 -> 4.8 (16)       9.1 -> 5.3            9.9 -> 5.9
-//   8192 x 7424                     10.1 -> 10.1 (4)      12.0 -> 10.6          15.8 -> 11.4
-//   3712 x 8192                      6.9 -> 7.2 (3)        8.4 -> 7.7 (3)       11.0 -> 8.2 (4)
+//   8192 x 7424                     10.1 -> 10.1 (4)      12.0 -> 10.6          15.8 -> 11.1
+//   3712 x 8192                      6.9 -> 7.2 (3)        8.4 -> 7.8 (3)       11.0 -> 8.0 (4)
 // The last two stay in ranges at one token (ts_cut).
 // What is left of 1024 x 8192 at M 1, in cycles from the end of the kernel before: 860 the tokens' way through L2, 1400
 // the MMAs of four units (22 each), 350 the last fold, 900 the cluster's sum, 450 the exit.
@@ -60,8 +60,9 @@
 //           (negative id) gets a row of zeros.
 // SPLIT, direct form: MODE 1 as a dense layer, every CTA with the same units of gate and up.  MODE 2: the CTAs of a
 // cluster have the slots of a token, each the whole matrix, and add the rounded rows in slot order, so that no kernel for
-// the sum follows.  Experts of 128 x 2048 x 768, one token, top-8 16.2 -> 14.45 us; 64 of 2048 x 1024 17.1 -> 15.4; two
-// tokens, top-4 15.5 -> 14.4.  (With zero points subtracted in the conversion 0.1 us slower, and other roundings than
+// the sum follows.  Each where the estimates say so.  Experts without the router, ranges and a kernel for the sum -> now:
+// 128 of 2048 x 768, one token, top-8 16.8 -> 14.5 us (gate_up in ranges, on clusters 15.3); 64 of 2048 x 1024, top-4 14.8
+// -> 13.2; 64 of 2048 x 768, two tokens, top-4 16.2 -> 14.1.  (With zero points subtracted in the conversion 0.1 us slower, and other roundings than
 // through the permutation.)
 //
 // unit_full counts the conversion warps, the announcement of the tokens and the fold warps of the unit
@@ -77,8 +78,8 @@
 // Lane 32 q + 8 i + g of tile t holds column
 // 128 t + 32 q + 8 (g / 2) + 2 i + g % 2 of the slab.  Every wait is bounded (tc_ptx.cuh).
 //
-// Measured (B200, K x N, first replays of a cool GPU; under the power limit of a long loop 8192 x 59136 takes 47 and
-// 55 us; before: mma.sync streaming kernel up to M = 8, its decode-layout copy in
+// Measured (B200, K x N, first replays of a cool GPU; a second later, at the power limit, 8192 x 59136 takes 45.6 us at M 4
+// and 49.8 at M 16; before: mma.sync streaming kernel up to M = 8, its decode-layout copy in
 // brackets, an earlier form of this kernel above; K-major copy in brackets):
 //   8192 x 59136   M 4: 56.2 (50.6) -> 41.6 us, 5.8 TB/s of int4    M 16: 82.1 (64.1) -> 45.3 us
 //   29568 x 8192   M 4: 35.0 (30.2) -> 24.7 us                        M 16: 40.0 (43.7) -> 27.3 us
@@ -274,10 +275,11 @@ __device__ __forceinline__ Work ts_split_work(const TsParams& p, int rank, int k
   return Work::range(tile * p.KT, (tile + 1) * p.KT, p.KT);
 }
 
-// BULK: scales and zero words of 256 columns of a group, of which `cols` exist, for plain bulk copies.  They are
-// contiguous, and a tensor map costs the host 0.2 us of a call, which is what bounds an eager call of a short layer (2048 x
-// 5120 at M 1: 5.1 -> 4.7 us; replayed 4.16 -> 4.2).  What a copy leaves as it is belongs to columns that are not stored.
-// Long layers keep their maps: bulk copies took 55 -> 58 us on 8192 x 59136 at M 32.
+// BULK: scales and zero words of 256 columns of a group, of which `cols` exist, for plain bulk copies: they are contiguous.
+// What a copy leaves as it is belongs to columns that are not stored.  Maps -> copies: the host needs two tensor maps less, 0.1
+// us of a call (eager, 2048 x 5120 at M 1 4.78 -> 4.72 us, which is less than runs differ by; replayed, clusters in groups of
+// 128 are 0.2 to 0.9 % slower, 4.21 -> 4.23); groups of 64 at M 24, 4096 x 11040 12.4 -> 11.7 (with maps some runs take
+// 11.5), eight other shapes of 17 to 32 tokens +- 0.9 %.  Long layers keep their maps: 8192 x 59136 at M 32 55 -> 58.
 struct TsRow {
   const __half* scales;
   const uint32_t* zeros;
