@@ -62,8 +62,8 @@
 // cluster have the slots of a token, each the whole matrix, and add the rounded rows in slot order, so that no kernel for
 // the sum follows.  Each where the estimates say so.  Experts without the router, ranges and a kernel for the sum -> now:
 // 128 of 2048 x 768, one token, top-8 16.8 -> 14.5 us (gate_up in ranges, on clusters 15.3); 64 of 2048 x 1024, top-4 14.8
-// -> 13.2; 64 of 2048 x 768, two tokens, top-4 16.2 -> 14.1.  (With zero points subtracted in the conversion 0.1 us slower, and other roundings than
-// through the permutation.)
+// -> 13.2; 64 of 2048 x 768, two tokens, top-4 16.2 -> 14.1.  (With zero points subtracted in the conversion 0.1 us slower,
+// and other roundings than through the permutation.)
 //
 // unit_full counts the conversion warps, the announcement of the tokens and the fold warps of the unit
 // NDB before, whose accumulators the MMAs overwrite.  mma_done counts the MMA warp's commit and the

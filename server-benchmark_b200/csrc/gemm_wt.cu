@@ -1156,7 +1156,8 @@ int wt_rings(WtParams* p, int mode, int group) {
   p->nx = p->xstage <= (16 << 10) ? 8 : 4;
   // Two accumulators, so that the next tile's MMAs run under the epilogue, while they fit beside six A slots, or beside four
   // where a CTA has many tiles; what TMEM is left over goes to A slots.
-  const bool one = p->nt > 128 || (p->nt > 64 && (p->share.tiles == 1 || wt_one_accumulator(p->nt, p->chunk, p->KT, group)));
+  const bool one =
+      p->nt > 128 || (p->nt > 64 && (p->share.tiles == 1 || wt_one_accumulator(p->nt, p->chunk, p->KT, group)));
   p->nbuf = one ? 1 : 2;
   // One accumulator and whole tiles: the WIDE kernel.
   p->stage_bytes = p->nbuf == 2 || p->chunk > 0 || p->share.pairs > 0 ? 0 : (p->nt + 31) / 32 * 32 * kWtCols * (mode == 1 ? 1 : 2);
